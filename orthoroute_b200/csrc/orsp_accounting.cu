@@ -7,6 +7,7 @@
 // float32 numpy expression of the reference function it replaces (numpy >= 2
 // keeps Python-float scalars "weak", so every operand is rounded to float32).
 #include <algorithm>
+#include <initializer_list>
 
 #include "accounting.cuh"
 
@@ -20,44 +21,100 @@ inline int grid_for(int64_t n, int threads = 256) {
   return (int)std::max<int64_t>(1, std::min<int64_t>(b, 148 * 32));
 }
 
-// EdgeAccountant.update_costs (UPF:973-1043).
-__global__ void update_costs_kernel(int64_t E, const float *__restrict__ base,
-                                    const float *__restrict__ ema,
-                                    const float *__restrict__ cap,
-                                    const float *__restrict__ hist,
-                                    const uint8_t *__restrict__ layer,
-                                    const uint8_t *__restrict__ kind,
-                                    const float *__restrict__ lbias, float pres_fac,
-                                    float hist_w, float via_mult, float base_w,
-                                    int jitter, float *__restrict__ out) {
+// The whole-array updates read and write each edge once, so they are bound by
+// HBM; what keeps them there is bytes in flight.  Four edges per thread in
+// 16-byte accesses (4-byte for the uint8 arrays) do that; arrays whose
+// addresses are not 16-byte (4-byte) aligned, such as an offset view, and the
+// last E mod 4 edges take the same step one edge at a time.  Measured on
+// 25.2 M edges, before -> after: history 80 -> 69 us, present EMA 67 -> 47 us
+// (6.4 TB/s), overuse 53 -> 42 us, present from usage 33 -> 28 us.
+template <int V, typename T>
+struct alignas(sizeof(T) * V) Vec {
+  T v[V];
+};
+template <int V, typename T>
+__device__ __forceinline__ Vec<V, T> ldv(const T *p, int64_t i) {
+  return *reinterpret_cast<const Vec<V, T> *>(p + i * V);
+}
+template <int V, typename T>
+__device__ __forceinline__ void stv(T *p, int64_t i, const Vec<V, T> &x) {
+  *reinterpret_cast<Vec<V, T> *>(p + i * V) = x;
+}
+
+inline bool aligned_to(size_t a, std::initializer_list<const void *> ps) {
+  for (const void *p : ps)
+    if ((uintptr_t)p % a) return false;
+  return true;
+}
+
+// EdgeAccountant.update_costs (UPF:973-1043) on one edge.
+struct CostParams {
+  const float *base, *ema, *cap, *hist;
+  const uint8_t *layer, *kind;
+  const float *lbias;
+  float pres_fac, hist_w, via_mult, base_w;
+  int jitter;
+  float *out;
+};
+
+template <bool BIAS>
+__device__ __forceinline__ float cost_of(const CostParams &p, int64_t e, float base, float ema, float cap, float hist,
+                                         uint8_t layer, uint8_t kind) {
+  // over = xp.maximum(0, present_ema - capacity)
+  float over = __fsub_rn(ema, cap);
+  over = over > 0.0f ? over : 0.0f;
+  float adjusted = __fmul_rn(__fmul_rn(base, p.via_mult), p.base_w);
+  float present_term;
+  if (BIAS) {
+    // per_edge_bias = where(edge_kind == 0, layer_bias[edge_layer], 1.0)
+    const bool planar = kind == 0;
+    const float peb = planar ? __ldg(&p.lbias[layer]) : 1.0f;
+    adjusted = __fmul_rn(adjusted, peb);
+    // inverted = where(peb != 0, 1/maximum(peb, 0.5), 1); where(kind==0, inv, 1)
+    float inv = 1.0f;
+    if (planar && peb != 0.0f) inv = __fdiv_rn(1.0f, peb > 0.5f ? peb : 0.5f);
+    present_term = __fmul_rn(__fmul_rn(p.pres_fac, inv), over);
+  } else {
+    adjusted = __fmul_rn(adjusted, 1.0f);
+    present_term = __fmul_rn(p.pres_fac, over);
+  }
+  float total = __fadd_rn(__fadd_rn(adjusted, present_term), __fmul_rn(p.hist_w, hist));
+  if (p.jitter) total = __fadd_rn(total, orsp::index_jitter(e));
+  return total;
+}
+
+template <int V, bool BIAS>
+__global__ void update_costs_kernel(int64_t first, int64_t n, CostParams p) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < E; e += stride) {
-    // over = xp.maximum(0, present_ema - capacity)
-    float over = __fsub_rn(ema[e], cap[e]);
-    over = over > 0.0f ? over : 0.0f;
-    float adjusted = __fmul_rn(__fmul_rn(base[e], via_mult), base_w);
-    float present_term;
-    if (lbias) {
-      // per_edge_bias = where(edge_kind == 0, layer_bias[edge_layer], 1.0)
-      const bool planar = kind[e] == 0;
-      const float peb = planar ? lbias[layer[e]] : 1.0f;
-      adjusted = __fmul_rn(adjusted, peb);
-      // inverted = where(peb != 0, 1/maximum(peb, 0.5), 1); where(kind==0, inv, 1)
-      float inv = 1.0f;
-      if (planar && peb != 0.0f) inv = __fdiv_rn(1.0f, peb > 0.5f ? peb : 0.5f);
-      present_term = __fmul_rn(__fmul_rn(pres_fac, inv), over);
-    } else {
-      adjusted = __fmul_rn(adjusted, 1.0f);
-      present_term = __fmul_rn(pres_fac, over);
+  for (int64_t i = first / V + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < first / V + n; i += stride) {
+    const Vec<V, float> b = ldv<V>(p.base, i), m = ldv<V>(p.ema, i), c = ldv<V>(p.cap, i), h = ldv<V>(p.hist, i);
+    Vec<V, uint8_t> l{}, k{};
+    if (BIAS) {
+      l = ldv<V>(p.layer, i);
+      k = ldv<V>(p.kind, i);
     }
-    float total = __fadd_rn(__fadd_rn(adjusted, present_term), __fmul_rn(hist_w, hist[e]));
-    if (jitter) {
-      // xp.arange(E, dtype=float32) % 9973 * 1e-6: the index is first rounded
-      // to float32 (exact below 2^24), the remainder is exact.
-      const float fi = __ll2float_rn(e);
-      total = __fadd_rn(total, __fmul_rn(fmodf(fi, 9973.0f), 1e-6f));
-    }
-    out[e] = total;
+    Vec<V, float> o;
+#pragma unroll
+    for (int j = 0; j < V; ++j) o.v[j] = cost_of<BIAS>(p, i * V + j, b.v[j], m.v[j], c.v[j], h.v[j], l.v[j], k.v[j]);
+    stv<V>(p.out, i, o);
+  }
+}
+
+// The live costs of all edges (edges == nullptr, V edges per step).
+template <int V>
+__global__ void live_costs_all_kernel(int64_t first, int64_t n, const float *__restrict__ base,
+                                      const int32_t *__restrict__ usage, const float *__restrict__ cap,
+                                      const float *__restrict__ hist, float pres_fac, float hist_w, float via_mult,
+                                      float base_w, int jitter, float *__restrict__ out) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = first / V + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < first / V + n; i += stride) {
+    const Vec<V, float> b = ldv<V>(base, i), c = ldv<V>(cap, i), h = ldv<V>(hist, i);
+    const Vec<V, int32_t> u = ldv<V>(usage, i);
+    Vec<V, float> o;
+#pragma unroll
+    for (int j = 0; j < V; ++j)
+      o.v[j] = orsp::live_cost_of(i * V + j, b.v[j], u.v[j], c.v[j], h.v[j], pres_fac, hist_w, via_mult, base_w, jitter);
+    stv<V>(out, i, o);
   }
 }
 
@@ -67,7 +124,7 @@ __global__ void live_costs_kernel(int64_t n, const int32_t *__restrict__ edges, 
                                   float via_mult, float base_w, int jitter, float *__restrict__ out) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-    const int64_t e = edges ? (int64_t)edges[i] : i;
+    const int64_t e = edges[i];
     if (e < 0) continue;
     out[e] = live_cost(e, base, usage, cap, hist, pres_fac, hist_w, via_mult, base_w, jitter);
   }
@@ -92,48 +149,74 @@ __global__ void live_costs_paths_kernel(int32_t K, const int32_t *__restrict__ p
 }
 
 // EdgeAccountant.update_present_ema (UPF:963-971).
-__global__ void ema_kernel(int64_t E, const float *__restrict__ present,
-                           float *__restrict__ ema, float beta, float omb) {
+template <int V>
+__global__ void ema_kernel(int64_t first, int64_t n, const float *__restrict__ present, float *__restrict__ ema,
+                           float beta, float omb) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < E; e += stride)
-    ema[e] = __fadd_rn(__fmul_rn(beta, present[e]), __fmul_rn(omb, ema[e]));
-}
-
-// EdgeAccountant.update_history (UPF:898-961).
-__global__ void history_kernel(int64_t E, float *__restrict__ hist,
-                               const float *__restrict__ present,
-                               const float *__restrict__ cap,
-                               const float *__restrict__ base, float gain,
-                               float cap_mult, float decay) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < E; e += stride) {
-    float h = __fmul_rn(hist[e], decay);
-    float over = __fsub_rn(present[e], cap[e]);
-    over = over > 0.0f ? over : 0.0f;
-    float inc = __fmul_rn(gain, over);
-    if (base) {
-      const float hc = __fmul_rn(cap_mult, base[e]);
-      inc = inc < hc ? inc : hc;  // xp.minimum (no NaNs here)
-    }
-    hist[e] = __fadd_rn(h, inc);
+  for (int64_t i = first / V + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < first / V + n; i += stride) {
+    const Vec<V, float> p = ldv<V>(present, i);
+    Vec<V, float> m = ldv<V>(ema, i);
+#pragma unroll
+    for (int j = 0; j < V; ++j) m.v[j] = __fadd_rn(__fmul_rn(beta, p.v[j]), __fmul_rn(omb, m.v[j]));
+    stv<V>(ema, i, m);
   }
 }
 
-// EdgeAccountant.compute_overuse (UPF:838-876), edge part.
-__global__ void overuse_kernel(int64_t E, const float *__restrict__ present,
-                               const float *__restrict__ cap,
-                               double *__restrict__ acc_sum,
-                               unsigned long long *__restrict__ acc_cnt) {
+// EdgeAccountant.update_history (UPF:898-961).
+template <int V>
+__global__ void history_kernel(int64_t first, int64_t n, float *__restrict__ hist,
+                               const float *__restrict__ present, const float *__restrict__ cap,
+                               const float *__restrict__ base, float gain, float cap_mult, float decay) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = first / V + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < first / V + n; i += stride) {
+    const Vec<V, float> p = ldv<V>(present, i), c = ldv<V>(cap, i);
+    Vec<V, float> h = ldv<V>(hist, i), b{};
+    if (base) b = ldv<V>(base, i);
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+      const float kept = __fmul_rn(h.v[j], decay);
+      float over = __fsub_rn(p.v[j], c.v[j]);
+      over = over > 0.0f ? over : 0.0f;
+      float inc = __fmul_rn(gain, over);
+      if (base) {
+        const float hc = __fmul_rn(cap_mult, b.v[j]);
+        inc = inc < hc ? inc : hc;  // xp.minimum (no NaNs here)
+      }
+      h.v[j] = __fadd_rn(kept, inc);
+    }
+    stv<V>(hist, i, h);
+  }
+}
+
+// EdgeAccountant.compute_overuse (UPF:838-876), edge part.  acc: the float64
+// sum, the count, and the number of blocks done; the last block writes the
+// result (int() truncation of the sum).
+struct OveruseAcc {
+  double sum;
+  unsigned long long cnt;
+  unsigned done, pad;
+};
+
+template <int V>
+__global__ void overuse_kernel(int64_t E, const float *__restrict__ present, const float *__restrict__ cap,
+                               OveruseAcc *__restrict__ acc, int64_t *__restrict__ out2) {
   double s = 0.0;
   unsigned long long c = 0;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < E; e += stride) {
-    float over = __fsub_rn(present[e], cap[e]);
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  auto add = [&](float p, float k) {
+    const float over = __fsub_rn(p, k);
     if (over > 0.0f) {
       s += (double)over;
       ++c;
     }
+  };
+  for (int64_t i = t; i < E / V; i += stride) {
+    const Vec<V, float> p = ldv<V>(present, i), k = ldv<V>(cap, i);
+#pragma unroll
+    for (int j = 0; j < V; ++j) add(p.v[j], k.v[j]);
   }
+  if (V > 1 && t < E % V) add(present[E - 1 - t], cap[E - 1 - t]);
   for (int o = 16; o > 0; o >>= 1) {
     s += __shfl_xor_sync(ORSP_FULL_MASK, s, o);
     c += __shfl_xor_sync(ORSP_FULL_MASK, c, o);
@@ -152,26 +235,49 @@ __global__ void overuse_kernel(int64_t E, const float *__restrict__ present,
       c += __shfl_xor_sync(ORSP_FULL_MASK, c, o);
     }
     if (lane == 0) {
-      atomicAdd(acc_sum, s);
-      atomicAdd(acc_cnt, c);
+      if (c) {
+        atomicAdd(&acc->sum, s);
+        atomicAdd(&acc->cnt, c);
+      }
+      __threadfence();
+      if (atomicAdd(&acc->done, 1u) == gridDim.x - 1) {
+        __threadfence();
+        out2[0] = (int64_t)__ldcg(&acc->sum);
+        out2[1] = (int64_t)__ldcg(&acc->cnt);
+      }
     }
   }
 }
 
-__global__ void overuse_finish_kernel(const double *acc_sum,
-                                      const unsigned long long *acc_cnt,
-                                      int64_t *out2) {
-  out2[0] = (int64_t)(*acc_sum);  // int() truncation
-  out2[1] = (int64_t)(*acc_cnt);
-}
-
-__global__ void present_from_usage_kernel(int64_t E, const int32_t *__restrict__ usage,
+template <int V>
+__global__ void present_from_usage_kernel(int64_t first, int64_t n, const int32_t *__restrict__ usage,
                                           float *__restrict__ present) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < E; e += stride)
-    present[e] = (float)usage[e];
+  for (int64_t i = first / V + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < first / V + n; i += stride) {
+    const Vec<V, int32_t> u = ldv<V>(usage, i);
+    Vec<V, float> p;
+#pragma unroll
+    for (int j = 0; j < V; ++j) p.v[j] = (float)u.v[j];
+    stv<V>(present, i, p);
+  }
 }
 
+// Launches `four(first, n)` over the n groups of four edges from edge `first`
+// when the arrays are aligned for it, and `one(first, n)` over the n single
+// edges left.
+template <class Four, class One>
+int over_edges(int64_t E, bool vec, Four four, One one) {
+  const int64_t n4 = vec ? E / 4 : 0;
+  if (n4) {
+    four((int64_t)0, n4);
+    ORSP_CUDA(cudaGetLastError());
+  }
+  if (E > 4 * n4) {
+    one(4 * n4, E - 4 * n4);
+    ORSP_CUDA(cudaGetLastError());
+  }
+  return ORSP_OK;
+}
 
 __global__ void commit_kernel(int64_t n, const int32_t *__restrict__ edges,
                               int32_t *__restrict__ usage, float *__restrict__ present,
@@ -254,20 +360,29 @@ extern "C" int orsp_update_costs(int64_t E, const float *base, const float *ema,
     return ORSP_ERR_ARG;
   }
   if (E == 0) return ORSP_OK;
-  update_costs_kernel<<<grid_for(E), 256, 0, (cudaStream_t)stream>>>(
-      E, base, ema, cap, hist, layer, kind, lbias, pres_fac, hist_w, via_mult,
-      base_w, add_jitter, out);
-  ORSP_CUDA(cudaGetLastError());
-  return ORSP_OK;
+  const CostParams p{base, ema, cap, hist, layer, kind, lbias, pres_fac, hist_w, via_mult, base_w, add_jitter, out};
+  cudaStream_t st = (cudaStream_t)stream;
+  return over_edges(
+      E, aligned_to(16, {base, ema, cap, hist, out}) && aligned_to(4, {layer, kind}),
+      [&](int64_t a, int64_t n) {
+        if (lbias) update_costs_kernel<4, true><<<grid_for(n), 256, 0, st>>>(a, n, p);
+        else update_costs_kernel<4, false><<<grid_for(n), 256, 0, st>>>(a, n, p);
+      },
+      [&](int64_t a, int64_t n) {
+        if (lbias) update_costs_kernel<1, true><<<grid_for(n), 256, 0, st>>>(a, n, p);
+        else update_costs_kernel<1, false><<<grid_for(n), 256, 0, st>>>(a, n, p);
+      });
 }
 
 extern "C" int orsp_update_present_ema(int64_t E, const float *present, float *ema,
                                        float beta, float omb, uintptr_t stream) {
   if (E < 0 || (E > 0 && (!present || !ema))) { set_error("ema: NULL array"); return ORSP_ERR_ARG; }
   if (E == 0) return ORSP_OK;
-  ema_kernel<<<grid_for(E), 256, 0, (cudaStream_t)stream>>>(E, present, ema, beta, omb);
-  ORSP_CUDA(cudaGetLastError());
-  return ORSP_OK;
+  cudaStream_t st = (cudaStream_t)stream;
+  return over_edges(
+      E, aligned_to(16, {present, ema}),
+      [&](int64_t a, int64_t n) { ema_kernel<4><<<grid_for(n), 256, 0, st>>>(a, n, present, ema, beta, omb); },
+      [&](int64_t a, int64_t n) { ema_kernel<1><<<grid_for(n), 256, 0, st>>>(a, n, present, ema, beta, omb); });
 }
 
 extern "C" int orsp_update_history(int64_t E, float *hist, const float *present,
@@ -275,10 +390,15 @@ extern "C" int orsp_update_history(int64_t E, float *hist, const float *present,
                                    float cap_mult, float decay, uintptr_t stream) {
   if (E < 0 || (E > 0 && (!hist || !present || !cap))) { set_error("history: NULL array"); return ORSP_ERR_ARG; }
   if (E == 0) return ORSP_OK;
-  history_kernel<<<grid_for(E), 256, 0, (cudaStream_t)stream>>>(E, hist, present, cap, base,
-                                                               gain, cap_mult, decay);
-  ORSP_CUDA(cudaGetLastError());
-  return ORSP_OK;
+  cudaStream_t st = (cudaStream_t)stream;
+  return over_edges(
+      E, aligned_to(16, {hist, present, cap, base}),
+      [&](int64_t a, int64_t n) {
+        history_kernel<4><<<grid_for(n), 256, 0, st>>>(a, n, hist, present, cap, base, gain, cap_mult, decay);
+      },
+      [&](int64_t a, int64_t n) {
+        history_kernel<1><<<grid_for(n), 256, 0, st>>>(a, n, hist, present, cap, base, gain, cap_mult, decay);
+      });
 }
 
 namespace orsp {
@@ -286,14 +406,11 @@ namespace orsp {
 // small per-device buffer owned by this translation unit.
 int overuse_into(int64_t E, const float *present, const float *cap, int64_t *out2,
                  void *acc, cudaStream_t st) {
-  ORSP_CUDA(cudaMemsetAsync(acc, 0, 16, st));
-  if (E > 0) {
-    overuse_kernel<<<grid_for(E), 256, 0, st>>>(E, present, cap, (double *)acc,
-                                                (unsigned long long *)((char *)acc + 8));
-    ORSP_CUDA(cudaGetLastError());
-  }
-  overuse_finish_kernel<<<1, 1, 0, st>>>((const double *)acc,
-                                         (const unsigned long long *)((char *)acc + 8), out2);
+  ORSP_CUDA(cudaMemsetAsync(acc, 0, sizeof(OveruseAcc), st));
+  if (aligned_to(16, {present, cap}))
+    overuse_kernel<4><<<grid_for((E + 3) / 4), 256, 0, st>>>(E, present, cap, (OveruseAcc *)acc, out2);
+  else
+    overuse_kernel<1><<<grid_for(E), 256, 0, st>>>(E, present, cap, (OveruseAcc *)acc, out2);
   ORSP_CUDA(cudaGetLastError());
   return ORSP_OK;
 }
@@ -307,7 +424,7 @@ extern "C" int orsp_overuse(int64_t E, const float *present, const float *cap,
   int dev = 0;
   ORSP_CUDA(cudaGetDevice(&dev));
   if (!acc || acc_dev != dev) {
-    ORSP_CUDA(cudaMalloc(&acc, 16));
+    ORSP_CUDA(cudaMalloc(&acc, sizeof(OveruseAcc)));
     acc_dev = dev;
   }
   cudaStream_t st = (cudaStream_t)stream;
@@ -324,9 +441,11 @@ extern "C" int orsp_present_from_usage(int64_t E, const int32_t *usage, float *p
                                        uintptr_t stream) {
   if (E < 0 || (E > 0 && (!usage || !present))) { set_error("present_from_usage: NULL array"); return ORSP_ERR_ARG; }
   if (E == 0) return ORSP_OK;
-  present_from_usage_kernel<<<grid_for(E), 256, 0, (cudaStream_t)stream>>>(E, usage, present);
-  ORSP_CUDA(cudaGetLastError());
-  return ORSP_OK;
+  cudaStream_t st = (cudaStream_t)stream;
+  return over_edges(
+      E, aligned_to(16, {usage, present}),
+      [&](int64_t a, int64_t n) { present_from_usage_kernel<4><<<grid_for(n), 256, 0, st>>>(a, n, usage, present); },
+      [&](int64_t a, int64_t n) { present_from_usage_kernel<1><<<grid_for(n), 256, 0, st>>>(a, n, usage, present); });
 }
 
 extern "C" int orsp_commit_edges(int64_t n, const int32_t *edges, int32_t *usage,
@@ -386,8 +505,20 @@ extern "C" int orsp_update_costs_live(int64_t E, const int32_t *edges, int64_t n
   }
   const int64_t n = edges ? n_edges : E;
   if (n == 0) return ORSP_OK;
-  live_costs_kernel<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(n, edges, base, usage, cap, hist, pres_fac,
-                                                                  hist_w, via_mult, base_w, add_jitter, out);
+  cudaStream_t st = (cudaStream_t)stream;
+  if (!edges)
+    return over_edges(
+        E, aligned_to(16, {base, usage, cap, hist, out}),
+        [&](int64_t a, int64_t m) {
+          live_costs_all_kernel<4><<<grid_for(m), 256, 0, st>>>(a, m, base, usage, cap, hist, pres_fac, hist_w,
+                                                                via_mult, base_w, add_jitter, out);
+        },
+        [&](int64_t a, int64_t m) {
+          live_costs_all_kernel<1><<<grid_for(m), 256, 0, st>>>(a, m, base, usage, cap, hist, pres_fac, hist_w,
+                                                                via_mult, base_w, add_jitter, out);
+        });
+  live_costs_kernel<<<grid_for(n), 256, 0, st>>>(n, edges, base, usage, cap, hist, pres_fac, hist_w, via_mult, base_w,
+                                                 add_jitter, out);
   ORSP_CUDA(cudaGetLastError());
   return ORSP_OK;
 }

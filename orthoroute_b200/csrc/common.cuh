@@ -97,6 +97,11 @@ struct Graph {
   // layer's routing axis or a via to an adjacent layer (see orsp_lattice.cu)
   bool lattice_ok = false;
   int8_t layer_axis[64] = {};     // 0: no planar edges, 1: x, 2: y
+  // every planar edge of each layer's axis and, for each pair of layers, the
+  // vias of all columns or of none are present: a node's neighbours follow
+  // from its coordinates and via_to[z] (the layers its vias lead to)
+  bool lat_uniform = false;
+  uint64_t via_to[64] = {};
   int32_t *slot_eid = nullptr;    // [4][N] in-edge id per slot (-1 absent)
   float *wslot = nullptr;         // [N] float4: gathered in-edge weights per node, by slot
   // column vias (the reference's Lattice3D: vias between any two layers of a

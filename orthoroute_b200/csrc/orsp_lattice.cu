@@ -1712,12 +1712,15 @@ namespace orsp {
 int analyze_lattice(Graph *g, const int32_t *indptr_h, const int32_t *indices_h) {
   g->lattice_ok = false;
   g->cvia = false;
+  g->lat_uniform = false;
   if (g->nx <= 0 || g->ny <= 0 || g->nz <= 0 || g->nz > 64) return ORSP_OK;
   const int32_t N = g->N, nx = g->nx, ny = g->ny;
   const int64_t nxy = (int64_t)nx * ny;
   std::vector<int8_t> axis(g->nz, -1);
   std::vector<int32_t> slot((size_t)4 * N, -1);
   bool adjacent_vias = true;  // every via spans one layer, no parallel vias
+  // edges present: planar ones per layer, columns with a via per layer pair
+  std::vector<int64_t> planar_n(g->nz, 0), via_n((size_t)g->nz * g->nz, 0);
   for (int32_t u = 0; u < N; ++u) {
     const int32_t zu = (int32_t)(u / nxy);
     const int32_t ru = (int32_t)(u - zu * nxy);
@@ -1753,6 +1756,8 @@ int analyze_lattice(Graph *g, const int32_t *indptr_h, const int32_t *indices_h)
         continue;
       }
       slotref = k;
+      if (s < 2) ++planar_n[zu];
+      else ++via_n[(size_t)zu * g->nz + zv];
     }
   }
   std::vector<int32_t> vcol;
@@ -1760,6 +1765,7 @@ int analyze_lattice(Graph *g, const int32_t *indptr_h, const int32_t *indices_h)
     // column vias: every via in-edge of v by source layer, two parallel
     // edges at most (edge ids ascend with u and k, so k = 0 is the smaller)
     vcol.assign((size_t)2 * g->nz * N, -1);
+    std::fill(via_n.begin(), via_n.end(), 0);
     for (int32_t u = 0; u < N; ++u) {
       const int32_t zu = (int32_t)(u / nxy);
       const int64_t cu = u - (int64_t)zu * nxy;
@@ -1769,14 +1775,27 @@ int analyze_lattice(Graph *g, const int32_t *indptr_h, const int32_t *indices_h)
         if (zv == zu || v - (int64_t)zv * nxy != cu) continue;  // planar (checked above)
         int32_t *e0 = &vcol[((size_t)0 * g->nz + zu) * N + v];
         int32_t *e1 = &vcol[((size_t)1 * g->nz + zu) * N + v];
-        if (*e0 < 0) *e0 = k;
-        else if (*e1 < 0) *e1 = k;
+        if (*e0 < 0) {
+          *e0 = k;
+          ++via_n[(size_t)zu * g->nz + zv];
+        } else if (*e1 < 0) *e1 = k;
         else return ORSP_OK;  // three parallel vias
       }
     }
     for (int32_t v = 0; v < N; ++v) slot[(size_t)2 * N + v] = slot[(size_t)3 * N + v] = -1;
   }
   for (int z = 0; z < g->nz; ++z) g->layer_axis[z] = axis[z] < 0 ? 0 : axis[z];
+  g->lat_uniform = true;
+  for (int z = 0; z < g->nz; ++z) {
+    const int64_t want = axis[z] == 1 ? 2 * (int64_t)(nx - 1) * ny : axis[z] == 2 ? 2 * (int64_t)nx * (ny - 1) : 0;
+    if (planar_n[z] != want) g->lat_uniform = false;
+    g->via_to[z] = 0;
+    for (int t = 0; t < g->nz; ++t) {
+      const int64_t n = via_n[(size_t)z * g->nz + t];
+      if (n == nxy) g->via_to[z] |= 1ull << t;
+      else if (n != 0) g->lat_uniform = false;
+    }
+  }
   ORSP_CUDA(cudaMalloc(&g->slot_eid, slot.size() * sizeof(int32_t)));
   ORSP_CUDA(cudaMemcpy(g->slot_eid, slot.data(), slot.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
   ORSP_CUDA(cudaMalloc(&g->wslot, slot.size() * sizeof(float)));

@@ -203,97 +203,261 @@ __global__ void __launch_bounds__(CMP_THREADS) write_tiles_kernel(const uint8_t 
   }
 }
 
-// Truncation to max_nodes with the reference's must-keep swap (UPF:1705-1722):
-// for the k-th kept node (in list order) at position p >= max_nodes, swap it
-// with position k; then keep the first max_nodes entries.
-__global__ void truncate_kernel(int32_t *roi, const int32_t *count_in, int32_t max_nodes,
-                                int32_t src, int32_t dst, int32_t *count_out) {
-  if (threadIdx.x != 0) return;
-  const int n = *count_in;
-  int cnt = n;
-  if (n > max_nodes) {
-    // positions of must-keep nodes in list order
-    int kept[2];
-    int nk = 0;
-    for (int i = 0; i < n && nk < 2; ++i) {
-      const int v = roi[i];
-      if (v == src || v == dst) kept[nk++] = i;
-    }
-    for (int k = 0; k < nk; ++k) {
-      const int p = kept[k];
-      if (p >= max_nodes) {
-        const int t = roi[p];
-        roi[p] = roi[k];
-        roi[k] = t;
-      }
-    }
-    cnt = max_nodes;
-  }
-  *count_out = cnt;
-}
-
-// The same truncation with a general must-keep list, as extract_roi_bfs does
-// with portal seeds (UPF:1700-1731): must_keep = [src, dst] followed by the
-// keep nodes not already in it (list order); the ones missing from the ROI
-// are appended after the ascending part in that order; then, if the list is
-// longer than max_nodes, the k-th must-keep position (ascending) at or past
-// max_nodes is swapped with position k and the list is cut to max_nodes.
-// One thread; the ascending part is binary-searched.  MAX_KEEP bounds the
-// list (checked on the host).
+// Truncation to max_nodes with the reference's must-keep list, as
+// extract_roi_bfs does it (UPF:1700-1731): must_keep = [src, dst] followed by
+// the keep nodes not already in it (list order); the ones missing from the
+// ROI are appended after the ascending part in that order; then, if the list
+// is longer than max_nodes, the k-th must-keep position (ascending) at or
+// past max_nodes is swapped with position k (UPF:1705-1722) and the list is
+// cut to max_nodes.  Called by a whole block after the list is written: one
+// thread per must-keep node drops repeats and searches the ascending part, so
+// the block pays one binary search (about 10 us of dependent loads) instead
+// of one thread's scan of the list (617 us for 75 K nodes).  MAX_KEEP bounds
+// the list (checked on the host).  Returns the length on thread 0.
 constexpr int MAX_KEEP = 256;
-__global__ void keep_truncate_kernel(int32_t *roi, const int32_t *count_in, int32_t max_nodes, int32_t src,
-                                     int32_t dst, const int32_t *keep, int32_t nkeep, int32_t *count_out) {
-  if (threadIdx.x != 0) return;
-  int32_t mk[MAX_KEEP + 2];
-  int nmk = 0;
-  mk[nmk++] = src;
-  if (dst != src) mk[nmk++] = dst;
-  for (int i = 0; i < nkeep; ++i) {
-    const int32_t v = keep[i];
+__device__ int truncate_block(int32_t *roi, int32_t n0, int32_t max_nodes, int32_t src, int32_t dst,
+                              const int32_t *keep, int32_t nkeep) {
+  __shared__ int32_t s_mk[MAX_KEEP + 2], s_pos[MAX_KEEP + 2];
+  const int nc = nkeep + 2;
+  for (int j = threadIdx.x; j < nc; j += blockDim.x) s_mk[j] = j == 0 ? src : j == 1 ? dst : keep[j - 2];
+  __syncthreads();
+  for (int j = threadIdx.x; j < nc; j += blockDim.x) {
+    const int32_t v = s_mk[j];
     bool dup = false;
-    for (int j = 0; j < nmk; ++j) dup |= mk[j] == v;
-    if (!dup) mk[nmk++] = v;
-  }
-  const int n0 = *count_in;
-  int n = n0;
-  int32_t pos[MAX_KEEP + 2];
-  for (int j = 0; j < nmk; ++j) {
-    int lo = 0, hi = n0;  // first position with roi[p] >= mk[j]
+    for (int i = 0; i < j; ++i) dup |= s_mk[i] == v;
+    int lo = 0, hi = dup ? 0 : n0;  // first position with roi[p] >= v
     while (lo < hi) {
       const int mid = (lo + hi) >> 1;
-      if (roi[mid] < mk[j]) lo = mid + 1;
+      if (__ldcg(&roi[mid]) < v) lo = mid + 1;
       else hi = mid;
     }
-    if (lo < n0 && roi[lo] == mk[j]) {
-      pos[j] = lo;
-    } else {
-      roi[n] = mk[j];
-      pos[j] = n++;
+    s_pos[j] = dup ? -2 : (lo < n0 && __ldcg(&roi[lo]) == v) ? lo : -1;
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return 0;
+  int n = n0, nmk = 0;
+  for (int j = 0; j < nc; ++j) {
+    int p = s_pos[j];
+    if (p == -2) continue;
+    if (p == -1) {
+      roi[n] = s_mk[j];
+      p = n++;
+    }
+    s_pos[nmk++] = p;
+  }
+  if (n <= max_nodes) return n;
+  // positions in ascending order (insertion sort of a short list)
+  for (int a = 1; a < nmk; ++a) {
+    const int32_t t = s_pos[a];
+    int b = a - 1;
+    while (b >= 0 && s_pos[b] > t) {
+      s_pos[b + 1] = s_pos[b];
+      --b;
+    }
+    s_pos[b + 1] = t;
+  }
+  for (int k = 0; k < nmk; ++k) {
+    const int p = s_pos[k];
+    if (p >= max_nodes) {
+      const int32_t t = roi[p];
+      roi[p] = roi[k];
+      roi[k] = t;
     }
   }
-  int cnt = n;
-  if (n > max_nodes) {
-    // positions in ascending order (insertion sort of a short list)
-    for (int a = 1; a < nmk; ++a) {
-      const int32_t t = pos[a];
-      int b = a - 1;
-      while (b >= 0 && pos[b] > t) {
-        pos[b + 1] = pos[b];
-        --b;
-      }
-      pos[b + 1] = t;
+  return max_nodes;
+}
+
+__global__ void truncate_kernel(int32_t *roi, const int32_t *count_in, int32_t max_nodes, int32_t src, int32_t dst,
+                                const int32_t *keep, int32_t nkeep, int32_t *count_out) {
+  const int cnt = truncate_block(roi, *count_in, max_nodes, src, dst, keep, nkeep);
+  if (threadIdx.x == 0) *count_out = cnt;
+}
+
+// The expansion on a uniform lattice (Graph::lat_uniform), one CTA.
+//
+// A level of the wave front is a chain of dependent accesses, about 100 to
+// 300 levels per ROI, so the kernel is bound by the latency of one level, not
+// by bandwidth.  roi_bfs_kernel above pays four round trips to L2 per level
+// (queue, row pointer, neighbour list, mark), the last one once per neighbour:
+// about 11 us.  Here the neighbours follow from the node's coordinates, the
+// queues hold packed coordinates in shared memory, and the marks (2 bits per
+// node) are in shared memory too when the lattice fits (SM), so a level makes
+// no trip to L2 and the marked nodes are compacted from shared memory by the
+// same launch.  Larger lattices keep their marks in global memory, up to
+// eight neighbours' marks in flight per node.  A queue that runs full sets
+// err; the host then runs the general kernel.  Semantics of the marks and of
+// the two waves as in roi_bfs_kernel.  (200 x 200 x 6 column-via
+// lattice, 75 K marked nodes: 1 295 us with roi_bfs_kernel, 324 us here.)
+struct LatBfs {
+  int32_t nx, ny, nz, N;
+  int32_t src, dst;      // node ids
+  int32_t psrc, pdst;    // packed coordinates x | y << 12 | z << 24
+  int32_t max_depth, max_nodes;
+  int32_t qcap;
+  const int32_t *keep;
+  int32_t nkeep;
+  uint8_t *seen;         // marks in global memory (!SM), zero on entry
+  int32_t *roi, *count;  // SM: the list and its length
+  BfsCtl *ctl;
+  int8_t axis[64];
+  uint64_t via_to[64];
+};
+
+template <bool SM>
+__global__ void __launch_bounds__(BFS_THREADS, 1) roi_bfs_lattice_kernel(const __grid_constant__ LatBfs p) {
+  extern __shared__ __align__(16) uint32_t s_dyn[];
+  __shared__ int s_next, s_met, s_err;
+  __shared__ int s_warp[32];
+  int32_t *qb[3];  // the two waves' fronts and the one being built
+  for (int i = 0; i < 3; ++i) qb[i] = (int32_t *)s_dyn + (int64_t)i * p.qcap;
+  uint32_t *marks = s_dyn + (int64_t)3 * p.qcap;
+  const int nwords = (p.N + 15) >> 4;
+  if (SM)
+    for (int i = threadIdx.x; i < nwords; i += BFS_THREADS) marks[i] = 0;
+  __syncthreads();
+  auto mark_node = [&](int32_t v, unsigned m) -> unsigned {
+    if (SM) {
+      const int sh = (v & 15) * 2;
+      return (atomicOr(&marks[v >> 4], m << sh) >> sh) & 3u;
     }
-    for (int k = 0; k < nmk; ++k) {
-      const int p = pos[k];
-      if (p >= max_nodes) {
-        const int32_t t = roi[p];
-        roi[p] = roi[k];
-        roi[k] = t;
-      }
-    }
-    cnt = max_nodes;
+    return or_mark(p.seen, v, m);
+  };
+  int cnt[2] = {1, 1};
+  int32_t *front[2] = {qb[0], qb[1]}, *spare = qb[2];
+  if (threadIdx.x == 0) {
+    if (p.src != p.dst) mark_node(p.src, 1u);
+    mark_node(p.dst, 2u);  // src == dst leaves mark 2, as the reference does
+    front[0][0] = p.psrc;
+    front[1][0] = p.pdst;
+    s_met = 0;
+    s_err = 0;
   }
-  *count_out = cnt;
+  int total = (p.src == p.dst) ? 1 : 2;
+  int depth = 0;
+  bool met = false;
+  const double limit = (double)p.max_nodes * 1.5;
+  const int32_t plane = p.nx * p.ny;
+  while (depth < p.max_depth && (cnt[0] > 0 || cnt[1] > 0) && !met) {
+#pragma unroll
+    for (int wave = 0; wave < 2; ++wave) {
+      if (wave == 1 && met) break;
+      const unsigned mark = wave == 0 ? 1u : 2u;
+      if (threadIdx.x == 0) s_next = 0;
+      __syncthreads();
+      bool met_local = false;
+      const int n = cnt[wave];
+      for (int i = threadIdx.x; i < n; i += BFS_THREADS) {
+        const int32_t pk = front[wave][i];
+        const int32_t x = pk & 4095, y = (pk >> 12) & 4095, z = pk >> 24;
+        const int32_t id = (z * p.ny + y) * p.nx + x;
+        const int ax = p.axis[z];
+        const int32_t c = ax == 1 ? x : y, cmax = ax == 1 ? p.nx - 1 : p.ny - 1;
+        const int32_t step = ax == 1 ? 1 : p.nx, pstep = ax == 1 ? 1 : 4096;
+        uint64_t vm = p.via_to[z];
+        bool planar = ax != 0;
+        while (planar || vm) {
+          int32_t nid[8], npk[8];
+          bool has[8];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            has[k] = false;
+            nid[k] = npk[k] = 0;
+            if (k < 2 && planar) {
+              has[k] = k == 0 ? c > 0 : c < cmax;
+              nid[k] = k == 0 ? id - step : id + step;
+              npk[k] = k == 0 ? pk - pstep : pk + pstep;
+            } else if (vm) {
+              const int t = __ffsll((long long)vm) - 1;
+              vm &= vm - 1;
+              has[k] = true;
+              nid[k] = id + (t - z) * plane;
+              npk[k] = (pk & 0xffffff) | (t << 24);
+            }
+          }
+          planar = false;
+          unsigned old[8];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) old[k] = has[k] ? mark_node(nid[k], mark) : mark;
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            if (old[k] == 0) {
+              const int idx = atomicAdd(&s_next, 1);
+              if (idx < p.qcap) spare[idx] = npk[k];
+              else s_err = 1;
+            } else if (old[k] != mark) {
+              met_local = true;
+            }
+          }
+        }
+      }
+      if (met_local) s_met = 1;
+      __syncthreads();
+      const int nn = s_next;
+      met = s_met != 0;
+      const bool full = s_err != 0;
+      __syncthreads();  // s_next is reset by the next wave
+      total += nn;
+      cnt[wave] = nn;
+      int32_t *t = front[wave];
+      front[wave] = spare;
+      spare = t;
+      if (full) {
+        if (threadIdx.x == 0) p.ctl->err = 1;
+        return;
+      }
+    }
+    ++depth;
+    if ((double)total > limit) break;
+  }
+  if (threadIdx.x == 0) {
+    p.ctl->total = total;
+    p.ctl->depth = depth;
+    p.ctl->met = met ? 1 : 0;
+    p.ctl->err = 0;
+  }
+  if (!SM) return;
+  // the marked nodes in ascending order: each warp takes a contiguous range
+  // of mark words, lane after lane
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int per = (((nwords + 31) / 32) + 31) & ~31;
+  const int w0 = w * per, w1 = min(nwords, w0 + per);
+  int mine = 0;
+  for (int i = w0 + lane; i < w1; i += 32) mine += __popc((marks[i] | (marks[i] >> 1)) & 0x55555555u);
+  mine = __reduce_add_sync(ORSP_FULL_MASK, mine);
+  if (lane == 0) s_warp[w] = mine;
+  __syncthreads();
+  if (w == 0) {
+    const int v = s_warp[lane];
+    int x = v;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(ORSP_FULL_MASK, x, o);
+      if (lane >= o) x += y;
+    }
+    s_warp[lane] = x - v;
+    if (lane == 31) s_next = x;
+  }
+  __syncthreads();
+  int pos = s_warp[w];
+  for (int b = w0; b < w1; b += 32) {
+    uint32_t m = 0;
+    if (b + lane < w1) m = (marks[b + lane] | (marks[b + lane] >> 1)) & 0x55555555u;
+    const int c = __popc(m);
+    int x = c;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(ORSP_FULL_MASK, x, o);
+      if (lane >= o) x += y;
+    }
+    int at = pos + x - c;
+    while (m) {
+      const int j = __ffs(m) - 1;
+      m &= m - 1;
+      __stcg(&p.roi[at++], (b + lane) * 16 + (j >> 1));
+    }
+    pos += __shfl_sync(ORSP_FULL_MASK, x, 31);
+  }
+  __syncthreads();
+  const int n = truncate_block(p.roi, s_next, p.max_nodes, p.src, p.dst, p.keep, p.nkeep);
+  if (threadIdx.x == 0) *p.count = n;
 }
 
 __global__ void fill_i32_kernel(int32_t *p, int64_t n, int32_t v) {
@@ -368,6 +532,37 @@ extern "C" int orsp_roi_bfs_keep(orsp_graph *g, int32_t src, int32_t dst, int32_
   return roi_bfs_impl(g, src, dst, max_depth, max_nodes, keep_d, nkeep, roi_nodes_d, g2r_d, roi_count_h, stream);
 }
 
+// Compaction of the marks into the ascending list, and its truncation.
+static int compact_and_truncate(const uint8_t *seen, int32_t N, int32_t *tiles, int32_t *misc, int32_t max_nodes,
+                                int32_t src, int32_t dst, const int32_t *keep_d, int32_t nkeep, int32_t *roi_nodes_d,
+                                cudaStream_t st) {
+  const int ntiles = (int)(((int64_t)N + CMP_TILE - 1) / CMP_TILE);
+  count_tiles_kernel<<<ntiles, CMP_THREADS, 0, st>>>(seen, N, tiles);
+  ORSP_CUDA(cudaGetLastError());
+  scan_tiles_kernel<<<1, 1024, 0, st>>>(tiles, ntiles, misc + 4);
+  ORSP_CUDA(cudaGetLastError());
+  write_tiles_kernel<<<ntiles, CMP_THREADS, 0, st>>>(seen, N, tiles, roi_nodes_d);
+  ORSP_CUDA(cudaGetLastError());
+  truncate_kernel<<<1, 128, 0, st>>>(roi_nodes_d, misc + 4, max_nodes, src, dst, keep_d, nkeep, misc + 5);
+  ORSP_CUDA(cudaGetLastError());
+  return ORSP_OK;
+}
+
+static int write_g2r(const int32_t *roi_nodes_d, const int32_t *count_d, int64_t N, int32_t *g2r_d, cudaStream_t st) {
+  fill_i32_kernel<<<std::min<int64_t>((N + 255) / 256, 4096), 256, 0, st>>>(g2r_d, N, -1);
+  ORSP_CUDA(cudaGetLastError());
+  scatter_g2r_kernel<<<std::min<int64_t>((N + 255) / 256, 1024), 256, 0, st>>>(roi_nodes_d, count_d, g2r_d);
+  ORSP_CUDA(cudaGetLastError());
+  return ORSP_OK;
+}
+
+// Shared memory of the lattice expansion: a front on a lattice of moderate
+// depth holds up to a few thousand nodes; with the marks in shared memory too
+// the queues get 3 584 entries each, which leaves room for the marks of
+// 745 000 nodes, otherwise as many as fit.
+static constexpr int32_t kBfsSmem = 224 * 1024;
+static constexpr int32_t kBfsQueue = 3584;
+
 static int roi_bfs_impl(orsp_graph *g, int32_t src, int32_t dst, int32_t max_depth, int32_t max_nodes,
                         const int32_t *keep_d, int32_t nkeep, int32_t *roi_nodes_d, int32_t *g2r_d,
                         int32_t *roi_count_h, uintptr_t stream) {
@@ -392,33 +587,65 @@ static int roi_bfs_impl(orsp_graph *g, int32_t src, int32_t dst, int32_t max_dep
   int32_t *tiles = (int32_t *)(base + seen_b + 4 * q_b);
   int32_t *misc = (int32_t *)(base + seen_b + 4 * q_b + tiles_b);  // [0..3] BfsCtl, [4] total, [5] count
   BfsCtl *ctl = (BfsCtl *)misc;
-
-  ORSP_CUDA(cudaMemsetAsync(seen, 0, seen_b, st));
-  roi_bfs_kernel<<<1, BFS_THREADS, 0, st>>>(g->indptr, g->indices, g->N, src, dst, max_depth,
-                                            max_nodes, seen, q[0], q[1], q[2], q[3], ctl);
-  ORSP_CUDA(cudaGetLastError());
-  count_tiles_kernel<<<ntiles, CMP_THREADS, 0, st>>>(seen, g->N, tiles);
-  ORSP_CUDA(cudaGetLastError());
-  scan_tiles_kernel<<<1, 1024, 0, st>>>(tiles, ntiles, misc + 4);
-  ORSP_CUDA(cudaGetLastError());
-  write_tiles_kernel<<<ntiles, CMP_THREADS, 0, st>>>(seen, g->N, tiles, roi_nodes_d);
-  ORSP_CUDA(cudaGetLastError());
-  if (nkeep > 0)
-    keep_truncate_kernel<<<1, 32, 0, st>>>(roi_nodes_d, misc + 4, max_nodes, src, dst, keep_d, nkeep, misc + 5);
-  else
-    truncate_kernel<<<1, 32, 0, st>>>(roi_nodes_d, misc + 4, max_nodes, src, dst, misc + 5);
-  ORSP_CUDA(cudaGetLastError());
-  if (g2r_d) {
-    fill_i32_kernel<<<std::min<int64_t>((N + 255) / 256, 4096), 256, 0, st>>>(g2r_d, N, -1);
-    scatter_g2r_kernel<<<std::min<int64_t>((N + 255) / 256, 1024), 256, 0, st>>>(roi_nodes_d,
-                                                                                 misc + 5, g2r_d);
-    ORSP_CUDA(cudaGetLastError());
-  }
-  ORSP_CUDA(cudaMemcpyAsync(g->pinned, misc, 24, cudaMemcpyDeviceToHost, st));
-  ORSP_CUDA(cudaStreamSynchronize(st));
   const int32_t *h = (const int32_t *)g->pinned;
-  if (h[3]) { set_error("roi_bfs: queue overflow"); return ORSP_ERR_OVERFLOW; }
+
+  // uniform lattices (12-bit coordinates in the queues): the lattice
+  // expansion, then, if a queue ran full, the general one
+  const bool lattice = g->lattice_ok && g->lat_uniform && g->nx <= 4096 && g->ny <= 4096;
+  for (int general = lattice ? 0 : 1; general < 2; ++general) {
+    if (!general) {
+      LatBfs p{};
+      p.nx = g->nx;
+      p.ny = g->ny;
+      p.nz = g->nz;
+      p.N = g->N;
+      p.src = src;
+      p.dst = dst;
+      const int32_t plane = g->nx * g->ny;
+      auto pack = [&](int32_t v) { return (v % g->nx) | ((v % plane) / g->nx) << 12 | (v / plane) << 24; };
+      p.psrc = pack(src);
+      p.pdst = pack(dst);
+      p.max_depth = max_depth;
+      p.max_nodes = max_nodes;
+      p.keep = keep_d;
+      p.nkeep = nkeep;
+      p.seen = seen;
+      p.roi = roi_nodes_d;
+      p.count = misc + 5;
+      p.ctl = ctl;
+      for (int z = 0; z < g->nz; ++z) {
+        p.axis[z] = g->layer_axis[z];
+        p.via_to[z] = g->via_to[z];
+      }
+      const int64_t marks_b = ((N + 15) >> 4) * 4;
+      const bool sm = marks_b + 3 * (int64_t)kBfsQueue * 4 <= kBfsSmem;
+      p.qcap = sm ? kBfsQueue : kBfsSmem / 12;
+      const int smem = (int)(3 * (int64_t)p.qcap * 4 + (sm ? marks_b : 0));
+      void (*kfn)(LatBfs) = sm ? roi_bfs_lattice_kernel<true> : roi_bfs_lattice_kernel<false>;
+      ORSP_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, kBfsSmem));
+      if (!sm) ORSP_CUDA(cudaMemsetAsync(seen, 0, seen_b, st));
+      kfn<<<1, BFS_THREADS, smem, st>>>(p);
+      ORSP_CUDA(cudaGetLastError());
+      if (!sm) rc = compact_and_truncate(seen, g->N, tiles, misc, max_nodes, src, dst, keep_d, nkeep, roi_nodes_d, st);
+    } else {
+      ORSP_CUDA(cudaMemsetAsync(seen, 0, seen_b, st));
+      roi_bfs_kernel<<<1, BFS_THREADS, 0, st>>>(g->indptr, g->indices, g->N, src, dst, max_depth,
+                                                max_nodes, seen, q[0], q[1], q[2], q[3], ctl);
+      ORSP_CUDA(cudaGetLastError());
+      rc = compact_and_truncate(seen, g->N, tiles, misc, max_nodes, src, dst, keep_d, nkeep, roi_nodes_d, st);
+    }
+    if (rc) return rc;
+    ORSP_CUDA(cudaMemcpyAsync(g->pinned, misc, 24, cudaMemcpyDeviceToHost, st));
+    ORSP_CUDA(cudaStreamSynchronize(st));
+    if (!h[3]) break;
+    if (general) { set_error("roi_bfs: queue overflow"); return ORSP_ERR_OVERFLOW; }
+  }
   *roi_count_h = h[5];
+  if (g2r_d) {
+    rc = write_g2r(roi_nodes_d, misc + 5, N, g2r_d, st);
+    if (rc) return rc;
+    ORSP_CUDA(cudaStreamSynchronize(st));
+  }
   return ORSP_OK;
 }
 
@@ -493,7 +720,6 @@ extern "C" int orsp_roi_bfs_noalloc(orsp_graph *g, int32_t src, int32_t dst, int
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t N = g->N;
-  const int ntiles = (int)((N + CMP_TILE - 1) / CMP_TILE);
   uint8_t *seen = base;
   int32_t *q[4];
   for (int i = 0; i < 4; ++i) q[i] = (int32_t *)(base + kNaSeenBytes + i * kNaQueueBytes);
@@ -507,19 +733,11 @@ extern "C" int orsp_roi_bfs_noalloc(orsp_graph *g, int32_t src, int32_t dst, int
   roi_bfs_kernel<<<1, BFS_THREADS, 0, st>>>(g->indptr, g->indices, g->N, src, dst, max_depth,
                                             max_nodes, seen, q[0], q[1], q[2], q[3], ctl);
   ORSP_CUDA(cudaGetLastError());
-  count_tiles_kernel<<<ntiles, CMP_THREADS, 0, st>>>(seen, g->N, tiles);
-  ORSP_CUDA(cudaGetLastError());
-  scan_tiles_kernel<<<1, 1024, 0, st>>>(tiles, ntiles, misc + 4);
-  ORSP_CUDA(cudaGetLastError());
-  write_tiles_kernel<<<ntiles, CMP_THREADS, 0, st>>>(seen, g->N, tiles, roi_nodes_d);
-  ORSP_CUDA(cudaGetLastError());
-  truncate_kernel<<<1, 32, 0, st>>>(roi_nodes_d, misc + 4, max_nodes, src, dst, misc + 5);
-  ORSP_CUDA(cudaGetLastError());
+  int rc_c = compact_and_truncate(seen, g->N, tiles, misc, max_nodes, src, dst, nullptr, 0, roi_nodes_d, st);
+  if (rc_c) return rc_c;
   if (g2r_d) {
-    fill_i32_kernel<<<std::min<int64_t>((N + 255) / 256, 4096), 256, 0, st>>>(g2r_d, N, -1);
-    scatter_g2r_kernel<<<std::min<int64_t>((N + 255) / 256, 1024), 256, 0, st>>>(roi_nodes_d,
-                                                                                 misc + 5, g2r_d);
-    ORSP_CUDA(cudaGetLastError());
+    rc_c = write_g2r(roi_nodes_d, misc + 5, N, g2r_d, st);
+    if (rc_c) return rc_c;
   }
   // g->pinned was allocated when the graph was created, not here; it is one
   // buffer per graph, so overlapping calls on one graph race on it too.

@@ -163,16 +163,13 @@ struct LatBox {
   int64_t dbase;     // -1: distances indexed by node id in the shared array;
                      // >= 0: the box's own slice, box-local row-major from here
 };
-// Tile width of the lattice search (ORSP_LAT_TILE: 16 or 32); the height is 16.
-int lattice_tile_w();
-// Whether a tile of nzb layers at tile width tile_w (0: lattice_tile_w())
-// fits in shared memory.
+// Whether a tile of nzb layers at tile width tile_w (16 or 32; 0: 16, the
+// width of every tile) fits in shared memory.
 bool lattice_tile_fits(int nzb, int tile_w = 0);
-// Fills out[i] for boxes_h[6i..6i+5] (tile width tile_w, 0 = lattice_tile_w(),
-// shared distances) and returns the total tile count.
-int64_t make_lat_boxes(const int32_t *boxes_h, int32_t nbox, LatBox *out, int tile_w = 0);
+// Fills out[i] for boxes_h[6i..6i+5] (shared distances) and returns the total
+// count of their 16 x 16 tiles.
+int64_t make_lat_boxes(const int32_t *boxes_h, int32_t nbox, LatBox *out);
 struct LatOptions {
-  int tile_w = 0;              // tile width (0: lattice_tile_w()); the tables must use the same
   bool private_dist = false;   // boxes have their own slices (dbase >= 0): seed i starts box i, and
                                // `dist` is the slice arena of private_count entries, all reset
   int64_t private_count = 0;

@@ -632,7 +632,7 @@ int run_batch_cta(orsp_graph *g, const float *cost_d, int32_t K, const std::vect
 // chunks whose slices fit the arena (ORSP_BATCH_LAT_MB, default 4096 MB).
 int run_batch_lat(orsp_graph *g, const float *cost_d, int32_t K, const std::vector<int32_t> &items,
                   const std::vector<int32_t> &bb, const std::vector<int32_t> &src_h,
-                  const std::vector<int32_t> &dst_h, int tile_w, int32_t *path_nodes_d, int32_t *path_edges_d,
+                  const std::vector<int32_t> &dst_h, int32_t *path_nodes_d, int32_t *path_edges_d,
                   int32_t path_cap, int32_t *path_len_d, cudaStream_t st) {
   (void)K;
   const size_t n = items.size();
@@ -678,7 +678,7 @@ int run_batch_lat(orsp_graph *g, const float *cost_d, int32_t K, const std::vect
       h_src[j] = src_h[k];
       h_dst[j] = dst_h[k];
     }
-    const int64_t ntiles = make_lat_boxes(boxes.data(), m, hb, tile_w);
+    const int64_t ntiles = make_lat_boxes(boxes.data(), m, hb);
     int64_t base = 0;
     for (int32_t j = 0; j < m; ++j) {
       hb[j].dbase = base;
@@ -693,8 +693,12 @@ int run_batch_lat(orsp_graph *g, const float *cost_d, int32_t K, const std::vect
     rc = reserve_lattice_ws(g, ntiles);
     if (rc) return rc;
     LatOptions opt;
-    opt.tile_w = tile_w;
     opt.private_dist = true;
+    // many boxes: two CTAs per SM and the warp-specialised schedule, as for
+    // many sources (2 048 boxes of up to 400 x 400 x 16: 10.5 ms, against
+    // 14.6 ms without the schedule and 13.2 ms with it at one CTA per SM)
+    opt.blocks_per_sm = 2;
+    opt.spec = 1;
     opt.private_count = cells;
     opt.copy_ctl = false;
     rc = run_lattice_boxes(g, cost_d, m, d_src, nullptr, m, boxes.data(), db, g->blat_dist, st, &opt);
@@ -793,7 +797,7 @@ static int run_batch(orsp_graph *g, const float *cost_d, int32_t K, const int32_
     const int32_t k = ord[i];
     bucket[tuned ? plan_bucket(g, box_volume(&bb[(size_t)per * k], range_mode)) : 0].push_back(k);
   }
-  // Tile-sweep buckets first (one launch per tile width), then every
+  // Tile-sweep buckets first (one launch), then every
   // one-CTA-per-search item in a single launch, each with its bucket's width,
   // so that searches of all sizes share the GPU.
   std::vector<int32_t> src_h, dst_h;
@@ -806,32 +810,29 @@ static int run_batch(orsp_graph *g, const float *cost_d, int32_t K, const int32_
     const int32_t *b = &bb[(size_t)per * k];
     return lattice_tile_fits(b[5] - b[4] + 1, tw);
   };
-  for (int tw : {16, 32}) {
-    std::vector<int32_t> lat_items;
-    for (int i = 0; i < nb; ++i)
-      if (tuned && g->plan_impl[i] == 1 && g->lattice_ok && !(g->cvia && tw != 16) && g->plan_tile[i] == tw)
-        for (int32_t k : bucket[i])
-          if (tile_ok(k, tw)) lat_items.push_back(k);
-    if (lat_items.empty()) continue;
-    if (src_h.empty()) {
-      src_h.resize(K);
-      dst_h.resize(K);
-      ORSP_CUDA(cudaMemcpyAsync(src_h.data(), src_d, (size_t)K * 4, cudaMemcpyDeviceToHost, st));
-      ORSP_CUDA(cudaMemcpyAsync(dst_h.data(), dst_d, (size_t)K * 4, cudaMemcpyDeviceToHost, st));
-      ORSP_CUDA(cudaStreamSynchronize(st));
-    }
-    int rc = run_batch_lat(g, cost_d, K, lat_items, bb, src_h, dst_h, tw, path_nodes_d, path_edges_d, path_cap,
-                           path_len_d, st);
+  auto swept = [&](int i, int32_t k) {
+    return tuned && g->plan_impl[i] == 1 && g->lattice_ok && !(g->cvia && g->plan_tile[i] != 16) &&
+           tile_ok(k, g->plan_tile[i]);
+  };
+  std::vector<int32_t> lat_items;
+  for (int32_t i = 0; i < K; ++i) {
+    const int32_t k = ord[i];
+    if (tuned && swept(plan_bucket(g, box_volume(&bb[(size_t)per * k], range_mode)), k)) lat_items.push_back(k);
+  }
+  if (!lat_items.empty()) {
+    src_h.resize(K);
+    dst_h.resize(K);
+    ORSP_CUDA(cudaMemcpyAsync(src_h.data(), src_d, (size_t)K * 4, cudaMemcpyDeviceToHost, st));
+    ORSP_CUDA(cudaMemcpyAsync(dst_h.data(), dst_d, (size_t)K * 4, cudaMemcpyDeviceToHost, st));
+    ORSP_CUDA(cudaStreamSynchronize(st));
+    int rc = run_batch_lat(g, cost_d, K, lat_items, bb, src_h, dst_h, path_nodes_d, path_edges_d, path_cap, path_len_d,
+                           st);
     if (rc) return rc;
   }
   for (int i = 0; i < nb; ++i) {
     std::vector<int32_t> items;
-    if (tuned && g->plan_impl[i] == 1 && g->lattice_ok && !(g->cvia && g->plan_tile[i] != 16)) {
-      for (int32_t k : bucket[i])
-        if (!tile_ok(k, g->plan_tile[i])) items.push_back(k);
-    } else {
-      items = bucket[i];
-    }
+    for (int32_t k : bucket[i])
+      if (!swept(i, k)) items.push_back(k);
     if (items.empty()) continue;
     if (tuned) {
       if (delta_k.empty()) delta_k.assign(K, 0.0f);
@@ -992,14 +993,13 @@ extern "C" int orsp_sssp_sources(orsp_graph *g, const float *cost_d, int32_t nsr
     opt.private_count = (int64_t)m * g->N;
     opt.tma_slices = m;
     // many wave fronts keep two CTAs per SM busy: one's queue handoff
-    // overlaps the other's sweeps (measured 0.50 against 0.77 ms per source
-    // on 1000x1000x12 at 16 sources per launch)
+    // overlaps the other's sweeps (4.95 against 6.43 ms for 16 sources on
+    // 1000x1000x12)
     opt.blocks_per_sm = 2;
-    // and, for tiles of up to 12 layers (the instantiation sized for two
-    // CTAs per SM), the warp-specialised schedule: its scheduler warp takes
-    // the queue handoff off the workers' path (0.449 against 0.473 ms per
-    // source on 1000x1000x12)
-    opt.spec = g->nz <= 12 ? 1 : 0;
+    // and the warp-specialised schedule: its scheduler warp takes the queue
+    // handoff off the workers' path (4.95 against 5.61 ms for 16 sources on
+    // 1000x1000x12)
+    opt.spec = 1;
     // every chunk after the first reuses the gathered weights of this call
     if (decl) g->decl_cost = cost_d, g->decl_gen = decl;
     else if (a > 0) g->decl_cost = cost_d, g->decl_gen = ~0ull;

@@ -29,6 +29,7 @@
 #include <climits>
 #include <cstdlib>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -89,6 +90,10 @@ struct LatParams {
   const float *wcol;       // column vias: gathered via weights [N][nzp] (Graph::wcol)
   int32_t nzp;             // nz rounded up to 4
   int64_t N;
+  // layers by axis, as bit sets and as ascending lists (run visits)
+  uint64_t hmask, vmask;
+  int8_t hlist[64], vlist[64];
+  const int32_t *tbox;  // box of each tile (asynchronous schedule)
 };
 
 __global__ void fill_kernel(uint32_t *p, int64_t n, uint32_t v) {
@@ -398,6 +403,20 @@ __device__ __forceinline__ int tile_of(const LatBox &B, int32_t gx, int32_t gy) 
   return B.tile0 + ((gy - B.y0) / TY) * B.ntx + (gx - B.x0) / TX;
 }
 
+// Asynchronous schedule: every tile idle, the queue empty, each tile's box.
+__global__ void lattice_init_kernel(LatParams p, int32_t ntiles) {
+  const int64_t s = (int64_t)gridDim.x * blockDim.x;
+  const int64_t n = max((int64_t)ntiles, (int64_t)p.qcap);
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += s) {
+    if (i < ntiles) {
+      p.tstate[i] = 0;
+      p.stamp[i] = 0;
+      p.list0[i] = p.nbox == 1 ? 0 : box_of_tile(p, (int)i);
+    }
+    if (i < p.qcap) p.qslot[i] = -1;
+  }
+}
+
 template <int TX, int TY>
 __global__ void lattice_seed_kernel(LatParams p, int32_t nseeds, const int32_t *seeds,
                                     const float *seed_cost) {
@@ -445,6 +464,8 @@ __global__ void lattice_seed_kernel(LatParams p, int32_t nseeds, const int32_t *
     // on a tile edge reaches the next tile through that tile's halo only.
     const int t = tile_of<TX, TY>(B, x, y);
     const int lt = t - B.tile0, tx = lt % B.ntx, ty = lt / B.ntx;
+    // its columns start unrelaxed: the first visit takes all of them
+    if (p.qslot) p.stamp[t] = 1u;
     const int nb[5] = {t, tx > 0 ? t - 1 : -1, tx < B.ntx - 1 ? t + 1 : -1, ty > 0 ? t - B.ntx : -1,
                        ty < B.nty - 1 ? t + B.ntx : -1};
     for (int j = 0; j < 5; ++j) {
@@ -700,13 +721,13 @@ __device__ __forceinline__ void tma_stage(const LatParams &p, int32_t X0, int32_
 // box (Gauss-Seidel, so a later layer sees an earlier one's new value), the
 // in-weights read as float4 rows wcol[v * nzp ..] (+inf where no via).  col:
 // the column's distances in shared memory, layer stride PS; v0: the node of
-// the column's layer z0.  Returns whether any distance decreased.  The sweep
-// cycles of the visit repeat it until nothing changes.
+// the column's layer z0.  Returns the set of layers that decreased.  The
+// visit repeats it until nothing changes.
 template <int PS>
-__device__ __forceinline__ bool zcol_pass(float *col, const float *__restrict__ wcol, int32_t nzp, int64_t v0,
+__device__ __forceinline__ unsigned long long zcol_pass(float *col, const float *__restrict__ wcol, int32_t nzp, int64_t v0,
                                           int64_t nxy, int32_t z0, int32_t nzb) {
   const float INF_F = __int_as_float(0x7f800000);
-  bool chg = false;
+  unsigned long long chg = 0;
   const int q0 = z0 >> 2, q1 = (z0 + nzb - 1) >> 2;
   for (int zb = 0; zb < nzb; ++zb) {
     const float4 *wr = reinterpret_cast<const float4 *>(wcol + (v0 + (int64_t)zb * nxy) * nzp);
@@ -722,7 +743,7 @@ __device__ __forceinline__ bool zcol_pass(float *col, const float *__restrict__ 
     }
     if (best < col[zb * PS]) {
       col[zb * PS] = best;
-      chg = true;
+      chg |= 1ull << zb;
     }
   }
   return chg;
@@ -986,7 +1007,7 @@ __device__ __forceinline__ void process_tile(const LatParams &p, int t, float *s
       const int xx = c % tw + 1, yy = c / tw + 1;
       if constexpr (CV) {
         const int64_t v0 = (int64_t)B.z0 * nxy + col0 + (int64_t)(yy - 1) * p.nx + (xx - 1);
-        chg |= zcol_pass<PS>(sd + yy * SX + xx, p.wcol, p.nzp, v0, nxy, B.z0, nzb);
+        chg |= zcol_pass<PS>(sd + yy * SX + xx, p.wcol, p.nzp, v0, nxy, B.z0, nzb) != 0;
       } else {
         const int wo = (yy - 1) * WSX + (xx - 1);
         chg |= zrun<PS, WPS>(sd + yy * SX + xx, wdn + wo, wup + wo, nzb);
@@ -1037,6 +1058,356 @@ __device__ __forceinline__ void process_tile(const LatParams &p, int t, float *s
     atomicAdd(&p.ctl->ns[1], ts2 - ts1);
     atomicAdd(&p.ctl->ns[2], ts3 - ts2);
   }
+}
+
+// ---------------------------------------------------------------------------
+// Run visit: the tile visit of 16 x 16 tiles of up to NZM layers.
+//
+// The visit above keeps everything in shared memory: each relaxation reads a
+// distance and a weight from it, each sweep cycle walks every run forward
+// and then backward, and one more cycle that changes nothing ends the visit.
+// It is bound by shared-memory accesses and by the length of the dependent
+// add-min chains (1.6 us per sweep cycle of a 12-layer tile, 3.2 cycles a
+// visit).  Here
+//  - a thread owns one planar run (16 cells of a row on an H layer or of a
+//    column on a V layer) and one via column for the whole visit, with the
+//    weights of both in registers and its run's two halo values too; only
+//    the distances are in shared memory, so the planar and the via passes
+//    read and write them and nothing else;
+//  - the forward and the backward walk of a run start from the same values,
+//    run side by side and are combined with a min.  With non-negative weights
+//    a shortest path inside a run never turns (the cell where it turned was
+//    reached with no more), and the sums along it are those of the one-sided
+//    walk, so the result is the run's fixpoint as before, bit for bit, with
+//    half the chain;
+//  - a pass takes only the runs (columns) in which the other pass changed a
+//    cell since they were last taken, by bit sets in shared memory.  A run or
+//    column just taken is at its own fixpoint, so when a pass changes
+//    nothing that the other one reads, the tile is at its fixpoint and the
+//    visit ends, with no confirming cycle.
+// Cells outside the box hold +inf with +inf weights, so every run has its
+// full length.
+// Measured (before -> after, per visit: load / passes / write-back): one
+// 18-layer box 2.55 / 6.77 / 1.17 -> 1.65 / 2.66 / 1.78 us; 600 x 600 x 12,
+// one source, 795 -> 612 us; 1000 x 1000 x 12, 16 sources, 6.50 -> 4.95 ms;
+// 2 048 boxes of up to 400 x 400 x 16, 19.1 -> 9.9 ms (against 32-wide tiles).
+//
+// Threads: 16 runs per layer, H runs first: 256 threads up to 16 layers, 288
+// above.  Shared memory: nzb x 3 x 280 floats (distances, the two planar
+// weight arrays as they pass from the column loads to the runs), with ZS
+// nzb x 5 x 280 (the via weights too, where two CTAs share an SM's registers).
+constexpr int kRunWS = 17;                // row stride (odd: rows and columns hit distinct banks)
+constexpr int kRunPS = tile_wps(16, 16);  // layer stride
+template <int NZM, bool ZS>
+struct RunTile {
+  static constexpr int NW = NZM > 16 ? 288 : 256;
+  float lo[16], hi[16];    // the run's in-edge weights from its lower / upper neighbours
+  float dn[ZS ? 1 : NZM], up[ZS ? 1 : NZM];  // the column's in-edge weights from below / above
+  float ha, hb;            // the run's halo values
+};
+
+struct RunShared {
+  // columns changed by the last planar pass: by row (bits x), by column (bits y)
+  unsigned rowx[2][16], coly[2][16];
+  // layers changed by the last via pass: by row, by column
+  unsigned rowz[2][16], colz[2][16];
+  unsigned cells[32 * 16];  // cells changed by the visit's planar passes: [layer][line]
+  // thread 0: times in load, passes and write-back and the cycles made,
+  // summed over the block's visits and added to the control block at its end
+  unsigned long long ns[3], last;
+  unsigned cycles;
+  __device__ __forceinline__ void start() { ns[0] = ns[1] = ns[2] = 0, cycles = 0; }
+  __device__ __forceinline__ void lap(int i) {
+    const unsigned long long t = dev_globaltimer();
+    if (i >= 0) ns[i] += t - last;
+    last = t;
+  }
+  __device__ __forceinline__ void flush(LatCtl *c) const {
+    atomicAdd(&c->cycles, (unsigned long long)cycles);
+    for (int i = 0; i < 3; ++i) atomicAdd(&c->ns[i], ns[i]);
+  }
+};
+
+__host__ __device__ constexpr int run_smem_floats(int nzb, bool zs) { return nzb * (zs ? 5 : 3) * kRunPS; }
+
+// Asynchronous 8-byte copy from global to shared memory.
+__device__ __forceinline__ void copy8_async(void *dst, const void *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+
+// OR of `v` over the visiting threads, with their barrier.
+template <int NW, bool SPEC>
+__device__ __forceinline__ bool tile_sync_or(bool v) {
+  if (SPEC) {
+    unsigned r;
+    asm volatile(
+        "{\n .reg .pred P, Q;\n setp.ne.u32 P, %1, 0;\n bar.red.or.pred Q, 1, %2, P;\n selp.u32 %0, 1, 0, Q;\n}"
+        : "=r"(r)
+        : "r"((unsigned)v), "n"(NW)
+        : "memory");
+    return r != 0;
+  }
+  return __syncthreads_or(v) != 0;
+}
+
+// Both walks over N cells: LD(i) the cells' values, LO(i) / HI(i) the weights
+// from the lower / upper neighbour, a / b the values before the first and
+// after the last cell, ST(i, v) stores a decreased cell.  The walks meet in
+// the middle; from there on each step completes one cell on either side, so
+// at most half of each walk is kept.  Returns the set of decreased cells.
+template <int N, class LD, class LO, class HI, class ST>
+__device__ __forceinline__ unsigned walk_both(float a, float b, LD ld, LO lo, HI hi, ST st) {
+  float o[N], k[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) o[i] = ld(i);
+  unsigned m = 0;
+  auto put = [&](int i, float v) {
+    if (v < o[i]) {
+      st(i, v);
+      m |= 1u << i;
+    }
+  };
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const int j = N - 1 - i;
+    a = fminf(__fadd_rn(a, lo(i)), o[i]);
+    b = fminf(__fadd_rn(b, hi(j)), o[j]);
+    if (i < j) {
+      k[i] = a;
+      k[j] = b;
+    } else if (i == j) {
+      put(i, fminf(a, b));
+    } else {
+      put(i, fminf(a, k[i]));
+      put(j, fminf(b, k[j]));
+    }
+  }
+  return m;
+}
+
+// The same visit contract as process_tile.  warm: the tile was visited last
+// by this block (its distances are in shared memory, its weights in R), only
+// the halo is read again and only the runs whose halo improved are taken
+// first.  force (shared with the block): the last visit stopped at MAX_CYCLES.
+//
+// B: the tile's box, in shared memory.  (Looked up by the visit itself, the
+// binary search over the boxes and the box's fields were dependent trips to
+// L2 - the streamed weights evict them from L1 - and cost 3 us of an 11 us
+// visit with 16 boxes and two CTAs per SM.)
+template <int NZM, bool PRIV, bool SPEC, bool CV, bool ZS>
+__device__ __forceinline__ void visit_runs(const LatParams &p, int t, const LatBox &SB, float *sd, RunTile<NZM, ZS> &R, RunShared &S,
+                                           int *s_act, int *s_nb, bool warm) {
+  constexpr int NW = RunTile<NZM, ZS>::NW, WS = kRunWS, PS = kRunPS;
+  const float INF_F = __int_as_float(0x7f800000);
+  const LatBox B = SB;
+  const int lt = t - B.tile0;
+  const int ty = lt / B.ntx, tx = lt - ty * B.ntx;
+  const int32_t X0 = B.x0 + tx * 16, Y0 = B.y0 + ty * 16;
+  const int tw = min(16, B.x1 - X0 + 1), th = min(16, B.y1 - Y0 + 1);
+  const int nzb = B.z1 - B.z0 + 1;
+  const int64_t nxy = (int64_t)p.nx * p.ny;
+  const uint64_t lay = nzb >= 64 ? ~0ull : (1ull << nzb) - 1ull;
+  const unsigned hm = (unsigned)((p.hmask >> B.z0) & lay), vm = (unsigned)((p.vmask >> B.z0) & lay);
+  const int nh = __popc(hm), nv = __popc(vm);
+  const int tid = threadIdx.x;
+  if (tid == 0) S.lap(-1);
+  if (tid < 5) s_act[tid] = 0;
+  if (s_nb && tid < 4) {  // neighbour tiles in the box: left, right, down, up (-1: box edge)
+    s_nb[tid] = tid == 0 ? (tx > 0 ? t - 1 : -1)
+                         : tid == 1 ? (tx < B.ntx - 1 ? t + 1 : -1)
+                                    : tid == 2 ? (ty > 0 ? t - B.ntx : -1) : (ty < B.nty - 1 ? t + B.ntx : -1);
+  }
+  if (tid < 32) {
+    const int k = tid >> 4, i = tid & 15;
+    S.rowx[k][i] = S.coly[k][i] = S.rowz[k][i] = S.colz[k][i] = 0;
+  }
+  // the thread's run: layer rz, line rl
+  const int v0 = nh * 16;
+  const bool isv = tid >= v0;
+  const int ri = isv ? tid - v0 : tid;
+  const int rl = ri & 15;
+  bool run = ri < 16 * (isv ? nv : nh) && rl < (isv ? tw : th);
+  int rz = 0;
+  if (run) rz = isv ? p.vlist[__popcll(p.vmask & ((1ull << B.z0) - 1ull)) + (ri >> 4)] - B.z0
+                    : p.hlist[__popcll(p.hmask & ((1ull << B.z0) - 1ull)) + (ri >> 4)] - B.z0;
+  // the thread's column
+  const int xx = tid & 15, yy = tid >> 4;
+  const bool col = tid < 256 && xx < tw && yy < th;
+  // ---- load: the run's halo cells (where the box has them), then the column
+  float ha = INF_F, hb = INF_F;
+  if (run) {
+    const int32_t gx = isv ? X0 + rl : X0, gy = isv ? Y0 : Y0 + rl, gz = B.z0 + rz;
+    if (isv) {
+      if (Y0 > B.y0) ha = bits_f(__ldcg(&p.dist[dist_index<PRIV>(p, B, gx, gy - 1, gz)]));
+      if (Y0 + 16 <= B.y1) hb = bits_f(__ldcg(&p.dist[dist_index<PRIV>(p, B, gx, gy + 16, gz)]));
+    } else {
+      if (X0 > B.x0) ha = bits_f(__ldcg(&p.dist[dist_index<PRIV>(p, B, gx - 1, gy, gz)]));
+      if (X0 + 16 <= B.x1) hb = bits_f(__ldcg(&p.dist[dist_index<PRIV>(p, B, gx + 16, gy, gz)]));
+    }
+  }
+  const bool force = __ldcg(&p.stamp[t]) != 0;
+  const int64_t n0 = (int64_t)B.z0 * nxy + (int64_t)(Y0 + yy) * p.nx + (X0 + xx);  // the column's node at z0
+  const int64_t dz = (!PRIV || B.dbase < 0) ? nxy : (int64_t)(B.x1 - B.x0 + 1) * (B.y1 - B.y0 + 1);
+  float *const cd = sd + yy * WS + xx;  // the column's distances
+  float2 *const wp = (float2 *)(sd + nzb * PS);  // planar weight pairs
+  float2 *const wz = wp + nzb * PS;              // via weight pairs (ZS)
+  const int rbase = isv ? rz * PS + rl : rz * PS + rl * WS;
+  bool dirty = run;
+  if (!warm) {
+    if (tid < 256) {
+      const int64_t d0 = col ? dist_index<PRIV>(p, B, X0 + xx, Y0 + yy, B.z0) : 0;
+      const int w0 = yy * WS + xx;
+      if constexpr (ZS) {
+        // the weights go to shared memory as they are, 8 bytes per copy, all
+        // in flight and without registers to hold them
+        const float4 *src = p.w4 + n0;
+#pragma unroll
+        for (int z = 0; z < NZM; ++z)
+          if (z < nzb) {
+            if (col) {
+              copy8_async(&wp[z * PS + w0], src + z * nxy);
+              copy8_async(&wz[z * PS + w0], (const float2 *)(src + z * nxy) + 1);
+            } else {
+              wp[z * PS + w0] = wz[z * PS + w0] = make_float2(INF_F, INF_F);
+            }
+          }
+      }
+      float dv[NZM];
+      float4 wv[ZS ? 1 : NZM];
+#pragma unroll
+      for (int z = 0; z < NZM; ++z) {
+        dv[z] = INF_F;
+        if (!ZS) wv[ZS ? 0 : z] = make_float4(INF_F, INF_F, INF_F, INF_F);
+        if (col && z < nzb) {
+          dv[z] = bits_f(__ldcg(&p.dist[d0 + z * dz]));
+          if (!ZS) wv[ZS ? 0 : z] = __ldg(&p.w4[n0 + z * nxy]);
+        }
+      }
+#pragma unroll
+      for (int z = 0; z < NZM; ++z) {
+        if (z < nzb) {
+          cd[z * PS] = dv[z];
+          if (!ZS) wp[z * PS + w0] = make_float2(wv[ZS ? 0 : z].x, wv[ZS ? 0 : z].y);
+        }
+        if constexpr (!ZS) {
+          R.dn[z] = wv[z].z;
+          R.up[z] = wv[z].w;
+        }
+      }
+      if (ZS) asm volatile("cp.async.wait_all;" ::: "memory");
+    }
+    tile_sync<NW, SPEC>();
+    if (run) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const float2 w = wp[rbase + i * (isv ? WS : 1)];
+        R.lo[i] = w.x;
+        R.hi[i] = w.y;
+      }
+    }
+  } else {
+    dirty = run && (force || ha < R.ha || hb < R.hb);
+    tile_sync<NW, SPEC>();
+  }
+  R.ha = ha;
+  R.hb = hb;
+  if (tid == 0) S.lap(0);
+
+  // ---- passes
+  const float2 *const cw = wz + yy * WS + xx;
+  auto run_pass = [&](float *c, auto stride) {
+    constexpr int DS = decltype(stride)::value;
+    return walk_both<16>(
+        ha, hb, [&](int i) { return c[i * DS]; }, [&](int i) { return R.lo[i]; }, [&](int i) { return R.hi[i]; },
+        [&](int i, float v) { c[i * DS] = v; });
+  };
+  unsigned runm = 0, colm = 0;  // cells changed by this visit: the run's, the column's (by layer)
+  bool converged = false, again = false;
+  int cyc = 0;
+  for (; cyc < MAX_CYCLES; ++cyc) {
+    const int k = cyc & 1;
+    unsigned m = 0;
+    if (dirty) {
+      if (isv) {
+        m = run_pass(sd + rbase, std::integral_constant<int, WS>());
+        if (m) atomicOr(&S.coly[k][rl], m);
+      } else {
+        m = run_pass(sd + rbase, std::integral_constant<int, 1>());
+        if (m) atomicOr(&S.rowx[k][rl], m);
+      }
+      runm |= m;
+    }
+    const bool all = force && cyc == 0;
+    if (!tile_sync_or<NW, SPEC>(m != 0 || again) && !all) {
+      converged = true;
+      break;
+    }
+    unsigned mz = 0;
+    const bool take = col && (all || again || (((S.rowx[k][yy] >> xx) | (S.coly[k][xx] >> yy)) & 1u));
+    if (take) {
+      if constexpr (CV) mz = (unsigned)zcol_pass<PS>(cd, p.wcol, p.nzp, n0, nxy, B.z0, nzb);
+      else
+        mz = walk_both<NZM>(
+            INF_F, INF_F, [&](int z) { return z < nzb ? cd[z * PS] : INF_F; },
+            [&](int z) { return ZS ? (z < nzb ? cw[z * PS].x : INF_F) : R.dn[ZS ? 0 : z]; },
+            [&](int z) { return ZS ? (z < nzb ? cw[z * PS].y : INF_F) : R.up[ZS ? 0 : z]; },
+            [&](int z, float v) { cd[z * PS] = v; });
+      if (mz) {
+        if (mz & hm) atomicOr(&S.rowz[k][yy], mz & hm);
+        if (mz & vm) atomicOr(&S.colz[k][xx], mz & vm);
+        colm |= mz;
+      }
+    }
+    // one Gauss-Seidel pass over a column's layer pairs is not its fixpoint:
+    // a column-via column that changed is taken again
+    if (CV) again = mz != 0;
+    if (tid < 16) {
+      S.rowx[k ^ 1][tid] = S.coly[k ^ 1][tid] = 0;
+      S.rowz[k ^ 1][tid] = S.colz[k ^ 1][tid] = 0;
+    }
+    if (!tile_sync_or<NW, SPEC>(CV ? mz != 0 : (mz & (hm | vm)) != 0)) {
+      converged = true;
+      break;
+    }
+    dirty = run && (((isv ? S.colz[k][rl] : S.rowz[k][rl]) >> rz) & 1u);
+  }
+  if (tid == 0) {
+    S.lap(1);
+    S.cycles += cyc + 1;
+  }
+
+  // ---- publish improvements; mark neighbour tiles whose halo changed.  One
+  // thread per column: the layers its own passes changed, and its bits of the
+  // runs' changed cells.
+  if (run) S.cells[rz * 16 + rl] = runm;
+  tile_sync<NW, SPEC>();
+  if (col) {
+    const int64_t d0 = dist_index<PRIV>(p, B, X0 + xx, Y0 + yy, B.z0);
+#pragma unroll
+    for (int z = 0; z < NZM; ++z)
+      if (((hm | vm) >> z) & 1u) {
+        const bool h = (hm >> z) & 1u;
+        if ((S.cells[z * 16 + (h ? yy : xx)] >> (h ? xx : yy)) & 1u) colm |= 1u << z;
+      }
+#pragma unroll
+    for (int z = 0; z < NZM; ++z)
+      if ((colm >> z) & 1u) __stcg(&p.dist[d0 + z * dz], f_bits(cd[z * PS]));
+    if (colm & hm) {
+      if (xx == 0) s_act[0] = 1;
+      if (xx == tw - 1) s_act[1] = 1;
+    }
+    if (colm & vm) {
+      if (yy == 0) s_act[2] = 1;
+      if (yy == th - 1) s_act[3] = 1;
+    }
+  }
+  if (tid == 0) {
+    if (!converged) s_act[4] = 1;
+    if (force == converged) p.stamp[t] = converged ? 0u : 1u;
+  }
+  tile_sync<NW, SPEC>();
+  if (tid == 0) S.lap(2);
 }
 
 // Tiles to revisit after a visit of tile t: the neighbours whose halo value
@@ -1152,8 +1523,11 @@ __device__ bool activate_tile(const LatParams &p, int t) {
 // the whole lattice (the tensor maps and the staging are sized for p.nz
 // layers), distances in slices of N cells (LatBox.pad = slice).  tmw / tmd
 // are unused otherwise.
-template <int TX, int TY, bool PRIV, bool DEEP = false, int MINB = 1, bool TMA = false, bool CV = false>
-__global__ void __launch_bounds__(TX * TY, MINB)
+//
+// NZM > 0: run visits (visit_runs) of tiles of up to NZM layers.
+template <int TX, int TY, bool PRIV, bool DEEP = false, int MINB = 1, bool TMA = false, bool CV = false, int NZM = 0,
+          bool ZS = false>
+__global__ void __launch_bounds__(NZM > 0 ? RunTile<NZM ? NZM : 1, ZS>::NW : TX *TY, MINB)
     lattice_async_kernel(LatParams p, const __grid_constant__ CUtensorMap tmw, const __grid_constant__ CUtensorMap tmd) {
   extern __shared__ __align__(128) float sd[];
   __shared__ LayerLists s_layers;
@@ -1180,7 +1554,11 @@ __global__ void __launch_bounds__(TX * TY, MINB)
       asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&tmd) : "memory");
     }
   }
-  if (threadIdx.x == 0) s_layers.box = -1;
+  __shared__ RunShared s_run;
+  if (threadIdx.x == 0) s_layers.box = -1, s_run.start();
+  __shared__ LatBox s_box;
+  int box = -1;  // thread 0: the box in s_box
+  RunTile<NZM ? NZM : 1, ZS> R;
   __syncthreads();
   unsigned visits = 0;
   unsigned long long sched_ns = 0;
@@ -1214,7 +1592,12 @@ __global__ void __launch_bounds__(TX * TY, MINB)
         }
       }
       if (t >= 0) {
+        const int bi = NZM > 0 ? __ldg(&p.tbox[t]) : 0;
         atomicExch(&p.tstate[t], 2);
+        if (NZM > 0 && bi != box) {
+          s_box = load_box(p, bi);
+          box = bi;
+        }
         __threadfence();
       }
       s_tile = t;
@@ -1225,7 +1608,8 @@ __global__ void __launch_bounds__(TX * TY, MINB)
     const int t = warm ? s_cont : s_tile;
     __syncthreads();
     if (t < 0) break;
-    process_tile<TX, TY, PRIV, false, DEEP, TMA, CV>(p, t, sd, s_layers, s_flags, s_act, s_nb, warm, &tma);
+    if constexpr (NZM > 0) visit_runs<NZM, PRIV, false, CV, ZS>(p, t, s_box, sd, R, s_run, s_act, s_nb, warm);
+    else process_tile<TX, TY, PRIV, false, DEEP, TMA, CV>(p, t, sd, s_layers, s_flags, s_act, s_nb, warm, &tma);
     // neighbours are activated by threads 0..3 in parallel, after this
     // tile's distances are visible
     unsigned long long ta = 0;
@@ -1264,28 +1648,49 @@ __global__ void __launch_bounds__(TX * TY, MINB)
   if (threadIdx.x == 0) {
     atomicAdd(&ctl->visits, visits);
     atomicAdd(&ctl->ns[3], sched_ns);
+    if (NZM > 0) s_run.flush(ctl);
   }
 }
 
-// Scheduler side of a finished visit of tile t with neighbour flags act:
-// activate the neighbours whose halo improved, then leave the visiting state
-// (idle, or queued again when dirty or not converged).  `pending` drops only
-// after everything the visit activated is queued.
-__device__ void finish_visit(const LatParams &p, int t, const int *act) {
+// Scheduler side of a finished visit of tile t with neighbour flags act, by
+// one full warp: activate the neighbours whose halo improved (lanes 0..3) and
+// leave the visiting state - idle, or queued again when dirty or not
+// converged (lane 4).  Everything newly queued takes consecutive queue
+// places; `pending` counts it (and drops this visit) before it is visible in
+// the queue, so it reaches 0 only at the fixpoint.  Three dependent trips to
+// L2 in all; one lane doing the same tile after tile took about 6 us, more
+// than the visit it overlaps.
+__device__ void finish_visit(const LatParams &p, int t, const LatBox &B, const int *act, int lane) {
   __threadfence();
-  const LatBox B = load_box(p, box_of_tile(p, t));
-  const int lt = t - B.tile0, tx = lt % B.ntx, ty = lt / B.ntx;
-  const int nbs[4] = {(act[0] && tx > 0) ? t - 1 : -1, (act[1] && tx < B.ntx - 1) ? t + 1 : -1,
-                      (act[2] && ty > 0) ? t - B.ntx : -1, (act[3] && ty < B.nty - 1) ? t + B.ntx : -1};
-#pragma unroll
-  for (int d = 0; d < 4; ++d)
-    if (nbs[d] >= 0 && !activate_tile(p, nbs[d])) atomicCAS(&p.ctl->err, DEV_OK, DEV_ERR_INTERNAL);
-  if (act[4] || atomicCAS(&p.tstate[t], 2, 0) != 2) {
-    atomicExch(&p.tstate[t], 1);
-    queue_tile(p, t);
-  } else {
-    atomicSub(&p.ctl->pending, 1);
+  const int lt = t - B.tile0, ty = lt / B.ntx, tx = lt - ty * B.ntx;
+  int q = -1;
+  if (lane == 0 && act[0] && tx > 0) q = t - 1;
+  if (lane == 1 && act[1] && tx < B.ntx - 1) q = t + 1;
+  if (lane == 2 && act[2] && ty > 0) q = t - B.ntx;
+  if (lane == 3 && act[3] && ty < B.nty - 1) q = t + B.ntx;
+  bool queue = false, bad = q >= 0;
+  for (int tries = 0; bad && tries < 1024; ++tries) {
+    const int st = atomicCAS(&p.tstate[q], 0, 1);
+    queue = st == 0;
+    bad = !(st == 0 || st == 1 || st == 3 || atomicCAS(&p.tstate[q], 2, 3) == 2);
   }
+  if (lane == 4 && (act[4] || atomicCAS(&p.tstate[t], 2, 0) != 2)) {
+    atomicExch(&p.tstate[t], 1);
+    q = t;
+    queue = true;
+  }
+  const unsigned m = __ballot_sync(ORSP_FULL_MASK, queue);
+  const int n = __popc(m);
+  unsigned base = 0;
+  if (lane == 0) {
+    if (n) base = atomicAdd(&p.ctl->tail, (unsigned)n);
+    // (this visit is one of `pending`; the returned value is awaited before
+    // the tiles are queued)
+    if (n != 1 && atomicAdd(&p.ctl->pending, n - 1) < 1) bad = true;
+  }
+  base = __shfl_sync(ORSP_FULL_MASK, base, 0);
+  if (queue) atomicExch(&p.qslot[(base + __popc(m & lanemask_lt())) % p.qcap], q);
+  if (bad) atomicCAS(&p.ctl->err, DEV_OK, DEV_ERR_INTERNAL);
 }
 
 // Warp-specialised asynchronous schedule.  The block has NW = TX*TY worker
@@ -1299,8 +1704,7 @@ __device__ void finish_visit(const LatParams &p, int t, const int *act) {
 // once per handoff (the scheduler warp passes it once per loop iteration, the
 // workers once before each visit; both stop after the handoff that carries
 // -1).  The workers visit cur_k with their own named barrier 1, write the
-// visit's neighbour flags into s_act[k & 1] and, after a device fence, set
-// s_done = k.  The scheduler finishes visit k (activations, state
+// visit's neighbour flags into s_act[k & 1] and set s_done = k.  The scheduler finishes visit k (activations, state
 // transition) once s_done == k - in its wait loop for the next tile, or just
 // after the next handoff - so it never waits for work that only its own
 // finished tile would create.  The flags of visit k stay intact until visit
@@ -1311,8 +1715,8 @@ __device__ void finish_visit(const LatParams &p, int t, const int *act) {
 // below the tile where the box has them (the y-halo).  Every address
 // prefetched lies inside the weight array or the box's distances.
 template <int TX, int TY, bool PRIV>
-__device__ __forceinline__ void prefetch_tile_l2(const LatParams &p, int t, int lane) {
-  const LatBox B = load_box(p, box_of_tile(p, t));
+__device__ __forceinline__ void prefetch_tile_l2(const LatParams &p, int t, const LatBox &SB, int lane) {
+  const LatBox B = SB;
   const int lt = t - B.tile0;
   const int tx = lt % B.ntx, ty = lt / B.ntx;
   const int32_t X0 = B.x0 + tx * TX, Y0 = B.y0 + ty * TY;
@@ -1336,22 +1740,23 @@ __device__ __forceinline__ void prefetch_tile_l2(const LatParams &p, int t, int 
   }
 }
 
-template <int TX, int TY, bool PRIV, int MINB = 1>
-__global__ void __launch_bounds__(TX * TY + 32, MINB) lattice_spec_kernel(LatParams p) {
-  constexpr int NW = TX * TY;
+template <int NZM, bool PRIV, int MINB, bool ZS>
+__global__ void __launch_bounds__(RunTile<NZM, ZS>::NW + 32, MINB) lattice_spec_kernel(LatParams p) {
+  constexpr int NW = RunTile<NZM, ZS>::NW;
   extern __shared__ float sd[];
-  __shared__ LayerLists s_layers;
-  __shared__ int s_flags[6];
   __shared__ int s_act[2][5];
   __shared__ volatile int s_cur;
   __shared__ volatile int s_done;
+  __shared__ LatBox s_box[2];  // boxes of the handed-over tiles, by parity of the handoff
   LatCtl *ctl = p.ctl;
-  if (threadIdx.x == 0) s_layers.box = -1;
+  __shared__ RunShared s_run;
+  if (threadIdx.x == 0) s_run.start();
   if (threadIdx.x == NW) s_done = 0;
   __syncthreads();
   if (threadIdx.x < NW) {
     // ---------------------------------------------------------- workers
-    unsigned long long idle_ns = 0;
+    RunTile<NZM, ZS> R;
+      unsigned long long idle_ns = 0;
     for (int k = 1;; ++k) {
       unsigned long long tw = 0;
       if (threadIdx.x == 0) tw = dev_globaltimer();
@@ -1359,14 +1764,19 @@ __global__ void __launch_bounds__(TX * TY + 32, MINB) lattice_spec_kernel(LatPar
       if (threadIdx.x == 0) idle_ns += dev_globaltimer() - tw;
       const int t = s_cur;
       if (t < 0) break;
-      process_tile<TX, TY, PRIV, true>(p, t, sd, s_layers, s_flags, s_act[k & 1]);
-      // process_tile ended with barrier 1: every write of the visit is done
+      visit_runs<NZM, PRIV, true, false, ZS>(p, t, s_box[k & 1], sd, R, s_run, s_act[k & 1], nullptr, false);
+      // the visit ended with barrier 1: every write of it is done, and
+      // finish_visit's device fence makes them visible before it activates
+      // any tile (the workers do not wait for that fence)
       if (threadIdx.x == 0) {
-        __threadfence();
+        __threadfence_block();
         s_done = k;
       }
     }
-    if (threadIdx.x == 0) atomicAdd(&ctl->ns[3], idle_ns);
+    if (threadIdx.x == 0) {
+      atomicAdd(&ctl->ns[3], idle_ns);
+      s_run.flush(ctl);
+    }
     return;
   }
   // ------------------------------------------------------------ scheduler
@@ -1378,47 +1788,59 @@ __global__ void __launch_bounds__(TX * TY + 32, MINB) lattice_spec_kernel(LatPar
   unsigned visits = 0;
   for (;;) {
     int next = -1;
-    if (lane == 0) {
-      long long pos = -1;
-      const unsigned long long t0 = dev_globaltimer();
-      for (unsigned spins = 0;; ++spins) {
-        if (!finished && s_done == k) {
-          finish_visit(p, cur, s_act[k & 1]);
-          ++visits;
-          finished = true;
-        }
-        if (ld_acquire_u32((const unsigned *)&ctl->err)) break;
+    long long pos = -1;
+    const unsigned long long t0 = dev_globaltimer();
+    for (unsigned spins = 0;; ++spins) {
+      // (one lane reads it: the warp takes the branch as one)
+      if (!finished && __shfl_sync(0xffffffffu, s_done, 0) == k) {
+        finish_visit(p, cur, s_box[k & 1], s_act[k & 1], lane);
+        ++visits;
+        finished = true;
+      }
+      int got = 0;  // 1: a tile, 2: stop
+      if (lane == 0) {
         if (pos < 0) pos = (long long)atomicAdd(&ctl->head, 1u);
         int *slot = &p.qslot[(unsigned)pos % p.qcap];
-        const int v = (int)ld_acquire_u32((const unsigned *)slot);
-        if (v >= 0) {
+        next = (int)ld_acquire_u32((const unsigned *)slot);
+        if (next >= 0) {
           atomicExch(slot, -1);
-          atomicExch(&p.tstate[v], 2);
-          __threadfence();
-          next = v;
-          break;
-        }
-        if (finished && ld_acquire_u32((const unsigned *)&ctl->pending) == 0) break;  // fixpoint reached
-        if ((spins & 31u) == 31u) {
+          atomicExch(&p.tstate[next], 2);
+          got = 1;
+        } else if (ld_acquire_u32((const unsigned *)&ctl->err)) {
+          got = 2;
+        } else if (finished && ld_acquire_u32((const unsigned *)&ctl->pending) == 0) {
+          got = 2;  // fixpoint reached
+        } else if ((spins & 31u) == 31u) {
           const unsigned long long now = dev_globaltimer();
           if (now - t0 > p.wait_ns || now - t_start > p.budget_ns) {
             atomicCAS(&ctl->err, DEV_OK, DEV_ERR_TIMEOUT);
-            break;
+            got = 2;
           }
           __nanosleep(64);
         }
       }
-      s_cur = next;
-      __threadfence_block();
+      got = __shfl_sync(0xffffffffu, got, 0);
+      if (got == 2) next = -1;
+      if (got) break;
     }
     next = __shfl_sync(0xffffffffu, next, 0);
-    // the workers are still on visit k: bring the next tile's rows into L2
-    if (next >= 0 && p.prefetch) prefetch_tile_l2<TX, TY, PRIV>(p, next, lane);
+    if (lane == 0) {
+      s_cur = next;
+      __threadfence();  // the tile is marked as visited before its halo is read
+    }
+    // the workers are still on visit k: hand over the next tile's box and
+    // bring its rows into L2
+    if (next >= 0) {
+      const int32_t *src = (const int32_t *)(p.boxes + __ldg(&p.tbox[next]));
+      if (lane < (int)(sizeof(LatBox) / 4)) ((int32_t *)&s_box[(k + 1) & 1])[lane] = __ldg(src + lane);
+      __syncwarp();
+      if (p.prefetch) prefetch_tile_l2<16, 16, PRIV>(p, next, s_box[(k + 1) & 1], lane);
+    }
     __syncwarp();
     asm volatile("bar.sync 2, %0;" ::"r"(NW + 32) : "memory");  // handoff k + 1
     // the workers reached this barrier only after finishing visit k
-    if (lane == 0 && !finished) {
-      finish_visit(p, cur, s_act[k & 1]);
+    if (!finished) {
+      finish_visit(p, cur, s_box[k & 1], s_act[k & 1], lane);
       ++visits;
       finished = true;
     }
@@ -1534,9 +1956,32 @@ bool encode_lattice_maps(const orsp::Graph *g, const LatParams &p, int TX, int T
   return true;
 }
 
-template <int TX, int TY>
+// Layer bound of the run visit for boxes of up to nzb layers, or 0 where it
+// does not apply (more than 18 layers).
+int run_visit_layers(int nzb) { return nzb <= 6 ? 6 : nzb <= 12 ? 12 : nzb <= 18 ? 18 : 0; }
+
+// The asynchronous kernels with run visits: column vias (one CTA per SM), the
+// warp-specialised schedule, or the plain one; with two CTAs per SM the via
+// weights are in shared memory (RunTile ZS: the registers of two CTAs do not
+// hold them; 16 sources on 1000 x 1000 x 12: 4.95 ms against 5.64 ms with the
+// spills, 2 048 boxes of up to 16 layers: 10.5 against 16.9 ms).
+template <int NZM, bool PRIV>
+void *run_visit_kernel(bool cv, bool spec, bool two) {
+  if (cv) return (void *)lattice_async_kernel<16, 16, PRIV, false, 1, false, true, NZM>;
+  if (spec)
+    return two ? (void *)lattice_spec_kernel<NZM, PRIV, 2, true> : (void *)lattice_spec_kernel<NZM, PRIV, 1, false>;
+  return two ? (void *)lattice_async_kernel<16, 16, PRIV, false, 2, false, false, NZM, true>
+             : (void *)lattice_async_kernel<16, 16, PRIV, false, 1, false, false, NZM>;
+}
+template <bool PRIV>
+void *run_visit_kernel(int nzm, bool cv, bool spec, bool two) {
+  return nzm == 6 ? run_visit_kernel<6, PRIV>(cv, spec, two)
+                  : nzm == 12 ? run_visit_kernel<12, PRIV>(cv, spec, two) : run_visit_kernel<18, PRIV>(cv, spec, two);
+}
+
 int launch_lattice(orsp::Graph *g, LatParams &p, int64_t ntiles, int nzb, int32_t nseeds, const int32_t *seeds,
                    const float *seed_cost, cudaStream_t st, orsp::LatOptions *opt) {
+  constexpr int TX = 16, TY = 16;
   // (column vias always take the asynchronous schedule)
   const bool async = p.wcol != nullptr || env_u64("ORSP_LAT_ASYNC", 1) != 0;
   const WsLayout L = ws_layout(g, ntiles);
@@ -1553,70 +1998,63 @@ int launch_lattice(orsp::Graph *g, LatParams &p, int64_t ntiles, int nzb, int32_
   p.qcap = qcap;
   p.ctl = (LatCtl *)(b + 4 * list_b + q_b);
   if (opt) opt->err_d = &p.ctl->err;
-  if (!async) ORSP_CUDA(cudaMemsetAsync(p.stamp, 0, (size_t)ntiles * 4, st));
-  ORSP_CUDA(cudaMemsetAsync(p.tstate, 0, (size_t)ntiles * 4, st));
-  if (async) ORSP_CUDA(cudaMemsetAsync(p.qslot, 0xff, (size_t)qcap * 4, st));
+  p.tbox = async ? p.list0 : nullptr;
+  if (async) {
+    const int64_t n = std::max<int64_t>(ntiles, qcap);
+    lattice_init_kernel<<<(int)std::min<int64_t>((n + 255) / 256, (int64_t)g->num_sms * 8), 256, 0, st>>>(p, (int32_t)ntiles);
+    ORSP_CUDA(cudaGetLastError());
+  } else {
+    ORSP_CUDA(cudaMemsetAsync(p.stamp, 0, list_b + (size_t)ntiles * 4, st));  // stamps and states
+  }
   lattice_seed_kernel<TX, TY><<<1, 256, 0, st>>>(p, nseeds, seeds, seed_cost);
   ORSP_CUDA(cudaGetLastError());
-  size_t smem = (size_t)nzb * tile_floats_per_layer(TX, TY) * sizeof(float);
+  p.hmask = p.vmask = 0;
+  for (int z = 0, h = 0, v = 0; z < p.nz && z < 64; ++z) {
+    if (p.axis[z] == 1) p.hmask |= 1ull << z, p.hlist[h++] = (int8_t)z;
+    else if (p.axis[z] == 2) p.vmask |= 1ull << z, p.vlist[v++] = (int8_t)z;
+  }
+  // run visits up to 18 layers; deeper tiles take process_tile
+  const int nzm = async ? run_visit_layers(nzb) : 0;
+  // ORSP_LAT_BLOCKS_PER_SM: CTAs per SM
+  const int want = (int)env_u64("ORSP_LAT_BLOCKS_PER_SM", (opt && opt->blocks_per_sm > 0) ? opt->blocks_per_sm : 1);
+  const bool two = nzm && !p.wcol && want >= 2;
+  size_t smem = nzm ? (size_t)run_smem_floats(nzb, two) * sizeof(float)
+                    : (size_t)nzb * tile_floats_per_layer(TX, TY) * sizeof(float);
   if (smem > 227 * 1024) {
     orsp::set_error("lattice search: too many layers for the shared-memory tile");
     return ORSP_ERR_ARG;
   }
   const bool priv = opt && opt->private_dist;
   // ORSP_LAT_SPEC=1: the warp-specialised asynchronous schedule
-  const bool spec = async && !p.wcol && env_u64("ORSP_LAT_SPEC", (opt && opt->spec) ? 1 : 0) != 0;
-  // ORSP_LAT_BLOCKS_PER_SM: CTAs per SM (tiles of up to 12 layers at width
-  // 16 have an instantiation sized for 2)
-  const int want = (int)env_u64("ORSP_LAT_BLOCKS_PER_SM", (opt && opt->blocks_per_sm > 0) ? opt->blocks_per_sm : 1);
+  const bool spec = nzm && !p.wcol && env_u64("ORSP_LAT_SPEC", (opt && opt->spec) ? 1 : 0) != 0;
   // ORSP_LAT_TMA=1: tensor-load staging of fresh visits, for whole-lattice
   // boxes (opt->tma_slices: distance slices of N cells, box j in slice j)
   CUtensorMap tmw{}, tmd{};
   bool tma = false;
-  if constexpr (TX == 16) {
-    if (async && !spec && !p.wcol && want < 2 && nzb <= 12 && nzb == g->nz && opt && opt->tma_slices > 0 &&
-        env_u64("ORSP_LAT_TMA", 0) != 0)
-      tma = encode_lattice_maps(g, p, TX, TY, nzb, opt->tma_slices, &tmw, &tmd);
-  }
+  if (async && !spec && !p.wcol && want < 2 && nzb <= 12 && nzb == g->nz && opt && opt->tma_slices > 0 &&
+      env_u64("ORSP_LAT_TMA", 0) != 0)
+    tma = encode_lattice_maps(g, p, TX, TY, nzb, opt->tma_slices, &tmw, &tmd);
+  const bool runs = nzm != 0 && !tma;
   if (tma) {
     const size_t base = ((size_t)nzb * tile_floats_per_layer(TX, TY) + 31) & ~(size_t)31;
     smem = (base + (size_t)nzb * TY * TX * 4 + (size_t)nzb * (TY + 2) * (TX + 8)) * sizeof(float);
   }
   void *kfn;
-  if (p.wcol) {
-    // column vias: the asynchronous schedule with the column via pass, one
-    // CTA per SM, tile width 16
-    if constexpr (TX == 16) {
-      kfn = nzb > 12 ? (priv ? (void *)lattice_async_kernel<TX, TY, true, true, 1, false, true>
-                             : (void *)lattice_async_kernel<TX, TY, false, true, 1, false, true>)
-                     : (priv ? (void *)lattice_async_kernel<TX, TY, true, false, 1, false, true>
-                             : (void *)lattice_async_kernel<TX, TY, false, false, 1, false, true>);
-    } else {
-      orsp::set_error("lattice search: column vias need tile width 16");
-      return ORSP_ERR_ARG;
-    }
-  } else if (spec) {
-    kfn = priv ? (void *)lattice_spec_kernel<TX, TY, true> : (void *)lattice_spec_kernel<TX, TY, false>;
-    if constexpr (TX == 16) {  // two CTAs per SM: the instantiation held to their register share
-      if (want >= 2 && nzb <= 12)
-        kfn = priv ? (void *)lattice_spec_kernel<TX, TY, true, 2> : (void *)lattice_spec_kernel<TX, TY, false, 2>;
-    }
+  if (runs) {
+    kfn = priv ? run_visit_kernel<true>(nzm, p.wcol != nullptr, spec, two)
+               : run_visit_kernel<false>(nzm, p.wcol != nullptr, spec, two);
+  } else if (p.wcol) {
+    kfn = priv ? (void *)lattice_async_kernel<16, 16, true, true, 1, false, true>
+               : (void *)lattice_async_kernel<16, 16, false, true, 1, false, true>;
+  } else if (tma) {
+    kfn = priv ? (void *)lattice_async_kernel<16, 16, true, false, 1, true>
+               : (void *)lattice_async_kernel<16, 16, false, false, 1, true>;
+  } else if (async) {
+    kfn = priv ? (void *)lattice_async_kernel<16, 16, true, true> : (void *)lattice_async_kernel<16, 16, false, true>;
+  } else {
+    kfn = priv ? (void *)lattice_tile_kernel<16, 16, true> : (void *)lattice_tile_kernel<16, 16, false>;
   }
-  else if (async) {
-    kfn = priv ? (void *)lattice_async_kernel<TX, TY, true> : (void *)lattice_async_kernel<TX, TY, false>;
-    if constexpr (TX == 16) {  // deeper tiles: the instantiation with 18-layer column loads
-      if (tma)
-        kfn = priv ? (void *)lattice_async_kernel<TX, TY, true, false, 1, true>
-                   : (void *)lattice_async_kernel<TX, TY, false, false, 1, true>;
-      else if (nzb > 12)
-        kfn = priv ? (void *)lattice_async_kernel<TX, TY, true, true> : (void *)lattice_async_kernel<TX, TY, false, true>;
-      else if (want >= 2)
-        kfn = priv ? (void *)lattice_async_kernel<TX, TY, true, false, 2>
-                   : (void *)lattice_async_kernel<TX, TY, false, false, 2>;
-    }
-  }
-  else kfn = priv ? (void *)lattice_tile_kernel<TX, TY, true> : (void *)lattice_tile_kernel<TX, TY, false>;
-  const int threads = TX * TY + (spec ? 32 : 0);
+  const int threads = (runs && nzm > 16 ? 288 : TX * TY) + (spec ? 32 : 0);
   // The shared-memory cap is a per-kernel attribute: it is raised to the
   // largest tile once per (kernel, device), never lowered, so a launch with a
   // smaller tile does not invalidate a cached larger one.  The occupancy is
@@ -1830,18 +2268,18 @@ void free_lattice(Graph *g) {
   g->lat_ctl_h = nullptr;
 }
 
-int lattice_tile_w() { return env_u64("ORSP_LAT_TILE", 16) == 32 ? 32 : 16; }
-
+// (tile_w 32: the depth up to which a batch plan's width-32 bucket takes the
+// tile sweeps)
 bool lattice_tile_fits(int nzb, int tile_w) {
-  const int TX = tile_w ? tile_w : lattice_tile_w(), TY = 16;
+  const int TX = tile_w ? tile_w : 16, TY = 16;
   const size_t smem = (size_t)nzb * tile_floats_per_layer(TX, TY) * sizeof(float);
   return smem <= 227 * 1024;
 }
 
 int reserve_lattice_ws(Graph *g, int64_t ntiles) { return grow_ws(g, ws_layout(g, ntiles).total); }
 
-int64_t make_lat_boxes(const int32_t *boxes_h, int32_t nbox, LatBox *out, int tile_w) {
-  const int TX = tile_w ? tile_w : lattice_tile_w(), TY = 16;
+int64_t make_lat_boxes(const int32_t *boxes_h, int32_t nbox, LatBox *out) {
+  constexpr int TX = 16, TY = 16;
   int64_t t0 = 0;
   for (int32_t i = 0; i < nbox; ++i) {
     const int32_t *b = boxes_h + 6 * (int64_t)i;
@@ -1871,8 +2309,7 @@ int run_lattice_boxes(Graph *g, const float *cost_d, int32_t nseeds, const int32
                       const float *seed_cost_d, int32_t nbox, const int32_t *boxes_h, const LatBox *lboxes_d,
                       uint32_t *dist, cudaStream_t st, LatOptions *opt) {
   const int64_t N = g->N;
-  const int TX = (opt && opt->tile_w) ? opt->tile_w : lattice_tile_w(), TY = 16;
-  if (TX != 16 && TX != 32) { set_error("lattice search: tile width must be 16 or 32"); return ORSP_ERR_ARG; }
+  constexpr int TX = 16, TY = 16;
   const bool priv = opt && opt->private_dist;
   int64_t vol_sum = 0;
   int64_t ntiles = 0;
@@ -1979,8 +2416,7 @@ int run_lattice_boxes(Graph *g, const float *cost_d, int32_t nseeds, const int32
   p.N = N;
   p.dist = dist;
   for (int z = 0; z < 64; ++z) p.axis[z] = z < g->nz ? g->layer_axis[z] : 0;
-  if (TX == 32) return launch_lattice<32, 16>(g, p, ntiles, nzb, nseeds, seeds_d, seed_cost_d, st, opt);
-  return launch_lattice<16, 16>(g, p, ntiles, nzb, nseeds, seeds_d, seed_cost_d, st, opt);
+  return launch_lattice(g, p, ntiles, nzb, nseeds, seeds_d, seed_cost_d, st, opt);
 }
 
 int run_lattice_search(Graph *g, const float *cost_d, int32_t nseeds, const int32_t *seeds_d,
@@ -2000,7 +2436,7 @@ int run_lattice_roi(Graph *g, const float *cost_d, int32_t nseeds, const int32_t
                     const float *seed_cost_d, const int32_t *roi_map_d, const int32_t *roi_nodes_d,
                     int64_t n_roi, const uint8_t *sink_d, uint32_t *dist, cudaStream_t st) {
   const int64_t N = g->N;
-  const int TX = lattice_tile_w(), TY = 16;
+  constexpr int TX = 16, TY = 16;
   if (!g->lat_box_d) ORSP_CUDA(cudaMalloc(&g->lat_box_d, sizeof(LatBox)));
   int rc = ensure_roi_arrays(g);
   if (rc) return rc;
@@ -2009,7 +2445,7 @@ int run_lattice_roi(Graph *g, const float *cost_d, int32_t nseeds, const int32_t
   if (!roi_map_d && !roi_nodes_d) {
     const int32_t full[6] = {0, g->nx - 1, 0, g->ny - 1, 0, g->nz - 1};
     LatBox *hb = (LatBox *)((char *)g->pinned + 1024);
-    make_lat_boxes(full, 1, hb, TX);
+    make_lat_boxes(full, 1, hb);
     ORSP_CUDA(cudaMemcpyAsync(box_d, hb, sizeof(LatBox), cudaMemcpyHostToDevice, st));
   } else {
     // running maxima start at 0x80808080, below every coordinate
@@ -2018,8 +2454,7 @@ int run_lattice_roi(Graph *g, const float *cost_d, int32_t nseeds, const int32_t
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, gblocks));
     roi_bbox_kernel<<<blocks, 256, 0, st>>>(roi_nodes_d, n, roi_map_d, g->nx, g->ny, N, g->roi_bb);
     ORSP_CUDA(cudaGetLastError());
-    if (TX == 32) roi_box_finish_kernel<32, 16><<<1, 1, 0, st>>>(g->roi_bb, box_d);
-    else roi_box_finish_kernel<16, 16><<<1, 1, 0, st>>>(g->roi_bb, box_d);
+    roi_box_finish_kernel<16, 16><<<1, 1, 0, st>>>(g->roi_bb, box_d);
     ORSP_CUDA(cudaGetLastError());
   }
   RoiGeom G{};
@@ -2056,8 +2491,7 @@ int run_lattice_roi(Graph *g, const float *cost_d, int32_t nseeds, const int32_t
   for (int z = 0; z < 64; ++z) p.axis[z] = z < g->nz ? g->layer_axis[z] : 0;
   // the box is known on the device only: size the tile arrays for the lattice
   const int64_t ntiles = (int64_t)((g->nx - 1 + TX) / TX) * ((g->ny - 1 + TY) / TY);
-  if (TX == 32) return launch_lattice<32, 16>(g, p, ntiles, g->nz, nseeds, seeds_d, seed_cost_d, st, nullptr);
-  return launch_lattice<16, 16>(g, p, ntiles, g->nz, nseeds, seeds_d, seed_cost_d, st, nullptr);
+  return launch_lattice(g, p, ntiles, g->nz, nseeds, seeds_d, seed_cost_d, st, nullptr);
 }
 
 int finish_lattice_search(Graph *g, int32_t *rounds_h) {

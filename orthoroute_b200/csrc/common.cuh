@@ -114,6 +114,8 @@ struct Graph {
   float *wcol = nullptr;
   void *lat_ws = nullptr;         // tile lists, stamps and control block
   size_t lat_ws_bytes = 0;
+  void *own_ws = nullptr;         // owner schedule: control, exchange rows, message counts
+  size_t own_ws_bytes = 0;
   void *lat_ctl_h = nullptr;      // pinned mirror of the control block
   void *lat_box_d = nullptr;      // tile table of a single-box search
   // ROI searches (orsp_sssp_roi_nodes, ROI-masked tile sweeps): a global_to_roi

@@ -1116,6 +1116,10 @@ struct RunShared {
   // summed over the block's visits and added to the control block at its end
   unsigned long long ns[3], last;
   unsigned cycles;
+  __device__ __forceinline__ void clear() {  // the change sets, by the first warp
+    const int k = threadIdx.x >> 4, i = threadIdx.x & 15;
+    rowx[k][i] = coly[k][i] = rowz[k][i] = colz[k][i] = 0;
+  }
   __device__ __forceinline__ void start() { ns[0] = ns[1] = ns[2] = 0, cycles = 0; }
   __device__ __forceinline__ void lap(int i) {
     const unsigned long long t = dev_globaltimer();
@@ -1186,155 +1190,140 @@ __device__ __forceinline__ unsigned walk_both(float a, float b, LD ld, LO lo, HI
   return m;
 }
 
-// The same visit contract as process_tile.  warm: the tile was visited last
-// by this block (its distances are in shared memory, its weights in R), only
-// the halo is read again and only the runs whose halo improved are taken
-// first.  force (shared with the block): the last visit stopped at MAX_CYCLES.
-//
-// B: the tile's box, in shared memory.  (Looked up by the visit itself, the
-// binary search over the boxes and the box's fields were dependent trips to
-// L2 - the streamed weights evict them from L1 - and cost 3 us of an 11 us
-// visit with 16 boxes and two CTAs per SM.)
-template <int NZM, bool PRIV, bool SPEC, bool CV, bool ZS>
-__device__ __forceinline__ void visit_runs(const LatParams &p, int t, const LatBox &SB, float *sd, RunTile<NZM, ZS> &R, RunShared &S,
-                                           int *s_act, int *s_nb, bool warm) {
+// Where a thread's run and column lie in tile t of box B.
+struct RunGeom {
+  int32_t X0, Y0, z0;  // the tile's first cell
+  int tx, ty, tw, th, nzb;
+  unsigned hm, vm;     // the box's H and V layers (bit 0: layer z0)
+  bool run, isv, col;
+  int rz, rl, rbase;   // the run: layer, line, offset of its first cell
+  int xx, yy;          // the column
+  int64_t n0;          // its node at z0
+};
+__device__ __forceinline__ RunGeom run_geom(const LatParams &p, const LatBox &B, int t) {
+  RunGeom G;
+  const int lt = t - B.tile0;
+  G.ty = lt / B.ntx;
+  G.tx = lt - G.ty * B.ntx;
+  G.X0 = B.x0 + G.tx * 16;
+  G.Y0 = B.y0 + G.ty * 16;
+  G.z0 = B.z0;
+  G.tw = min(16, B.x1 - G.X0 + 1);
+  G.th = min(16, B.y1 - G.Y0 + 1);
+  G.nzb = B.z1 - B.z0 + 1;
+  const uint64_t lay = G.nzb >= 64 ? ~0ull : (1ull << G.nzb) - 1ull, below = (1ull << B.z0) - 1ull;
+  G.hm = (unsigned)((p.hmask >> B.z0) & lay);
+  G.vm = (unsigned)((p.vmask >> B.z0) & lay);
+  const int nh = __popc(G.hm), nv = __popc(G.vm), tid = threadIdx.x;
+  G.isv = tid >= nh * 16;
+  const int ri = G.isv ? tid - nh * 16 : tid;
+  G.rl = ri & 15;
+  G.run = ri < 16 * (G.isv ? nv : nh) && G.rl < (G.isv ? G.tw : G.th);
+  G.rz = 0;
+  if (G.run) G.rz = (G.isv ? p.vlist[__popcll(p.vmask & below) + (ri >> 4)]
+                           : p.hlist[__popcll(p.hmask & below) + (ri >> 4)]) - B.z0;
+  G.rbase = G.isv ? G.rz * kRunPS + G.rl : G.rz * kRunPS + G.rl * kRunWS;
+  G.xx = tid & 15;
+  G.yy = tid >> 4;
+  G.col = tid < 256 && G.xx < G.tw && G.yy < G.th;
+  G.n0 = ((int64_t)B.z0 * p.ny + (G.Y0 + G.yy)) * p.nx + (G.X0 + G.xx);
+  return G;
+}
+
+// Loads the tile's weights (and, with a column's own distances D0.. in global
+// memory, those): the columns' loads, one thread each, then the runs' planar
+// weights out of shared memory.  A barrier lies in between, so every thread
+// of the visit calls it.
+template <int NZM, bool SPEC, bool ZS, bool DIST>
+__device__ __forceinline__ void load_tile(const LatParams &p, const RunGeom &G, RunTile<NZM, ZS> &R, float *sd,
+                                          float2 *wp, float2 *wz, int64_t d0, int64_t dz) {
   constexpr int NW = RunTile<NZM, ZS>::NW, WS = kRunWS, PS = kRunPS;
   const float INF_F = __int_as_float(0x7f800000);
-  const LatBox B = SB;
-  const int lt = t - B.tile0;
-  const int ty = lt / B.ntx, tx = lt - ty * B.ntx;
-  const int32_t X0 = B.x0 + tx * 16, Y0 = B.y0 + ty * 16;
-  const int tw = min(16, B.x1 - X0 + 1), th = min(16, B.y1 - Y0 + 1);
-  const int nzb = B.z1 - B.z0 + 1;
   const int64_t nxy = (int64_t)p.nx * p.ny;
-  const uint64_t lay = nzb >= 64 ? ~0ull : (1ull << nzb) - 1ull;
-  const unsigned hm = (unsigned)((p.hmask >> B.z0) & lay), vm = (unsigned)((p.vmask >> B.z0) & lay);
-  const int nh = __popc(hm), nv = __popc(vm);
-  const int tid = threadIdx.x;
-  if (tid == 0) S.lap(-1);
-  if (tid < 5) s_act[tid] = 0;
-  if (s_nb && tid < 4) {  // neighbour tiles in the box: left, right, down, up (-1: box edge)
-    s_nb[tid] = tid == 0 ? (tx > 0 ? t - 1 : -1)
-                         : tid == 1 ? (tx < B.ntx - 1 ? t + 1 : -1)
-                                    : tid == 2 ? (ty > 0 ? t - B.ntx : -1) : (ty < B.nty - 1 ? t + B.ntx : -1);
-  }
-  if (tid < 32) {
-    const int k = tid >> 4, i = tid & 15;
-    S.rowx[k][i] = S.coly[k][i] = S.rowz[k][i] = S.colz[k][i] = 0;
-  }
-  // the thread's run: layer rz, line rl
-  const int v0 = nh * 16;
-  const bool isv = tid >= v0;
-  const int ri = isv ? tid - v0 : tid;
-  const int rl = ri & 15;
-  bool run = ri < 16 * (isv ? nv : nh) && rl < (isv ? tw : th);
-  int rz = 0;
-  if (run) rz = isv ? p.vlist[__popcll(p.vmask & ((1ull << B.z0) - 1ull)) + (ri >> 4)] - B.z0
-                    : p.hlist[__popcll(p.hmask & ((1ull << B.z0) - 1ull)) + (ri >> 4)] - B.z0;
-  // the thread's column
-  const int xx = tid & 15, yy = tid >> 4;
-  const bool col = tid < 256 && xx < tw && yy < th;
-  // ---- load: the run's halo cells (where the box has them), then the column
-  float ha = INF_F, hb = INF_F;
-  if (run) {
-    const int32_t gx = isv ? X0 + rl : X0, gy = isv ? Y0 : Y0 + rl, gz = B.z0 + rz;
-    if (isv) {
-      if (Y0 > B.y0) ha = bits_f(__ldcg(&p.dist[dist_index<PRIV>(p, B, gx, gy - 1, gz)]));
-      if (Y0 + 16 <= B.y1) hb = bits_f(__ldcg(&p.dist[dist_index<PRIV>(p, B, gx, gy + 16, gz)]));
-    } else {
-      if (X0 > B.x0) ha = bits_f(__ldcg(&p.dist[dist_index<PRIV>(p, B, gx - 1, gy, gz)]));
-      if (X0 + 16 <= B.x1) hb = bits_f(__ldcg(&p.dist[dist_index<PRIV>(p, B, gx + 16, gy, gz)]));
-    }
-  }
-  const bool force = __ldcg(&p.stamp[t]) != 0;
-  const int64_t n0 = (int64_t)B.z0 * nxy + (int64_t)(Y0 + yy) * p.nx + (X0 + xx);  // the column's node at z0
-  const int64_t dz = (!PRIV || B.dbase < 0) ? nxy : (int64_t)(B.x1 - B.x0 + 1) * (B.y1 - B.y0 + 1);
-  float *const cd = sd + yy * WS + xx;  // the column's distances
-  float2 *const wp = (float2 *)(sd + nzb * PS);  // planar weight pairs
-  float2 *const wz = wp + nzb * PS;              // via weight pairs (ZS)
-  const int rbase = isv ? rz * PS + rl : rz * PS + rl * WS;
-  bool dirty = run;
-  if (!warm) {
-    if (tid < 256) {
-      const int64_t d0 = col ? dist_index<PRIV>(p, B, X0 + xx, Y0 + yy, B.z0) : 0;
-      const int w0 = yy * WS + xx;
-      if constexpr (ZS) {
-        // the weights go to shared memory as they are, 8 bytes per copy, all
-        // in flight and without registers to hold them
-        const float4 *src = p.w4 + n0;
+  const int nzb = G.nzb;
+  if (threadIdx.x < 256) {
+    const int w0 = G.yy * WS + G.xx;
+    const float4 *src = p.w4 + G.n0;
+    if constexpr (ZS) {
+      // the weights go to shared memory as they are, 8 bytes per copy, all
+      // in flight and without registers to hold them
 #pragma unroll
-        for (int z = 0; z < NZM; ++z)
-          if (z < nzb) {
-            if (col) {
-              copy8_async(&wp[z * PS + w0], src + z * nxy);
-              copy8_async(&wz[z * PS + w0], (const float2 *)(src + z * nxy) + 1);
-            } else {
-              wp[z * PS + w0] = wz[z * PS + w0] = make_float2(INF_F, INF_F);
-            }
-          }
-      }
-      float dv[NZM];
-      float4 wv[ZS ? 1 : NZM];
-#pragma unroll
-      for (int z = 0; z < NZM; ++z) {
-        dv[z] = INF_F;
-        if (!ZS) wv[ZS ? 0 : z] = make_float4(INF_F, INF_F, INF_F, INF_F);
-        if (col && z < nzb) {
-          dv[z] = bits_f(__ldcg(&p.dist[d0 + z * dz]));
-          if (!ZS) wv[ZS ? 0 : z] = __ldg(&p.w4[n0 + z * nxy]);
-        }
-      }
-#pragma unroll
-      for (int z = 0; z < NZM; ++z) {
+      for (int z = 0; z < NZM; ++z)
         if (z < nzb) {
-          cd[z * PS] = dv[z];
-          if (!ZS) wp[z * PS + w0] = make_float2(wv[ZS ? 0 : z].x, wv[ZS ? 0 : z].y);
+          if (G.col) {
+            copy8_async(&wp[z * PS + w0], src + z * nxy);
+            copy8_async(&wz[z * PS + w0], (const float2 *)(src + z * nxy) + 1);
+          } else {
+            wp[z * PS + w0] = wz[z * PS + w0] = make_float2(INF_F, INF_F);
+          }
         }
-        if constexpr (!ZS) {
-          R.dn[z] = wv[z].z;
-          R.up[z] = wv[z].w;
-        }
-      }
-      if (ZS) asm volatile("cp.async.wait_all;" ::: "memory");
     }
-    tile_sync<NW, SPEC>();
-    if (run) {
+    float dv[DIST ? NZM : 1];
+    float4 wv[ZS ? 1 : NZM];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const float2 w = wp[rbase + i * (isv ? WS : 1)];
-        R.lo[i] = w.x;
-        R.hi[i] = w.y;
+    for (int z = 0; z < NZM; ++z) {
+      if (DIST) dv[DIST ? z : 0] = INF_F;
+      if (!ZS) wv[ZS ? 0 : z] = make_float4(INF_F, INF_F, INF_F, INF_F);
+      if (G.col && z < nzb) {
+        if (DIST) dv[DIST ? z : 0] = bits_f(__ldcg(&p.dist[d0 + z * dz]));
+        if (!ZS) wv[ZS ? 0 : z] = __ldg(src + z * nxy);
       }
     }
-  } else {
-    dirty = run && (force || ha < R.ha || hb < R.hb);
-    tile_sync<NW, SPEC>();
+#pragma unroll
+    for (int z = 0; z < NZM; ++z) {
+      if (z < nzb) {
+        if (DIST) sd[z * PS + w0] = dv[DIST ? z : 0];
+        if (!ZS) wp[z * PS + w0] = make_float2(wv[ZS ? 0 : z].x, wv[ZS ? 0 : z].y);
+      }
+      if constexpr (!ZS) {
+        R.dn[z] = wv[z].z;
+        R.up[z] = wv[z].w;
+      }
+    }
+    if (ZS) asm volatile("cp.async.wait_all;" ::: "memory");
   }
-  R.ha = ha;
-  R.hb = hb;
-  if (tid == 0) S.lap(0);
+  tile_sync<NW, SPEC>();
+  if (G.run) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const float2 w = wp[G.rbase + i * (G.isv ? WS : 1)];
+      R.lo[i] = w.x;
+      R.hi[i] = w.y;
+    }
+  }
+}
 
-  // ---- passes
-  const float2 *const cw = wz + yy * WS + xx;
+// The passes of a visit, from the runs marked `dirty` (and, with force, every
+// column) to the tile's fixpoint, at most max_cycles.  runm / colm collect
+// the cells changed in the thread's run and column.  Ends with a barrier
+// after the last change; returns whether the fixpoint was reached.
+template <int NZM, bool SPEC, bool CV, bool ZS>
+__device__ __forceinline__ bool run_passes(const LatParams &p, const RunGeom &G, const RunTile<NZM, ZS> &R,
+                                           RunShared &S, float *sd, const float2 *wz, float ha, float hb, bool dirty,
+                                           bool force, int max_cycles, unsigned &runm, unsigned &colm) {
+  constexpr int NW = RunTile<NZM, ZS>::NW, WS = kRunWS, PS = kRunPS;
+  const float INF_F = __int_as_float(0x7f800000);
+  const int nzb = G.nzb;
+  float *const cd = sd + G.yy * WS + G.xx;  // the column's distances
+  const float2 *const cw = wz + G.yy * WS + G.xx;
   auto run_pass = [&](float *c, auto stride) {
     constexpr int DS = decltype(stride)::value;
     return walk_both<16>(
         ha, hb, [&](int i) { return c[i * DS]; }, [&](int i) { return R.lo[i]; }, [&](int i) { return R.hi[i]; },
         [&](int i, float v) { c[i * DS] = v; });
   };
-  unsigned runm = 0, colm = 0;  // cells changed by this visit: the run's, the column's (by layer)
-  bool converged = false, again = false;
+  bool again = false, converged = false;
   int cyc = 0;
-  for (; cyc < MAX_CYCLES; ++cyc) {
+  for (; cyc < max_cycles; ++cyc) {
     const int k = cyc & 1;
     unsigned m = 0;
     if (dirty) {
-      if (isv) {
-        m = run_pass(sd + rbase, std::integral_constant<int, WS>());
-        if (m) atomicOr(&S.coly[k][rl], m);
+      if (G.isv) {
+        m = run_pass(sd + G.rbase, std::integral_constant<int, WS>());
+        if (m) atomicOr(&S.coly[k][G.rl], m);
       } else {
-        m = run_pass(sd + rbase, std::integral_constant<int, 1>());
-        if (m) atomicOr(&S.rowx[k][rl], m);
+        m = run_pass(sd + G.rbase, std::integral_constant<int, 1>());
+        if (m) atomicOr(&S.rowx[k][G.rl], m);
       }
       runm |= m;
     }
@@ -1344,9 +1333,8 @@ __device__ __forceinline__ void visit_runs(const LatParams &p, int t, const LatB
       break;
     }
     unsigned mz = 0;
-    const bool take = col && (all || again || (((S.rowx[k][yy] >> xx) | (S.coly[k][xx] >> yy)) & 1u));
-    if (take) {
-      if constexpr (CV) mz = (unsigned)zcol_pass<PS>(cd, p.wcol, p.nzp, n0, nxy, B.z0, nzb);
+    if (G.col && (all || again || (((S.rowx[k][G.yy] >> G.xx) | (S.coly[k][G.xx] >> G.yy)) & 1u))) {
+      if constexpr (CV) mz = (unsigned)zcol_pass<PS>(cd, p.wcol, p.nzp, G.n0, (int64_t)p.nx * p.ny, G.z0, nzb);
       else
         mz = walk_both<NZM>(
             INF_F, INF_F, [&](int z) { return z < nzb ? cd[z * PS] : INF_F; },
@@ -1354,52 +1342,111 @@ __device__ __forceinline__ void visit_runs(const LatParams &p, int t, const LatB
             [&](int z) { return ZS ? (z < nzb ? cw[z * PS].y : INF_F) : R.up[ZS ? 0 : z]; },
             [&](int z, float v) { cd[z * PS] = v; });
       if (mz) {
-        if (mz & hm) atomicOr(&S.rowz[k][yy], mz & hm);
-        if (mz & vm) atomicOr(&S.colz[k][xx], mz & vm);
+        if (mz & G.hm) atomicOr(&S.rowz[k][G.yy], mz & G.hm);
+        if (mz & G.vm) atomicOr(&S.colz[k][G.xx], mz & G.vm);
         colm |= mz;
       }
     }
     // one Gauss-Seidel pass over a column's layer pairs is not its fixpoint:
     // a column-via column that changed is taken again
     if (CV) again = mz != 0;
-    if (tid < 16) {
-      S.rowx[k ^ 1][tid] = S.coly[k ^ 1][tid] = 0;
-      S.rowz[k ^ 1][tid] = S.colz[k ^ 1][tid] = 0;
+    if (threadIdx.x < 16) {
+      S.rowx[k ^ 1][threadIdx.x] = S.coly[k ^ 1][threadIdx.x] = 0;
+      S.rowz[k ^ 1][threadIdx.x] = S.colz[k ^ 1][threadIdx.x] = 0;
     }
-    if (!tile_sync_or<NW, SPEC>(CV ? mz != 0 : (mz & (hm | vm)) != 0)) {
+    if (!tile_sync_or<NW, SPEC>(CV ? mz != 0 : (mz & (G.hm | G.vm)) != 0)) {
       converged = true;
       break;
     }
-    dirty = run && (((isv ? S.colz[k][rl] : S.rowz[k][rl]) >> rz) & 1u);
+    dirty = G.run && (((G.isv ? S.colz[k][G.rl] : S.rowz[k][G.rl]) >> G.rz) & 1u);
   }
-  if (tid == 0) {
-    S.lap(1);
-    S.cycles += cyc + 1;
+  if (threadIdx.x == 0) S.cycles += cyc + 1;
+  return converged;
+}
+
+// The same visit contract as process_tile.  warm: the tile was visited last
+// by this block (its distances are in shared memory, its weights in R), only
+// the halo is read again and only the runs whose halo improved are taken
+// first.  A tile whose last visit stopped at MAX_CYCLES, or that holds a
+// seed, has its stamp set: then every column is taken too.
+//
+// B: the tile's box, in shared memory.  (Looked up by the visit itself, the
+// binary search over the boxes and the box's fields were dependent trips to
+// L2 - the streamed weights evict them from L1 - and cost 3 us of an 11 us
+// visit with 16 boxes and two CTAs per SM.)
+template <int NZM, bool PRIV, bool SPEC, bool CV, bool ZS>
+__device__ __forceinline__ void visit_runs(const LatParams &p, int t, const LatBox &SB, float *sd,
+                                           RunTile<NZM, ZS> &R, RunShared &S, int *s_act, int *s_nb, bool warm) {
+  constexpr int NW = RunTile<NZM, ZS>::NW, PS = kRunPS;
+  const float INF_F = __int_as_float(0x7f800000);
+  const LatBox B = SB;
+  const RunGeom G = run_geom(p, B, t);
+  const int tid = threadIdx.x;
+  if (tid == 0) S.lap(-1);
+  if (tid < 5) s_act[tid] = 0;
+  if (s_nb && tid < 4) {  // neighbour tiles in the box: left, right, down, up (-1: box edge)
+    s_nb[tid] = tid == 0 ? (G.tx > 0 ? t - 1 : -1)
+                         : tid == 1 ? (G.tx < B.ntx - 1 ? t + 1 : -1)
+                                    : tid == 2 ? (G.ty > 0 ? t - B.ntx : -1) : (G.ty < B.nty - 1 ? t + B.ntx : -1);
   }
+  if (tid < 32) S.clear();
+  // ---- load: the run's halo cells (where the box has them), then the column
+  float ha = INF_F, hb = INF_F;
+  if (G.run) {
+    const int32_t gx = G.isv ? G.X0 + G.rl : G.X0, gy = G.isv ? G.Y0 : G.Y0 + G.rl, gz = B.z0 + G.rz;
+    if (G.isv) {
+      if (G.Y0 > B.y0) ha = bits_f(__ldcg(&p.dist[dist_index<PRIV>(p, B, gx, gy - 1, gz)]));
+      if (G.Y0 + 16 <= B.y1) hb = bits_f(__ldcg(&p.dist[dist_index<PRIV>(p, B, gx, gy + 16, gz)]));
+    } else {
+      if (G.X0 > B.x0) ha = bits_f(__ldcg(&p.dist[dist_index<PRIV>(p, B, gx - 1, gy, gz)]));
+      if (G.X0 + 16 <= B.x1) hb = bits_f(__ldcg(&p.dist[dist_index<PRIV>(p, B, gx + 16, gy, gz)]));
+    }
+  }
+  const bool force = __ldcg(&p.stamp[t]) != 0;
+  const int64_t dz =
+      (!PRIV || B.dbase < 0) ? (int64_t)p.nx * p.ny : (int64_t)(B.x1 - B.x0 + 1) * (B.y1 - B.y0 + 1);
+  const int64_t d0 = G.col ? dist_index<PRIV>(p, B, G.X0 + G.xx, G.Y0 + G.yy, B.z0) : 0;
+  float2 *const wp = (float2 *)(sd + G.nzb * PS);  // planar weight pairs
+  float2 *const wz = wp + G.nzb * PS;              // via weight pairs (ZS)
+  bool dirty = G.run;
+  if (!warm) {
+    load_tile<NZM, SPEC, ZS, true>(p, G, R, sd, wp, wz, d0, dz);
+  } else {
+    dirty = G.run && (force || ha < R.ha || hb < R.hb);
+    tile_sync<NW, SPEC>();
+  }
+  R.ha = ha;
+  R.hb = hb;
+  if (tid == 0) S.lap(0);
+
+  unsigned runm = 0, colm = 0;
+  const bool converged =
+      run_passes<NZM, SPEC, CV, ZS>(p, G, R, S, sd, wz, ha, hb, dirty, force, MAX_CYCLES, runm, colm);
+  if (tid == 0) S.lap(1);
 
   // ---- publish improvements; mark neighbour tiles whose halo changed.  One
   // thread per column: the layers its own passes changed, and its bits of the
   // runs' changed cells.
-  if (run) S.cells[rz * 16 + rl] = runm;
+  if (G.run) S.cells[G.rz * 16 + G.rl] = runm;
   tile_sync<NW, SPEC>();
-  if (col) {
-    const int64_t d0 = dist_index<PRIV>(p, B, X0 + xx, Y0 + yy, B.z0);
+  if (G.col) {
+    const float *const cd = sd + G.yy * kRunWS + G.xx;
 #pragma unroll
     for (int z = 0; z < NZM; ++z)
-      if (((hm | vm) >> z) & 1u) {
-        const bool h = (hm >> z) & 1u;
-        if ((S.cells[z * 16 + (h ? yy : xx)] >> (h ? xx : yy)) & 1u) colm |= 1u << z;
+      if (((G.hm | G.vm) >> z) & 1u) {
+        const bool h = (G.hm >> z) & 1u;
+        if ((S.cells[z * 16 + (h ? G.yy : G.xx)] >> (h ? G.xx : G.yy)) & 1u) colm |= 1u << z;
       }
 #pragma unroll
     for (int z = 0; z < NZM; ++z)
       if ((colm >> z) & 1u) __stcg(&p.dist[d0 + z * dz], f_bits(cd[z * PS]));
-    if (colm & hm) {
-      if (xx == 0) s_act[0] = 1;
-      if (xx == tw - 1) s_act[1] = 1;
+    if (colm & G.hm) {
+      if (G.xx == 0) s_act[0] = 1;
+      if (G.xx == G.tw - 1) s_act[1] = 1;
     }
-    if (colm & vm) {
-      if (yy == 0) s_act[2] = 1;
-      if (yy == th - 1) s_act[3] = 1;
+    if (colm & G.vm) {
+      if (G.yy == 0) s_act[2] = 1;
+      if (G.yy == G.th - 1) s_act[3] = 1;
     }
   }
   if (tid == 0) {
@@ -1408,6 +1455,329 @@ __device__ __forceinline__ void visit_runs(const LatParams &p, int t, const LatB
   }
   tile_sync<NW, SPEC>();
   if (tid == 0) S.lap(2);
+}
+
+// ---------------------------------------------------------------------------
+// Owner schedule: launches with at most one tile per resident CTA.
+//
+// One search is bound by the chain of tile visits along its wave front, and a
+// visit of the queue schedule spends more on handing the tile over (the
+// queue's atomics, loading distances and weights, writing back) than on its
+// passes, which in turn start on values that improve while they run.  Here
+// tile t belongs to CTA t for the whole search: distances in shared memory,
+// weights in registers, loaded once, and the CTAs relax their tiles
+// continuously.  Neighbours exchange only the values of boundary cells: each
+// tile has an exchange row per side of its runs (exch[tile][side][run]), which
+// the neighbour's runs write with plain stores as soon as a pass has improved
+// a boundary cell.  A distance is an upper bound at any time and only falls,
+// so a halo value needs no flag to go with it: every cycle reads the rows
+// anew (coalesced, one value per run and side, the loads overlapping the via
+// pass), takes what improved, and an idle tile polls them.  A hop of the wave
+// front costs one pass, one store and one load.
+//
+// Termination.  Publications are also counted as messages (inbox[tile]), by a
+// helper warp beside the workers, so that no worker waits for an atomic.  The
+// helper reads the inbox count c and asks the workers (s_req); when a whole
+// cycle whose halo loads came after that changed nothing, they answer
+// (s_ack), and the helper first sends the messages for everything published
+// so far (sent count, fence, inbox of the neighbour) and then counts c as
+// dealt with.  CTA 0's helper adds up the dealt-with counts and then the sent
+// counts; equal sums mean that nothing is under way: both only grow, the
+// sent sum was read later, and a tile that works on values whose message has
+// not come yet is covered by the sender, which still owes that message.  The
+// seeds' tiles start with one message each, sent by the launch.
+//
+// Measured, search kernel, queue schedule with run visits -> owners: 49 tiles
+// of 18 layers 193 -> 57 us, 100 x 100 x 4 board 77 (before run visits) -> 19
+// us, 91 tiles of a 200 x 200 x 6 column-via lattice 248 -> 133 us.
+struct OwnParams {
+  LatParams l;
+  int32_t tcap, nr;              // tiles (at most), values per exchange row
+  int32_t nzb;
+  float *exch;                   // [tcap][2][nr]
+  unsigned *inbox, *sent, *got;  // [tcap], [tcap + 1], [tcap + 1]
+  int *done;
+  int32_t *seedt;                // tile of each seed, -1: outside
+  int32_t nseeds;
+  const int32_t *seeds;
+  const float *seed_cost;
+};
+constexpr int kOwnSeeds = 4096;
+
+// Prepares a launch: block 0 the control words and the seeds' messages, the
+// other blocks the exchange rows.
+__global__ void own_init_kernel(const __grid_constant__ OwnParams o) {
+  const LatParams &p = o.l;
+  const float INF_F = __int_as_float(0x7f800000);
+  if (blockIdx.x > 0) {
+    const int64_t n = (int64_t)o.tcap * 2 * o.nr / 4, s = (int64_t)(gridDim.x - 1) * blockDim.x;
+    for (int64_t i = (int64_t)(blockIdx.x - 1) * blockDim.x + threadIdx.x; i < n; i += s)
+      ((float4 *)o.exch)[i] = make_float4(INF_F, INF_F, INF_F, INF_F);
+    return;
+  }
+  LatCtl *c = p.ctl;
+  if (threadIdx.x == 0) {
+    c->err = 0;
+    c->rounds = c->visits = 0;
+    c->cycles = 0;
+    for (int i = 0; i < 4; ++i) c->ns[i] = 0;
+    *o.done = 0;
+  }
+  for (int i = threadIdx.x; i < o.tcap; i += blockDim.x) o.inbox[i] = 0;
+  for (int i = threadIdx.x; i <= o.tcap; i += blockDim.x) o.sent[i] = o.got[i] = 0;
+  __syncthreads();
+  const int32_t plane = p.nx * p.ny;
+  for (int i = threadIdx.x; i < o.nseeds; i += blockDim.x) {
+    const int32_t s = o.seeds[i];
+    int t = -1;
+    const float c0 = o.seed_cost ? o.seed_cost[i] : 0.0f;
+    if (s >= 0 && s < plane * p.nz && (!p.roi_map || __ldg(&p.roi_map[s]) >= 0) && c0 >= 0.0f && c0 < INF_F) {
+      const int32_t z = s / plane, r = s - z * plane, y = r / p.nx, x = r - y * p.nx;
+      const int lo = p.seed_per_box ? i : 0, hi = p.seed_per_box ? min(i + 1, p.nbox) : p.nbox;
+      for (int b = lo; b < hi && t < 0; ++b) {
+        const LatBox B = load_box(p, b);
+        if (x >= B.x0 && x <= B.x1 && y >= B.y0 && y <= B.y1 && z >= B.z0 && z <= B.z1) t = tile_of<16, 16>(B, x, y);
+      }
+    }
+    o.seedt[i] = t;
+    if (t >= 0 && atomicExch(&o.inbox[t], 1u) == 0u) atomicAdd(&o.sent[o.tcap], 1u);
+  }
+}
+
+__device__ __forceinline__ float ld_relaxed_f32(const float *p) {
+  float v;
+  asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_relaxed_f32(float *p, float v) {
+  asm volatile("st.relaxed.gpu.global.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
+}
+
+template <int NZM, bool PRIV, bool CV, bool ZS, int MINB>
+__global__ void __launch_bounds__(RunTile<NZM, ZS>::NW + 32, MINB)
+    lattice_own_kernel(const __grid_constant__ OwnParams o) {
+  constexpr int NW = RunTile<NZM, ZS>::NW, WS = kRunWS, PS = kRunPS;
+  const float INF_F = __int_as_float(0x7f800000);
+  extern __shared__ __align__(128) float sd[];
+  __shared__ RunShared S;
+  __shared__ volatile unsigned s_req, s_ack;  // inbox count to deal with, last one dealt with
+  __shared__ int s_pub[4];                    // sides with publications not yet sent as messages
+  __shared__ volatile int s_stop;
+  const LatParams &p = o.l;
+  const int t = blockIdx.x, tid = threadIdx.x;
+  // the tile's box (a box sized on the device may have fewer tiles than the launch)
+  const LatBox B = load_box(p, p.nbox == 1 ? 0 : box_of_tile(p, t));
+  const bool mine = t < B.tile0 + B.ntx * B.nty;
+  const unsigned long long t_start = dev_globaltimer();
+  if (tid < 4) s_pub[tid] = 0;
+  if (tid < 32) S.clear();
+  if (tid == 0) {
+    s_req = s_ack = 0;
+    s_stop = 0;
+    S.start();
+    S.lap(-1);
+  }
+  __syncthreads();
+
+  if (tid >= NW) {
+    // ------------------------------------------------------------ helper
+    const int lane = tid - NW;
+    unsigned sent = 0, got = 0, asked = 0;
+    for (unsigned spins = 0;; ++spins) {
+      // publications become messages: one lane per side, the sent count first
+      const bool pub = lane < 4 && atomicExch(&s_pub[lane], 0) != 0;
+      const unsigned pm = __ballot_sync(ORSP_FULL_MASK, pub);
+      const bool acked = asked != got && __shfl_sync(ORSP_FULL_MASK, s_ack, 0) == asked;
+      if (acked) {
+        // everything published up to the answer: flags raised since the
+        // exchange above are part of it
+        __threadfence_block();
+        const bool more = lane < 4 && atomicExch(&s_pub[lane], 0) != 0;
+        const unsigned mm = __ballot_sync(ORSP_FULL_MASK, more);
+        const unsigned both = pm | mm;
+        if (both) {
+          sent += __popc(both);
+          if (lane == 0) __stcg(&o.sent[t], sent);
+          __threadfence();
+          __syncwarp();
+          if (lane == 0) {
+            if (both & 1u) atomicAdd(&o.inbox[t - 1], 1u);
+            if (both & 2u) atomicAdd(&o.inbox[t + 1], 1u);
+            if (both & 4u) atomicAdd(&o.inbox[t - B.ntx], 1u);
+            if (both & 8u) atomicAdd(&o.inbox[t + B.ntx], 1u);
+          }
+        }
+        got = asked;
+        if (lane == 0) asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&o.got[t]), "r"(got) : "memory");
+      } else if (pm) {
+        sent += __popc(pm);
+        if (lane == 0) {
+          __stcg(&o.sent[t], sent);
+          __threadfence();
+          if (pm & 1u) atomicAdd(&o.inbox[t - 1], 1u);
+          if (pm & 2u) atomicAdd(&o.inbox[t + 1], 1u);
+          if (pm & 4u) atomicAdd(&o.inbox[t - B.ntx], 1u);
+          if (pm & 8u) atomicAdd(&o.inbox[t + B.ntx], 1u);
+        }
+      }
+      unsigned in = 0;
+      int stop = 0;
+      if (lane == 0) {
+        in = ld_acquire_u32(&o.inbox[t]);
+        stop = ld_acquire_u32((const unsigned *)o.done) != 0 || ld_acquire_u32((const unsigned *)&p.ctl->err) != 0;
+      }
+      in = __shfl_sync(ORSP_FULL_MASK, in, 0);
+      if (asked == got && in != got) {
+        asked = in;
+        if (lane == 0) s_req = in;
+      }
+      if (t == 0 && asked == got) {
+        unsigned a = 0, b = 0;
+        for (int i = lane; i <= o.tcap; i += 32) a += ld_acquire_u32(&o.got[i]);
+        a = __reduce_add_sync(ORSP_FULL_MASK, a);
+        __threadfence();
+        for (int i = lane; i <= o.tcap; i += 32) b += ld_acquire_u32(&o.sent[i]);
+        b = __reduce_add_sync(ORSP_FULL_MASK, b);
+        if (a == b) {
+          stop = 1;
+          if (lane == 0) atomicExch(o.done, 1);
+        }
+      }
+      if (lane == 0 && (spins & 31u) == 31u && dev_globaltimer() - t_start > min(p.wait_ns * 4, p.budget_ns)) {
+        atomicCAS(&p.ctl->err, DEV_OK, DEV_ERR_TIMEOUT);
+        stop = 1;
+      }
+      if (__shfl_sync(ORSP_FULL_MASK, stop, 0)) break;
+    }
+    if (lane == 0) s_stop = 1;
+    return;
+  }
+
+  // -------------------------------------------------------------- workers
+  const RunGeom G = run_geom(p, B, t);
+  const bool run = mine && G.run, col = mine && G.col;
+  RunTile<NZM, ZS> R;
+  float2 *const wp = (float2 *)(sd + o.nzb * PS), *const wz = wp + o.nzb * PS;
+  float *const ex = o.exch + (int64_t)t * 2 * o.nr + tid;
+  bool seeded = false;
+  if (mine) {
+    for (int i = tid; i < o.nzb * PS; i += NW) sd[i] = INF_F;
+    load_tile<NZM, true, ZS, false>(p, G, R, nullptr, wp, wz, 0, 0);  // (with a barrier)
+    for (int i = tid; i < o.nseeds; i += NW) {
+      if (o.seedt[i] != t) continue;
+      seeded = true;
+      const int32_t v = o.seeds[i], plane = p.nx * p.ny, z = v / plane, r = v - z * plane, y = r / p.nx, x = r - y * p.nx;
+      atomicMin((unsigned *)&sd[(z - B.z0) * PS + (y - G.Y0) * WS + (x - G.X0)],
+                f_bits(o.seed_cost ? o.seed_cost[i] : 0.0f));
+    }
+  }
+  seeded = tile_sync_or<NW, true>(seeded);
+  if (tid == 0) S.lap(0);
+  // the neighbours' exchange values that this thread's run writes
+  const int step = (G.isv ? B.ntx : 1) * 2 * o.nr;
+  const bool lo = run && (G.isv ? G.ty > 0 : G.tx > 0), hi = run && (G.isv ? G.ty < B.nty - 1 : G.tx < B.ntx - 1);
+  float ha = INF_F, hb = INF_F;  // halo values taken
+  float pa = INF_F, pb = INF_F;  // boundary values published
+  bool dirty = run && seeded, all = seeded, again = false, idle = false;
+  unsigned snap = 0, cycles = 0;
+  float *const cd = sd + G.yy * WS + G.xx;
+  const float2 *const cw = wz + G.yy * WS + G.xx;
+  float na = INF_F, nb = INF_F;
+  for (int k = 0; mine; k ^= 1) {
+    // ---- halo values read since the last look
+    unsigned next_snap = 0;
+    if (na < ha) ha = na, dirty = true;
+    if (nb < hb) hb = nb, dirty = true;
+    if (idle) {  // nothing to do at the last look
+      const bool stop = s_stop != 0;
+      if (!tile_sync_or<NW, true>(dirty || stop)) {
+        if (tid == 0) {
+          s_ack = snap;
+          snap = s_req;
+        }
+        tile_sync<NW, true>();
+        if (run) na = ld_relaxed_f32(ex), nb = ld_relaxed_f32(ex + o.nr);
+        continue;
+      }
+      if (!tile_sync_or<NW, true>(dirty)) break;
+      idle = false;
+    }
+    // ---- planar pass, boundary improvements published
+    unsigned m = 0;
+    if (dirty) {
+      auto pass = [&](float *c, auto stride) {
+        constexpr int DS = decltype(stride)::value;
+        m = walk_both<16>(
+            ha, hb, [&](int i) { return c[i * DS]; }, [&](int i) { return R.lo[i]; }, [&](int i) { return R.hi[i]; },
+            [&](int i, float v) { c[i * DS] = v; });
+        const float v0 = c[0], v1 = c[15 * DS];
+        if (lo && v0 < pa) {
+          pa = v0;
+          st_relaxed_f32(ex - step + o.nr, v0);
+          __threadfence_block();
+          s_pub[G.isv ? 2 : 0] = 1;
+        }
+        if (hi && v1 < pb) {
+          pb = v1;
+          st_relaxed_f32(ex + step, v1);
+          __threadfence_block();
+          s_pub[G.isv ? 3 : 1] = 1;
+        }
+      };
+      if (G.isv) {
+        pass(sd + G.rbase, std::integral_constant<int, WS>());
+        if (m) atomicOr(&S.coly[k][G.rl], m);
+      } else {
+        pass(sd + G.rbase, std::integral_constant<int, 1>());
+        if (m) atomicOr(&S.rowx[k][G.rl], m);
+      }
+    }
+    if (tid == 0) next_snap = s_req;
+    const bool any = tile_sync_or<NW, true>(m != 0 || again);
+    // the next cycle's halo values; their round trip overlaps the via pass
+    if (run) na = ld_relaxed_f32(ex), nb = ld_relaxed_f32(ex + o.nr);
+    // ---- via pass
+    unsigned mz = 0;
+    if ((any || all) && col && (all || again || (((S.rowx[k][G.yy] >> G.xx) | (S.coly[k][G.xx] >> G.yy)) & 1u))) {
+      if constexpr (CV) mz = (unsigned)zcol_pass<PS>(cd, p.wcol, p.nzp, G.n0, (int64_t)p.nx * p.ny, G.z0, G.nzb);
+      else
+        mz = walk_both<NZM>(
+            INF_F, INF_F, [&](int z) { return z < G.nzb ? cd[z * PS] : INF_F; },
+            [&](int z) { return ZS ? (z < G.nzb ? cw[z * PS].x : INF_F) : R.dn[ZS ? 0 : z]; },
+            [&](int z) { return ZS ? (z < G.nzb ? cw[z * PS].y : INF_F) : R.up[ZS ? 0 : z]; },
+            [&](int z, float v) { cd[z * PS] = v; });
+      if (mz & G.hm) atomicOr(&S.rowz[k][G.yy], mz & G.hm);
+      if (mz & G.vm) atomicOr(&S.colz[k][G.xx], mz & G.vm);
+    }
+    if (CV) again = mz != 0;
+    all = false;
+    if (tid < 16) {
+      S.rowx[k ^ 1][tid] = S.coly[k ^ 1][tid] = 0;
+      S.rowz[k ^ 1][tid] = S.colz[k ^ 1][tid] = 0;
+    }
+    const bool zany = tile_sync_or<NW, true>(mz != 0);
+    dirty = run && (((G.isv ? S.colz[k][G.rl] : S.rowz[k][G.rl]) >> G.rz) & 1u);
+    ++cycles;
+    idle = !any && !zany;
+    if (tid == 0) {
+      // a cycle without a change answers the request read before its halo loads
+      if (idle) s_ack = snap;
+      snap = next_snap;
+    }
+  }
+  // ---- the box's distances
+  tile_sync<NW, true>();
+  if (col) {
+    const int64_t dz = (!PRIV || B.dbase < 0) ? (int64_t)p.nx * p.ny : (int64_t)(B.x1 - B.x0 + 1) * (B.y1 - B.y0 + 1);
+    const int64_t d0 = dist_index<PRIV>(p, B, G.X0 + G.xx, G.Y0 + G.yy, B.z0);
+    for (int z = 0; z < G.nzb; ++z) p.dist[d0 + z * dz] = f_bits(cd[z * PS]);
+  }
+  if (tid == 0 && mine) {
+    S.lap(1);
+    S.cycles = cycles;
+    atomicAdd(&p.ctl->visits, 1u);
+    S.flush(p.ctl);
+  }
 }
 
 // Tiles to revisit after a visit of tile t: the neighbours whose halo value
@@ -1979,82 +2349,10 @@ void *run_visit_kernel(int nzm, bool cv, bool spec, bool two) {
                   : nzm == 12 ? run_visit_kernel<12, PRIV>(cv, spec, two) : run_visit_kernel<18, PRIV>(cv, spec, two);
 }
 
-int launch_lattice(orsp::Graph *g, LatParams &p, int64_t ntiles, int nzb, int32_t nseeds, const int32_t *seeds,
-                   const float *seed_cost, cudaStream_t st, orsp::LatOptions *opt) {
-  constexpr int TX = 16, TY = 16;
-  // (column vias always take the asynchronous schedule)
-  const bool async = p.wcol != nullptr || env_u64("ORSP_LAT_ASYNC", 1) != 0;
-  const WsLayout L = ws_layout(g, ntiles);
-  const size_t list_b = L.list_b, q_b = L.q_b;
-  const unsigned qcap = L.qcap;
-  int rc0 = grow_ws(g, L.total);
-  if (rc0) return rc0;
-  char *b = (char *)g->lat_ws;
-  p.list0 = (int32_t *)b;
-  p.list1 = (int32_t *)(b + list_b);
-  p.stamp = (unsigned *)(b + 2 * list_b);
-  p.tstate = (int *)(b + 3 * list_b);
-  p.qslot = async ? (int32_t *)(b + 4 * list_b) : nullptr;
-  p.qcap = qcap;
-  p.ctl = (LatCtl *)(b + 4 * list_b + q_b);
-  if (opt) opt->err_d = &p.ctl->err;
-  p.tbox = async ? p.list0 : nullptr;
-  if (async) {
-    const int64_t n = std::max<int64_t>(ntiles, qcap);
-    lattice_init_kernel<<<(int)std::min<int64_t>((n + 255) / 256, (int64_t)g->num_sms * 8), 256, 0, st>>>(p, (int32_t)ntiles);
-    ORSP_CUDA(cudaGetLastError());
-  } else {
-    ORSP_CUDA(cudaMemsetAsync(p.stamp, 0, list_b + (size_t)ntiles * 4, st));  // stamps and states
-  }
-  lattice_seed_kernel<TX, TY><<<1, 256, 0, st>>>(p, nseeds, seeds, seed_cost);
-  ORSP_CUDA(cudaGetLastError());
-  p.hmask = p.vmask = 0;
-  for (int z = 0, h = 0, v = 0; z < p.nz && z < 64; ++z) {
-    if (p.axis[z] == 1) p.hmask |= 1ull << z, p.hlist[h++] = (int8_t)z;
-    else if (p.axis[z] == 2) p.vmask |= 1ull << z, p.vlist[v++] = (int8_t)z;
-  }
-  // run visits up to 18 layers; deeper tiles take process_tile
-  const int nzm = async ? run_visit_layers(nzb) : 0;
-  // ORSP_LAT_BLOCKS_PER_SM: CTAs per SM
-  const int want = (int)env_u64("ORSP_LAT_BLOCKS_PER_SM", (opt && opt->blocks_per_sm > 0) ? opt->blocks_per_sm : 1);
-  const bool two = nzm && !p.wcol && want >= 2;
-  size_t smem = nzm ? (size_t)run_smem_floats(nzb, two) * sizeof(float)
-                    : (size_t)nzb * tile_floats_per_layer(TX, TY) * sizeof(float);
-  if (smem > 227 * 1024) {
-    orsp::set_error("lattice search: too many layers for the shared-memory tile");
-    return ORSP_ERR_ARG;
-  }
-  const bool priv = opt && opt->private_dist;
-  // ORSP_LAT_SPEC=1: the warp-specialised asynchronous schedule
-  const bool spec = nzm && !p.wcol && env_u64("ORSP_LAT_SPEC", (opt && opt->spec) ? 1 : 0) != 0;
-  // ORSP_LAT_TMA=1: tensor-load staging of fresh visits, for whole-lattice
-  // boxes (opt->tma_slices: distance slices of N cells, box j in slice j)
-  CUtensorMap tmw{}, tmd{};
-  bool tma = false;
-  if (async && !spec && !p.wcol && want < 2 && nzb <= 12 && nzb == g->nz && opt && opt->tma_slices > 0 &&
-      env_u64("ORSP_LAT_TMA", 0) != 0)
-    tma = encode_lattice_maps(g, p, TX, TY, nzb, opt->tma_slices, &tmw, &tmd);
-  const bool runs = nzm != 0 && !tma;
-  if (tma) {
-    const size_t base = ((size_t)nzb * tile_floats_per_layer(TX, TY) + 31) & ~(size_t)31;
-    smem = (base + (size_t)nzb * TY * TX * 4 + (size_t)nzb * (TY + 2) * (TX + 8)) * sizeof(float);
-  }
-  void *kfn;
-  if (runs) {
-    kfn = priv ? run_visit_kernel<true>(nzm, p.wcol != nullptr, spec, two)
-               : run_visit_kernel<false>(nzm, p.wcol != nullptr, spec, two);
-  } else if (p.wcol) {
-    kfn = priv ? (void *)lattice_async_kernel<16, 16, true, true, 1, false, true>
-               : (void *)lattice_async_kernel<16, 16, false, true, 1, false, true>;
-  } else if (tma) {
-    kfn = priv ? (void *)lattice_async_kernel<16, 16, true, false, 1, true>
-               : (void *)lattice_async_kernel<16, 16, false, false, 1, true>;
-  } else if (async) {
-    kfn = priv ? (void *)lattice_async_kernel<16, 16, true, true> : (void *)lattice_async_kernel<16, 16, false, true>;
-  } else {
-    kfn = priv ? (void *)lattice_tile_kernel<16, 16, true> : (void *)lattice_tile_kernel<16, 16, false>;
-  }
-  const int threads = (runs && nzm > 16 ? 288 : TX * TY) + (spec ? 32 : 0);
+// Launches a persistent kernel of `want` CTAs per SM where they fit (ctas > 0:
+// of that many CTAs), timed when profiling is on.
+int launch_persistent(orsp::Graph *g, void *kfn, int threads, size_t smem, int want, int ctas, void **args,
+                      cudaStream_t st) {
   // The shared-memory cap is a per-kernel attribute: it is raised to the
   // largest tile once per (kernel, device), never lowered, so a launch with a
   // smaller tile does not invalidate a cached larger one.  The occupancy is
@@ -2102,15 +2400,7 @@ int launch_lattice(orsp::Graph *g, LatParams &p, int64_t ntiles, int nzb, int32_
     orsp::set_error("lattice search: kernel does not fit on an SM");
     return ORSP_ERR_ARG;
   }
-  const int bps = std::max(1, std::min(occ, want));
-  p.max_rounds = (unsigned)std::min<unsigned long long>(64ull * (unsigned long long)ntiles + 4096ull, 1ull << 30);
-  p.wait_ns = env_u64("ORSP_WAIT_NS", 2000000000ull);
-  // ORSP_LAT_SELF=0: a tile to visit again goes back to the queue instead
-  p.selfcont = (int)env_u64("ORSP_LAT_SELF", 1);
-  // ORSP_LAT_PREFETCH=0: no L2 prefetch of the next tile by the scheduler warp
-  p.prefetch = (int)env_u64("ORSP_LAT_PREFETCH", 1);
-  p.budget_ns = env_u64("ORSP_BUDGET_NS", 20000000000ull);
-  void *args[] = {&p, &tmw, &tmd};  // the tile and spec kernels take p only
+  if (ctas <= 0) ctas = g->num_sms * std::max(1, std::min(occ, want));
   if (orsp::g_timer.on) ORSP_CUDA(cudaEventRecord(orsp::g_timer.a, st));
   // Cooperative launch in both schedules: every CTA is resident, so a CTA
   // waiting for a queue slot never blocks the CTA that will fill it.
@@ -2118,7 +2408,7 @@ int launch_lattice(orsp::Graph *g, LatParams &p, int64_t ntiles, int nzb, int32_
   // cudaLaunchCooperativeKernel, so that a stream capture keeps the
   // co-residency guarantee in the graph's kernel node)
   cudaLaunchConfig_t lc{};
-  lc.gridDim = dim3(g->num_sms * bps);
+  lc.gridDim = dim3(ctas);
   lc.blockDim = dim3(threads);
   lc.dynamicSmemBytes = smem;
   lc.stream = st;
@@ -2132,6 +2422,189 @@ int launch_lattice(orsp::Graph *g, LatParams &p, int64_t ntiles, int nzb, int32_
     ORSP_CUDA(cudaEventRecord(orsp::g_timer.b, st));
     orsp::g_timer.pending = true;
   }
+  return ORSP_OK;
+}
+
+// Shape of a launch under the owner schedule.  False when it does not apply:
+// more than 18 layers, more tiles than resident CTAs (one per SM, or two with
+// the via weights in shared memory), more seeds than it lists.  (Several
+// tiles per CTA, weights reloaded at each visit, took more visits than the
+// queue makes: 776 against 602 us for 1 444 tiles of 600 x 600 x 12.)
+struct OwnShape {
+  int per_sm, nzb;
+  size_t smem, ws;
+};
+bool own_shape(const orsp::Graph *g, int64_t ntiles, int nzb, int64_t nseeds, OwnShape *o) {
+  if (!run_visit_layers(nzb) || nseeds > kOwnSeeds || ntiles < 1 || ntiles > 2 * (int64_t)g->num_sms) return false;
+  o->per_sm = ntiles > g->num_sms ? 2 : 1;
+  o->nzb = nzb;
+  o->smem = (size_t)run_smem_floats(nzb, o->per_sm == 2) * sizeof(float);
+  // exchange rows, seeds' tiles, inbox, sent and dealt-with counts, control
+  o->ws = 512 + ((size_t)ntiles * (2 * 16 * nzb + 3) + kOwnSeeds + 2) * 4;
+  return true;
+}
+
+int grow_own_ws(orsp::Graph *g, size_t need) {
+  if (g->own_ws_bytes >= need) return ORSP_OK;
+  cudaFree(g->own_ws);
+  g->own_ws = nullptr;
+  g->own_ws_bytes = 0;
+  ORSP_CUDA(cudaMalloc(&g->own_ws, need));
+  g->own_ws_bytes = need;
+  return ORSP_OK;
+}
+
+template <int NZM, bool PRIV>
+void *own_kernel(bool cv, bool two) {
+  if (cv)
+    return two ? (void *)lattice_own_kernel<NZM, PRIV, true, true, 2> : (void *)lattice_own_kernel<NZM, PRIV, true, false, 1>;
+  return two ? (void *)lattice_own_kernel<NZM, PRIV, false, true, 2>
+             : (void *)lattice_own_kernel<NZM, PRIV, false, false, 1>;
+}
+template <bool PRIV>
+void *own_kernel(int nzm, bool cv, bool two) {
+  return nzm == 6 ? own_kernel<6, PRIV>(cv, two) : nzm == 12 ? own_kernel<12, PRIV>(cv, two) : own_kernel<18, PRIV>(cv, two);
+}
+
+void fill_axes(LatParams &p) {
+  p.hmask = p.vmask = 0;
+  for (int z = 0, h = 0, v = 0; z < p.nz && z < 64; ++z) {
+    if (p.axis[z] == 1) p.hmask |= 1ull << z, p.hlist[h++] = (int8_t)z;
+    else if (p.axis[z] == 2) p.vmask |= 1ull << z, p.vlist[v++] = (int8_t)z;
+  }
+}
+
+int launch_own(orsp::Graph *g, LatParams &p, int64_t ntiles, const OwnShape &sh, int32_t nseeds, const int32_t *seeds,
+               const float *seed_cost, cudaStream_t st, orsp::LatOptions *opt) {
+  int rc = grow_own_ws(g, sh.ws);
+  if (rc) return rc;
+  if (!g->lat_ctl_h) ORSP_CUDA(cudaMallocHost(&g->lat_ctl_h, sizeof(LatCtl)));
+  fill_axes(p);
+  OwnParams o{};
+  char *b = (char *)g->own_ws;
+  p.ctl = (LatCtl *)b;
+  o.done = (int *)(b + 256);
+  o.nr = 16 * sh.nzb;
+  o.exch = (float *)(b + 512);
+  o.inbox = (unsigned *)(o.exch + ntiles * 2 * o.nr);
+  o.sent = o.inbox + ntiles;
+  o.got = o.sent + ntiles + 1;
+  o.seedt = (int32_t *)(o.got + ntiles + 1);
+  if (opt) opt->err_d = &p.ctl->err;
+  p.wait_ns = env_u64("ORSP_WAIT_NS", 2000000000ull);
+  p.budget_ns = env_u64("ORSP_BUDGET_NS", 20000000000ull);
+  o.l = p;
+  o.tcap = (int32_t)ntiles;
+  o.nzb = sh.nzb;
+  o.nseeds = nseeds;
+  o.seeds = seeds;
+  o.seed_cost = seed_cost;
+  const int64_t rows = ntiles * 2 * o.nr / 4;
+  own_init_kernel<<<1 + (int)std::max<int64_t>(1, std::min<int64_t>((rows + 255) / 256, g->num_sms)), 256, 0, st>>>(o);
+  ORSP_CUDA(cudaGetLastError());
+  const int nzm = run_visit_layers(sh.nzb);
+  const bool cv = p.wcol != nullptr, two = sh.per_sm == 2;
+  void *kfn = opt && opt->private_dist ? own_kernel<true>(nzm, cv, two) : own_kernel<false>(nzm, cv, two);
+  void *args[] = {&o};
+  rc = launch_persistent(g, kfn, (nzm > 16 ? 288 : 256) + 32, sh.smem, sh.per_sm, (int)ntiles, args, st);
+  if (rc) return rc;
+  if (!opt || opt->copy_ctl)
+    ORSP_CUDA(cudaMemcpyAsync(g->lat_ctl_h, p.ctl, sizeof(LatCtl), cudaMemcpyDeviceToHost, st));
+  return ORSP_OK;
+}
+
+// Whether a launch takes the owner schedule (ORSP_LAT_OWN=0: none does): one
+// that fits it and was not given the schedule of many wave fronts.
+bool use_own(const orsp::Graph *g, int64_t ntiles, int nzb, int64_t nseeds, const orsp::LatOptions *opt, OwnShape *sh) {
+  if (env_u64("ORSP_LAT_OWN", 1) == 0 || env_u64("ORSP_LAT_ASYNC", 1) == 0 || env_u64("ORSP_LAT_TMA", 0) != 0)
+    return false;
+  if (env_u64("ORSP_LAT_SPEC", 0) != 0 || env_u64("ORSP_LAT_BLOCKS_PER_SM", 1) > 1) return false;
+  if (opt && (opt->spec || opt->blocks_per_sm > 1 || opt->active)) return false;
+  return own_shape(g, ntiles, nzb, nseeds, sh) && sh->per_sm <= (int)env_u64("ORSP_OWN_PER_SM", 2);
+}
+
+int launch_lattice(orsp::Graph *g, LatParams &p, int64_t ntiles, int nzb, int32_t nseeds, const int32_t *seeds,
+                   const float *seed_cost, cudaStream_t st, orsp::LatOptions *opt) {
+  constexpr int TX = 16, TY = 16;
+  // (column vias always take the asynchronous schedule)
+  const bool async = p.wcol != nullptr || env_u64("ORSP_LAT_ASYNC", 1) != 0;
+  const WsLayout L = ws_layout(g, ntiles);
+  const size_t list_b = L.list_b, q_b = L.q_b;
+  const unsigned qcap = L.qcap;
+  int rc0 = grow_ws(g, L.total);
+  if (rc0) return rc0;
+  char *b = (char *)g->lat_ws;
+  p.list0 = (int32_t *)b;
+  p.list1 = (int32_t *)(b + list_b);
+  p.stamp = (unsigned *)(b + 2 * list_b);
+  p.tstate = (int *)(b + 3 * list_b);
+  p.qslot = async ? (int32_t *)(b + 4 * list_b) : nullptr;
+  p.qcap = qcap;
+  p.ctl = (LatCtl *)(b + 4 * list_b + q_b);
+  if (opt) opt->err_d = &p.ctl->err;
+  p.tbox = async ? p.list0 : nullptr;
+  if (async) {
+    const int64_t n = std::max<int64_t>(ntiles, qcap);
+    lattice_init_kernel<<<(int)std::min<int64_t>((n + 255) / 256, (int64_t)g->num_sms * 8), 256, 0, st>>>(p, (int32_t)ntiles);
+    ORSP_CUDA(cudaGetLastError());
+  } else {
+    ORSP_CUDA(cudaMemsetAsync(p.stamp, 0, list_b + (size_t)ntiles * 4, st));  // stamps and states
+  }
+  lattice_seed_kernel<TX, TY><<<1, 256, 0, st>>>(p, nseeds, seeds, seed_cost);
+  ORSP_CUDA(cudaGetLastError());
+  fill_axes(p);
+  // run visits up to 18 layers; deeper tiles take process_tile
+  const int nzm = async ? run_visit_layers(nzb) : 0;
+  // ORSP_LAT_BLOCKS_PER_SM: CTAs per SM
+  const int want = (int)env_u64("ORSP_LAT_BLOCKS_PER_SM", (opt && opt->blocks_per_sm > 0) ? opt->blocks_per_sm : 1);
+  const bool two = nzm && !p.wcol && want >= 2;
+  size_t smem = nzm ? (size_t)run_smem_floats(nzb, two) * sizeof(float)
+                    : (size_t)nzb * tile_floats_per_layer(TX, TY) * sizeof(float);
+  if (smem > 227 * 1024) {
+    orsp::set_error("lattice search: too many layers for the shared-memory tile");
+    return ORSP_ERR_ARG;
+  }
+  const bool priv = opt && opt->private_dist;
+  // ORSP_LAT_SPEC=1: the warp-specialised asynchronous schedule
+  const bool spec = nzm && !p.wcol && env_u64("ORSP_LAT_SPEC", (opt && opt->spec) ? 1 : 0) != 0;
+  // ORSP_LAT_TMA=1: tensor-load staging of fresh visits, for whole-lattice
+  // boxes (opt->tma_slices: distance slices of N cells, box j in slice j)
+  CUtensorMap tmw{}, tmd{};
+  bool tma = false;
+  if (async && !spec && !p.wcol && want < 2 && nzb <= 12 && nzb == g->nz && opt && opt->tma_slices > 0 &&
+      env_u64("ORSP_LAT_TMA", 0) != 0)
+    tma = encode_lattice_maps(g, p, TX, TY, nzb, opt->tma_slices, &tmw, &tmd);
+  const bool runs = nzm != 0 && !tma;
+  if (tma) {
+    const size_t base = ((size_t)nzb * tile_floats_per_layer(TX, TY) + 31) & ~(size_t)31;
+    smem = (base + (size_t)nzb * TY * TX * 4 + (size_t)nzb * (TY + 2) * (TX + 8)) * sizeof(float);
+  }
+  void *kfn;
+  if (runs) {
+    kfn = priv ? run_visit_kernel<true>(nzm, p.wcol != nullptr, spec, two)
+               : run_visit_kernel<false>(nzm, p.wcol != nullptr, spec, two);
+  } else if (p.wcol) {
+    kfn = priv ? (void *)lattice_async_kernel<16, 16, true, true, 1, false, true>
+               : (void *)lattice_async_kernel<16, 16, false, true, 1, false, true>;
+  } else if (tma) {
+    kfn = priv ? (void *)lattice_async_kernel<16, 16, true, false, 1, true>
+               : (void *)lattice_async_kernel<16, 16, false, false, 1, true>;
+  } else if (async) {
+    kfn = priv ? (void *)lattice_async_kernel<16, 16, true, true> : (void *)lattice_async_kernel<16, 16, false, true>;
+  } else {
+    kfn = priv ? (void *)lattice_tile_kernel<16, 16, true> : (void *)lattice_tile_kernel<16, 16, false>;
+  }
+  const int threads = (runs && nzm > 16 ? 288 : TX * TY) + (spec ? 32 : 0);
+  p.max_rounds = (unsigned)std::min<unsigned long long>(64ull * (unsigned long long)ntiles + 4096ull, 1ull << 30);
+  p.wait_ns = env_u64("ORSP_WAIT_NS", 2000000000ull);
+  // ORSP_LAT_SELF=0: a tile to visit again goes back to the queue instead
+  p.selfcont = (int)env_u64("ORSP_LAT_SELF", 1);
+  // ORSP_LAT_PREFETCH=0: no L2 prefetch of the next tile by the scheduler warp
+  p.prefetch = (int)env_u64("ORSP_LAT_PREFETCH", 1);
+  p.budget_ns = env_u64("ORSP_BUDGET_NS", 20000000000ull);
+  void *args[] = {&p, &tmw, &tmd};  // the tile and spec kernels take p only
+  int rc = launch_persistent(g, kfn, threads, smem, want, 0, args, st);
+  if (rc) return rc;
   if (!opt || opt->copy_ctl)
     ORSP_CUDA(cudaMemcpyAsync(g->lat_ctl_h, p.ctl, sizeof(LatCtl), cudaMemcpyDeviceToHost, st));
   return ORSP_OK;
@@ -2259,6 +2732,8 @@ void free_lattice(Graph *g) {
   g->wcol = nullptr;
   g->cvia = false;
   cudaFree(g->lat_ws);
+  cudaFree(g->own_ws);
+  g->own_ws = nullptr;
   cudaFree(g->lat_box_d);
   if (g->lat_ctl_h) cudaFreeHost(g->lat_ctl_h);
   g->lat_box_d = nullptr;
@@ -2276,7 +2751,15 @@ bool lattice_tile_fits(int nzb, int tile_w) {
   return smem <= 227 * 1024;
 }
 
-int reserve_lattice_ws(Graph *g, int64_t ntiles) { return grow_ws(g, ws_layout(g, ntiles).total); }
+int reserve_lattice_ws(Graph *g, int64_t ntiles) {
+  OwnShape sh;  // launches of up to that many tiles that take the owner schedule
+  const int64_t most = 2 * (int64_t)g->num_sms;
+  if (own_shape(g, std::min(std::max<int64_t>(ntiles, 1), most), std::min(g->nz, 18), 0, &sh)) {
+    int rc = grow_own_ws(g, sh.ws);
+    if (rc) return rc;
+  }
+  return grow_ws(g, ws_layout(g, ntiles).total);
+}
 
 int64_t make_lat_boxes(const int32_t *boxes_h, int32_t nbox, LatBox *out) {
   constexpr int TX = 16, TY = 16;
@@ -2383,7 +2866,11 @@ int run_lattice_boxes(Graph *g, const float *cost_d, int32_t nseeds, const int32
       }
     }
   }
-  if (by_flag) {
+  OwnShape own;
+  const bool owned = use_own(g, ntiles, nzb, nseeds, opt, &own);
+  if (owned && (priv || whole || (opt && opt->fill_box_only))) {
+    // the owners write every cell of the boxes
+  } else if (by_flag) {
     fill_slices_kernel<<<dim3(per_box, (unsigned)nbox), 256, 0, st>>>(dist, lboxes_d, opt->active, ORSP_INF_BITS);
     ORSP_CUDA(cudaGetLastError());
   } else if (priv) {
@@ -2416,6 +2903,7 @@ int run_lattice_boxes(Graph *g, const float *cost_d, int32_t nseeds, const int32
   p.N = N;
   p.dist = dist;
   for (int z = 0; z < 64; ++z) p.axis[z] = z < g->nz ? g->layer_axis[z] : 0;
+  if (owned) return launch_own(g, p, ntiles, own, nseeds, seeds_d, seed_cost_d, st, opt);
   return launch_lattice(g, p, ntiles, nzb, nseeds, seeds_d, seed_cost_d, st, opt);
 }
 
@@ -2491,6 +2979,9 @@ int run_lattice_roi(Graph *g, const float *cost_d, int32_t nseeds, const int32_t
   for (int z = 0; z < 64; ++z) p.axis[z] = z < g->nz ? g->layer_axis[z] : 0;
   // the box is known on the device only: size the tile arrays for the lattice
   const int64_t ntiles = (int64_t)((g->nx - 1 + TX) / TX) * ((g->ny - 1 + TY) / TY);
+  OwnShape own;
+  if (use_own(g, ntiles, g->nz, nseeds, nullptr, &own))
+    return launch_own(g, p, ntiles, own, nseeds, seeds_d, seed_cost_d, st, nullptr);
   return launch_lattice(g, p, ntiles, g->nz, nseeds, seeds_d, seed_cost_d, st, nullptr);
 }
 

@@ -658,6 +658,7 @@ static int sssp_impl(orsp_graph *g, const float *cost_d, int32_t nseeds, const i
   } else if (lattice) {
     LatOptions lopt;
     lopt.tma_slices = box_h ? 0 : 1;  // the whole lattice: TMA staging allowed
+    lopt.fill_box_only = box_h && !dist_out_d;  // the walk stays inside the box
     rc = run_lattice_search(g, cost_d, nseeds, seeds_d, seed_cost_d, box_h, dist, st, &lopt);
     if (rc) return rc;
     ORSP_CUDA(cudaMemsetAsync(g->ctl, 0, sizeof(SsspCtl), st));

@@ -26,6 +26,11 @@
 #include <climits>
 #include <cstdint>
 
+#include <mutex>
+#include <type_traits>
+
+#include <cuda.h>
+#include <cudaTypedefs.h>
 #include <cuda_bf16.h>
 
 #include "common.cuh"
@@ -841,6 +846,583 @@ __global__ void __launch_bounds__(TC_THREADS, 1) wgrad_tc_kernel(
   }
 }
 
+// ---------------------------------------------------------------------------
+// Plane kernels: convolution and weight gradient of 16- and 32-channel layers
+// with up to 32 channels on the other side.
+//
+// The kernels above copy rows with cp.async into a layout built by hand, run
+// MMAs of N = Cout (32) columns, and re-read the 4 KB A operand for every tap:
+// 40 clocks of shared memory for 16 of tensor work per MMA, behind a serial
+// copy (127 TFLOP/s; the weight gradient, one barrier and one wait per 32
+// voxels, 40).  Here
+//  - a plane of the tile (32 voxels x 8 rows and its halo) arrives by one TMA
+//    load, zero-filled outside the grid, in the swizzled layout that the
+//    MMA reads; a CTA marches along z, so a plane is loaded once for the
+//    three output planes that use it;
+//  - the taps that differ in x share one MMA: N = 3 Cout columns hold their
+//    partial products of the same input voxels, and the epilogue adds the
+//    three with a shift of one voxel (a TMEM quarter is one row of 32 voxels,
+//    so the shift is a shuffle).  27 x Cin / 16 MMAs of 32 columns become
+//    9 x Cin / 16 of 96, whose tensor time covers their operand reads;
+//  - warps are specialised: TMA, MMA, ReLU-mask (in place in shared memory,
+//    only when a mask is given), epilogue on a second accumulator pair.
+// Every wait is bounded; one that expires sets the abort flag that ends the
+// others, the TMA thread waits (bounded) for its loads in flight, and TMEM is
+// freed.  No load is multicast.
+constexpr int PL_X = 32;              // voxels per patch row, one TMEM quarter
+constexpr int PL_Y = 8;               // rows of a tile
+constexpr int PL_ROWS = PL_Y + 2;     // with the halo rows
+
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c1, int c2, int c3) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
+      : "memory");
+}
+
+// Shared-memory descriptor of a swizzled operand whose rows are C channels of
+// bf16 (64-byte swizzle for 32, 32-byte for 16): sbo between groups of eight
+// rows, lbo between blocks of C channels (M- or N-major operands only).
+template <int C>
+__device__ __forceinline__ uint64_t plane_desc(uint32_t addr, uint32_t lbo) {
+  constexpr uint64_t layout = C == 32 ? 4 : 6;
+  return umma_smem_desc(addr, lbo, 8 * C * 2) | (layout << 61);
+}
+
+// The tiles of a launch: nxs x nys columns of tiles, each cut into nzc
+// chunks of zc planes; unit u is chunk u / (nxs nys) of column u mod (nxs nys).
+struct PlanePlan {
+  int nxs, nys, zc, units;
+};
+
+struct PlaneUnit {
+  int x, y, z0, z1;  // column, planes [z0, z1)
+  __device__ __forceinline__ PlaneUnit(const PlanePlan &pl, int u, int D) {
+    const int cols = pl.nxs * pl.nys, c = u % cols;
+    x = c % pl.nxs;
+    y = c / pl.nxs;
+    z0 = (u / cols) * pl.zc;
+    z1 = min(D, z0 + pl.zc);
+  }
+};
+
+// Keeps the elements of n bytes of bf16 at v where the mask m is positive.
+__device__ __forceinline__ void mask_plane(unsigned char *v, const unsigned char *m, int n, int tid, int threads) {
+  for (int i = tid * 16; i < n; i += threads * 16) {
+    uint4 a = *reinterpret_cast<uint4 *>(v + i);
+    const uint4 b = *reinterpret_cast<const uint4 *>(m + i);
+    uint32_t *pa = reinterpret_cast<uint32_t *>(&a);
+    const uint32_t *pb = reinterpret_cast<const uint32_t *>(&b);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      // positive and not NaN: bits 1 .. 0x7f80
+      const uint32_t lo = ((pb[q] & 0xffffu) - 1u) < 0x7f80u ? 0xffffu : 0u;
+      const uint32_t hi = ((pb[q] >> 16) - 1u) < 0x7f80u ? 0xffff0000u : 0u;
+      pa[q] &= lo | hi;
+    }
+    *reinterpret_cast<uint4 *>(v + i) = a;
+  }
+}
+
+__device__ __forceinline__ void mbar_init(void *bar, int count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(void *bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(void *bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mma_commit(void *bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar))
+               : "memory");
+}
+
+constexpr int PL_MAXB = 8;  // plane buffers at most
+struct PlaneBars {
+  unsigned long long full[PL_MAXB], ready[PL_MAXB], empty[PL_MAXB];  // loaded, masked, consumed
+  unsigned long long mfree[2];                                       // mask buffer read
+  unsigned long long xfull[2], xempty[2];                            // weight gradient: X planes
+  unsigned long long accf[2], acce[2];
+  uint32_t tmem;
+  volatile int abort;
+};
+
+// Waits for `parity` of a barrier, bounded; ends early when another role has
+// given up, and makes the others give up when it expires.
+__device__ __forceinline__ bool plane_wait(PlaneBars &pb, void *bar, int parity) {
+  const uint32_t a = smem_addr(bar);
+  if (mbar_try(a, static_cast<uint32_t>(parity))) return true;
+  const unsigned long long t0 = dev_globaltimer();
+  for (;;) {
+    if (mbar_try(a, static_cast<uint32_t>(parity))) return true;
+    if (pb.abort) return false;
+    if (dev_globaltimer() - t0 > TC_WAIT_NS) {
+      pb.abort = 1;
+      atomicExch(&g_tc_err, 1);
+      return false;
+    }
+  }
+}
+
+constexpr int PC_THREADS = 384;  // TMA, MMA, two mask warps, eight epilogue warps
+
+template <int CIN>
+__host__ __device__ constexpr int plane_bytes() { return PL_X * PL_ROWS * CIN * 2; }
+template <int CIN>
+__host__ __device__ constexpr size_t pc_weight_bytes(int Cout) { return static_cast<size_t>(27) * CIN * Cout * 2; }
+
+// Convolution.  An MMA tile is four rows of 32 voxels (M = 128), a step two of
+// them (8 rows) of one output plane; patch columns overlap by two voxels, so a
+// row gives 30 outputs.
+template <int CIN, bool MASK>
+__global__ void __launch_bounds__(PC_THREADS, 1) conv3d_planes_kernel(
+    const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmm,
+    const __nv_bfloat16 *__restrict__ Wt, const float *__restrict__ bias, __nv_bfloat16 *__restrict__ Y,
+    float *__restrict__ Yf, int D, int H, int W, int Cout, int relu, PlanePlan plan, int NB) {
+  extern __shared__ __align__(1024) unsigned char sm[];
+  __shared__ PlaneBars pb;
+  constexpr int KC = CIN / 16, PB = plane_bytes<CIN>();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  unsigned char *const planes = sm;                                    // [NB] planes, 1024-byte aligned
+  unsigned char *const masks = planes + static_cast<size_t>(NB) * PB;  // [2] mask planes (MASK)
+  unsigned char *const sB = masks + (MASK ? 2 * PB : 0);
+  const int N = 3 * Cout, bblk = N * 32;
+  // weights: block (dz, dy; 16-wide K slice) of rows n = dx * Cout + co, K-major
+  // without swizzle: 8-row groups 256 bytes apart, K halves 128
+  for (int i = tid; i < 9 * KC * 2 * N; i += PC_THREADS) {
+    const int n = i % N, r = i / N, kh = r & 1, kc = (r >> 1) % KC, zy = (r >> 1) / KC;
+    const int dx = n / Cout, co = n - dx * Cout;
+    const __nv_bfloat16 *src = Wt + (static_cast<int64_t>(zy * 3 + dx) * CIN + kc * 16 + kh * 8) * Cout + co;
+    uint32_t v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      v[j] = static_cast<uint32_t>(__bfloat16_as_ushort(src[(2 * j) * Cout])) |
+             (static_cast<uint32_t>(__bfloat16_as_ushort(src[(2 * j + 1) * Cout])) << 16);
+    *reinterpret_cast<uint4 *>(sB + (zy * KC + kc) * bblk + (n >> 3) * 256 + kh * 128 + (n & 7) * 16) =
+        make_uint4(v[0], v[1], v[2], v[3]);
+  }
+  if (tid == 0) {
+    pb.abort = 0;
+    for (int b = 0; b < NB; ++b) {
+      mbar_init(&pb.full[b], 1);
+      mbar_init(&pb.ready[b], 64);
+      mbar_init(&pb.empty[b], 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(&pb.mfree[a], 64);
+      mbar_init(&pb.accf[a], 1);
+      mbar_init(&pb.acce[a], 256);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  const uint32_t ncols = 4 * N <= 256 ? 256u : 512u;  // two steps of two accumulators
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&pb.tmem)),
+                 "r"(ncols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = pb.tmem;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      // -------------------------------------------------------------- TMA
+      int n = 0;  // planes issued
+      bool ok = true;
+      for (int u = blockIdx.x; u < plan.units && ok; u += gridDim.x) {
+        const PlaneUnit un(plan, u, D);
+        for (int z = max(un.z0 - 1, 0); z <= min(un.z1, D - 1); ++z, ++n) {
+          const int b = n % NB;
+          if (n >= NB && !plane_wait(pb, &pb.empty[b], (n / NB - 1) & 1)) { ok = false; break; }
+          if (MASK && n >= 2 && !plane_wait(pb, &pb.mfree[n & 1], ((n >> 1) - 1) & 1)) { ok = false; break; }
+          mbar_expect(&pb.full[b], MASK ? 2 * PB : PB);
+          const int x = un.x * (PL_X - 2) - 1, y = un.y * PL_Y - 1;
+          tma_load_4d(smem_addr(planes + static_cast<size_t>(b) * PB), &tmx, smem_addr(&pb.full[b]), x, y, z);
+          if (MASK) tma_load_4d(smem_addr(masks + (n & 1) * PB), &tmm, smem_addr(&pb.full[b]), x, y, z);
+        }
+      }
+      // the loads in flight land before the block ends, also after a failure
+      for (int k = max(0, n - NB); k < n; ++k) mbar_wait(smem_addr(&pb.full[k % NB]), (k / NB) & 1);
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      // -------------------------------------------------------------- MMA
+      const uint32_t idesc = umma_idesc_bf16(TC_M, N);
+      int n = 0, step = 0, lastb = -1, lastp = 0;  // planes seen, steps made, last commit
+      bool ok = true;
+      for (int u = blockIdx.x; u < plan.units && ok; u += gridDim.x) {
+        const PlaneUnit un(plan, u, D);
+        const int zlo = max(un.z0 - 1, 0), zhi = min(un.z1, D - 1), n0 = n;
+        for (int z = un.z0; z < un.z1; ++z, ++step) {
+          const int a = step & 1;
+          while (ok && n - n0 <= min(z + 1, zhi) - zlo) {
+            const int b = n % NB;
+            ok = plane_wait(pb, MASK ? &pb.ready[b] : &pb.full[b], (n / NB) & 1);
+            ++n;
+          }
+          if (ok && step >= 2) ok = plane_wait(pb, &pb.acce[a], ((step >> 1) - 1) & 1);
+          if (!ok) break;
+          tc_fence_after();
+          for (int j = 0; j < 2; ++j) {
+            const uint32_t acc = tmem + static_cast<uint32_t>((a * 2 + j) * N);
+            uint32_t add = 0;
+            for (int dz = -1; dz <= 1; ++dz) {
+              if (z + dz < 0 || z + dz >= D) continue;
+              const uint32_t pl = smem_addr(planes + static_cast<size_t>((n0 + z + dz - zlo) % NB) * PB);
+#pragma unroll
+              for (int dy = 0; dy < 3; ++dy)
+#pragma unroll
+                for (int kc = 0; kc < KC; ++kc) {
+                  const uint64_t ad = plane_desc<CIN>(pl + (j * 4 + dy) * (PL_X * CIN * 2) + kc * 32, 16);
+                  const uint64_t bd =
+                      umma_smem_desc(smem_addr(sB + (((dz + 1) * 3 + dy) * KC + kc) * bblk), 128, 256);
+                  mma_bf16(acc, ad, bd, idesc, add);
+                  add = 1;
+                }
+            }
+          }
+          mma_commit(&pb.accf[a]);
+          lastb = a;
+          lastp = (step >> 1) & 1;
+          if (z - 1 >= zlo) mma_commit(&pb.empty[(n0 + z - 1 - zlo) % NB]);
+        }
+        if (ok)  // the planes still held: the last one written and the halo above it
+          for (int z = un.z1 - 1; z <= zhi; ++z) mma_commit(&pb.empty[(n0 + z - zlo) % NB]);
+      }
+      // after a failed wait the MMAs in flight get one more bounded wait
+      if (!ok && lastb >= 0) mbar_wait(smem_addr(&pb.accf[lastb]), static_cast<uint32_t>(lastp));
+    }
+  } else if (warp < 4) {
+    // ---------------------------------------------------------------- mask
+    if (MASK) {
+      int n = 0;
+      bool ok = true;
+      for (int u = blockIdx.x; u < plan.units && ok; u += gridDim.x) {
+        const PlaneUnit un(plan, u, D);
+        for (int z = max(un.z0 - 1, 0); z <= min(un.z1, D - 1) && ok; ++z, ++n) {
+          const int b = n % NB;
+          ok = plane_wait(pb, &pb.full[b], (n / NB) & 1);
+          if (!ok) break;
+          mask_plane(planes + static_cast<size_t>(b) * PB, masks + (n & 1) * PB, PB, tid - 64, 64);
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          mbar_arrive(&pb.ready[b]);
+          mbar_arrive(&pb.mfree[n & 1]);
+        }
+      }
+    }
+  } else {
+    // ------------------------------------------------------------ epilogue
+    // warp e: TMEM quarter e % 4 (one row of 32 voxels) of MMA tile e / 4
+    const int e = warp - 4, qd = e & 3, j = e >> 2;
+    const int nch = Cout >> 4;
+    int step = 0;
+    bool ok = true;
+    for (int u = blockIdx.x; u < plan.units && ok; u += gridDim.x) {
+      const PlaneUnit un(plan, u, D);
+      const int y = un.y * PL_Y + j * 4 + qd, x = un.x * (PL_X - 2) - 1 + lane;
+      const bool in = lane >= 1 && lane <= 30 && x < W && y < H;
+      for (int z = un.z0; z < un.z1; ++z, ++step) {
+        const int a = step & 1;
+        ok = plane_wait(pb, &pb.accf[a], (step >> 1) & 1);
+        if (!ok) break;
+        __syncwarp();
+        tc_fence_after();
+        const uint32_t t0 = tmem + (static_cast<uint32_t>(qd * 32) << 16) + static_cast<uint32_t>((a * 2 + j) * N);
+        for (int c = 0; c < nch; ++c) {
+          uint32_t r0[16], r1[16], r2[16];
+          tmem_ld16(t0 + c * 16, r0);
+          tmem_ld16(t0 + Cout + c * 16, r1);
+          tmem_ld16(t0 + 2 * Cout + c * 16, r2);
+          float f[16];
+#pragma unroll
+          for (int k = 0; k < 16; ++k) {
+            const float l = __shfl_up_sync(0xffffffffu, __uint_as_float(r0[k]), 1);
+            const float r = __shfl_down_sync(0xffffffffu, __uint_as_float(r2[k]), 1);
+            const float v = ((l + __uint_as_float(r1[k])) + r) + (bias ? __ldg(&bias[c * 16 + k]) : 0.0f);
+            f[k] = relu ? fmaxf(v, 0.0f) : v;
+          }
+          if (c == nch - 1) {  // the accumulator is read
+            tc_fence_before();
+            mbar_arrive(&pb.acce[a]);
+          }
+          if (!in) continue;
+          const int64_t o = ((static_cast<int64_t>(z) * H + y) * W + x) * Cout + c * 16;
+          if (Yf) {
+#pragma unroll
+            for (int k = 0; k < 16; k += 4)
+              *reinterpret_cast<float4 *>(Yf + o + k) = make_float4(f[k], f[k + 1], f[k + 2], f[k + 3]);
+          } else {
+            uint32_t p[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+              p[k] = static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16(f[2 * k]))) |
+                     (static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16(f[2 * k + 1]))) << 16);
+            *reinterpret_cast<uint4 *>(Y + o) = make_uint4(p[0], p[1], p[2], p[3]);
+            *reinterpret_cast<uint4 *>(Y + o + 8) = make_uint4(p[4], p[5], p[6], p[7]);
+          }
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols) : "memory");
+  }
+}
+
+constexpr int PW_THREADS = 256;  // TMA, MMA, two mask warps, four epilogue warps
+
+template <int CIN>
+__host__ __device__ constexpr int pw_x_bytes() { return PL_X * PL_Y * CIN * 2; }  // one shifted X plane
+template <int COUT>
+__host__ __device__ constexpr int pw_g_bytes() { return PL_X * PL_ROWS * COUT * 2; }
+
+// Weight gradient: for each plane z' of X, row y' and voxel x of a tile,
+//   D[dz][(dx, ci)][(dy, co)] += X[z'][y'][x + dx][ci] G[z' - dz][y' - dy][x][co]
+// as M = 128 (three dx blocks of CIN channels, the rest of M unused) by N = 3
+// COUT (three dy blocks) MMAs over K = 16 voxels; both operands are M- or
+// N-major (channels contiguous).  The dx blocks are three TMA loads of the X
+// plane, one voxel apart, the dy blocks the G plane one row apart, so one MMA
+// serves nine taps.  The three accumulators (dz) stay in TMEM over all of a
+// CTA's tiles and are added to dW once, four values per atomic.
+template <int CIN, int COUT, bool MASK>
+__global__ void __launch_bounds__(PW_THREADS, 1) wgrad_planes_kernel(
+    const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmg,
+    const __grid_constant__ CUtensorMap tmm, float *__restrict__ dW, int D, PlanePlan plan) {
+  extern __shared__ __align__(1024) unsigned char sm[];
+  __shared__ PlaneBars pb;
+  constexpr int XB = pw_x_bytes<CIN>(), GB = pw_g_bytes<COUT>(), NG = 4, N = 3 * COUT;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  unsigned char *const xs = sm;               // [2][3] shifted X planes
+  unsigned char *const gs = xs + 6 * XB;      // [NG] G planes
+  unsigned char *const ms = gs + NG * GB;     // [2] mask planes (MASK)
+  if (tid == 0) {
+    pb.abort = 0;
+    for (int b = 0; b < NG; ++b) {
+      mbar_init(&pb.full[b], 1);
+      mbar_init(&pb.ready[b], 64);
+      mbar_init(&pb.empty[b], 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(&pb.mfree[a], 64);
+      mbar_init(&pb.xfull[a], 1);
+      mbar_init(&pb.xempty[a], 1);
+    }
+    mbar_init(&pb.accf[0], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  constexpr uint32_t ncols = 3 * N <= 256 ? 256u : 512u;
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&pb.tmem)),
+                 "r"(ncols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = pb.tmem;
+  const bool any = static_cast<int>(blockIdx.x) < plan.units;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      // -------------------------------------------------------------- TMA
+      int n = 0, m = 0;  // G planes, X planes issued
+      bool ok = true;
+      auto load_g = [&](const PlaneUnit &un, int z) {
+        const int b = n % NG;
+        if (n >= NG && !plane_wait(pb, &pb.empty[b], (n / NG - 1) & 1)) return false;
+        if (MASK && n >= 2 && !plane_wait(pb, &pb.mfree[n & 1], ((n >> 1) - 1) & 1)) return false;
+        mbar_expect(&pb.full[b], MASK ? 2 * GB : GB);
+        tma_load_4d(smem_addr(gs + b * GB), &tmg, smem_addr(&pb.full[b]), un.x * PL_X, un.y * PL_Y - 1, z);
+        if (MASK) tma_load_4d(smem_addr(ms + (n & 1) * GB), &tmm, smem_addr(&pb.full[b]), un.x * PL_X, un.y * PL_Y - 1, z);
+        ++n;
+        return true;
+      };
+      for (int u = blockIdx.x; u < plan.units && ok; u += gridDim.x) {
+        const PlaneUnit un(plan, u, D);
+        const int zhi = min(un.z1, D - 1);
+        int zg = max(un.z0 - 1, 0);
+        for (int z = un.z0; z < un.z1 && ok; ++z, ++m) {
+          while (ok && zg <= min(z + 1, zhi)) ok = load_g(un, zg++);
+          const int b = m & 1;
+          if (!ok || (m >= 2 && !plane_wait(pb, &pb.xempty[b], ((m >> 1) - 1) & 1))) { ok = false; break; }
+          mbar_expect(&pb.xfull[b], 3 * XB);
+          for (int dx = 0; dx < 3; ++dx)
+            tma_load_4d(smem_addr(xs + (b * 3 + dx) * XB), &tmx, smem_addr(&pb.xfull[b]), un.x * PL_X + dx - 1,
+                        un.y * PL_Y, z);
+        }
+      }
+      for (int k = max(0, n - NG); k < n; ++k) mbar_wait(smem_addr(&pb.full[k % NG]), (k / NG) & 1);
+      for (int k = max(0, m - 2); k < m; ++k) mbar_wait(smem_addr(&pb.xfull[k & 1]), (k >> 1) & 1);
+    }
+  } else if (warp == 1) {
+    if (lane == 0 && any) {
+      // -------------------------------------------------------------- MMA
+      const uint32_t idesc = umma_idesc_bf16_mn(TC_M, N);
+      int n = 0, m = 0;
+      uint32_t used[3] = {0, 0, 0};
+      bool ok = true;
+      for (int u = blockIdx.x; u < plan.units && ok; u += gridDim.x) {
+        const PlaneUnit un(plan, u, D);
+        const int zlo = max(un.z0 - 1, 0), zhi = min(un.z1, D - 1), n0 = n;
+        for (int z = un.z0; z < un.z1; ++z, ++m) {
+          while (ok && n - n0 <= min(z + 1, zhi) - zlo) {
+            const int b = n % NG;
+            ok = plane_wait(pb, MASK ? &pb.ready[b] : &pb.full[b], (n / NG) & 1);
+            ++n;
+          }
+          if (ok) ok = plane_wait(pb, &pb.xfull[m & 1], (m >> 1) & 1);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t xa = smem_addr(xs + (m & 1) * 3 * XB);
+#pragma unroll
+          for (int dz = 0; dz < 3; ++dz) {
+            const int zg = z - (dz - 1);
+            if (zg < 0 || zg >= D) continue;
+            const uint32_t ga = smem_addr(gs + ((n0 + zg - zlo) % NG) * GB);
+            const uint32_t acc = tmem + static_cast<uint32_t>(dz * N);
+            uint32_t add = used[dz];
+#pragma unroll 4
+            for (int k = 0; k < PL_Y * 2; ++k) {
+              const uint64_t ad = plane_desc<CIN>(xa + k * (16 * CIN * 2), XB);
+              const uint64_t bd = plane_desc<COUT>(ga + k * (16 * COUT * 2), PL_X * COUT * 2);
+              mma_bf16(acc, ad, bd, idesc, add);
+              add = 1;
+            }
+            used[dz] = 1;
+          }
+          mma_commit(&pb.xempty[m & 1]);
+          if (z - 1 >= zlo) mma_commit(&pb.empty[(n0 + z - 1 - zlo) % NG]);
+        }
+        if (ok)
+          for (int z = un.z1 - 1; z <= zhi; ++z) mma_commit(&pb.empty[(n0 + z - zlo) % NG]);
+      }
+      mma_commit(&pb.accf[0]);  // after every MMA of the CTA, also after a failed wait
+      if (!ok) mbar_wait(smem_addr(&pb.accf[0]), 0);
+    }
+  } else if (warp < 4) {
+    if (MASK) {
+      int n = 0;
+      bool ok = true;
+      for (int u = blockIdx.x; u < plan.units && ok; u += gridDim.x) {
+        const PlaneUnit un(plan, u, D);
+        for (int z = max(un.z0 - 1, 0); z <= min(un.z1, D - 1) && ok; ++z, ++n) {
+          const int b = n % NG;
+          ok = plane_wait(pb, &pb.full[b], (n / NG) & 1);
+          if (!ok) break;
+          mask_plane(gs + b * GB, ms + (n & 1) * GB, GB, tid - 64, 64);
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          mbar_arrive(&pb.ready[b]);
+          mbar_arrive(&pb.mfree[n & 1]);
+        }
+      }
+    }
+  } else if (any) {
+    // ------------------------------------------------------------ epilogue
+    const int qd = warp & 3, mrow = qd * 32 + lane, dx = mrow / CIN, ci = mrow % CIN;
+    // accumulators that some plane of this CTA wrote: a plane has no G plane
+    // above it at the top of the grid, none below at the bottom
+    bool used[3] = {false, true, false};
+    for (int u = blockIdx.x; u < plan.units; u += gridDim.x) {
+      const PlaneUnit un(plan, u, D);
+      used[0] = used[0] || un.z0 < D - 1;
+      used[2] = used[2] || un.z1 > 1;
+    }
+    if (qd * 32 < 3 * CIN && plane_wait(pb, &pb.accf[0], 0) && !pb.abort) {
+      __syncwarp();
+      tc_fence_after();
+#pragma unroll
+      for (int dz = 0; dz < 3; ++dz) {
+        if (!used[dz]) continue;
+        for (int c0 = 0; c0 < N; c0 += 16) {
+          uint32_t r[16];
+          tmem_ld16(tmem + (static_cast<uint32_t>(qd * 32) << 16) + static_cast<uint32_t>(dz * N + c0), r);
+          const int dy = 2 - c0 / COUT;  // block 0 pairs row y' with G row y' - 1
+          if (dx < 3) {
+            float *dst = dW + (static_cast<int64_t>(dz * 9 + dy * 3 + dx) * CIN + ci) * COUT + c0 % COUT;
+            if ((reinterpret_cast<uintptr_t>(dW) & 15) == 0) {
+#pragma unroll
+              for (int k = 0; k < 16; k += 4)
+                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + k),
+                             "f"(__uint_as_float(r[k])), "f"(__uint_as_float(r[k + 1])),
+                             "f"(__uint_as_float(r[k + 2])), "f"(__uint_as_float(r[k + 3]))
+                             : "memory");
+            } else {
+#pragma unroll
+              for (int k = 0; k < 16; ++k) atomicAdd(dst + k, __uint_as_float(r[k]));
+            }
+          }
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols) : "memory");
+  }
+}
+
+// cuTensorMapEncodeTiled through the runtime's driver entry point (no link
+// against the driver library); nullptr when unavailable.
+PFN_cuTensorMapEncodeTiled_v12000 warm_map_encoder() {
+  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    void *f = nullptr;
+    cudaDriverEntryPointQueryResult q{};
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      fn = (PFN_cuTensorMapEncodeTiled_v12000)f;
+    else
+      (void)cudaGetLastError();
+  });
+  return fn;
+}
+
+// Map of a [D][H][W][C] bf16 array, box C x 32 voxels x `rows` x 1, swizzled by
+// the row of channels; false when the address is not 16-byte aligned or the
+// encoder refuses.
+bool plane_map(CUtensorMap *m, const void *X, int D, int H, int W, int C, int rows) {
+  PFN_cuTensorMapEncodeTiled_v12000 enc = warm_map_encoder();
+  if (!enc || (reinterpret_cast<uintptr_t>(X) & 15)) return false;
+  const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)D};
+  const cuuint64_t str[3] = {(cuuint64_t)C * 2, (cuuint64_t)C * 2 * W, (cuuint64_t)C * 2 * W * H};
+  const cuuint32_t box[4] = {(cuuint32_t)C, PL_X, (cuuint32_t)rows, 1}, es[4] = {1, 1, 1, 1};
+  return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void *>(X), dims, str, box, es,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, C == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
+             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Cuts D planes of `cols` tile columns into chunks so that the CTA with the
+// most work has the fewest planes (a chunk loads about one plane's worth more
+// than it computes).
+PlanePlan plane_plan(int nxs, int nys, int D, int ctas) {
+  PlanePlan best{nxs, nys, D, 0};
+  double cost = 1e30;
+  const int64_t cols = (int64_t)nxs * nys;
+  for (int zc = 1; zc <= D; ++zc) {
+    const int64_t units = cols * ((D + zc - 1) / zc);
+    if (units > INT32_MAX) continue;
+    const double c = (double)((units + ctas - 1) / ctas) * (zc + 0.6);
+    if (c < cost) {
+      cost = c;
+      best.zc = zc;
+      best.units = (int)units;
+    }
+  }
+  return best;
+}
+
 // db[co] += sum_v G[v][co] (G = dY, or dY where Yo > 0): one block per
 // chunk of voxels, per-thread channel sums, one atomic per channel and block.
 __global__ void bias_sum_kernel(const __nv_bfloat16 *__restrict__ dY, const __nv_bfloat16 *__restrict__ Yo,
@@ -866,6 +1448,59 @@ __global__ void bias_sum_kernel(const __nv_bfloat16 *__restrict__ dY, const __nv
 
 using namespace orsp;
 
+// The plane kernel's launch; ORSP_NO_PATH when its loads do not apply (input
+// or mask not 16-byte aligned).
+static int conv3d_planes(const void *X, const void *mask, const void *Wt, const float *bias, void *Y, float *Yf, int D,
+                         int H, int W, int Cin, int Cout, int relu, cudaStream_t st) {
+  CUtensorMap tx, tm;
+  if (!plane_map(&tx, X, D, H, W, Cin, PL_ROWS)) return ORSP_NO_PATH;
+  tm = tx;
+  if (mask && !plane_map(&tm, mask, D, H, W, Cin, PL_ROWS)) return ORSP_NO_PATH;
+  int dev = 0, sms = 0;
+  ORSP_CUDA(cudaGetDevice(&dev));
+  ORSP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const PlanePlan plan = plane_plan((W + PL_X - 3) / (PL_X - 2), (H + PL_Y - 1) / PL_Y, D, sms);
+  if (plan.units <= 0) return ORSP_NO_PATH;
+  const size_t pb = Cin == 32 ? plane_bytes<32>() : plane_bytes<16>();
+  const size_t wb = Cin == 32 ? pc_weight_bytes<32>(Cout) : pc_weight_bytes<16>(Cout);
+  const size_t room = 224 * 1024 - wb - (mask ? 2 * pb : 0);
+  const int nb = (int)std::min<size_t>(PL_MAXB, room / pb);
+  const size_t smem = nb * pb + (mask ? 2 * pb : 0) + wb;
+  auto kfn = Cin == 32 ? (mask ? conv3d_planes_kernel<32, true> : conv3d_planes_kernel<32, false>)
+                       : (mask ? conv3d_planes_kernel<16, true> : conv3d_planes_kernel<16, false>);
+  ORSP_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kfn<<<std::min(plan.units, sms), PC_THREADS, smem, st>>>(tx, tm, (const __nv_bfloat16 *)Wt, bias, (__nv_bfloat16 *)Y,
+                                                           Yf, D, H, W, Cout, relu, plan, nb);
+  ORSP_CUDA(cudaGetLastError());
+  return ORSP_OK;
+}
+
+static int wgrad_planes(const void *X, const void *dY, const void *Yo, float *dW, int D, int H, int W, int Cin,
+                        int Cout, cudaStream_t st) {
+  CUtensorMap tx, tg, tm;
+  if (!plane_map(&tx, X, D, H, W, Cin, PL_Y) || !plane_map(&tg, dY, D, H, W, Cout, PL_ROWS)) return ORSP_NO_PATH;
+  tm = tg;
+  if (Yo && !plane_map(&tm, Yo, D, H, W, Cout, PL_ROWS)) return ORSP_NO_PATH;
+  int dev = 0, sms = 0;
+  ORSP_CUDA(cudaGetDevice(&dev));
+  ORSP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const PlanePlan plan = plane_plan((W + PL_X - 1) / PL_X, (H + PL_Y - 1) / PL_Y, D, sms);
+  if (plan.units <= 0) return ORSP_NO_PATH;
+  const size_t xb = Cin == 32 ? pw_x_bytes<32>() : pw_x_bytes<16>(), gb = Cout == 32 ? pw_g_bytes<32>() : pw_g_bytes<16>();
+  // (the unused rows of M read past the third X plane, within the allocation)
+  const size_t smem = std::max(6 * xb + 4 * gb + (Yo ? 2 * gb : 0), 3 * xb + 128 / Cin * xb);
+  auto pick = [&](auto masked) {
+    constexpr bool M = decltype(masked)::value;
+    return Cin == 32 ? (Cout == 32 ? wgrad_planes_kernel<32, 32, M> : wgrad_planes_kernel<32, 16, M>)
+                     : (Cout == 32 ? wgrad_planes_kernel<16, 32, M> : wgrad_planes_kernel<16, 16, M>);
+  };
+  auto kfn = Yo ? pick(std::true_type()) : pick(std::false_type());
+  ORSP_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kfn<<<std::min(plan.units, sms), PW_THREADS, smem, st>>>(tx, tg, tm, dW, D, plan);
+  ORSP_CUDA(cudaGetLastError());
+  return ORSP_OK;
+}
+
 extern "C" int orsp_warm_conv3d_tc(const void *X, const void *mask, const void *Wt, const float *bias, void *Y,
                                    float *Yf, int32_t D, int32_t H, int32_t W, int32_t Cin, int32_t Cout,
                                    int32_t relu, uintptr_t stream) {
@@ -873,6 +1508,12 @@ extern "C" int orsp_warm_conv3d_tc(const void *X, const void *mask, const void *
       Cout % 16 || Cout > 64) {
     set_error("warm_conv3d_tc: bad arguments (Cin, Cout multiples of 16, Cout <= 64)");
     return ORSP_ERR_ARG;
+  }
+  const char *ws = getenv("ORSP_WARM_TC_WS");
+  const bool stage_barrier = ws && ws[0] == '0';
+  if (!stage_barrier && (Cin == 16 || Cin == 32) && Cout <= 32) {
+    int rc = conv3d_planes(X, mask, Wt, bias, Y, Yf, D, H, W, Cin, Cout, relu, (cudaStream_t)stream);
+    if (rc != ORSP_NO_PATH) return rc;
   }
   const int ns = cv_stages(Cin, Cout);
   if (ns < 2) {
@@ -900,8 +1541,7 @@ extern "C" int orsp_warm_conv3d_tc(const void *X, const void *mask, const void *
   // the warp-specialised kernel (producer warps and an MMA warp handing
   // stages over through mbarriers); ORSP_WARM_TC_WS=0: the kernel with one
   // block barrier per stage
-  const char *ws = getenv("ORSP_WARM_TC_WS");
-  if (!(ws && ws[0] == '0')) {
+  if (!stage_barrier) {
     decltype(kfn) kws = Cin == 16 ? conv3d_tc_ws_kernel<2> : Cin == 32 ? conv3d_tc_ws_kernel<4>
                                                                        : conv3d_tc_ws_kernel<8>;
     const size_t smem_ws = ws_smem_bytes(Cin, Cout, ns);
@@ -936,20 +1576,25 @@ extern "C" int orsp_warm_wgrad_tc(const void *X, const void *dY, const void *Yo,
     return ORSP_ERR_ARG;
   }
   cudaStream_t st = (cudaStream_t)stream;
-  const size_t smem = wg_smem_bytes(Cin, Cout);
   int dev = 0, sms = 0;
   ORSP_CUDA(cudaGetDevice(&dev));
   ORSP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  ORSP_CUDA(cudaFuncSetAttribute(wgrad_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int64_t nchunks = static_cast<int64_t>(D) * H * ((W + WG_K - 1) / WG_K);
-  if (nchunks > INT32_MAX) {
-    set_error("warm_wgrad_tc: grid too large (the chunk counter is 32-bit)");
-    return ORSP_ERR_ARG;
+  int rc = ORSP_NO_PATH;
+  if ((Cin == 16 || Cin == 32) && (Cout == 16 || Cout == 32)) rc = wgrad_planes(X, dY, Yo, dW, D, H, W, Cin, Cout, st);
+  if (rc < 0) return rc;
+  if (rc == ORSP_NO_PATH) {
+    const size_t smem = wg_smem_bytes(Cin, Cout);
+    ORSP_CUDA(cudaFuncSetAttribute(wgrad_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int64_t nchunks = static_cast<int64_t>(D) * H * ((W + WG_K - 1) / WG_K);
+    if (nchunks > INT32_MAX) {
+      set_error("warm_wgrad_tc: grid too large (the chunk counter is 32-bit)");
+      return ORSP_ERR_ARG;
+    }
+    const int grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(nchunks, sms)));
+    wgrad_tc_kernel<<<grid, TC_THREADS, smem, st>>>((const __nv_bfloat16 *)X, (const __nv_bfloat16 *)dY,
+                                                    (const __nv_bfloat16 *)Yo, dW, D, H, W, Cin, Cout);
+    ORSP_CUDA(cudaGetLastError());
   }
-  const int grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(nchunks, sms)));
-  wgrad_tc_kernel<<<grid, TC_THREADS, smem, st>>>((const __nv_bfloat16 *)X, (const __nv_bfloat16 *)dY,
-                                                  (const __nv_bfloat16 *)Yo, dW, D, H, W, Cin, Cout);
-  ORSP_CUDA(cudaGetLastError());
   if (db) {
     const int64_t nvox = static_cast<int64_t>(D) * H * W;
     const int threads = (256 / Cout) * Cout;

@@ -258,9 +258,11 @@ ORSP_API int orsp_sssp_batch_ranges(orsp_graph *g, const float *cost_d, int32_t 
  *            one launch of the largest ctas_per_sm of their buckets CTAs per
  *            SM (0: default 2);
  *   impl 1   tile sweeps over many boxes per launch, each box with its own
- *            distance slice, tile width tile_w[i] (16 or 32); used on graphs
- *            recognised as H/V lattices, impl 0 otherwise.
- * nb = 0 restores the default (impl 0 for every box).  Every plan gives the
+ *            distance slice; used on graphs recognised as H/V lattices, impl 0
+ *            otherwise.  tile_w[i] (16 or 32) only bounds the depth of the
+ *            boxes swept (orsp_lattice_max_layers); tiles are 16 wide.
+ * nb = 0 restores the default: tile sweeps for boxes of up to 18 layers on
+ * H/V lattices with adjacent vias, impl 0 otherwise.  Every plan gives the
  * same paths, bit for bit; the plan only changes the time.  No counterpart in
  * the reference. */
 ORSP_API int orsp_batch_set_plan(orsp_graph *g, int32_t nb, const int64_t *max_nodes, const int32_t *impl,

@@ -694,12 +694,15 @@ int run_batch_lat(orsp_graph *g, const float *cost_d, int32_t K, const std::vect
     if (rc) return rc;
     LatOptions opt;
     opt.private_dist = true;
+    opt.private_count = cells;
     // many boxes: two CTAs per SM and the warp-specialised schedule, as for
     // many sources (2 048 boxes of up to 400 x 400 x 16: 10.5 ms, against
-    // 14.6 ms without the schedule and 13.2 ms with it at one CTA per SM)
-    opt.blocks_per_sm = 2;
-    opt.spec = 1;
-    opt.private_count = cells;
+    // 14.6 ms without the schedule and 13.2 ms with it at one CTA per SM);
+    // boxes of no more tiles than the owner schedule holds take that one
+    if (ntiles > 2 * (int64_t)g->num_sms) {
+      opt.blocks_per_sm = 2;
+      opt.spec = 1;
+    }
     opt.copy_ctl = false;
     rc = run_lattice_boxes(g, cost_d, m, d_src, nullptr, m, boxes.data(), db, g->blat_dist, st, &opt);
     if (rc) return rc;
@@ -810,14 +813,23 @@ static int run_batch(orsp_graph *g, const float *cost_d, int32_t K, const int32_
     const int32_t *b = &bb[(size_t)per * k];
     return lattice_tile_fits(b[5] - b[4] + 1, tw);
   };
+  // without a plan, boxes on an H/V lattice with adjacent vias, up to 18 layers
+  // deep (the depth of the run visits), are swept: that is the faster form
+  // at every count and size measured (one box of up to 30 x 30 x 6: 0.21 ms
+  // against 0.29 ms with one CTA per search, 2 048 of 24 x 24 x 4: 0.63
+  // against 1.38, 512 of up to 400 x 400 x 16: 2.7 against 19.3).  Column-via
+  // and deeper boxes keep one CTA per search: not measured.
+  const bool sweep_all = !range_mode && g->plan_nb == 0 && g->lattice_ok && !g->cvia;
   auto swept = [&](int i, int32_t k) {
+    const int32_t *b = &bb[(size_t)per * k];
+    if (sweep_all) return b[5] - b[4] < 18;
     return tuned && g->plan_impl[i] == 1 && g->lattice_ok && !(g->cvia && g->plan_tile[i] != 16) &&
            tile_ok(k, g->plan_tile[i]);
   };
   std::vector<int32_t> lat_items;
   for (int32_t i = 0; i < K; ++i) {
     const int32_t k = ord[i];
-    if (tuned && swept(plan_bucket(g, box_volume(&bb[(size_t)per * k], range_mode)), k)) lat_items.push_back(k);
+    if (swept(tuned ? plan_bucket(g, box_volume(&bb[(size_t)per * k], range_mode)) : 0, k)) lat_items.push_back(k);
   }
   if (!lat_items.empty()) {
     src_h.resize(K);

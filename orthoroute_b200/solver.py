@@ -247,7 +247,7 @@ class DeviceGraph:
     def batch_bbox(self, cost: torch.Tensor, src: torch.Tensor, dst: torch.Tensor, bbox: torch.Tensor,
                    order: Optional[torch.Tensor] = None, delta: Optional[float] = None,
                    path_cap: int = 4096, with_edges: bool = True):
-        """K box-ROI searches in one launch.  Returns (nodes[K,cap], edges[K,cap]
+        """K box-ROI searches in one call.  Returns (nodes[K,cap], edges[K,cap]
         or None, lens[K]) as device tensors; lens < 2 means no path."""
         lib = _lib.load()
         K = int(src.numel())

@@ -325,6 +325,12 @@ ORSP_API int orsp_route_nets_snapshot(orsp_graph *g, int32_t M, const int32_t *s
                     const float *hist_d, float pres_fac, float hist_w, float via_mult, float base_w,
                     int32_t jitter, int64_t *searches_out, uintptr_t stream);
 
+/* First-fit rounds of boxes (host): round_h[j] = the first round that holds no
+ * earlier box meeting box j (boxes_h[6j..6j+5], inclusive bounds), so the boxes
+ * of a round are pairwise disjoint.  The order in which the routing loop's
+ * groups take the nets; no counterpart in the reference. */
+ORSP_API int orsp_first_fit_rounds(int32_t n, const int32_t *boxes_h, int32_t *round_h);
+
 /* ---- negotiation bookkeeping ------------------------------------------- */
 /* The per-iteration loops the reference runs in Python over all committed
  * nets.  Nets come in the router's dict order as concatenated node paths or

@@ -102,6 +102,7 @@ _SIGS = {
     "orsp_update_history": (ctypes.c_int, [_i64, _P, _P, _P, _P, _f32, _f32, _f32, _u]),
     "orsp_overuse": (ctypes.c_int, [_i64, _P, _P, _P, _P, _u]),
     "orsp_present_from_usage": (ctypes.c_int, [_i64, _P, _P, _u]),
+    "orsp_first_fit_rounds": (ctypes.c_int, [_i32, _P, _P]),
     "orsp_commit_edges": (ctypes.c_int, [_i64, _P, _P, _P, _i32, _u]),
     "orsp_commit_batch": (ctypes.c_int, [_i32, _P, _P, _i32, _P, _P, _i32, _u]),
 }

@@ -6,10 +6,11 @@ namespace orsp {
 
 // commit_path / clear_path on one edge (UPF:821-836): usage +-1 (never below
 // 0) and present kept equal to it; atomic, so paths of a batch may share edges.
-__device__ __forceinline__ void apply_usage(int32_t *usage, float *present, int32_t e,
-                                            int32_t sign) {
+__device__ __forceinline__ int32_t apply_usage(int32_t *usage, float *present, int32_t e,
+                                               int32_t sign) {
+  int32_t left;
   if (sign >= 0) {
-    atomicAdd(&usage[e], sign);
+    left = atomicAdd(&usage[e], sign) + sign;
     if (present) atomicAdd(&present[e], 1.0f);
   } else {
     // clear_path: canonical count drops (never below 0) and
@@ -18,6 +19,7 @@ __device__ __forceinline__ void apply_usage(int32_t *usage, float *present, int3
     for (;;) {
       const int32_t nv = old > 0 ? old - 1 : 0;
       const int32_t prev = atomicCAS(&usage[e], old, nv);
+      left = nv;
       if (prev == old) break;
       old = prev;
     }
@@ -33,6 +35,7 @@ __device__ __forceinline__ void apply_usage(int32_t *usage, float *present, int3
       }
     }
   }
+  return left;
 }
 
 // The edge-index jitter of the cost formulas, xp.arange(E, dtype=float32) %

@@ -407,11 +407,11 @@ int env_int(const char *name, int dflt) {
 }
 
 // Backtrace of the searches done by tile sweeps with their own distance
-// slices: one warp per search (block j: item[j], box boxes[j]).  The warp
-// walks with lat_walk_warp (the parent rule of block_backtrace), reading distances from the box's slice (box-local row-major order,
-// which is the node-id order, so the ranks agree); then the lanes reverse the
-// path and map each step u -> v to the in-edge of v in u's slot (the first CSR
-// edge u -> v: the lattice has no parallel edges).  Same status codes as
+// slices: one block per search (block j: item[j], box boxes[j]).  Warp 0
+// walks with lat_walk_warp (the parent rule of block_backtrace), reading
+// distances from the box's slice (box-local row-major order, which is the
+// node-id order, so the ranks agree); then the block maps each step u -> v to
+// the in-edge of v in u's slot and reverses the path.  Same status codes as
 // block_backtrace.
 struct LatBt {
   const float4 *w4;         // gathered in-edge weights (fresh inside the boxes)
@@ -431,8 +431,9 @@ __device__ __forceinline__ bool lat_in_box(const orsp::LatBox &B, int32_t x, int
   return x >= B.x0 && x <= B.x1 && y >= B.y0 && y <= B.y1 && z >= B.z0 && z <= B.z1;
 }
 
-__global__ void lat_batch_backtrace_kernel(LatBt p) {
-  const int lane = threadIdx.x & 31;
+__global__ void __launch_bounds__(orsp::kWalkBlock) lat_batch_backtrace_kernel(LatBt p) {
+  __shared__ int s_len;
+  const int lane = threadIdx.x;
   const int j = blockIdx.x;
   const int32_t k = p.item[j];
   const orsp::LatBox B = p.boxes[j];
@@ -457,42 +458,25 @@ __global__ void lat_batch_backtrace_kernel(LatBt p) {
   auto dget = [dist, bw, bh, bx0, by0, bz0](int32_t a, int32_t b, int32_t c) {
     return __ldcg(&dist[((int64_t)(c - bz0) * bh + (b - by0)) * bw + (a - bx0)]);
   };
-  unsigned dv = dget(x, y, z);
-  if (dv == ORSP_INF_BITS) {
-    if (lane == 0) p.path_len[k] = 0;
-    return;
-  }
   auto at_src = [src](int64_t v, unsigned) { return v == src; };
-  int len = orsp::lat_walk_warp(p.geom, B, p.w4, dget, at_src, x, y, z, dv, nodes, p.path_cap);
-  int status = 0;
-  if (len == -1) status = ST_PATHCAP;
-  else if (len < 0) status = ST_INTERNAL;
-  __syncwarp();
-  if (status) {
-    if (lane == 0) p.path_len[k] = status;
+  if (lane < 32) {
+    const int n = orsp::lat_walk_warp(p.geom, B, p.w4, dget, at_src, x, y, z, nodes, p.path_cap);
+    if (lane == 0) s_len = n;
+  }
+  __syncthreads();
+  const int len = s_len;
+  if (len <= 0) {
+    if (lane == 0) p.path_len[k] = len == 0 ? 0 : len == -1 ? ST_PATHCAP : ST_INTERNAL;
     return;
   }
-  for (int i = lane; i < len / 2; i += 32) {
-    const int32_t a = nodes[i], zz = nodes[len - 1 - i];
-    nodes[i] = zz;
-    nodes[len - 1 - i] = a;
-  }
-  __syncwarp();
   if (edges) {
-    for (int i = lane; i < len - 1; i += 32) {
-      const int32_t u = nodes[i], w = nodes[i + 1];
-      const int64_t plane = (int64_t)p.geom.nx * p.geom.ny;
-      const int64_t zu = u / plane, zw = w / plane;
-      if (p.vcol_eid && zu != zw)  // a column via: the first CSR edge u -> w (the smaller id)
-        edges[i] = __ldg(&p.vcol_eid[zu * p.N + w]);
-      else
-        edges[i] = __ldg(&p.slot_eid[(int64_t)orsp::lat_edge_slot(p.geom, u, w) * p.N + w]);
-    }
+    for (int i = lane; i < len - 1; i += blockDim.x)
+      edges[i] = orsp::lat_step_edge(p.geom, p.slot_eid, p.vcol_eid, p.N, nodes[len - 1 - i], nodes[len - 2 - i]);
+    __syncthreads();
   }
-  __syncwarp();
+  orsp::lat_reverse(nodes, len);
   if (lane == 0) p.path_len[k] = len;
 }
-
 
 }  // namespace
 
@@ -727,7 +711,7 @@ int run_batch_lat(orsp_graph *g, const float *cost_d, int32_t K, const std::vect
     bt.path_len = path_len_d;
     bt.path_cap = path_cap;
     bt.search_err = opt.err_d;
-    lat_batch_backtrace_kernel<<<m, 32, 0, st>>>(bt);
+    lat_batch_backtrace_kernel<<<m, orsp::kWalkBlock, 0, st>>>(bt);
     ORSP_CUDA(cudaGetLastError());
     ORSP_CUDA(cudaStreamSynchronize(st));
     a = b;

@@ -35,12 +35,15 @@
 namespace {
 
 using orsp::apply_usage;
-using orsp::lat_edge_slot;
+using orsp::kWalkBlock;
+using orsp::lat_reverse;
+using orsp::lat_step_edge;
 using orsp::lat_walk_warp;
 using orsp::lat_xyz;
 using orsp::LatBox;
 using orsp::LatWalkGeom;
 using orsp::live_cost;
+using orsp::live_cost_of;
 
 struct LiveParams {
   int32_t *usage;
@@ -51,12 +54,21 @@ struct LiveParams {
   float *cost;
 };
 
-// Steps 1 and 4 for the nets of one group: block j takes net order[j], the
-// len-1 edges of its row, usage +-1 and live costs.  mode 0: both per edge
-// (the edges of a shortest path are distinct and the group's boxes are
-// disjoint, so each edge is handled by one thread); 1: usage only; 2: live
-// costs only, launched after the usage pass of a group whose paths may share
-// edges, so that every edge's cost is computed from its final usage.
+// Usage +-1 on edge e and its live cost from the usage left, where no other
+// thread of the launch takes the same edge: one round trip, the usage comes
+// back with the atomic.
+__device__ __forceinline__ void use_edge(const LiveParams &lp, int32_t e, int32_t sign) {
+  const float base = lp.base[e], capa = lp.capa[e], hist = lp.hist[e];
+  const int32_t left = apply_usage(lp.usage, lp.present, e, sign);
+  lp.cost[e] = live_cost_of(e, base, left, capa, hist, lp.pres_fac, lp.hist_w, lp.via_mult, lp.base_w, lp.jitter);
+}
+
+// Step 1 for the nets of one group (block j takes net order[j], the len-1
+// edges of its row), and the cost pass of snapshot groups.  mode 0: usage and
+// live cost per edge (the edges of a shortest path are distinct and the group's
+// boxes are disjoint, so each edge is handled by one thread); 1: usage only;
+// 2: live costs only, launched after the usage pass of a group whose paths may
+// share edges, so that every edge's cost is computed from its final usage.
 // active (NULL: every net) skips net order[j] when active[j] == 0.
 __global__ void route_commit_kernel(const int32_t *order, const int32_t *edges, const int32_t *lens, int32_t cap,
                                     int32_t sign, int32_t mode, const int32_t *active, LiveParams lp) {
@@ -69,8 +81,9 @@ __global__ void route_commit_kernel(const int32_t *order, const int32_t *edges, 
   for (int32_t i = threadIdx.x; i < ne; i += blockDim.x) {
     const int32_t e = row[i];
     if (e < 0) continue;
-    if (mode != 2) apply_usage(lp.usage, lp.present, e, sign);
-    if (mode != 1)
+    if (mode == 0) use_edge(lp, e, sign);
+    else if (mode == 1) apply_usage(lp.usage, lp.present, e, sign);
+    else
       lp.cost[e] = live_cost(e, lp.base, lp.usage, lp.capa, lp.hist, lp.pres_fac, lp.hist_w, lp.via_mult,
                              lp.base_w, lp.jitter);
   }
@@ -78,31 +91,20 @@ __global__ void route_commit_kernel(const int32_t *order, const int32_t *edges, 
 
 // Snapshot groups: after a round, the nets whose new path uses an edge that
 // a net earlier in the group (smaller j) of the same round also uses.  The
-// three steps are separate launches: every mark lands before any test reads
-// it, and every test reads before the reset.
+// three steps ride on launches that the round makes anyway, each after the
+// other: the mark on the backtrace, the test on the cost pass and the reset on
+// the next round's rip-up, so every mark lands before any test reads it, and
+// every test reads before the reset.
 constexpr int32_t kOwnerFree = 0x7f7f7f7f;  // byte fill of the owner array
 
-// mark: owner[e] = the smallest j of the round's nets whose path holds e
-__global__ void snap_mark_kernel(const int32_t *order, const int32_t *edges, const int32_t *lens, int32_t cap,
-                                 const int32_t *active, int32_t *owner) {
-  const int32_t j = blockIdx.x;
-  if (active && !active[j]) return;
-  const int32_t k = order[j], len = lens[k];
-  if (len < 2) return;
-  const int32_t ne = min(len - 1, cap);
-  const int32_t *row = edges + (int64_t)k * cap;
-  for (int32_t i = threadIdx.x; i < ne; i += blockDim.x) {
-    const int32_t e = row[i];
-    if (e >= 0) atomicMin(&owner[e], j);
-  }
-}
-
-// test: next[j] = 1 (and seeds[j] = the net's source) when an edge of net j
-// is held by an earlier net of the round; 0 (seeds[j] = -1) otherwise.
-// searches counts the nets flagged.
+// Live costs of the round's new paths (their usage is final), and the test:
+// next[j] = 1 (and seeds[j] = the net's source) when an edge of net j is held
+// by an earlier net of the round; 0 (seeds[j] = -1) otherwise.  owner[e] is
+// the smallest j of the round's nets whose path holds e.  searches counts the
+// nets flagged.
 __global__ void snap_test_kernel(const int32_t *order, const int32_t *edges, const int32_t *lens, int32_t cap,
                                  const int32_t *active, const int32_t *owner, const int32_t *src, int32_t *next,
-                                 int32_t *seeds, unsigned long long *searches) {
+                                 int32_t *seeds, unsigned long long *searches, LiveParams lp) {
   __shared__ int hit;
   const int32_t j = blockIdx.x;
   if (threadIdx.x == 0) hit = 0;
@@ -114,7 +116,10 @@ __global__ void snap_test_kernel(const int32_t *order, const int32_t *edges, con
     const int32_t *row = edges + (int64_t)k * cap;
     for (int32_t i = threadIdx.x; i < ne; i += blockDim.x) {
       const int32_t e = row[i];
-      if (e >= 0 && __ldcg(&owner[e]) < j) atomicOr(&hit, 1);
+      if (e < 0) continue;
+      lp.cost[e] = live_cost(e, lp.base, lp.usage, lp.capa, lp.hist, lp.pres_fac, lp.hist_w, lp.via_mult,
+                             lp.base_w, lp.jitter);
+      if (__ldcg(&owner[e]) < j) atomicOr(&hit, 1);
     }
   }
   __syncthreads();
@@ -126,18 +131,23 @@ __global__ void snap_test_kernel(const int32_t *order, const int32_t *edges, con
   }
 }
 
-// reset: the round's edges back to kOwnerFree
-__global__ void snap_reset_kernel(const int32_t *order, const int32_t *edges, const int32_t *lens, int32_t cap,
-                                  const int32_t *active, int32_t *owner) {
+// The last round's edges back to kOwnerFree (nets with was[j] != 0, NULL: all),
+// and the rip-up of the nets that its test flagged (now[j] != 0, NULL: none):
+// usage -1 on the same rows.
+__global__ void snap_next_kernel(const int32_t *order, const int32_t *edges, const int32_t *lens, int32_t cap,
+                                 const int32_t *was, const int32_t *now, int32_t *owner, LiveParams lp) {
   const int32_t j = blockIdx.x;
-  if (active && !active[j]) return;
+  if (was && !was[j]) return;  // a flagged net was in the round
+  const bool rip = now && now[j];
   const int32_t k = order[j], len = lens[k];
   if (len < 2) return;
   const int32_t ne = min(len - 1, cap);
   const int32_t *row = edges + (int64_t)k * cap;
   for (int32_t i = threadIdx.x; i < ne; i += blockDim.x) {
     const int32_t e = row[i];
-    if (e >= 0) owner[e] = kOwnerFree;
+    if (e < 0) continue;
+    owner[e] = kOwnerFree;
+    if (rip) apply_usage(lp.usage, lp.present, e, -1);
   }
 }
 
@@ -156,19 +166,24 @@ struct RouteBt {
   int32_t cap;
   const int *search_err;  // the group search's error word
   int *route_err;
+  bool shared;     // snapshot groups: nets may share edges, so only the usage is counted here
+  int32_t *owner;  // snapshot groups with another round to come: marks of the edges used
+  LiveParams lp;
 };
 
-// Step 3, one warp per net of the group (block j: net order[j]).  The warp
-// walks from the target to the source with lat_walk_warp (the parent rule of
+// Steps 3 and 4, one block per net of the group (block j: net order[j]).  Warp
+// 0 walks from the target to the source with lat_walk_warp (the parent rule of
 // orsp_sssp, rank = node id = box-local order); the source (distance 0) ends
 // the walk.  The walk never leaves the box: with shared distances the nodes
 // outside it hold distances of other boxes or of earlier searches, and a box
-// with its own slice (dbase >= 0) has distances for its cells only.  Then the lanes reverse
-// the path and map each step u -> v to its CSR edge, the in-edge of v in the
-// slot that u occupies (the lattice has no parallel edges, so this is the
-// first CSR edge u -> v of path_to_edges).
-__global__ void route_backtrace_kernel(RouteBt p) {
-  const int lane = threadIdx.x & 31;
+// with its own slice (dbase >= 0) has distances for its cells only.  Then the
+// block maps each step u -> v to its CSR edge, the in-edge of v in the slot
+// that u occupies (the lattice has no parallel edges, so this is the first CSR
+// edge u -> v of path_to_edges), commits it and reverses the path.
+// Bound by the walk's chain of loads and by the launch: the commit as a launch
+// of its own cost 2.1 us of a 100 x 100 x 4 net's 40.
+__global__ void __launch_bounds__(kWalkBlock) route_backtrace_kernel(RouteBt p) {
+  __shared__ int s_len;
   const int j = blockIdx.x;
   if (p.active && !p.active[j]) return;
   const int32_t k = p.order[j];
@@ -178,58 +193,47 @@ __global__ void route_backtrace_kernel(RouteBt p) {
   int32_t *edges = p.net_edges + (int64_t)k * p.cap;
   int32_t *len_out = p.net_lens + k;
   const int serr = *p.search_err;
-  if (serr) {
-    if (lane == 0) {
-      atomicCAS(p.route_err, DEV_OK, serr);
-      *len_out = 0;
+  if (threadIdx.x < 32) {
+    int len = 0;
+    if (!serr) {
+      int32_t x, y, z;
+      lat_xyz(p.geom, dst, x, y, z);
+      const bool dst_in = x >= B.x0 && x <= B.x1 && y >= B.y0 && y <= B.y1 && z >= B.z0 && z <= B.z1;
+      // distances: by node id, or box-local rows of the box's own slice
+      const bool own = B.dbase >= 0;
+      const uint32_t *dist = own ? p.dist + B.dbase : p.dist;
+      const int32_t rx = own ? B.x1 - B.x0 + 1 : p.geom.nx, ry = own ? B.y1 - B.y0 + 1 : p.geom.ny;
+      const int32_t ox = own ? B.x0 : 0, oy = own ? B.y0 : 0, oz = own ? B.z0 : 0;
+      auto dget = [dist, rx, ry, ox, oy, oz](int32_t a, int32_t b, int32_t c) {
+        return __ldcg(&dist[((int64_t)(c - oz) * ry + (b - oy)) * rx + (a - ox)]);
+      };
+      if (src >= 0 && dst_in && dst != src) {
+        auto at_src = [src](int64_t v, unsigned d) { return v == src && d == 0u; };
+        len = lat_walk_warp(p.geom, B, p.w4, dget, at_src, x, y, z, nodes, p.cap);
+      }
     }
-    return;
-  }
-  int len = 0, err = 0;
-  int32_t x, y, z;
-  lat_xyz(p.geom, dst, x, y, z);
-  const bool dst_in = x >= B.x0 && x <= B.x1 && y >= B.y0 && y <= B.y1 && z >= B.z0 && z <= B.z1;
-  // distances: by node id, or box-local rows of the box's own slice
-  const bool own = B.dbase >= 0;
-  const uint32_t *dist = own ? p.dist + B.dbase : p.dist;
-  const int32_t rx = own ? B.x1 - B.x0 + 1 : p.geom.nx, ry = own ? B.y1 - B.y0 + 1 : p.geom.ny;
-  const int32_t ox = own ? B.x0 : 0, oy = own ? B.y0 : 0, oz = own ? B.z0 : 0;
-  auto dget = [dist, rx, ry, ox, oy, oz](int32_t a, int32_t b, int32_t c) {
-    return __ldcg(&dist[((int64_t)(c - oz) * ry + (b - oy)) * rx + (a - ox)]);
-  };
-  const unsigned dv = (src >= 0 && dst_in) ? dget(x, y, z) : ORSP_INF_BITS;
-  if (dv != ORSP_INF_BITS && dst != src) {
-    auto at_src = [src](int64_t v, unsigned d) { return v == src && d == 0u; };
-    len = lat_walk_warp(p.geom, B, p.w4, dget, at_src, x, y, z, dv, nodes, p.cap);
-    if (len == -1) err = DEV_ERR_PATH_OVERFLOW;
-    else if (len < 0) err = DEV_ERR_INTERNAL;
-    if (err) len = 0;
-  }
-  __syncwarp();
-  if (err) {
-    if (lane == 0) {
-      atomicCAS(p.route_err, DEV_OK, err);
-      *len_out = 0;
+    if (threadIdx.x == 0) {
+      s_len = max(len, 0);
+      const int err = serr ? serr : len == -1 ? DEV_ERR_PATH_OVERFLOW : len < 0 ? DEV_ERR_INTERNAL : 0;
+      if (err) atomicCAS(p.route_err, DEV_OK, err);
+      *len_out = max(len, 0);
     }
-    return;
   }
-  for (int i = lane; i < len / 2; i += 32) {
-    const int a = nodes[i], z = nodes[len - 1 - i];
-    nodes[i] = z;
-    nodes[len - 1 - i] = a;
+  __syncthreads();
+  const int len = s_len;
+  for (int i = threadIdx.x; i < len - 1; i += blockDim.x) {
+    const int32_t e = lat_step_edge(p.geom, p.slot_eid, p.vcol_eid, p.N, nodes[len - 1 - i], nodes[len - 2 - i]);
+    edges[i] = e;
+    if (e < 0) continue;
+    if (!p.shared) {
+      use_edge(p.lp, e, 1);
+    } else {
+      apply_usage(p.lp.usage, p.lp.present, e, 1);
+      if (p.owner) atomicMin(&p.owner[e], j);
+    }
   }
-  __syncwarp();
-  for (int i = lane; i < len - 1; i += 32) {
-    const int32_t u = nodes[i], w = nodes[i + 1];
-    const int64_t plane = (int64_t)p.geom.nx * p.geom.ny;
-    const int64_t zu = u / plane, zw = w / plane;
-    if (p.vcol_eid && zu != zw)  // a column via: the first CSR edge u -> w (the smaller id)
-      edges[i] = __ldg(&p.vcol_eid[zu * p.N + w]);
-    else
-      edges[i] = __ldg(&p.slot_eid[(int64_t)lat_edge_slot(p.geom, u, w) * p.N + w]);
-  }
-  __syncwarp();
-  if (lane == 0) *len_out = len;
+  __syncthreads();
+  lat_reverse(nodes, len);
 }
 
 bool box_ok(const orsp::Graph *g, const int32_t *b) {
@@ -413,8 +417,13 @@ static int route_nets_impl(orsp_graph *g, int32_t M, const int32_t *src_h, const
     int32_t *seeds = g->route_flags + 2 * kMaxGroup;
     const int32_t *act = nullptr;
     const int32_t *seed_r = d_src + a;
+    const int32_t *was = nullptr;  // the nets of the round before
     for (int32_t r = 0; r <= repair; ++r) {
-      route_commit_kernel<<<n, 256, 0, st>>>(d_order + a, net_edges_d, net_lens_d, path_cap, -1, 1, act, lp);
+      if (r == 0)
+        route_commit_kernel<<<n, 256, 0, st>>>(d_order + a, net_edges_d, net_lens_d, path_cap, -1, 1, nullptr, lp);
+      else
+        snap_next_kernel<<<n, 256, 0, st>>>(d_order + a, net_edges_d, net_lens_d, path_cap, was, act,
+                                            g->route_owner, lp);
       ORSP_CUDA(cudaGetLastError());
       route_commit_kernel<<<n, 256, 0, st>>>(d_order + a, net_edges_d, net_lens_d, path_cap, -1, 2, act, lp);
       ORSP_CUDA(cudaGetLastError());
@@ -444,21 +453,21 @@ static int route_nets_impl(orsp_graph *g, int32_t M, const int32_t *src_h, const
       bt.cap = path_cap;
       bt.search_err = opt.err_d;
       bt.route_err = route_err;
-      route_backtrace_kernel<<<n, 32, 0, st>>>(bt);
+      bt.shared = true;
+      bt.owner = r < repair ? g->route_owner : nullptr;
+      bt.lp = lp;
+      route_backtrace_kernel<<<n, kWalkBlock, 0, st>>>(bt);
       ORSP_CUDA(cudaGetLastError());
-      route_commit_kernel<<<n, 256, 0, st>>>(d_order + a, net_edges_d, net_lens_d, path_cap, 1, 1, act, lp);
-      ORSP_CUDA(cudaGetLastError());
-      route_commit_kernel<<<n, 256, 0, st>>>(d_order + a, net_edges_d, net_lens_d, path_cap, 1, 2, act, lp);
-      ORSP_CUDA(cudaGetLastError());
-      if (r == repair) break;
+      if (r == repair) {
+        route_commit_kernel<<<n, 256, 0, st>>>(d_order + a, net_edges_d, net_lens_d, path_cap, 1, 2, act, lp);
+        ORSP_CUDA(cudaGetLastError());
+        break;
+      }
       int32_t *next = flags[r & 1];
-      snap_mark_kernel<<<n, 256, 0, st>>>(d_order + a, net_edges_d, net_lens_d, path_cap, act, g->route_owner);
-      ORSP_CUDA(cudaGetLastError());
       snap_test_kernel<<<n, 256, 0, st>>>(d_order + a, net_edges_d, net_lens_d, path_cap, act, g->route_owner,
-                                          d_src + a, next, seeds, repair_count);
+                                          d_src + a, next, seeds, repair_count, lp);
       ORSP_CUDA(cudaGetLastError());
-      snap_reset_kernel<<<n, 256, 0, st>>>(d_order + a, net_edges_d, net_lens_d, path_cap, act, g->route_owner);
-      ORSP_CUDA(cudaGetLastError());
+      was = act;
       act = next;
       seed_r = seeds;
     }
@@ -495,9 +504,8 @@ static int route_nets_impl(orsp_graph *g, int32_t M, const int32_t *src_h, const
     bt.cap = path_cap;
     bt.search_err = opt.err_d;
     bt.route_err = route_err;
-    route_backtrace_kernel<<<n, 32, 0, st>>>(bt);
-    ORSP_CUDA(cudaGetLastError());
-    route_commit_kernel<<<n, 256, 0, st>>>(d_order + a, net_edges_d, net_lens_d, path_cap, 1, 0, nullptr, lp);
+    bt.lp = lp;
+    route_backtrace_kernel<<<n, kWalkBlock, 0, st>>>(bt);
     ORSP_CUDA(cudaGetLastError());
     return rc;
   };

@@ -345,7 +345,7 @@ __global__ void backtrace_kernel(BacktraceParams p) {
 }
 
 // The same walk on a recognised H/V lattice after a tile-sweep search inside
-// box B: lat_walk_warp, up to 32 nodes of a straight run per memory round
+// box B: lat_walk_warp, one run of the path per memory round
 // trip (ranks are node ids, as in the tile-sweep search).
 using orsp::lat_walk_warp;
 using orsp::lat_xyz;
@@ -368,22 +368,17 @@ struct LatBacktraceParams {
   SsspCtl *ctl;
 };
 
-__global__ void lat_backtrace_kernel(LatBacktraceParams p) {
-  const int lane = threadIdx.x & 31;
+__global__ void __launch_bounds__(orsp::kWalkBlock) lat_backtrace_kernel(LatBacktraceParams p) {
+  __shared__ int s_len;
   SsspCtl *ctl = p.ctl;
   if (ctl->err) return;
   const LatBox &B = p.box;
   const int32_t dst = p.dst_d ? *p.dst_d : p.dst;
-  if (dst < 0) {
-    if (lane == 0) { ctl->path_len = 0; ctl->status = 1; }
-    return;
-  }
-  int32_t x, y, z;
-  lat_xyz(p.geom, dst, x, y, z);
+  int32_t x = -1, y = 0, z = 0;
+  if (dst >= 0) lat_xyz(p.geom, dst, x, y, z);
   const bool in = x >= B.x0 && x <= B.x1 && y >= B.y0 && y <= B.y1 && z >= B.z0 && z <= B.z1;
-  unsigned dv = in ? __ldcg(&p.dist[dst]) : ORSP_INF_BITS;
-  if (dv == ORSP_INF_BITS) {
-    if (lane == 0) { ctl->path_len = 0; ctl->status = 1; }
+  if (dst < 0 || !in) {
+    if (threadIdx.x == 0) { ctl->path_len = 0; ctl->status = 1; }
     return;
   }
   const uint32_t *dist = p.dist;
@@ -396,29 +391,26 @@ __global__ void lat_backtrace_kernel(LatBacktraceParams p) {
   const int32_t nseeds = p.nseeds;
   // a seed whose distance still equals its start cost ends the walk
   auto at_start = [seeds, seed_cost, nseeds](int64_t v, unsigned d) {
-    for (int i = 0; i < nseeds; ++i)
-      if (seeds[i] == v && f_bits(seed_cost ? seed_cost[i] : 0.0f) == d) return true;
-    return false;
+    bool hit = false;
+#pragma unroll 4
+    for (int i = 0; i < nseeds; ++i) hit |= seeds[i] == v && f_bits(seed_cost ? seed_cost[i] : 0.0f) == d;
+    return hit;
   };
-  int len;
-  if (p.rank_map) len = lat_walk_warp(p.geom, B, p.w4, dget, at_start, x, y, z, dv, p.path_out, p.path_cap,
-                                      orsp::LatRankRoi{p.rank_map});
-  else len = lat_walk_warp(p.geom, B, p.w4, dget, at_start, x, y, z, dv, p.path_out, p.path_cap);
-  int err = 0;
-  if (len == -1) err = DEV_ERR_PATH_OVERFLOW;
-  else if (len < 0) err = DEV_ERR_INTERNAL;
-  __syncwarp();
-  if (err) {
-    if (lane == 0) atomicCAS(&ctl->err, DEV_OK, err);
+  if (threadIdx.x < 32) {
+    int len;
+    if (p.rank_map) len = lat_walk_warp(p.geom, B, p.w4, dget, at_start, x, y, z, p.path_out, p.path_cap,
+                                        orsp::LatRankRoi{p.rank_map});
+    else len = lat_walk_warp(p.geom, B, p.w4, dget, at_start, x, y, z, p.path_out, p.path_cap);
+    if (threadIdx.x == 0) s_len = len;
+  }
+  __syncthreads();
+  const int len = s_len;
+  if (len < 0) {
+    if (threadIdx.x == 0) atomicCAS(&ctl->err, DEV_OK, len == -1 ? DEV_ERR_PATH_OVERFLOW : DEV_ERR_INTERNAL);
     return;
   }
-  for (int i = lane; i < len / 2; i += 32) {
-    const int a = p.path_out[i];
-    const int zz = p.path_out[len - 1 - i];
-    p.path_out[i] = zz;
-    p.path_out[len - 1 - i] = a;
-  }
-  if (lane == 0) { ctl->path_len = len; ctl->status = 0; }
+  orsp::lat_reverse(p.path_out, len);
+  if (threadIdx.x == 0) { ctl->path_len = len; ctl->status = len ? 0 : 1; }
 }
 
 // Multi-sink winner, as find_path_multisource_multisink (UPF:1941-1975): the
@@ -694,7 +686,7 @@ static int sssp_impl(orsp_graph *g, const float *cost_d, int32_t nseeds, const i
     b.path_out = path_out_d;
     b.path_cap = path_cap;
     b.ctl = (SsspCtl *)g->ctl;
-    lat_backtrace_kernel<<<1, 32, 0, st>>>(b);
+    lat_backtrace_kernel<<<1, orsp::kWalkBlock, 0, st>>>(b);
     ORSP_CUDA(cudaGetLastError());
   } else if (dst >= 0) {
     BacktraceParams b{};
@@ -822,7 +814,7 @@ extern "C" int orsp_sssp_roi_nodes(orsp_graph *g, const float *cost_d, int32_t s
     ORSP_CUDA(cudaMemsetAsync(g->ctl, 0, sizeof(SsspCtl), st));
     LatBacktraceParams b = lat_bt_full(g, g->dist, g->seed_one, nullptr, 1, dst, nullptr, g->roi_map, path_out_d,
                                        path_cap);
-    lat_backtrace_kernel<<<1, 32, 0, st>>>(b);
+    lat_backtrace_kernel<<<1, orsp::kWalkBlock, 0, st>>>(b);
     ORSP_CUDA(cudaGetLastError());
   } else if (use_roi_cta(n_roi)) {
     // one CTA: block-local near-far rounds over ROI-local distances
@@ -945,7 +937,7 @@ extern "C" int orsp_sssp_multi(orsp_graph *g, const float *cost_d, int32_t nseed
     ORSP_CUDA(cudaGetLastError());
     LatBacktraceParams b = lat_bt_full(g, g->dist, seeds_d, seed_cost_d, nseeds, -1, best_l, roi_map_d, path_out_d,
                                        path_cap);
-    lat_backtrace_kernel<<<1, 32, 0, st>>>(b);
+    lat_backtrace_kernel<<<1, orsp::kWalkBlock, 0, st>>>(b);
     ORSP_CUDA(cudaGetLastError());
     mark_kernel<<<mblocks, 256, 0, st>>>(g->sink_mask, ntargets, targets_d, g->N, 0);
     ORSP_CUDA(cudaGetLastError());

@@ -62,7 +62,7 @@ struct LatCtl {
   unsigned long long cycles;
   unsigned head, tail;  // tile queue positions (asynchronous schedule)
   int pending;          // tiles queued or being visited
-  unsigned pad;
+  int avail;            // visiting owners: queued tiles less the CTAs waiting for one
   unsigned long long ns[4];  // time in load, sweeps, write-back, scheduling (sum over visits)
 };
 
@@ -94,6 +94,7 @@ struct LatParams {
   uint64_t hmask, vmask;
   int8_t hlist[64], vlist[64];
   const int32_t *tbox;  // box of each tile (asynchronous schedule)
+  unsigned *inbox;      // messages to each tile (visiting owners; else NULL)
 };
 
 __global__ void fill_kernel(uint32_t *p, int64_t n, uint32_t v) {
@@ -403,14 +404,19 @@ __device__ __forceinline__ int tile_of(const LatBox &B, int32_t gx, int32_t gy) 
   return B.tile0 + ((gy - B.y0) / TY) * B.ntx + (gx - B.x0) / TX;
 }
 
-// Asynchronous schedule: every tile idle, the queue empty, each tile's box.
-__global__ void lattice_init_kernel(LatParams p, int32_t ntiles) {
+// Asynchronous schedule: every tile idle, the queue empty, each tile's box
+// (and, for visiting owners, no messages and the exchange rows at +inf).
+__global__ void lattice_init_kernel(LatParams p, int32_t ntiles, unsigned *got, float4 *rows, int64_t nrows) {
   const int64_t s = (int64_t)gridDim.x * blockDim.x;
+  const float INF_F = __int_as_float(0x7f800000);
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nrows; i += s)
+    rows[i] = make_float4(INF_F, INF_F, INF_F, INF_F);
   const int64_t n = max((int64_t)ntiles, (int64_t)p.qcap);
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += s) {
     if (i < ntiles) {
       p.tstate[i] = 0;
       p.stamp[i] = 0;
+      if (p.inbox) p.inbox[i] = got[i] = 0;
       p.list0[i] = p.nbox == 1 ? 0 : box_of_tile(p, (int)i);
     }
     if (i < p.qcap) p.qslot[i] = -1;
@@ -432,6 +438,7 @@ __global__ void lattice_seed_kernel(LatParams p, int32_t nseeds, const int32_t *
     c->head = 0;
     c->tail = 0;
     c->pending = 0;
+    c->avail = 0;
     for (int i = 0; i < 4; ++i) c->ns[i] = 0;
   }
   __syncthreads();
@@ -471,7 +478,15 @@ __global__ void lattice_seed_kernel(LatParams p, int32_t nseeds, const int32_t *
     for (int j = 0; j < 5; ++j) {
       const int q = nb[j];
       if (q < 0) continue;
-      if (p.qslot) {
+      if (p.inbox) {
+        // a message for the seed's tile; its neighbours are only taken early
+        if (j == 0 && atomicExch(&p.inbox[q], 1u) == 0u) atomicAdd(&c->pending, 1);
+        if (atomicCAS(&p.tstate[q], 0, 1) == 0) {
+          atomicAdd(&c->avail, 1);
+          const unsigned k = atomicAdd(&c->tail, 1u);
+          atomicExch(&p.qslot[k % p.qcap], q);
+        }
+      } else if (p.qslot) {
         if (atomicCAS(&p.tstate[q], 0, 1) == 0) {
           atomicAdd(&c->pending, 1);
           const unsigned k = atomicAdd(&c->tail, 1u);
@@ -1553,6 +1568,124 @@ __device__ __forceinline__ void st_relaxed_f32(float *p, float v) {
   asm volatile("st.relaxed.gpu.global.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
 }
 
+// What the workers and the helper warp of an owner share.
+struct OwnShared {
+  volatile unsigned req, ack;  // inbox count to deal with, last one dealt with
+  int pub[4];                  // sides with publications not yet sent as messages
+  volatile int stop, rel;      // the search is over; the tile is given back once it is idle
+  volatile int idle, out;      // no work at the last look; the tile's distances are written
+  int tile;
+  LatBox box;
+};
+
+// The cycles of an owned tile, from the halo values na / nb until it is idle
+// and asked to stop.  pa / pb: the boundary values last published; snap: the
+// inbox count read before na and nb.  Returns the number of cycles.
+template <int NZM, bool CV, bool ZS>
+__device__ __forceinline__ unsigned own_cycles(const OwnParams &o, const LatBox &B, const RunGeom &G,
+                                               const RunTile<NZM, ZS> &R, RunShared &S, OwnShared &Q, float *sd,
+                                               const float2 *wz, float *ex, float na, float nb, float pa, float pb,
+                                               bool dirty, bool all, unsigned snap) {
+  constexpr int NW = RunTile<NZM, ZS>::NW, WS = kRunWS, PS = kRunPS;
+  const float INF_F = __int_as_float(0x7f800000);
+  const LatParams &p = o.l;
+  const int tid = threadIdx.x;
+  const bool run = G.run, col = G.col;
+  // the neighbours' exchange values that this thread's run writes
+  const int step = (G.isv ? B.ntx : 1) * 2 * o.nr;
+  const bool lo = run && (G.isv ? G.ty > 0 : G.tx > 0), hi = run && (G.isv ? G.ty < B.nty - 1 : G.tx < B.ntx - 1);
+  float ha = INF_F, hb = INF_F;  // halo values taken
+  bool again = false, idle = false;
+  unsigned cycles = 0;
+  float *const cd = sd + G.yy * WS + G.xx;
+  const float2 *const cw = wz + G.yy * WS + G.xx;
+  for (int k = 0;; k ^= 1) {
+    // ---- halo values read since the last look
+    unsigned next_snap = 0;
+    if (na < ha) ha = na, dirty = true;
+    if (nb < hb) hb = nb, dirty = true;
+    if (idle) {  // nothing to do at the last look
+      const bool stop = Q.stop != 0 || Q.rel != 0;
+      if (!tile_sync_or<NW, true>(dirty || stop)) {
+        if (tid == 0) {
+          Q.ack = snap;
+          Q.idle = 1;
+          snap = Q.req;
+        }
+        tile_sync<NW, true>();
+        if (run) na = ld_relaxed_f32(ex), nb = ld_relaxed_f32(ex + o.nr);
+        continue;
+      }
+      if (!tile_sync_or<NW, true>(dirty)) break;
+      idle = false;
+      if (tid == 0) Q.idle = 0;
+    }
+    // ---- planar pass, boundary improvements published
+    unsigned m = 0;
+    if (dirty) {
+      auto pass = [&](float *c, auto stride) {
+        constexpr int DS = decltype(stride)::value;
+        m = walk_both<16>(
+            ha, hb, [&](int i) { return c[i * DS]; }, [&](int i) { return R.lo[i]; }, [&](int i) { return R.hi[i]; },
+            [&](int i, float v) { c[i * DS] = v; });
+        const float v0 = c[0], v1 = c[15 * DS];
+        if (lo && v0 < pa) {
+          pa = v0;
+          st_relaxed_f32(ex - step + o.nr, v0);
+          __threadfence_block();
+          Q.pub[G.isv ? 2 : 0] = 1;
+        }
+        if (hi && v1 < pb) {
+          pb = v1;
+          st_relaxed_f32(ex + step, v1);
+          __threadfence_block();
+          Q.pub[G.isv ? 3 : 1] = 1;
+        }
+      };
+      if (G.isv) {
+        pass(sd + G.rbase, std::integral_constant<int, WS>());
+        if (m) atomicOr(&S.coly[k][G.rl], m);
+      } else {
+        pass(sd + G.rbase, std::integral_constant<int, 1>());
+        if (m) atomicOr(&S.rowx[k][G.rl], m);
+      }
+    }
+    if (tid == 0) next_snap = Q.req;
+    const bool any = tile_sync_or<NW, true>(m != 0 || again);
+    // the next cycle's halo values; their round trip overlaps the via pass
+    if (run) na = ld_relaxed_f32(ex), nb = ld_relaxed_f32(ex + o.nr);
+    // ---- via pass
+    unsigned mz = 0;
+    if ((any || all) && col && (all || again || (((S.rowx[k][G.yy] >> G.xx) | (S.coly[k][G.xx] >> G.yy)) & 1u))) {
+      if constexpr (CV) mz = (unsigned)zcol_pass<PS>(cd, p.wcol, p.nzp, G.n0, (int64_t)p.nx * p.ny, G.z0, G.nzb);
+      else
+        mz = walk_both<NZM>(
+            INF_F, INF_F, [&](int z) { return z < G.nzb ? cd[z * PS] : INF_F; },
+            [&](int z) { return ZS ? (z < G.nzb ? cw[z * PS].x : INF_F) : R.dn[ZS ? 0 : z]; },
+            [&](int z) { return ZS ? (z < G.nzb ? cw[z * PS].y : INF_F) : R.up[ZS ? 0 : z]; },
+            [&](int z, float v) { cd[z * PS] = v; });
+      if (mz & G.hm) atomicOr(&S.rowz[k][G.yy], mz & G.hm);
+      if (mz & G.vm) atomicOr(&S.colz[k][G.xx], mz & G.vm);
+    }
+    if (CV) again = mz != 0;
+    all = false;
+    if (tid < 16) {
+      S.rowx[k ^ 1][tid] = S.coly[k ^ 1][tid] = 0;
+      S.rowz[k ^ 1][tid] = S.colz[k ^ 1][tid] = 0;
+    }
+    const bool zany = tile_sync_or<NW, true>(mz != 0);
+    dirty = run && (((G.isv ? S.colz[k][G.rl] : S.rowz[k][G.rl]) >> G.rz) & 1u);
+    ++cycles;
+    idle = !any && !zany;
+    if (tid == 0) {
+      // a cycle without a change answers the request read before its halo loads
+      if (idle) Q.ack = snap;
+      snap = next_snap;
+    }
+  }
+  return cycles;
+}
+
 template <int NZM, bool PRIV, bool CV, bool ZS, int MINB>
 __global__ void __launch_bounds__(RunTile<NZM, ZS>::NW + 32, MINB)
     lattice_own_kernel(const __grid_constant__ OwnParams o) {
@@ -1560,20 +1693,18 @@ __global__ void __launch_bounds__(RunTile<NZM, ZS>::NW + 32, MINB)
   const float INF_F = __int_as_float(0x7f800000);
   extern __shared__ __align__(128) float sd[];
   __shared__ RunShared S;
-  __shared__ volatile unsigned s_req, s_ack;  // inbox count to deal with, last one dealt with
-  __shared__ int s_pub[4];                    // sides with publications not yet sent as messages
-  __shared__ volatile int s_stop;
+  __shared__ OwnShared Q;
   const LatParams &p = o.l;
   const int t = blockIdx.x, tid = threadIdx.x;
   // the tile's box (a box sized on the device may have fewer tiles than the launch)
   const LatBox B = load_box(p, p.nbox == 1 ? 0 : box_of_tile(p, t));
   const bool mine = t < B.tile0 + B.ntx * B.nty;
   const unsigned long long t_start = dev_globaltimer();
-  if (tid < 4) s_pub[tid] = 0;
+  if (tid < 4) Q.pub[tid] = 0;
   if (tid < 32) S.clear();
   if (tid == 0) {
-    s_req = s_ack = 0;
-    s_stop = 0;
+    Q.req = Q.ack = 0;
+    Q.stop = Q.rel = 0;
     S.start();
     S.lap(-1);
   }
@@ -1585,14 +1716,14 @@ __global__ void __launch_bounds__(RunTile<NZM, ZS>::NW + 32, MINB)
     unsigned sent = 0, got = 0, asked = 0;
     for (unsigned spins = 0;; ++spins) {
       // publications become messages: one lane per side, the sent count first
-      const bool pub = lane < 4 && atomicExch(&s_pub[lane], 0) != 0;
+      const bool pub = lane < 4 && atomicExch(&Q.pub[lane], 0) != 0;
       const unsigned pm = __ballot_sync(ORSP_FULL_MASK, pub);
-      const bool acked = asked != got && __shfl_sync(ORSP_FULL_MASK, s_ack, 0) == asked;
+      const bool acked = asked != got && __shfl_sync(ORSP_FULL_MASK, Q.ack, 0) == asked;
       if (acked) {
         // everything published up to the answer: flags raised since the
         // exchange above are part of it
         __threadfence_block();
-        const bool more = lane < 4 && atomicExch(&s_pub[lane], 0) != 0;
+        const bool more = lane < 4 && atomicExch(&Q.pub[lane], 0) != 0;
         const unsigned mm = __ballot_sync(ORSP_FULL_MASK, more);
         const unsigned both = pm | mm;
         if (both) {
@@ -1629,7 +1760,7 @@ __global__ void __launch_bounds__(RunTile<NZM, ZS>::NW + 32, MINB)
       in = __shfl_sync(ORSP_FULL_MASK, in, 0);
       if (asked == got && in != got) {
         asked = in;
-        if (lane == 0) s_req = in;
+        if (lane == 0) Q.req = in;
       }
       if (t == 0 && asked == got) {
         unsigned a = 0, b = 0;
@@ -1649,7 +1780,7 @@ __global__ void __launch_bounds__(RunTile<NZM, ZS>::NW + 32, MINB)
       }
       if (__shfl_sync(ORSP_FULL_MASK, stop, 0)) break;
     }
-    if (lane == 0) s_stop = 1;
+    if (lane == 0) Q.stop = 1;
     return;
   }
 
@@ -1673,103 +1804,16 @@ __global__ void __launch_bounds__(RunTile<NZM, ZS>::NW + 32, MINB)
   }
   seeded = tile_sync_or<NW, true>(seeded);
   if (tid == 0) S.lap(0);
-  // the neighbours' exchange values that this thread's run writes
-  const int step = (G.isv ? B.ntx : 1) * 2 * o.nr;
-  const bool lo = run && (G.isv ? G.ty > 0 : G.tx > 0), hi = run && (G.isv ? G.ty < B.nty - 1 : G.tx < B.ntx - 1);
-  float ha = INF_F, hb = INF_F;  // halo values taken
-  float pa = INF_F, pb = INF_F;  // boundary values published
-  bool dirty = run && seeded, all = seeded, again = false, idle = false;
-  unsigned snap = 0, cycles = 0;
-  float *const cd = sd + G.yy * WS + G.xx;
-  const float2 *const cw = wz + G.yy * WS + G.xx;
-  float na = INF_F, nb = INF_F;
-  for (int k = 0; mine; k ^= 1) {
-    // ---- halo values read since the last look
-    unsigned next_snap = 0;
-    if (na < ha) ha = na, dirty = true;
-    if (nb < hb) hb = nb, dirty = true;
-    if (idle) {  // nothing to do at the last look
-      const bool stop = s_stop != 0;
-      if (!tile_sync_or<NW, true>(dirty || stop)) {
-        if (tid == 0) {
-          s_ack = snap;
-          snap = s_req;
-        }
-        tile_sync<NW, true>();
-        if (run) na = ld_relaxed_f32(ex), nb = ld_relaxed_f32(ex + o.nr);
-        continue;
-      }
-      if (!tile_sync_or<NW, true>(dirty)) break;
-      idle = false;
-    }
-    // ---- planar pass, boundary improvements published
-    unsigned m = 0;
-    if (dirty) {
-      auto pass = [&](float *c, auto stride) {
-        constexpr int DS = decltype(stride)::value;
-        m = walk_both<16>(
-            ha, hb, [&](int i) { return c[i * DS]; }, [&](int i) { return R.lo[i]; }, [&](int i) { return R.hi[i]; },
-            [&](int i, float v) { c[i * DS] = v; });
-        const float v0 = c[0], v1 = c[15 * DS];
-        if (lo && v0 < pa) {
-          pa = v0;
-          st_relaxed_f32(ex - step + o.nr, v0);
-          __threadfence_block();
-          s_pub[G.isv ? 2 : 0] = 1;
-        }
-        if (hi && v1 < pb) {
-          pb = v1;
-          st_relaxed_f32(ex + step, v1);
-          __threadfence_block();
-          s_pub[G.isv ? 3 : 1] = 1;
-        }
-      };
-      if (G.isv) {
-        pass(sd + G.rbase, std::integral_constant<int, WS>());
-        if (m) atomicOr(&S.coly[k][G.rl], m);
-      } else {
-        pass(sd + G.rbase, std::integral_constant<int, 1>());
-        if (m) atomicOr(&S.rowx[k][G.rl], m);
-      }
-    }
-    if (tid == 0) next_snap = s_req;
-    const bool any = tile_sync_or<NW, true>(m != 0 || again);
-    // the next cycle's halo values; their round trip overlaps the via pass
-    if (run) na = ld_relaxed_f32(ex), nb = ld_relaxed_f32(ex + o.nr);
-    // ---- via pass
-    unsigned mz = 0;
-    if ((any || all) && col && (all || again || (((S.rowx[k][G.yy] >> G.xx) | (S.coly[k][G.xx] >> G.yy)) & 1u))) {
-      if constexpr (CV) mz = (unsigned)zcol_pass<PS>(cd, p.wcol, p.nzp, G.n0, (int64_t)p.nx * p.ny, G.z0, G.nzb);
-      else
-        mz = walk_both<NZM>(
-            INF_F, INF_F, [&](int z) { return z < G.nzb ? cd[z * PS] : INF_F; },
-            [&](int z) { return ZS ? (z < G.nzb ? cw[z * PS].x : INF_F) : R.dn[ZS ? 0 : z]; },
-            [&](int z) { return ZS ? (z < G.nzb ? cw[z * PS].y : INF_F) : R.up[ZS ? 0 : z]; },
-            [&](int z, float v) { cd[z * PS] = v; });
-      if (mz & G.hm) atomicOr(&S.rowz[k][G.yy], mz & G.hm);
-      if (mz & G.vm) atomicOr(&S.colz[k][G.xx], mz & G.vm);
-    }
-    if (CV) again = mz != 0;
-    all = false;
-    if (tid < 16) {
-      S.rowx[k ^ 1][tid] = S.coly[k ^ 1][tid] = 0;
-      S.rowz[k ^ 1][tid] = S.colz[k ^ 1][tid] = 0;
-    }
-    const bool zany = tile_sync_or<NW, true>(mz != 0);
-    dirty = run && (((G.isv ? S.colz[k][G.rl] : S.rowz[k][G.rl]) >> G.rz) & 1u);
-    ++cycles;
-    idle = !any && !zany;
-    if (tid == 0) {
-      // a cycle without a change answers the request read before its halo loads
-      if (idle) s_ack = snap;
-      snap = next_snap;
-    }
-  }
+  unsigned cycles = 0;
+  if (mine)
+    cycles = own_cycles<NZM, CV, ZS>(o, B, G, R, S, Q, sd, wz, ex, INF_F, INF_F, INF_F, INF_F, run && seeded, seeded,
+                                     0u);
   // ---- the box's distances
   tile_sync<NW, true>();
   if (col) {
     const int64_t dz = (!PRIV || B.dbase < 0) ? (int64_t)p.nx * p.ny : (int64_t)(B.x1 - B.x0 + 1) * (B.y1 - B.y0 + 1);
     const int64_t d0 = dist_index<PRIV>(p, B, G.X0 + G.xx, G.Y0 + G.yy, B.z0);
+    const float *const cd = sd + G.yy * kRunWS + G.xx;
     for (int z = 0; z < G.nzb; ++z) p.dist[d0 + z * dz] = f_bits(cd[z * PS]);
   }
   if (tid == 0 && mine) {
@@ -1778,6 +1822,252 @@ __global__ void __launch_bounds__(RunTile<NZM, ZS>::NW + 32, MINB)
     atomicAdd(&p.ctl->visits, 1u);
     S.flush(p.ctl);
   }
+}
+
+// Visiting owners: launches with more tiles than resident CTAs and wave fronts
+// that do not fill the chip.  Like the owners' bound by the chain of hops along
+// the front, but a tile has an owner only while the front is near it: a CTA
+// takes a tile from the queue, owns it as above - distances in shared memory,
+// weights in registers, boundary values exchanged while it works - until it is
+// idle and CTAs are short, writes its distances and takes the next.
+//
+// tstate: 0 never owned, 1 queued, 2 owned, 4 given back.  `pending` counts
+// messages not dealt with: a helper raises it before it sends and lowers it by
+// what its workers have dealt with, after it has sent what they published
+// meanwhile, so it reaches 0 only at the fixpoint.  A message to a tile that no
+// CTA owns queues the tile.  The owner stores its count and leaves state 2
+// before it looks at the inbox for the last time, and a sender raises the inbox
+// before it looks at the state, so no message is lost between the two.
+//
+// A CTA without a tile takes a place in the queue (head) and waits for it to be
+// filled.  `avail` is the queued tiles less the CTAs that wait; owners of idle
+// tiles give them up until kFreeCtas CTAs wait, so a tile that the front
+// reaches is taken at once.  (Each takes its place by lowering avail, and puts
+// it back where others were first; a compare-and-swap on head let through 0.7
+// tiles per us.)  Where CTAs wait, a tile's first message queues its
+// neighbours too, before the front reaches them: their weights are on chip when
+// it does.  Each tile is taken about once, where the queue schedule visits it
+// 4 to 5 times.
+//
+// Measured, whole search, queue schedule -> visiting owners: 600 x 600 x 12
+// 750 -> 540 us (kFreeCtas 0: 760, 16: 570, 64: 540; without the early
+// neighbours 560; one CTA per SM 610), 1000 x 1000 x 12 1.62 -> 0.95 ms, 400 x
+// 400 x 5 with column vias 620 -> 380 us.
+constexpr int kFreeCtas = 32;
+template <int NZM, bool PRIV, bool CV>
+__global__ void __launch_bounds__(RunTile<NZM, true>::NW + 32, 2)
+    lattice_live_kernel(const __grid_constant__ OwnParams o) {
+  constexpr bool ZS = true;
+  constexpr int NW = RunTile<NZM, ZS>::NW, PS = kRunPS;
+  const float INF_F = __int_as_float(0x7f800000);
+  extern __shared__ __align__(128) float sd[];
+  __shared__ RunShared S;
+  __shared__ OwnShared Q;
+  const LatParams &p = o.l;
+  LatCtl *const ctl = p.ctl;
+  const int tid = threadIdx.x;
+  auto handover = [&] { asm volatile("bar.sync 2, %0;" ::"n"(NW + 32) : "memory"); };
+
+  if (tid >= NW) {
+    // ------------------------------------------------------------ helper
+    const unsigned long long t_start = dev_globaltimer();
+    const unsigned long long limit = min(p.wait_ns * 4, p.budget_ns);
+    const int lane = tid - NW;
+    int box = -1;
+    bool have = false;  // a place in the queue is taken: pos
+    unsigned pos = 0, visits = 0;
+    // tiles `q` of the lanes with `push`, already in state 1, into the queue
+    auto enqueue = [&](bool push, int q) {
+      const unsigned m = __ballot_sync(ORSP_FULL_MASK, push);
+      if (!m) return;
+      __threadfence();
+      unsigned base = 0;
+      if (lane == 0) base = atomicAdd(&ctl->tail, (unsigned)__popc(m));
+      base = __shfl_sync(ORSP_FULL_MASK, base, 0);
+      if (lane == 0) atomicAdd(&ctl->avail, __popc(m));
+      if (push) atomicExch(&p.qslot[(base + __popc(m & lanemask_lt())) % p.qcap], q);
+    };
+    for (;;) {
+      // ---- the next tile
+      if (!have) {
+        if (lane == 0) {
+          atomicSub(&ctl->avail, 1);
+          pos = atomicAdd(&ctl->head, 1u);
+        }
+        pos = __shfl_sync(ORSP_FULL_MASK, pos, 0);
+      }
+      have = false;
+      const unsigned *slot = (const unsigned *)&p.qslot[pos % p.qcap];
+      const unsigned *look = lane == 0 ? slot : lane == 1 ? (const unsigned *)&ctl->pending : (const unsigned *)&ctl->err;
+      int t = -1;
+      for (unsigned spins = 0;; ++spins) {
+        const unsigned v = lane < 3 ? ld_acquire_u32(look) : 0u;
+        if (__shfl_sync(ORSP_FULL_MASK, v, 1) == 0u || __shfl_sync(ORSP_FULL_MASK, v, 2) != 0u) break;
+        t = (int)__shfl_sync(ORSP_FULL_MASK, v, 0);
+        if (t >= 0) break;
+        if (lane == 0 && (spins & 31u) == 31u && dev_globaltimer() - t_start > limit)
+          atomicCAS(&ctl->err, DEV_OK, DEV_ERR_TIMEOUT);
+      }
+      unsigned got = 0;
+      if (t >= 0) {
+        const int bi = p.nbox == 1 ? 0 : __ldg(&p.tbox[t]);
+        got = __ldcg(&o.got[t]);
+        if (lane == 0) {
+          atomicExch((int *)slot, -1);
+          atomicExch(&p.tstate[t], 2);
+          if (bi != box) Q.box = load_box(p, bi);
+          Q.req = Q.ack = got;
+          Q.stop = Q.rel = Q.idle = Q.out = 0;
+        }
+        box = bi;
+        if (lane < 4) Q.pub[lane] = 0;
+      }
+      if (lane == 0) Q.tile = t;
+      __syncwarp();
+      handover();
+      if (t < 0) break;
+      ++visits;
+      const int ntx = Q.box.ntx, nty = Q.box.nty, lt = t - Q.box.tile0, ty = lt / ntx, tx = lt - ty * ntx;
+      const int nb = lane == 0 ? (tx > 0 ? t - 1 : -1)
+                               : lane == 1 ? (tx < ntx - 1 ? t + 1 : -1)
+                                           : lane == 2 ? (ty > 0 ? t - ntx : -1)
+                                                       : lane == 3 ? (ty < nty - 1 ? t + ntx : -1) : -1;
+      // messages to the neighbours on the sides in m
+      auto send = [&](unsigned m) {
+        if (lane == 0) atomicAdd(&ctl->pending, __popc(m));
+        __threadfence();
+        __syncwarp();
+        bool push = false;
+        if ((m >> lane) & 1u) {
+          atomicAdd(&o.inbox[nb], 1u);
+          __threadfence();
+          const int st = atomicCAS(&p.tstate[nb], 0, 1);
+          push = st == 0 || (st == 4 && atomicCAS(&p.tstate[nb], 4, 1) == 4);
+        }
+        enqueue(push, nb);
+      };
+      unsigned asked = got;
+      bool reached = false, over = false;
+      for (unsigned spins = 0;; ++spins) {
+        const bool acked = asked != got && __shfl_sync(ORSP_FULL_MASK, Q.ack, 0) == asked;
+        const bool out = __shfl_sync(ORSP_FULL_MASK, Q.out, 0) != 0;
+        const bool rest = __shfl_sync(ORSP_FULL_MASK, Q.idle, 0) != 0;
+        __threadfence_block();
+        // everything published up to the answer is sent before the count is
+        // dealt with
+        const unsigned pm = __ballot_sync(ORSP_FULL_MASK, lane < 4 && atomicExch(&Q.pub[lane & 3], 0) != 0);
+        if (pm) send(pm);
+        if (acked) {
+          if (lane == 0) {
+            __threadfence();
+            atomicSub(&ctl->pending, (int)(asked - got));
+          }
+          got = asked;
+        }
+        if (out) break;
+        unsigned v = 0;
+        if (lane == 0) v = ld_acquire_u32(&o.inbox[t]);
+        if (lane == 1) v = ld_acquire_u32((const unsigned *)&ctl->pending);
+        if (lane == 2) v = ld_acquire_u32((const unsigned *)&ctl->err);
+        if (lane == 3) v = ld_acquire_u32((const unsigned *)&ctl->avail);
+        const unsigned in = __shfl_sync(ORSP_FULL_MASK, v, 0);
+        over = __shfl_sync(ORSP_FULL_MASK, v, 1) == 0u || __shfl_sync(ORSP_FULL_MASK, v, 2) != 0u;
+        const int waiting = (int)__shfl_sync(ORSP_FULL_MASK, v, 3);  // < 0: free CTAs
+        if (over && lane == 0) Q.stop = 1;
+        if (asked == got && in != got) {
+          asked = in;
+          if (lane == 0) Q.req = in;
+          if (!reached && waiting < 0) enqueue(nb >= 0 && atomicCAS(&p.tstate[nb], 0, 1) == 0, nb);
+          reached = true;
+        }
+        if (!have && waiting > -kFreeCtas && rest && asked == got && !pm) {
+          if (lane == 0) {
+            have = atomicSub(&ctl->avail, 1) > -kFreeCtas;
+            if (have) pos = atomicAdd(&ctl->head, 1u);
+            else atomicAdd(&ctl->avail, 1);
+          }
+          have = __shfl_sync(ORSP_FULL_MASK, (int)have, 0);
+          pos = __shfl_sync(ORSP_FULL_MASK, pos, 0);
+          if (have) {
+            if (lane == 0) Q.rel = 1;
+          }
+        }
+        if (lane == 0 && (spins & 31u) == 31u && dev_globaltimer() - t_start > limit)
+          atomicCAS(&ctl->err, DEV_OK, DEV_ERR_TIMEOUT);
+      }
+      handover();  // the tile's distances are in memory
+      if (over) {
+        if (lane == 0) Q.tile = -1;
+        __syncwarp();
+        handover();
+        break;
+      }
+      // ---- give the tile back
+      bool push = false;
+      if (lane == 0) {
+        __stcg(&o.got[t], got);
+        __threadfence();
+        atomicExch(&p.tstate[t], 4);
+        __threadfence();
+        push = ld_acquire_u32(&o.inbox[t]) != got && atomicCAS(&p.tstate[t], 4, 1) == 4;
+      }
+      enqueue(push, t);
+    }
+    if (lane == 0) atomicAdd(&ctl->visits, visits);
+    return;
+  }
+
+  // -------------------------------------------------------------- workers
+  RunTile<NZM, ZS> R;
+  float2 *const wp = (float2 *)(sd + o.nzb * PS), *const wz = wp + o.nzb * PS;
+  if (tid == 0) S.start();
+  for (;;) {
+    handover();
+    const int t = Q.tile;
+    if (t < 0) break;
+    if (tid == 0) S.lap(-1);
+    const LatBox B = Q.box;
+    const RunGeom G = run_geom(p, B, t);
+    const unsigned snap = Q.ack;
+    if (tid < 32) S.clear();
+    // the rows' values, what was published to the neighbours, the tile
+    float *const ex = o.exch + (int64_t)t * 2 * o.nr + tid;
+    const int step = (G.isv ? B.ntx : 1) * 2 * o.nr;
+    float na = INF_F, nb = INF_F, pa = INF_F, pb = INF_F;
+    if (G.run) {
+      na = ld_relaxed_f32(ex);
+      nb = ld_relaxed_f32(ex + o.nr);
+      if (G.isv ? G.ty > 0 : G.tx > 0) pa = ld_relaxed_f32(ex - step + o.nr);
+      if (G.isv ? G.ty < B.nty - 1 : G.tx < B.ntx - 1) pb = ld_relaxed_f32(ex + step);
+    }
+    const bool force = __ldcg(&p.stamp[t]) != 0;
+    const int64_t dz = (!PRIV || B.dbase < 0) ? (int64_t)p.nx * p.ny : (int64_t)(B.x1 - B.x0 + 1) * (B.y1 - B.y0 + 1);
+    const int64_t d0 = G.col ? dist_index<PRIV>(p, B, G.X0 + G.xx, G.Y0 + G.yy, B.z0) : 0;
+    load_tile<NZM, true, ZS, true>(p, G, R, sd, wp, wz, d0, dz);  // (with a barrier)
+    if (tid == 0) {
+      S.lap(0);
+      if (force) p.stamp[t] = 0;
+    }
+    const unsigned cycles = own_cycles<NZM, CV, ZS>(o, B, G, R, S, Q, sd, wz, ex, na, nb, pa, pb, G.run && force, force, snap);
+    if (tid == 0) S.lap(1);
+    if (cycles) {
+      if (G.col) {
+        const float *const cd = sd + G.yy * kRunWS + G.xx;
+#pragma unroll
+        for (int z = 0; z < NZM; ++z)
+          if (z < G.nzb) __stcg(&p.dist[d0 + z * dz], f_bits(cd[z * PS]));
+      }
+      __threadfence();
+    }
+    tile_sync<NW, true>();
+    if (tid == 0) {
+      S.lap(2);
+      S.cycles += cycles;
+      Q.out = 1;
+    }
+    handover();
+  }
+  if (tid == 0) S.flush(ctl);
 }
 
 // Tiles to revisit after a visit of tile t: the neighbours whose halo value
@@ -2466,6 +2756,19 @@ void *own_kernel(int nzm, bool cv, bool two) {
   return nzm == 6 ? own_kernel<6, PRIV>(cv, two) : nzm == 12 ? own_kernel<12, PRIV>(cv, two) : own_kernel<18, PRIV>(cv, two);
 }
 
+constexpr int64_t kLiveTiles = 16384;  // tiles of a launch under visiting owners (38 MB of rows at 18 layers)
+size_t live_ws(int64_t ntiles, int nzb) { return ((size_t)ntiles * (2 * 16 * nzb + 2)) * 4 + 256; }
+
+template <bool PRIV, bool CV>
+void *live_kernel(int nzm) {
+  return nzm == 6 ? (void *)lattice_live_kernel<6, PRIV, CV>
+                  : nzm == 12 ? (void *)lattice_live_kernel<12, PRIV, CV> : (void *)lattice_live_kernel<18, PRIV, CV>;
+}
+template <bool PRIV>
+void *live_kernel(int nzm, bool cv) {
+  return cv ? live_kernel<PRIV, true>(nzm) : live_kernel<PRIV, false>(nzm);
+}
+
 void fill_axes(LatParams &p) {
   p.hmask = p.vmask = 0;
   for (int z = 0, h = 0, v = 0; z < p.nz && z < 64; ++z) {
@@ -2514,16 +2817,35 @@ int launch_own(orsp::Graph *g, LatParams &p, int64_t ntiles, const OwnShape &sh,
 }
 
 // Whether a launch takes the owner schedule (ORSP_LAT_OWN=0: none does): one
-// that fits it and was not given the schedule of many wave fronts.
+// that fits it, whose boxes are all searched.
 bool use_own(const orsp::Graph *g, int64_t ntiles, int nzb, int64_t nseeds, const orsp::LatOptions *opt, OwnShape *sh) {
   if (env_u64("ORSP_LAT_OWN", 1) == 0 || env_u64("ORSP_LAT_ASYNC", 1) == 0 || env_u64("ORSP_LAT_TMA", 0) != 0)
     return false;
   if (env_u64("ORSP_LAT_SPEC", 0) != 0 || env_u64("ORSP_LAT_BLOCKS_PER_SM", 1) > 1) return false;
-  if (opt && (opt->spec || opt->blocks_per_sm > 1 || opt->active)) return false;
+  if (opt && opt->active) return false;
   return own_shape(g, ntiles, nzb, nseeds, sh) && sh->per_sm <= (int)env_u64("ORSP_OWN_PER_SM", 2);
 }
 
-int launch_lattice(orsp::Graph *g, LatParams &p, int64_t ntiles, int nzb, int32_t nseeds, const int32_t *seeds,
+// Whether a launch takes visiting owners (ORSP_LAT_LIVE=0: none does).  `front`
+// is the sum of the boxes' sides in tiles, about the tiles that wave fronts
+// hold at a time; below one per resident CTA the owners are faster than the
+// queue schedules (sources on 1000 x 1000 x 12, 126 tiles each: 2 sources 1.58
+// against 2.15 ms, 4 2.86 against 2.57; on 400 x 400 x 6, 50 each: 6 sources
+// 0.64 against 0.66 ms, 8 0.79 against 0.67; boxes of 320 x 320 x 4, 40 each: 8
+// boxes 0.67 against 0.68 ms, 12 0.88 against 0.71).  Column vias, which have no
+// warp-specialised schedule, gain up to twice that (16 sources on 300 x 300 x 8,
+// 608 tiles: 1.30 against 1.42 ms).  Launches with activity flags search few of
+// their boxes (repair rounds of 32 boxes on 600 x 600 x 18: grouped routing 76
+// -> 70 ms).
+bool use_live(const orsp::Graph *g, int64_t ntiles, int64_t front, int nzb, const orsp::LatOptions *opt) {
+  if (env_u64("ORSP_LAT_LIVE", 1) == 0 || env_u64("ORSP_LAT_ASYNC", 1) == 0 || env_u64("ORSP_LAT_TMA", 0) != 0)
+    return false;
+  if (env_u64("ORSP_LAT_SPEC", 0) != 0 || env_u64("ORSP_LAT_BLOCKS_PER_SM", 1) > 1) return false;
+  if (!run_visit_layers(nzb) || ntiles > kLiveTiles) return false;
+  return (opt && opt->active) || front <= (g->cvia ? 4 : 2) * (int64_t)g->num_sms;
+}
+
+int launch_lattice(orsp::Graph *g, LatParams &p, int64_t ntiles, int64_t front, int nzb, int32_t nseeds, const int32_t *seeds,
                    const float *seed_cost, cudaStream_t st, orsp::LatOptions *opt) {
   constexpr int TX = 16, TY = 16;
   // (column vias always take the asynchronous schedule)
@@ -2543,9 +2865,23 @@ int launch_lattice(orsp::Graph *g, LatParams &p, int64_t ntiles, int nzb, int32_
   p.ctl = (LatCtl *)(b + 4 * list_b + q_b);
   if (opt) opt->err_d = &p.ctl->err;
   p.tbox = async ? p.list0 : nullptr;
+  const bool live = use_live(g, ntiles, front, nzb, opt);
+  OwnParams o{};
+  if (live) {
+    rc0 = grow_own_ws(g, live_ws(ntiles, nzb));
+    if (rc0) return rc0;
+    o.nr = 16 * nzb;
+    o.nzb = nzb;
+    o.tcap = (int32_t)ntiles;
+    o.exch = (float *)g->own_ws;
+    o.inbox = (unsigned *)(o.exch + ntiles * 2 * o.nr);
+    o.got = o.inbox + ntiles;
+    p.inbox = o.inbox;
+  }
   if (async) {
-    const int64_t n = std::max<int64_t>(ntiles, qcap);
-    lattice_init_kernel<<<(int)std::min<int64_t>((n + 255) / 256, (int64_t)g->num_sms * 8), 256, 0, st>>>(p, (int32_t)ntiles);
+    const int64_t rows = live ? ntiles * 2 * o.nr / 4 : 0, n = std::max<int64_t>(std::max<int64_t>(ntiles, qcap), rows);
+    lattice_init_kernel<<<(int)std::min<int64_t>((n + 255) / 256, (int64_t)g->num_sms * 8), 256, 0, st>>>(
+        p, (int32_t)ntiles, o.got, (float4 *)o.exch, rows);
     ORSP_CUDA(cudaGetLastError());
   } else {
     ORSP_CUDA(cudaMemsetAsync(p.stamp, 0, list_b + (size_t)ntiles * 4, st));  // stamps and states
@@ -2553,6 +2889,22 @@ int launch_lattice(orsp::Graph *g, LatParams &p, int64_t ntiles, int nzb, int32_
   lattice_seed_kernel<TX, TY><<<1, 256, 0, st>>>(p, nseeds, seeds, seed_cost);
   ORSP_CUDA(cudaGetLastError());
   fill_axes(p);
+  if (live) {
+    p.wait_ns = env_u64("ORSP_WAIT_NS", 2000000000ull);
+    p.budget_ns = env_u64("ORSP_BUDGET_NS", 20000000000ull);
+    o.l = p;
+    const int nzl = run_visit_layers(nzb);
+    void *kfn = opt && opt->private_dist ? live_kernel<true>(nzl, p.wcol != nullptr)
+                                         : live_kernel<false>(nzl, p.wcol != nullptr);
+    void *args[] = {&o};
+    // ORSP_LIVE_CTAS: that many CTAs instead of two per SM
+    int rc = launch_persistent(g, kfn, (nzl > 16 ? 288 : 256) + 32, (size_t)run_smem_floats(nzb, true) * sizeof(float), 2,
+                               (int)std::min<unsigned long long>(env_u64("ORSP_LIVE_CTAS", 0), g->num_sms), args, st);
+    if (rc) return rc;
+    if (!opt || opt->copy_ctl)
+      ORSP_CUDA(cudaMemcpyAsync(g->lat_ctl_h, p.ctl, sizeof(LatCtl), cudaMemcpyDeviceToHost, st));
+    return ORSP_OK;
+  }
   // run visits up to 18 layers; deeper tiles take process_tile
   const int nzm = async ? run_visit_layers(nzb) : 0;
   // ORSP_LAT_BLOCKS_PER_SM: CTAs per SM
@@ -2758,6 +3110,10 @@ int reserve_lattice_ws(Graph *g, int64_t ntiles) {
     int rc = grow_own_ws(g, sh.ws);
     if (rc) return rc;
   }
+  if (ntiles <= kLiveTiles && run_visit_layers(std::min(g->nz, 18))) {
+    int rc = grow_own_ws(g, live_ws(ntiles, std::min(g->nz, 18)));
+    if (rc) return rc;
+  }
   return grow_ws(g, ws_layout(g, ntiles).total);
 }
 
@@ -2795,12 +3151,14 @@ int run_lattice_boxes(Graph *g, const float *cost_d, int32_t nseeds, const int32
   constexpr int TX = 16, TY = 16;
   const bool priv = opt && opt->private_dist;
   int64_t vol_sum = 0;
-  int64_t ntiles = 0;
+  int64_t ntiles = 0, front = 0;
   int nzb = 1;
   bool whole = false;
   for (int32_t i = 0; i < nbox; ++i) {
     const int32_t *b = boxes_h + 6 * (int64_t)i;
-    ntiles += (int64_t)((b[1] - b[0] + TX) / TX) * ((b[3] - b[2] + TY) / TY);
+    const int64_t tx = (b[1] - b[0] + TX) / TX, ty = (b[3] - b[2] + TY) / TY;
+    ntiles += tx * ty;
+    front += tx + ty;
     nzb = std::max(nzb, b[5] - b[4] + 1);
     vol_sum += (int64_t)(b[1] - b[0] + 1) * (b[3] - b[2] + 1) * (b[5] - b[4] + 1);
     whole = whole || (b[0] == 0 && b[1] == g->nx - 1 && b[2] == 0 && b[3] == g->ny - 1 && b[4] == 0 &&
@@ -2904,7 +3262,7 @@ int run_lattice_boxes(Graph *g, const float *cost_d, int32_t nseeds, const int32
   p.dist = dist;
   for (int z = 0; z < 64; ++z) p.axis[z] = z < g->nz ? g->layer_axis[z] : 0;
   if (owned) return launch_own(g, p, ntiles, own, nseeds, seeds_d, seed_cost_d, st, opt);
-  return launch_lattice(g, p, ntiles, nzb, nseeds, seeds_d, seed_cost_d, st, opt);
+  return launch_lattice(g, p, ntiles, front, nzb, nseeds, seeds_d, seed_cost_d, st, opt);
 }
 
 int run_lattice_search(Graph *g, const float *cost_d, int32_t nseeds, const int32_t *seeds_d,
@@ -2978,11 +3336,11 @@ int run_lattice_roi(Graph *g, const float *cost_d, int32_t nseeds, const int32_t
   p.roi_map = roi_map_d;
   for (int z = 0; z < 64; ++z) p.axis[z] = z < g->nz ? g->layer_axis[z] : 0;
   // the box is known on the device only: size the tile arrays for the lattice
-  const int64_t ntiles = (int64_t)((g->nx - 1 + TX) / TX) * ((g->ny - 1 + TY) / TY);
+  const int64_t tx = (g->nx - 1 + TX) / TX, ty = (g->ny - 1 + TY) / TY, ntiles = tx * ty;
   OwnShape own;
   if (use_own(g, ntiles, g->nz, nseeds, nullptr, &own))
     return launch_own(g, p, ntiles, own, nseeds, seeds_d, seed_cost_d, st, nullptr);
-  return launch_lattice(g, p, ntiles, g->nz, nseeds, seeds_d, seed_cost_d, st, nullptr);
+  return launch_lattice(g, p, ntiles, tx + ty, g->nz, nseeds, seeds_d, seed_cost_d, st, nullptr);
 }
 
 int finish_lattice_search(Graph *g, int32_t *rounds_h) {

@@ -118,6 +118,7 @@ struct Graph {
   size_t own_ws_bytes = 0;
   void *lat_ctl_h = nullptr;      // pinned mirror of the control block
   void *lat_box_d = nullptr;      // tile table of a single-box search
+  int *wmin = nullptr;            // smallest planar and via weight of the last gather that asked for them
   // ROI searches (orsp_sssp_roi_nodes, ROI-masked tile sweeps): a global_to_roi
   // map kept at -1 between calls (each call scatters its ROI in and clears it
   // again), a sink mask kept at 0 the same way, the ROI's bounding box as it is
@@ -131,6 +132,7 @@ struct Graph {
   // (generation 0: not reusable), and the declaration for the next search
   const float *w4_cost = nullptr;
   uint64_t w4_gen = 0;
+  bool w4_min = false;  // that gather recorded wmin
   const float *decl_cost = nullptr;
   uint64_t decl_gen = 0;
 };
@@ -164,6 +166,8 @@ struct LatBox {
   int32_t pad;       // the box's distance slice for the TMA staging (LatOptions::tma_slices)
   int64_t dbase;     // -1: distances indexed by node id in the shared array;
                      // >= 0: the box's own slice, box-local row-major from here
+  int32_t gx, gy, gz;  // the target of a search of which only the path is wanted (gx -1: every distance is)
+  int32_t pad2;
 };
 // Whether a tile of nzb layers at tile width tile_w (16 or 32; 0: 16, the
 // width of every tile) fits in shared memory.
@@ -171,6 +175,13 @@ bool lattice_tile_fits(int nzb, int tile_w = 0);
 // Fills out[i] for boxes_h[6i..6i+5] (shared distances) and returns the total
 // count of their 16 x 16 tiles.
 int64_t make_lat_boxes(const int32_t *boxes_h, int32_t nbox, LatBox *out);
+// Sets the target of a box's search to node dst where the box holds it.
+inline void lat_box_target(const Graph *g, int32_t dst, LatBox *B) {
+  if (dst < 0 || dst >= g->N) return;
+  const int32_t plane = g->nx * g->ny, z = dst / plane, y = dst % plane / g->nx, x = dst % g->nx;
+  if (x < B->x0 || x > B->x1 || y < B->y0 || y > B->y1 || z < B->z0 || z > B->z1) return;
+  B->gx = x, B->gy = y, B->gz = z;
+}
 struct LatOptions {
   bool private_dist = false;   // boxes have their own slices (dbase >= 0): seed i starts box i, and
                                // `dist` is the slice arena of private_count entries, all reset
@@ -182,6 +193,8 @@ struct LatOptions {
   int spec = 0;                // 1: the warp-specialised schedule; ORSP_LAT_SPEC overrides
   int64_t tma_slices = 0;      // > 0: every box is the whole lattice, box j's distances in slice j of N
                                // cells from `dist` (LatBox.pad = j); allows the TMA staging
+  bool targets = false;        // private_dist: boxes have targets (LatBox::gx); only the distances that a
+                               // shortest path to the target needs are final
   const int32_t *active = nullptr;  // private_dist, device flags: a box with active[j] == 0 has no seed, and
                                     // its weights and distances are neither gathered nor reset
 };

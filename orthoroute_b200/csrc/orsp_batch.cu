@@ -667,6 +667,7 @@ int run_batch_lat(orsp_graph *g, const float *cost_d, int32_t K, const std::vect
     for (int32_t j = 0; j < m; ++j) {
       hb[j].dbase = base;
       base += box_volume(&boxes[(size_t)j * 6], 0);
+      lat_box_target(g, h_dst[j], &hb[j]);
     }
     ORSP_CUDA(cudaMemcpyAsync(g->blat_tab_d, g->blat_tab_h, (size_t)m * sizeof(LatBox) + (size_t)m * 12,
                               cudaMemcpyHostToDevice, st));
@@ -679,10 +680,11 @@ int run_batch_lat(orsp_graph *g, const float *cost_d, int32_t K, const std::vect
     LatOptions opt;
     opt.private_dist = true;
     opt.private_count = cells;
+    opt.targets = true;
     // many boxes: two CTAs per SM and the warp-specialised schedule, as for
-    // many sources (2 048 boxes of up to 400 x 400 x 16: 10.5 ms, against
-    // 14.6 ms without the schedule and 13.2 ms with it at one CTA per SM);
-    // boxes of no more tiles than the owner schedule holds take that one
+    // many sources (2 048 boxes of up to 400 x 400 x 16, before targets bounded
+    // the sweeps: 10.5 ms, against 14.6 ms without the schedule and 13.2 ms with
+    // it at one CTA per SM; now 6.5 ms); boxes of no more tiles than the owner schedule holds take that one
     if (ntiles > 2 * (int64_t)g->num_sms) {
       opt.blocks_per_sm = 2;
       opt.spec = 1;
@@ -801,7 +803,7 @@ static int run_batch(orsp_graph *g, const float *cost_d, int32_t K, const int32_
   // deep (the depth of the run visits), are swept: that is the faster form
   // at every count and size measured (one box of up to 30 x 30 x 6: 0.21 ms
   // against 0.29 ms with one CTA per search, 2 048 of 24 x 24 x 4: 0.63
-  // against 1.38, 512 of up to 400 x 400 x 16: 2.7 against 19.3).  Column-via
+  // against 1.38, 512 of up to 400 x 400 x 16: 1.9 against 19.3).  Column-via
   // and deeper boxes keep one CTA per search: not measured.
   const bool sweep_all = !range_mode && g->plan_nb == 0 && g->lattice_ok && !g->cvia;
   auto swept = [&](int i, int32_t k) {

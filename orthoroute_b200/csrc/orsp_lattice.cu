@@ -95,6 +95,7 @@ struct LatParams {
   int8_t hlist[64], vlist[64];
   const int32_t *tbox;  // box of each tile (asynchronous schedule)
   unsigned *inbox;      // messages to each tile (visiting owners; else NULL)
+  const int *wmin;      // boxes with targets: smallest planar and via weight (float bits; else NULL)
 };
 
 __global__ void fill_kernel(uint32_t *p, int64_t n, uint32_t v) {
@@ -157,17 +158,37 @@ struct BoxIndex {
   }
 };
 
+// Smallest planar and via weight, as float bits, of the nodes that a gather
+// passes (wmin NULL: not wanted).  Negative weights and -0 come out negative,
+// absent edges and NaN do not count.
+__device__ __forceinline__ void min_weight(int2 &m, const float4 &w) {
+  m.x = min(m.x, min(__float_as_int(w.x), __float_as_int(w.y)));
+  m.y = min(m.y, min(__float_as_int(w.z), __float_as_int(w.w)));
+}
+__device__ __forceinline__ void record_min(int *wmin, int2 m) {
+  m.x = __reduce_min_sync(ORSP_FULL_MASK, m.x);
+  m.y = __reduce_min_sync(ORSP_FULL_MASK, m.y);
+  if ((threadIdx.x & 31) == 0) {  // (the look first: most warps have nothing to add)
+    if (m.x < __ldcg(&wmin[0])) atomicMin(&wmin[0], m.x);
+    if (m.y < __ldcg(&wmin[1])) atomicMin(&wmin[1], m.y);
+  }
+}
+
 // In-edge weights of node v as one float4 {from lower axis neighbour, from
 // upper axis neighbour, via from below, via from above}; +inf where absent.
 __global__ void gather_kernel(const int32_t *__restrict__ slot_eid, const float *__restrict__ cost,
-                              float4 *__restrict__ w, int64_t n) {
+                              float4 *__restrict__ w, int64_t n, int *wmin) {
   const float INF_F = __int_as_float(0x7f800000);
+  int2 m = make_int2(INT_MAX, INT_MAX);
   const int64_t s = (int64_t)gridDim.x * blockDim.x;
   for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += s) {
     const int32_t e0 = slot_eid[v], e1 = slot_eid[n + v], e2 = slot_eid[2 * n + v], e3 = slot_eid[3 * n + v];
-    w[v] = make_float4(e0 >= 0 ? __ldg(&cost[e0]) : INF_F, e1 >= 0 ? __ldg(&cost[e1]) : INF_F,
-                       e2 >= 0 ? __ldg(&cost[e2]) : INF_F, e3 >= 0 ? __ldg(&cost[e3]) : INF_F);
+    const float4 o = make_float4(e0 >= 0 ? __ldg(&cost[e0]) : INF_F, e1 >= 0 ? __ldg(&cost[e1]) : INF_F,
+                                 e2 >= 0 ? __ldg(&cost[e2]) : INF_F, e3 >= 0 ? __ldg(&cost[e3]) : INF_F);
+    w[v] = o;
+    if (wmin) min_weight(m, o);
   }
+  if (wmin) record_min(wmin, m);
 }
 
 // The same gather for the nodes of a box only (x fastest, then y, then z).
@@ -195,9 +216,10 @@ __global__ void gather_box_kernel(const int32_t *__restrict__ slot_eid, const fl
 // two boxes are written twice with the same value.
 __global__ void gather_boxes_kernel(const int32_t *__restrict__ slot_eid, const float *__restrict__ cost,
                                     float4 *__restrict__ w, int64_t n, int32_t nx, int32_t ny,
-                                    const LatBox *__restrict__ boxes, const int32_t *__restrict__ active) {
+                                    const LatBox *__restrict__ boxes, const int32_t *__restrict__ active, int *wmin) {
   if (active && !active[blockIdx.y]) return;
   const float INF_F = __int_as_float(0x7f800000);
+  int2 m = make_int2(INT_MAX, INT_MAX);
   const LatBox B = boxes[blockIdx.y];
   const int32_t bw = B.x1 - B.x0 + 1, bh = B.y1 - B.y0 + 1;
   const int64_t plane = (int64_t)bw * bh, count = plane * (B.z1 - B.z0 + 1);
@@ -209,9 +231,12 @@ __global__ void gather_boxes_kernel(const int32_t *__restrict__ slot_eid, const 
     bi.split(i, plane, z, y, x);
     const int64_t v = ((int64_t)(B.z0 + z) * ny + (B.y0 + y)) * nx + (B.x0 + x);
     const int32_t e0 = slot_eid[v], e1 = slot_eid[n + v], e2 = slot_eid[2 * n + v], e3 = slot_eid[3 * n + v];
-    w[v] = make_float4(e0 >= 0 ? __ldg(&cost[e0]) : INF_F, e1 >= 0 ? __ldg(&cost[e1]) : INF_F,
-                       e2 >= 0 ? __ldg(&cost[e2]) : INF_F, e3 >= 0 ? __ldg(&cost[e3]) : INF_F);
+    const float4 o = make_float4(e0 >= 0 ? __ldg(&cost[e0]) : INF_F, e1 >= 0 ? __ldg(&cost[e1]) : INF_F,
+                                 e2 >= 0 ? __ldg(&cost[e2]) : INF_F, e3 >= 0 ? __ldg(&cost[e3]) : INF_F);
+    w[v] = o;
+    if (wmin) min_weight(m, o);
   }
+  if (wmin) record_min(wmin, m);
 }
 
 // ---------------------------------------------------------------------------
@@ -275,6 +300,8 @@ __global__ void roi_box_finish_kernel(const int *bb, LatBox *box) {
   B.tile0 = 0;
   B.pad = 0;
   B.dbase = -1;
+  B.gx = B.gy = B.gz = -1;
+  B.pad2 = 0;
   *box = B;
 }
 
@@ -374,6 +401,10 @@ __device__ __forceinline__ LatBox load_box(const LatParams &p, int b) {
   B.tile0 = __ldg(q + 8);
   B.pad = __ldg(q + 9);
   B.dbase = __ldg((const long long *)(p.boxes + b) + 5);
+  B.gx = __ldg(q + 12);
+  B.gy = __ldg(q + 13);
+  B.gz = __ldg(q + 14);
+  B.pad2 = 0;
   return B;
 }
 
@@ -1379,6 +1410,44 @@ __device__ __forceinline__ bool run_passes(const LatParams &p, const RunGeom &G,
   return converged;
 }
 
+// What a search with a target passes on to the next tile.
+//
+// U, the target's distance so far, only falls, and a distance x of cell v is
+// of use only if x and what is still to go from v do not exceed it.  To go are
+// at least |dx| + |dy| planar steps and |dz| vias, each at its smallest weight
+// in the launch (goal_weights), so an improvement with x + to go > goal_limit
+// activates no tile.  Every cell on a shortest path to the target, those that
+// tie among them, passes, so the path is the one of the whole search (cells
+// that do not pass keep upper bounds, which the backtrace never takes for a
+// parent: rounded sums are monotone).
+//
+// The margin.  The searched sums are rounded, the bound is not.  With r = U /
+// smallest weight below 2^20 each step of a path adds at least 15/16 of its
+// weight, so a path has at most r / 0.93 steps, each rounded by at most U
+// 2^-24: the sum falls short of the exact one by at most 6.5e-8 r U.  Beyond
+// that ratio, and with negative weights, nothing is held back; with zero
+// weights x > U decides (no margin: rounded sums never fall).
+//
+// Half of a box lies nearer than a target drawn from it, and the visits of the
+// other half, and corrections that come too late to matter, went into nothing:
+// 2 048 boxes of up to 400 x 400 x 16 9.8 -> 6.5 ms, 512 boxes 2.78 -> 1.91 ms.
+struct GoalWeights {
+  float xy, z;
+};
+__device__ __forceinline__ GoalWeights goal_weights(const int *wmin) {
+  const int mp = __ldg(&wmin[0]), mv = __ldg(&wmin[1]);
+  if (min(mp, mv) <= 0) return {0.0f, 0.0f};
+  return {__int_as_float(mp) * 0.9999f, __int_as_float(mv) * 0.9999f};
+}
+__device__ __forceinline__ float goal_limit(float u, const int *wmin) {
+  const float INF_F = __int_as_float(0x7f800000);
+  const int lo = min(__ldg(&wmin[0]), __ldg(&wmin[1]));
+  if (lo < 0) return INF_F;
+  if (lo == 0) return u;
+  const float r = u / __int_as_float(lo);
+  return r < 1048576.0f ? u + u * (r * 1.2e-7f + 1e-6f) : INF_F;
+}
+
 // The same visit contract as process_tile.  warm: the tile was visited last
 // by this block (its distances are in shared memory, its weights in R), only
 // the halo is read again and only the runs whose halo improved are taken
@@ -1389,7 +1458,10 @@ __device__ __forceinline__ bool run_passes(const LatParams &p, const RunGeom &G,
 // binary search over the boxes and the box's fields were dependent trips to
 // L2 - the streamed weights evict them from L1 - and cost 3 us of an 11 us
 // visit with 16 boxes and two CTAs per SM.)
-template <int NZM, bool PRIV, bool SPEC, bool CV, bool ZS>
+//
+// GOAL: the box has a target (SB.gx); s_act[0..3] are then the smallest
+// distances passed on at each side, to go included, as float bits.
+template <int NZM, bool PRIV, bool SPEC, bool CV, bool ZS, bool GOAL = false>
 __device__ __forceinline__ void visit_runs(const LatParams &p, int t, const LatBox &SB, float *sd,
                                            RunTile<NZM, ZS> &R, RunShared &S, int *s_act, int *s_nb, bool warm) {
   constexpr int NW = RunTile<NZM, ZS>::NW, PS = kRunPS;
@@ -1398,7 +1470,7 @@ __device__ __forceinline__ void visit_runs(const LatParams &p, int t, const LatB
   const RunGeom G = run_geom(p, B, t);
   const int tid = threadIdx.x;
   if (tid == 0) S.lap(-1);
-  if (tid < 5) s_act[tid] = 0;
+  if (tid < 5) s_act[tid] = GOAL && tid < 4 ? 0x7f800000 : 0;
   if (s_nb && tid < 4) {  // neighbour tiles in the box: left, right, down, up (-1: box edge)
     s_nb[tid] = tid == 0 ? (G.tx > 0 ? t - 1 : -1)
                          : tid == 1 ? (G.tx < B.ntx - 1 ? t + 1 : -1)
@@ -1455,13 +1527,35 @@ __device__ __forceinline__ void visit_runs(const LatParams &p, int t, const LatB
 #pragma unroll
     for (int z = 0; z < NZM; ++z)
       if ((colm >> z) & 1u) __stcg(&p.dist[d0 + z * dz], f_bits(cd[z * PS]));
-    if (colm & G.hm) {
-      if (G.xx == 0) s_act[0] = 1;
-      if (G.xx == G.tw - 1) s_act[1] = 1;
-    }
-    if (colm & G.vm) {
-      if (G.yy == 0) s_act[2] = 1;
-      if (G.yy == G.th - 1) s_act[3] = 1;
+    if constexpr (GOAL) {
+      // per side the smallest x + to go
+      const GoalWeights g = goal_weights(p.wmin);
+      const float to_go = g.xy * (float)(abs(G.X0 + G.xx - SB.gx) + abs(G.Y0 + G.yy - SB.gy));
+      float h = INF_F, v = INF_F;
+#pragma unroll
+      for (int z = 0; z < NZM; ++z)
+        if ((colm >> z) & 1u) {
+          const float f = cd[z * PS] + (to_go + g.z * (float)abs(B.z0 + z - SB.gz));
+          if ((G.hm >> z) & 1u) h = fminf(h, f);
+          else v = fminf(v, f);
+        }
+      if (h < INF_F) {
+        if (G.xx == 0) atomicMin(&s_act[0], __float_as_int(h));
+        if (G.xx == G.tw - 1) atomicMin(&s_act[1], __float_as_int(h));
+      }
+      if (v < INF_F) {
+        if (G.yy == 0) atomicMin(&s_act[2], __float_as_int(v));
+        if (G.yy == G.th - 1) atomicMin(&s_act[3], __float_as_int(v));
+      }
+    } else {
+      if (colm & G.hm) {
+        if (G.xx == 0) s_act[0] = 1;
+        if (G.xx == G.tw - 1) s_act[1] = 1;
+      }
+      if (colm & G.vm) {
+        if (G.yy == 0) s_act[2] = 1;
+        if (G.yy == G.th - 1) s_act[3] = 1;
+      }
     }
   }
   if (tid == 0) {
@@ -2320,14 +2414,22 @@ __global__ void __launch_bounds__(NZM > 0 ? RunTile<NZM ? NZM : 1, ZS>::NW : TX 
 // the queue, so it reaches 0 only at the fixpoint.  Three dependent trips to
 // L2 in all; one lane doing the same tile after tile took about 6 us, more
 // than the visit it overlaps.
+template <bool GOAL>
 __device__ void finish_visit(const LatParams &p, int t, const LatBox &B, const int *act, int lane) {
+  float lim = 0.0f;
+  if (GOAL) {
+    lim = __int_as_float(0x7f7fffff);
+    if (B.gx >= 0)
+      lim = fminf(lim, goal_limit(bits_f(__ldcg(&p.dist[dist_index<true>(p, B, B.gx, B.gy, B.gz)])), p.wmin));
+  }
+  auto side = [&](int i) { return GOAL ? __int_as_float(act[i]) <= lim : act[i] != 0; };
   __threadfence();
   const int lt = t - B.tile0, ty = lt / B.ntx, tx = lt - ty * B.ntx;
   int q = -1;
-  if (lane == 0 && act[0] && tx > 0) q = t - 1;
-  if (lane == 1 && act[1] && tx < B.ntx - 1) q = t + 1;
-  if (lane == 2 && act[2] && ty > 0) q = t - B.ntx;
-  if (lane == 3 && act[3] && ty < B.nty - 1) q = t + B.ntx;
+  if (lane == 0 && side(0) && tx > 0) q = t - 1;
+  if (lane == 1 && side(1) && tx < B.ntx - 1) q = t + 1;
+  if (lane == 2 && side(2) && ty > 0) q = t - B.ntx;
+  if (lane == 3 && side(3) && ty < B.nty - 1) q = t + B.ntx;
   bool queue = false, bad = q >= 0;
   for (int tries = 0; bad && tries < 1024; ++tries) {
     const int st = atomicCAS(&p.tstate[q], 0, 1);
@@ -2400,7 +2502,7 @@ __device__ __forceinline__ void prefetch_tile_l2(const LatParams &p, int t, cons
   }
 }
 
-template <int NZM, bool PRIV, int MINB, bool ZS>
+template <int NZM, bool PRIV, int MINB, bool ZS, bool GOAL = false>
 __global__ void __launch_bounds__(RunTile<NZM, ZS>::NW + 32, MINB) lattice_spec_kernel(LatParams p) {
   constexpr int NW = RunTile<NZM, ZS>::NW;
   extern __shared__ float sd[];
@@ -2424,7 +2526,7 @@ __global__ void __launch_bounds__(RunTile<NZM, ZS>::NW + 32, MINB) lattice_spec_
       if (threadIdx.x == 0) idle_ns += dev_globaltimer() - tw;
       const int t = s_cur;
       if (t < 0) break;
-      visit_runs<NZM, PRIV, true, false, ZS>(p, t, s_box[k & 1], sd, R, s_run, s_act[k & 1], nullptr, false);
+      visit_runs<NZM, PRIV, true, false, ZS, GOAL>(p, t, s_box[k & 1], sd, R, s_run, s_act[k & 1], nullptr, false);
       // the visit ended with barrier 1: every write of it is done, and
       // finish_visit's device fence makes them visible before it activates
       // any tile (the workers do not wait for that fence)
@@ -2453,7 +2555,7 @@ __global__ void __launch_bounds__(RunTile<NZM, ZS>::NW + 32, MINB) lattice_spec_
     for (unsigned spins = 0;; ++spins) {
       // (one lane reads it: the warp takes the branch as one)
       if (!finished && __shfl_sync(0xffffffffu, s_done, 0) == k) {
-        finish_visit(p, cur, s_box[k & 1], s_act[k & 1], lane);
+        finish_visit<GOAL>(p, cur, s_box[k & 1], s_act[k & 1], lane);
         ++visits;
         finished = true;
       }
@@ -2500,7 +2602,7 @@ __global__ void __launch_bounds__(RunTile<NZM, ZS>::NW + 32, MINB) lattice_spec_
     asm volatile("bar.sync 2, %0;" ::"r"(NW + 32) : "memory");  // handoff k + 1
     // the workers reached this barrier only after finishing visit k
     if (!finished) {
-      finish_visit(p, cur, s_box[k & 1], s_act[k & 1], lane);
+      finish_visit<GOAL>(p, cur, s_box[k & 1], s_act[k & 1], lane);
       ++visits;
       finished = true;
     }
@@ -2626,7 +2728,8 @@ int run_visit_layers(int nzb) { return nzb <= 6 ? 6 : nzb <= 12 ? 12 : nzb <= 18
 // hold them; 16 sources on 1000 x 1000 x 12: 4.95 ms against 5.64 ms with the
 // spills, 2 048 boxes of up to 16 layers: 10.5 against 16.9 ms).
 template <int NZM, bool PRIV>
-void *run_visit_kernel(bool cv, bool spec, bool two) {
+void *run_visit_kernel(bool cv, bool spec, bool two, bool goal) {
+  if (PRIV && goal) return (void *)lattice_spec_kernel<NZM, true, 2, true, true>;
   if (cv) return (void *)lattice_async_kernel<16, 16, PRIV, false, 1, false, true, NZM>;
   if (spec)
     return two ? (void *)lattice_spec_kernel<NZM, PRIV, 2, true> : (void *)lattice_spec_kernel<NZM, PRIV, 1, false>;
@@ -2634,9 +2737,10 @@ void *run_visit_kernel(bool cv, bool spec, bool two) {
              : (void *)lattice_async_kernel<16, 16, PRIV, false, 1, false, false, NZM>;
 }
 template <bool PRIV>
-void *run_visit_kernel(int nzm, bool cv, bool spec, bool two) {
-  return nzm == 6 ? run_visit_kernel<6, PRIV>(cv, spec, two)
-                  : nzm == 12 ? run_visit_kernel<12, PRIV>(cv, spec, two) : run_visit_kernel<18, PRIV>(cv, spec, two);
+void *run_visit_kernel(int nzm, bool cv, bool spec, bool two, bool goal) {
+  return nzm == 6    ? run_visit_kernel<6, PRIV>(cv, spec, two, goal)
+         : nzm == 12 ? run_visit_kernel<12, PRIV>(cv, spec, two, goal)
+                     : run_visit_kernel<18, PRIV>(cv, spec, two, goal);
 }
 
 // Launches a persistent kernel of `want` CTAs per SM where they fit (ctas > 0:
@@ -2933,8 +3037,8 @@ int launch_lattice(orsp::Graph *g, LatParams &p, int64_t ntiles, int64_t front, 
   }
   void *kfn;
   if (runs) {
-    kfn = priv ? run_visit_kernel<true>(nzm, p.wcol != nullptr, spec, two)
-               : run_visit_kernel<false>(nzm, p.wcol != nullptr, spec, two);
+    kfn = priv ? run_visit_kernel<true>(nzm, p.wcol != nullptr, spec, two, spec && two && p.wmin)
+               : run_visit_kernel<false>(nzm, p.wcol != nullptr, spec, two, false);
   } else if (p.wcol) {
     kfn = priv ? (void *)lattice_async_kernel<16, 16, true, true, 1, false, true>
                : (void *)lattice_async_kernel<16, 16, false, true, 1, false, true>;
@@ -3062,6 +3166,7 @@ int analyze_lattice(Graph *g, const int32_t *indptr_h, const int32_t *indices_h)
   ORSP_CUDA(cudaMalloc(&g->slot_eid, slot.size() * sizeof(int32_t)));
   ORSP_CUDA(cudaMemcpy(g->slot_eid, slot.data(), slot.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
   ORSP_CUDA(cudaMalloc(&g->wslot, slot.size() * sizeof(float)));
+  ORSP_CUDA(cudaMalloc(&g->wmin, 2 * sizeof(int)));
   if (!adjacent_vias) {
     ORSP_CUDA(cudaMalloc(&g->vcol_eid, vcol.size() * sizeof(int32_t)));
     ORSP_CUDA(cudaMemcpy(g->vcol_eid, vcol.data(), vcol.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
@@ -3086,6 +3191,8 @@ void free_lattice(Graph *g) {
   cudaFree(g->lat_ws);
   cudaFree(g->own_ws);
   g->own_ws = nullptr;
+  cudaFree(g->wmin);
+  g->wmin = nullptr;
   cudaFree(g->lat_box_d);
   if (g->lat_ctl_h) cudaFreeHost(g->lat_ctl_h);
   g->lat_box_d = nullptr;
@@ -3134,6 +3241,8 @@ int64_t make_lat_boxes(const int32_t *boxes_h, int32_t nbox, LatBox *out) {
     B.tile0 = (int32_t)t0;
     B.pad = 0;
     B.dbase = -1;
+    B.gx = B.gy = B.gz = -1;
+    B.pad2 = 0;
     t0 += (int64_t)B.ntx * B.nty;
   }
   return t0;
@@ -3181,16 +3290,29 @@ int run_lattice_boxes(Graph *g, const float *cost_d, int32_t nseeds, const int32
   }
   const unsigned per_box = (unsigned)std::max<int64_t>(1, std::min<int64_t>((vmax + 255) / 256,
                                                                             148 * 32 / std::max(1, nbox)));
+  OwnShape own;
+  const bool owned = use_own(g, ntiles, nzb, nseeds, opt, &own);
+  // Boxes with targets, in the warp-specialised schedule only, whose scheduler
+  // warp reads the target's distance off the workers' path (in the plain queue
+  // schedule, with the boxes of routed nets, whose targets lie at their far
+  // ends, 32 of them took 1.2 instead of 1.1 ms).  Not on column vias: a via
+  // may cross several layers, and their weights are gathered apart.
+  const bool goals = priv && opt->targets && opt->spec && !g->cvia && nbox <= 65535 && run_visit_layers(nzb) &&
+                     !owned && !use_live(g, ntiles, front, nzb, opt);
+  int *const wmin = goals ? g->wmin : nullptr;
+  const bool cached = decl != 0 && g->w4_cost == cost_d && g->w4_gen == decl && (!goals || g->w4_min);
+  const bool all = !by_flag && (whole || (priv && vol_sum >= N));
+  if (goals && !(all && cached)) ORSP_CUDA(cudaMemsetAsync(g->wmin, 0x7f, 2 * sizeof(int), st));
   if (by_flag) {
     g->w4_cost = nullptr;  // part of wslot is rewritten
     g->w4_gen = 0;
     gather_boxes_kernel<<<dim3(per_box, (unsigned)nbox), 256, 0, st>>>(g->slot_eid, cost_d, (float4 *)g->wslot, N,
-                                                                       g->nx, g->ny, lboxes_d, opt->active);
+                                                                       g->nx, g->ny, lboxes_d, opt->active, wmin);
     ORSP_CUDA(cudaGetLastError());
-  } else if (whole || (priv && vol_sum >= N)) {
-    if (!(decl != 0 && g->w4_cost == cost_d && g->w4_gen == decl)) {
+  } else if (all) {
+    if (!cached) {
       gather_kernel<<<(int)std::min<int64_t>((N + 255) / 256, 148 * 32), 256, 0, st>>>(
-          g->slot_eid, cost_d, (float4 *)g->wslot, N);
+          g->slot_eid, cost_d, (float4 *)g->wslot, N, wmin);
       ORSP_CUDA(cudaGetLastError());
       if (g->cvia) {
         const int32_t full[6] = {0, g->nx - 1, 0, g->ny - 1, 0, g->nz - 1};
@@ -3199,15 +3321,16 @@ int run_lattice_boxes(Graph *g, const float *cost_d, int32_t nseeds, const int32
       }
       g->w4_cost = cost_d;
       g->w4_gen = decl;
+      g->w4_min = goals;
     }
   } else {
     g->w4_cost = nullptr;  // part of wslot is rewritten
     g->w4_gen = 0;
-    if (!g->cvia && nbox > 1 && nbox <= 65535) {
+    if (!g->cvia && (nbox > 1 || goals) && nbox <= 65535) {
       // one launch for all boxes, as many blocks per box as the largest needs
       // (within a grid of about 32 blocks per SM)
       gather_boxes_kernel<<<dim3(per_box, (unsigned)nbox), 256, 0, st>>>(g->slot_eid, cost_d, (float4 *)g->wslot,
-                                                                         N, g->nx, g->ny, lboxes_d, nullptr);
+                                                                         N, g->nx, g->ny, lboxes_d, nullptr, wmin);
       ORSP_CUDA(cudaGetLastError());
     } else {
       for (int32_t i = 0; i < nbox; ++i) {
@@ -3224,8 +3347,6 @@ int run_lattice_boxes(Graph *g, const float *cost_d, int32_t nseeds, const int32
       }
     }
   }
-  OwnShape own;
-  const bool owned = use_own(g, ntiles, nzb, nseeds, opt, &own);
   if (owned && (priv || whole || (opt && opt->fill_box_only))) {
     // the owners write every cell of the boxes
   } else if (by_flag) {
@@ -3254,6 +3375,7 @@ int run_lattice_boxes(Graph *g, const float *cost_d, int32_t nseeds, const int32
   p.nz = g->nz;
   p.nbox = nbox;
   p.seed_per_box = priv ? 1 : 0;
+  p.wmin = wmin;
   p.boxes = lboxes_d;
   p.w4 = (const float4 *)g->wslot;
   p.wcol = g->cvia ? g->wcol : nullptr;

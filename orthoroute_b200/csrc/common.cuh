@@ -193,6 +193,7 @@ struct LatOptions {
   int spec = 0;                // 1: the warp-specialised schedule; ORSP_LAT_SPEC overrides
   int64_t tma_slices = 0;      // > 0: every box is the whole lattice, box j's distances in slice j of N
                                // cells from `dist` (LatBox.pad = j); allows the TMA staging
+  bool gathered = false;       // the weights of the boxes are gathered (gather_lattice) and up to date
   bool targets = false;        // private_dist: boxes have targets (LatBox::gx); only the distances that a
                                // shortest path to the target needs are final
   const int32_t *active = nullptr;  // private_dist, device flags: a box with active[j] == 0 has no seed, and
@@ -204,6 +205,9 @@ struct LatOptions {
 int run_lattice_search(Graph *g, const float *cost_d, int32_t nseeds, const int32_t *seeds_d,
                        const float *seed_cost_d, const int32_t *box, uint32_t *dist, cudaStream_t st,
                        LatOptions *opt = nullptr);
+// Gathers the weights of the whole lattice (adjacent vias) for searches with
+// LatOptions::gathered.
+int gather_lattice(Graph *g, const float *cost_d, cudaStream_t st);
 // Several pairwise disjoint boxes searched in one launch, sharing the
 // distance array: boxes_h (host, 6 ints per box) sizes the launch, lboxes_d
 // (device, from make_lat_boxes) is what the kernel reads and must stay valid

@@ -3248,6 +3248,16 @@ int64_t make_lat_boxes(const int32_t *boxes_h, int32_t nbox, LatBox *out) {
   return t0;
 }
 
+int gather_lattice(Graph *g, const float *cost_d, cudaStream_t st) {
+  g->w4_cost = nullptr;  // the caller changes them from here on
+  g->w4_gen = 0;
+  const int64_t N = g->N;
+  gather_kernel<<<(int)std::min<int64_t>((N + 255) / 256, 148 * 32), 256, 0, st>>>(g->slot_eid, cost_d,
+                                                                                   (float4 *)g->wslot, N, nullptr);
+  ORSP_CUDA(cudaGetLastError());
+  return ORSP_OK;
+}
+
 // Searches pairwise disjoint boxes in one launch.  Distances are reset to
 // +inf everywhere (or, with opt->fill_box_only, inside the boxes only - the
 // caller's backtrace must then test box membership); only the boxes' weights
@@ -3297,13 +3307,15 @@ int run_lattice_boxes(Graph *g, const float *cost_d, int32_t nseeds, const int32
   // schedule, with the boxes of routed nets, whose targets lie at their far
   // ends, 32 of them took 1.2 instead of 1.1 ms).  Not on column vias: a via
   // may cross several layers, and their weights are gathered apart.
-  const bool goals = priv && opt->targets && opt->spec && !g->cvia && nbox <= 65535 && run_visit_layers(nzb) &&
+  const bool goals = priv && opt->targets && !opt->gathered && opt->spec && !g->cvia && nbox <= 65535 && run_visit_layers(nzb) &&
                      !owned && !use_live(g, ntiles, front, nzb, opt);
   int *const wmin = goals ? g->wmin : nullptr;
   const bool cached = decl != 0 && g->w4_cost == cost_d && g->w4_gen == decl && (!goals || g->w4_min);
   const bool all = !by_flag && (whole || (priv && vol_sum >= N));
   if (goals && !(all && cached)) ORSP_CUDA(cudaMemsetAsync(g->wmin, 0x7f, 2 * sizeof(int), st));
-  if (by_flag) {
+  if (opt && opt->gathered) {
+    // by gather_lattice, kept since
+  } else if (by_flag) {
     g->w4_cost = nullptr;  // part of wslot is rewritten
     g->w4_gen = 0;
     gather_boxes_kernel<<<dim3(per_box, (unsigned)nbox), 256, 0, st>>>(g->slot_eid, cost_d, (float4 *)g->wslot, N,

@@ -36,6 +36,7 @@ namespace {
 
 using orsp::apply_usage;
 using orsp::kWalkBlock;
+using orsp::lat_edge_slot;
 using orsp::lat_reverse;
 using orsp::lat_step_edge;
 using orsp::lat_walk_warp;
@@ -52,15 +53,37 @@ struct LiveParams {
   float pres_fac, hist_w, via_mult, base_w;
   int jitter;
   float *cost;
+  // gathered weights kept equal to the costs while the nets are routed (NULL:
+  // each search gathers its own): float 4 v + slot is edge u -> v, its place
+  // found by its head and the slots' edge ids
+  float *w4;
+  const int32_t *heads, *slot_eid;
+  int64_t N;
 };
+
+// Place of edge e among the gathered weights, -1 where they are not kept.
+__device__ __forceinline__ int64_t weight_at(const LiveParams &lp, int32_t e) {
+  if (!lp.w4) return -1;
+  const int64_t v = __ldg(&lp.heads[e]);
+  int at = -1;
+#pragma unroll
+  for (int s = 0; s < 4; ++s)
+    if (__ldg(&lp.slot_eid[s * lp.N + v]) == e) at = s;
+  return at < 0 ? -1 : 4 * v + at;
+}
+__device__ __forceinline__ void set_cost(const LiveParams &lp, int32_t e, int64_t at, float c) {
+  lp.cost[e] = c;
+  if (at >= 0) lp.w4[at] = c;
+}
 
 // Usage +-1 on edge e and its live cost from the usage left, where no other
 // thread of the launch takes the same edge: one round trip, the usage comes
 // back with the atomic.
-__device__ __forceinline__ void use_edge(const LiveParams &lp, int32_t e, int32_t sign) {
+__device__ __forceinline__ void use_edge(const LiveParams &lp, int32_t e, int64_t at, int32_t sign) {
   const float base = lp.base[e], capa = lp.capa[e], hist = lp.hist[e];
   const int32_t left = apply_usage(lp.usage, lp.present, e, sign);
-  lp.cost[e] = live_cost_of(e, base, left, capa, hist, lp.pres_fac, lp.hist_w, lp.via_mult, lp.base_w, lp.jitter);
+  set_cost(lp, e, at,
+           live_cost_of(e, base, left, capa, hist, lp.pres_fac, lp.hist_w, lp.via_mult, lp.base_w, lp.jitter));
 }
 
 // Step 1 for the nets of one group (block j takes net order[j], the len-1
@@ -81,11 +104,12 @@ __global__ void route_commit_kernel(const int32_t *order, const int32_t *edges, 
   for (int32_t i = threadIdx.x; i < ne; i += blockDim.x) {
     const int32_t e = row[i];
     if (e < 0) continue;
-    if (mode == 0) use_edge(lp, e, sign);
+    if (mode == 0) use_edge(lp, e, weight_at(lp, e), sign);
     else if (mode == 1) apply_usage(lp.usage, lp.present, e, sign);
     else
-      lp.cost[e] = live_cost(e, lp.base, lp.usage, lp.capa, lp.hist, lp.pres_fac, lp.hist_w, lp.via_mult,
-                             lp.base_w, lp.jitter);
+      set_cost(lp, e, weight_at(lp, e),
+               live_cost(e, lp.base, lp.usage, lp.capa, lp.hist, lp.pres_fac, lp.hist_w, lp.via_mult, lp.base_w,
+                         lp.jitter));
   }
 }
 
@@ -117,8 +141,9 @@ __global__ void snap_test_kernel(const int32_t *order, const int32_t *edges, con
     for (int32_t i = threadIdx.x; i < ne; i += blockDim.x) {
       const int32_t e = row[i];
       if (e < 0) continue;
-      lp.cost[e] = live_cost(e, lp.base, lp.usage, lp.capa, lp.hist, lp.pres_fac, lp.hist_w, lp.via_mult,
-                             lp.base_w, lp.jitter);
+      set_cost(lp, e, weight_at(lp, e),
+               live_cost(e, lp.base, lp.usage, lp.capa, lp.hist, lp.pres_fac, lp.hist_w, lp.via_mult, lp.base_w,
+                         lp.jitter));
       if (__ldcg(&owner[e]) < j) atomicOr(&hit, 1);
     }
   }
@@ -222,11 +247,12 @@ __global__ void __launch_bounds__(kWalkBlock) route_backtrace_kernel(RouteBt p) 
   __syncthreads();
   const int len = s_len;
   for (int i = threadIdx.x; i < len - 1; i += blockDim.x) {
-    const int32_t e = lat_step_edge(p.geom, p.slot_eid, p.vcol_eid, p.N, nodes[len - 1 - i], nodes[len - 2 - i]);
+    const int32_t u = nodes[len - 1 - i], v = nodes[len - 2 - i];
+    const int32_t e = lat_step_edge(p.geom, p.slot_eid, p.vcol_eid, p.N, u, v);
     edges[i] = e;
     if (e < 0) continue;
     if (!p.shared) {
-      use_edge(p.lp, e, 1);
+      use_edge(p.lp, e, p.lp.w4 ? 4 * (int64_t)v + lat_edge_slot(p.geom, u, v) : -1, 1);
     } else {
       apply_usage(p.lp.usage, p.lp.present, e, 1);
       if (p.owner) atomicMin(&p.owner[e], j);
@@ -397,7 +423,26 @@ static int route_nets_impl(orsp_graph *g, int32_t M, const int32_t *src_h, const
     }
   }
 
-  LiveParams lp{usage_d, present_d, base_d, cap_d, hist_d, pres_fac, hist_w, via_mult, base_w, jitter, cost_d};
+  // The searches' weights: gathered once for the whole lattice, from then on
+  // kept by the launches that change costs, where the boxes of the call hold as
+  // many cells as the lattice; else gathered per search.  (Gathered per search,
+  // they were 1.2 of 12.9 ms of kernels for 270 nets on 100 x 100 x 4, whose
+  // routing went from 14.1 to 12.8 ms, and 5.7 of 69.6 ms for 1 000 nets in
+  // groups of 32 on 600 x 600 x 18, where the whole run shows no difference: the
+  // gathers had brought the weights into L2.)  Column vias keep
+  // the gather: theirs is the smaller of two edges.
+  int64_t cells = 0;
+  for (int32_t i = 0; i < K; ++i) {
+    const int32_t *b = boxes_o.data() + (size_t)i * 6;
+    cells += (int64_t)(b[1] - b[0] + 1) * (b[3] - b[2] + 1) * (b[5] - b[4] + 1);
+  }
+  const bool kept = !g->cvia && cells >= g->N;
+  if (kept) {
+    rc = gather_lattice(g, cost_d, st);
+    if (rc) return rc;
+  }
+  LiveParams lp{usage_d, present_d, base_d, cap_d,  hist_d, pres_fac, hist_w,
+                via_mult, base_w,   jitter, cost_d, kept ? g->wslot : nullptr, g->indices, g->slot_eid, g->N};
   LatWalkGeom geom{};
   geom.nx = g->nx;
   geom.ny = g->ny;
@@ -431,6 +476,7 @@ static int route_nets_impl(orsp_graph *g, int32_t M, const int32_t *src_h, const
       opt.private_dist = true;
       opt.private_count = gcells[q];
       opt.copy_ctl = false;
+      opt.gathered = kept;
       opt.active = act;  // repair rounds: only the flagged boxes are gathered and reset
       int rc = run_lattice_boxes(g, cost_d, n, seed_r, nullptr, n, boxes_o.data() + (size_t)a * 6, d_box + a,
                                  g->route_pdist, st, &opt);
@@ -484,6 +530,7 @@ static int route_nets_impl(orsp_graph *g, int32_t M, const int32_t *src_h, const
     LatOptions opt;
     opt.fill_box_only = true;
     opt.copy_ctl = false;
+    opt.gathered = kept;
     rc = run_lattice_boxes(g, cost_d, n, d_src + a, nullptr, n, boxes_o.data() + (size_t)a * 6, d_box + a, g->dist,
                            st, &opt);
     if (rc) return rc;

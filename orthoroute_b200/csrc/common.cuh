@@ -187,6 +187,8 @@ struct LatOptions {
                                // `dist` is the slice arena of private_count entries, all reset
   int64_t private_count = 0;
   bool fill_box_only = false;  // reset distances inside the boxes only (the caller's backtrace checks the box)
+  void *ctl_d = nullptr;       // out: the launch's control block; with copy_ctl off the caller may bring it
+                               // (lat_ctl_words words) to lat_ctl_h by itself
   bool copy_ctl = true;        // copy the control block to the pinned mirror (finish_lattice_search)
   int *err_d = nullptr;        // out: device address of the launch's error word
   int blocks_per_sm = 0;       // CTAs per SM (0: one); ORSP_LAT_BLOCKS_PER_SM overrides
@@ -205,6 +207,7 @@ struct LatOptions {
 int run_lattice_search(Graph *g, const float *cost_d, int32_t nseeds, const int32_t *seeds_d,
                        const float *seed_cost_d, const int32_t *box, uint32_t *dist, cudaStream_t st,
                        LatOptions *opt = nullptr);
+int lat_ctl_words();
 // Gathers the weights of the whole lattice (adjacent vias) for searches with
 // LatOptions::gathered.
 int gather_lattice(Graph *g, const float *cost_d, cudaStream_t st);
@@ -230,7 +233,7 @@ int finish_lattice_search(Graph *g, int32_t *rounds_h);
 // Seeds outside the ROI are ignored.  finish_lattice_search reports the status.
 int run_lattice_roi(Graph *g, const float *cost_d, int32_t nseeds, const int32_t *seeds_d,
                     const float *seed_cost_d, const int32_t *roi_map_d, const int32_t *roi_nodes_d,
-                    int64_t n_roi, const uint8_t *sink_d, uint32_t *dist, cudaStream_t st);
+                    int64_t n_roi, const uint8_t *sink_d, uint32_t *dist, cudaStream_t st, LatOptions *opt = nullptr);
 // One search over a node-list ROI whose global_to_roi map is roi_map_d (ROI
 // index = rank, -1 outside), by one CTA of the batch kernel; *len_h gets the
 // batch kernel's path_len (nodes, 0 = no path, < 0 a per-search status).

@@ -191,16 +191,17 @@ __global__ void gather_kernel(const int32_t *__restrict__ slot_eid, const float 
   if (wmin) record_min(wmin, m);
 }
 
-// The same gather for the nodes of a box only (x fastest, then y, then z).
-__global__ void gather_box_kernel(const int32_t *__restrict__ slot_eid, const float *__restrict__ cost,
-                                  float4 *__restrict__ w, int64_t n, int32_t nx, int32_t ny, int32_t x0,
-                                  int32_t bw, int32_t y0, int32_t bh, int32_t z0, int64_t count) {
+// The same gather for the nodes of a box only (x fastest, then y, then z): cells
+// i, i + s, ... of it.
+__device__ __forceinline__ void gather_cells(const int32_t *__restrict__ slot_eid, const float *__restrict__ cost,
+                                             float4 *__restrict__ w, int64_t n, int32_t nx, int32_t ny, int32_t x0,
+                                             int64_t bw, int32_t y0, int64_t bh, int32_t z0, int64_t count, int64_t i,
+                                             int64_t s) {
   const float INF_F = __int_as_float(0x7f800000);
-  const int64_t s = (int64_t)gridDim.x * blockDim.x;
-  const int64_t plane = (int64_t)bw * bh;
+  const int64_t plane = bw * bh;
   BoxIndex bi;
   bi.init(bw, bh, count);
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += s) {
+  for (; i < count; i += s) {
     int32_t z, y, x;
     bi.split(i, plane, z, y, x);
     const int64_t v = ((int64_t)(z0 + z) * ny + (y0 + y)) * nx + (x0 + x);
@@ -208,6 +209,13 @@ __global__ void gather_box_kernel(const int32_t *__restrict__ slot_eid, const fl
     w[v] = make_float4(e0 >= 0 ? __ldg(&cost[e0]) : INF_F, e1 >= 0 ? __ldg(&cost[e1]) : INF_F,
                        e2 >= 0 ? __ldg(&cost[e2]) : INF_F, e3 >= 0 ? __ldg(&cost[e3]) : INF_F);
   }
+}
+
+__global__ void gather_box_kernel(const int32_t *__restrict__ slot_eid, const float *__restrict__ cost,
+                                  float4 *__restrict__ w, int64_t n, int32_t nx, int32_t ny, int32_t x0,
+                                  int32_t bw, int32_t y0, int32_t bh, int32_t z0, int64_t count) {
+  gather_cells(slot_eid, cost, w, n, nx, ny, x0, bw, y0, bh, z0, count,
+               (int64_t)blockIdx.x * blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
 }
 
 // The same gather for the nodes of several boxes in one launch: blockIdx.y
@@ -1610,20 +1618,44 @@ struct OwnParams {
   int32_t nseeds;
   const int32_t *seeds;
   const float *seed_cost;
+  int one;      // a single box, by value
+  LatBox box1;
+  // weights gathered by the launch's preparation (0: they are there, 1: of the
+  // boxes, 2: of the whole lattice)
+  int gather;
+  const int32_t *slot_eid;
+  const float *cost;
+  float4 *w;
 };
 constexpr int kOwnSeeds = 4096;
 
-// Prepares a launch: block 0 the control words and the seeds' messages, the
-// other blocks the exchange rows.
+__device__ __forceinline__ LatBox own_box(const OwnParams &o, int b) { return o.one ? o.box1 : load_box(o.l, b); }
+
+// Prepares a launch: block (0, 0) the control words and the seeds' messages, the
+// other blocks the exchange rows and the weights of box blockIdx.y: a search is
+// short enough for a launch of its own to show.
 __global__ void own_init_kernel(const __grid_constant__ OwnParams o) {
   const LatParams &p = o.l;
   const float INF_F = __int_as_float(0x7f800000);
   if (blockIdx.x > 0) {
-    const int64_t n = (int64_t)o.tcap * 2 * o.nr / 4, s = (int64_t)(gridDim.x - 1) * blockDim.x;
-    for (int64_t i = (int64_t)(blockIdx.x - 1) * blockDim.x + threadIdx.x; i < n; i += s)
+    const int64_t bx = (int64_t)blockIdx.y * (gridDim.x - 1) + blockIdx.x - 1;
+    const int64_t n = (int64_t)o.tcap * 2 * o.nr / 4, s = (int64_t)(gridDim.x - 1) * gridDim.y * blockDim.x;
+    for (int64_t i = bx * blockDim.x + threadIdx.x; i < n; i += s)
       ((float4 *)o.exch)[i] = make_float4(INF_F, INF_F, INF_F, INF_F);
+    if (o.gather) {
+      int32_t x0 = 0, y0 = 0, z0 = 0;
+      int64_t bw = p.nx, bh = p.ny, bd = p.nz;
+      if (o.gather == 1) {
+        const LatBox B = own_box(o, blockIdx.y);
+        x0 = B.x0, y0 = B.y0, z0 = B.z0;
+        bw = B.x1 - B.x0 + 1, bh = B.y1 - B.y0 + 1, bd = B.z1 - B.z0 + 1;
+      }
+      gather_cells(o.slot_eid, o.cost, o.w, p.N, p.nx, p.ny, x0, bw, y0, bh, z0, bw * bh * bd,
+                   (int64_t)(blockIdx.x - 1) * blockDim.x + threadIdx.x, (int64_t)(gridDim.x - 1) * blockDim.x);
+    }
     return;
   }
+  if (blockIdx.y > 0) return;
   LatCtl *c = p.ctl;
   if (threadIdx.x == 0) {
     c->err = 0;
@@ -1644,7 +1676,7 @@ __global__ void own_init_kernel(const __grid_constant__ OwnParams o) {
       const int32_t z = s / plane, r = s - z * plane, y = r / p.nx, x = r - y * p.nx;
       const int lo = p.seed_per_box ? i : 0, hi = p.seed_per_box ? min(i + 1, p.nbox) : p.nbox;
       for (int b = lo; b < hi && t < 0; ++b) {
-        const LatBox B = load_box(p, b);
+        const LatBox B = own_box(o, b);
         if (x >= B.x0 && x <= B.x1 && y >= B.y0 && y <= B.y1 && z >= B.z0 && z <= B.z1) t = tile_of<16, 16>(B, x, y);
       }
     }
@@ -1791,7 +1823,7 @@ __global__ void __launch_bounds__(RunTile<NZM, ZS>::NW + 32, MINB)
   const LatParams &p = o.l;
   const int t = blockIdx.x, tid = threadIdx.x;
   // the tile's box (a box sized on the device may have fewer tiles than the launch)
-  const LatBox B = load_box(p, p.nbox == 1 ? 0 : box_of_tile(p, t));
+  const LatBox B = own_box(o, p.nbox == 1 ? 0 : box_of_tile(p, t));
   const bool mine = t < B.tile0 + B.ntx * B.nty;
   const unsigned long long t_start = dev_globaltimer();
   if (tid < 4) Q.pub[tid] = 0;
@@ -2881,8 +2913,11 @@ void fill_axes(LatParams &p) {
   }
 }
 
+// one: the box of a single search (else the device table p.boxes); gather: see
+// OwnParams, with up to `blocks` blocks a box.
 int launch_own(orsp::Graph *g, LatParams &p, int64_t ntiles, const OwnShape &sh, int32_t nseeds, const int32_t *seeds,
-               const float *seed_cost, cudaStream_t st, orsp::LatOptions *opt) {
+               const float *seed_cost, cudaStream_t st, orsp::LatOptions *opt, const LatBox *one = nullptr,
+               int gather = 0, const float *cost = nullptr, int blocks = 0) {
   int rc = grow_own_ws(g, sh.ws);
   if (rc) return rc;
   if (!g->lat_ctl_h) ORSP_CUDA(cudaMallocHost(&g->lat_ctl_h, sizeof(LatCtl)));
@@ -2897,17 +2932,26 @@ int launch_own(orsp::Graph *g, LatParams &p, int64_t ntiles, const OwnShape &sh,
   o.sent = o.inbox + ntiles;
   o.got = o.sent + ntiles + 1;
   o.seedt = (int32_t *)(o.got + ntiles + 1);
-  if (opt) opt->err_d = &p.ctl->err;
+  if (opt) opt->err_d = &p.ctl->err, opt->ctl_d = p.ctl;
   p.wait_ns = env_u64("ORSP_WAIT_NS", 2000000000ull);
   p.budget_ns = env_u64("ORSP_BUDGET_NS", 20000000000ull);
   o.l = p;
+  o.one = one != nullptr;
+  if (one) o.box1 = *one;
+  o.gather = gather;
+  o.slot_eid = g->slot_eid;
+  o.cost = cost;
+  o.w = (float4 *)g->wslot;
   o.tcap = (int32_t)ntiles;
   o.nzb = sh.nzb;
   o.nseeds = nseeds;
   o.seeds = seeds;
   o.seed_cost = seed_cost;
   const int64_t rows = ntiles * 2 * o.nr / 4;
-  own_init_kernel<<<1 + (int)std::max<int64_t>(1, std::min<int64_t>((rows + 255) / 256, g->num_sms)), 256, 0, st>>>(o);
+  const unsigned init_y = gather == 1 ? p.nbox : 1;
+  const unsigned init_x = 1 + (unsigned)std::max<int64_t>({1, gather ? blocks : 0,
+                                                           std::min<int64_t>((rows + 255) / 256, g->num_sms) / init_y});
+  own_init_kernel<<<dim3(init_x, init_y), 256, 0, st>>>(o);
   ORSP_CUDA(cudaGetLastError());
   const int nzm = run_visit_layers(sh.nzb);
   const bool cv = p.wcol != nullptr, two = sh.per_sm == 2;
@@ -2967,7 +3011,7 @@ int launch_lattice(orsp::Graph *g, LatParams &p, int64_t ntiles, int64_t front, 
   p.qslot = async ? (int32_t *)(b + 4 * list_b) : nullptr;
   p.qcap = qcap;
   p.ctl = (LatCtl *)(b + 4 * list_b + q_b);
-  if (opt) opt->err_d = &p.ctl->err;
+  if (opt) opt->err_d = &p.ctl->err, opt->ctl_d = p.ctl;
   p.tbox = async ? p.list0 : nullptr;
   const bool live = use_live(g, ntiles, front, nzb, opt);
   OwnParams o{};
@@ -3248,6 +3292,8 @@ int64_t make_lat_boxes(const int32_t *boxes_h, int32_t nbox, LatBox *out) {
   return t0;
 }
 
+int lat_ctl_words() { return (int)(sizeof(LatCtl) / 4); }
+
 int gather_lattice(Graph *g, const float *cost_d, cudaStream_t st) {
   g->w4_cost = nullptr;  // the caller changes them from here on
   g->w4_gen = 0;
@@ -3302,6 +3348,16 @@ int run_lattice_boxes(Graph *g, const float *cost_d, int32_t nseeds, const int32
                                                                             148 * 32 / std::max(1, nbox)));
   OwnShape own;
   const bool owned = use_own(g, ntiles, nzb, nseeds, opt, &own);
+  // a single box without a device table: the owners take it by value
+  LatBox one{};
+  if (!lboxes_d) {
+    LatBox *hb = owned ? &one : (LatBox *)((char *)g->pinned + 1024);
+    make_lat_boxes(boxes_h, 1, hb);
+    if (!owned) {
+      ORSP_CUDA(cudaMemcpyAsync(g->lat_box_d, hb, sizeof(LatBox), cudaMemcpyHostToDevice, st));
+      lboxes_d = (const LatBox *)g->lat_box_d;
+    }
+  }
   // Boxes with targets, in the warp-specialised schedule only, whose scheduler
   // warp reads the target's distance off the workers' path (in the plain queue
   // schedule, with the boxes of routed nets, whose targets lie at their far
@@ -3313,8 +3369,14 @@ int run_lattice_boxes(Graph *g, const float *cost_d, int32_t nseeds, const int32
   const bool cached = decl != 0 && g->w4_cost == cost_d && g->w4_gen == decl && (!goals || g->w4_min);
   const bool all = !by_flag && (whole || (priv && vol_sum >= N));
   if (goals && !(all && cached)) ORSP_CUDA(cudaMemsetAsync(g->wmin, 0x7f, 2 * sizeof(int), st));
+  // the owners' preparation gathers along with the rest it does
+  const int own_gather = !owned || g->cvia || (opt && opt->gathered) || (all && cached) ? 0 : all ? 2 : 1;
   if (opt && opt->gathered) {
     // by gather_lattice, kept since
+  } else if (own_gather) {
+    g->w4_cost = all ? cost_d : nullptr;
+    g->w4_gen = all ? decl : 0;
+    g->w4_min = false;
   } else if (by_flag) {
     g->w4_cost = nullptr;  // part of wslot is rewritten
     g->w4_gen = 0;
@@ -3395,7 +3457,9 @@ int run_lattice_boxes(Graph *g, const float *cost_d, int32_t nseeds, const int32
   p.N = N;
   p.dist = dist;
   for (int z = 0; z < 64; ++z) p.axis[z] = z < g->nz ? g->layer_axis[z] : 0;
-  if (owned) return launch_own(g, p, ntiles, own, nseeds, seeds_d, seed_cost_d, st, opt);
+  if (owned)
+    return launch_own(g, p, ntiles, own, nseeds, seeds_d, seed_cost_d, st, opt, lboxes_d ? nullptr : &one, own_gather,
+                      cost_d, (int)std::min<int64_t>(((own_gather == 2 ? N : vmax) + 255) / 256, 148 * 32 / std::max(1, nbox)));
   return launch_lattice(g, p, ntiles, front, nzb, nseeds, seeds_d, seed_cost_d, st, opt);
 }
 
@@ -3405,16 +3469,12 @@ int run_lattice_search(Graph *g, const float *cost_d, int32_t nseeds, const int3
   const int32_t full[6] = {0, g->nx - 1, 0, g->ny - 1, 0, g->nz - 1};
   const int32_t *b = box ? box : full;
   if (!g->lat_box_d) ORSP_CUDA(cudaMalloc(&g->lat_box_d, sizeof(LatBox)));
-  LatBox *hb = (LatBox *)((char *)g->pinned + 1024);
-  make_lat_boxes(b, 1, hb);
-  ORSP_CUDA(cudaMemcpyAsync(g->lat_box_d, hb, sizeof(LatBox), cudaMemcpyHostToDevice, st));
-  return run_lattice_boxes(g, cost_d, nseeds, seeds_d, seed_cost_d, 1, b, (const LatBox *)g->lat_box_d, dist, st,
-                           opt);
+  return run_lattice_boxes(g, cost_d, nseeds, seeds_d, seed_cost_d, 1, b, nullptr, dist, st, opt);
 }
 
 int run_lattice_roi(Graph *g, const float *cost_d, int32_t nseeds, const int32_t *seeds_d,
                     const float *seed_cost_d, const int32_t *roi_map_d, const int32_t *roi_nodes_d,
-                    int64_t n_roi, const uint8_t *sink_d, uint32_t *dist, cudaStream_t st) {
+                    int64_t n_roi, const uint8_t *sink_d, uint32_t *dist, cudaStream_t st, LatOptions *opt) {
   const int64_t N = g->N;
   constexpr int TX = 16, TY = 16;
   if (!g->lat_box_d) ORSP_CUDA(cudaMalloc(&g->lat_box_d, sizeof(LatBox)));
@@ -3472,9 +3532,9 @@ int run_lattice_roi(Graph *g, const float *cost_d, int32_t nseeds, const int32_t
   // the box is known on the device only: size the tile arrays for the lattice
   const int64_t tx = (g->nx - 1 + TX) / TX, ty = (g->ny - 1 + TY) / TY, ntiles = tx * ty;
   OwnShape own;
-  if (use_own(g, ntiles, g->nz, nseeds, nullptr, &own))
-    return launch_own(g, p, ntiles, own, nseeds, seeds_d, seed_cost_d, st, nullptr);
-  return launch_lattice(g, p, ntiles, tx + ty, g->nz, nseeds, seeds_d, seed_cost_d, st, nullptr);
+  if (use_own(g, ntiles, g->nz, nseeds, opt, &own))
+    return launch_own(g, p, ntiles, own, nseeds, seeds_d, seed_cost_d, st, opt);
+  return launch_lattice(g, p, ntiles, tx + ty, g->nz, nseeds, seeds_d, seed_cost_d, st, opt);
 }
 
 int finish_lattice_search(Graph *g, int32_t *rounds_h) {

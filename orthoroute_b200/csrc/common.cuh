@@ -187,6 +187,10 @@ struct LatOptions {
                                // `dist` is the slice arena of private_count entries, all reset
   int64_t private_count = 0;
   bool fill_box_only = false;  // reset distances inside the boxes only (the caller's backtrace checks the box)
+  bool parents = false;        // the distances serve one walk per box from its target to its one seed (cost 0)
+                               // only: the launch may record parents instead
+  const uint8_t *par_d = nullptr;  // out: the parents recorded (lattice_walk.cuh), NULL: distances as usual
+  int par_tile_bytes = 0, par_smem = 0;  // out: their bytes per tile, and in the box with the most tiles
   void *ctl_d = nullptr;       // out: the launch's control block; with copy_ctl off the caller may bring it
                                // (lat_ctl_words words) to lat_ctl_h by itself
   bool copy_ctl = true;        // copy the control block to the pinned mirror (finish_lattice_search)

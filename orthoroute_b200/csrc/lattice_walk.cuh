@@ -223,10 +223,12 @@ __device__ __forceinline__ bool lat_run_cell(const LatWalkGeom &G, const LatBox 
 // 1.51 ms, now 1.01.
 constexpr int kWalkSide = 14, kWalkVia = 3;  // 1 + 2 * kWalkSide + kWalkVia lanes
 
-template <class DIST, class STOP, class RANK = LatRankId>
-__device__ __forceinline__ int lat_walk_warp(const LatWalkGeom &G, const LatBox &B, const float4 *__restrict__ w4,
-                                             DIST dist, STOP stop, int32_t x, int32_t y, int32_t z, int32_t *out,
-                                             int32_t cap, RANK rank = RANK()) {
+//
+// PARENT(x, y, z, bits, px, py, pz): the slot of a cell's parent (-1: none), its
+// distance bits and the parent's coordinates.
+template <class PARENT, class STOP>
+__device__ __forceinline__ int lat_walk_by(const LatWalkGeom &G, const LatBox &B, PARENT parent, STOP stop, int32_t x,
+                                           int32_t y, int32_t z, int32_t *out, int32_t cap) {
   static_assert(1 + 2 * kWalkSide + kWalkVia == 32, "one warp");
   const int lane = threadIdx.x & 31;
   int len = 0;
@@ -246,8 +248,8 @@ __device__ __forceinline__ int lat_walk_warp(const LatWalkGeom &G, const LatBox 
     const int64_t c = ((int64_t)cz * G.ny + cy) * G.nx + cx;
     int ps = -1;
     int32_t px = 0, py = 0, pz = 0;
-    unsigned dc = ORSP_INF_BITS, pdu = 0;
-    if (valid) ps = lat_parent(G, B, w4, dist, cx, cy, cz, dc, px, py, pz, pdu, rank);
+    unsigned dc = ORSP_INF_BITS;
+    if (valid) ps = parent(cx, cy, cz, dc, px, py, pz);
     if (len == 0 && __shfl_sync(ORSP_FULL_MASK, dc, 0) == ORSP_INF_BITS) return 0;
     const bool is_stop = dc != ORSP_INF_BITS && stop(c, dc);
     const unsigned m = __ballot_sync(ORSP_FULL_MASK, lane && !is_stop && ps == sl && step < n);
@@ -274,6 +276,60 @@ __device__ __forceinline__ int lat_walk_warp(const LatWalkGeom &G, const LatBox 
     y = __shfl_sync(ORSP_FULL_MASK, py, end);
     z = __shfl_sync(ORSP_FULL_MASK, pz, end);
   }
+}
+
+// The walk on distances and weights.
+template <class DIST, class STOP, class RANK = LatRankId>
+__device__ __forceinline__ int lat_walk_warp(const LatWalkGeom &G, const LatBox &B, const float4 *__restrict__ w4,
+                                             DIST dist, STOP stop, int32_t x, int32_t y, int32_t z, int32_t *out,
+                                             int32_t cap, RANK rank = RANK()) {
+  auto parent = [&](int32_t cx, int32_t cy, int32_t cz, unsigned &dc, int32_t &px, int32_t &py, int32_t &pz) {
+    unsigned pdu;
+    return lat_parent(G, B, w4, dist, cx, cy, cz, dc, px, py, pz, pdu, rank);
+  };
+  return lat_walk_by(G, B, parent, stop, x, y, z, out, cap);
+}
+
+// Parents recorded by the search (owner schedule, LatOptions::parents): four
+// bits per cell - the slot, kParNone, or kParFar where the cell is not reached -
+// two layers to a byte, 16 x 16 bytes per pair of layers, tile after tile.
+constexpr unsigned kParNone = 4, kParFar = 7;
+struct LatParents {
+  const uint8_t *par;  // NULL: not recorded
+  int32_t tile_bytes;
+};
+
+// Brings box B's parents to shared memory, by the whole block; every thread's
+// copies have landed when it returns (a barrier is still due).
+__device__ __forceinline__ void lat_load_parents(const LatParents &P, const LatBox &B, uint8_t *sm) {
+  const int n = B.ntx * B.nty * P.tile_bytes;
+  const uint8_t *src = P.par + (int64_t)B.tile0 * P.tile_bytes;
+  const uint32_t to = (uint32_t)__cvta_generic_to_shared(sm);
+  for (int i = threadIdx.x * 16; i < n; i += blockDim.x * 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + i), "l"(src + i) : "memory");
+  asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+// The walk on recorded parents, from (x, y, z) to node src, whose distance is 0.
+// A round takes a trip to shared memory instead of one to L2.
+__device__ __forceinline__ int lat_walk_parents(const LatWalkGeom &G, const LatBox &B, const LatParents &P,
+                                                const uint8_t *sm, int64_t src, int32_t x, int32_t y, int32_t z,
+                                                int32_t *out, int32_t cap) {
+  auto parent = [&](int32_t cx, int32_t cy, int32_t cz, unsigned &dc, int32_t &px, int32_t &py, int32_t &pz) {
+    const int lx = cx - B.x0, ly = cy - B.y0, lz = cz - B.z0;
+    const int at = ((ly >> 4) * B.ntx + (lx >> 4)) * P.tile_bytes + (lz >> 1) * 256 + (ly & 15) * 16 + (lx & 15);
+    const unsigned s = (sm[at] >> ((lz & 1) * 4)) & 15u;
+    dc = s == kParFar ? ORSP_INF_BITS : 0u;
+    if (s >= kParNone) return -1;
+    const bool h = G.axis[cz] == 1;
+    const int d = s & 1 ? 1 : -1;
+    px = cx + (s < 2 && h ? d : 0);
+    py = cy + (s < 2 && !h ? d : 0);
+    pz = cz + (s < 2 ? 0 : d);
+    return (int)s;
+  };
+  auto at_src = [src](int64_t v, unsigned) { return v == src; };
+  return lat_walk_by(G, B, parent, at_src, x, y, z, out, cap);
 }
 
 // Whether the lattice edge u -> v is a via: a planar step changes the id by 1
@@ -308,5 +364,7 @@ __device__ __forceinline__ int32_t lat_step_edge(const LatWalkGeom &G, const int
 }
 
 constexpr int kWalkBlock = 128;  // warp 0 walks, the block reverses the path and maps its edges
+constexpr int kParBlock = 512;   // the same with recorded parents, which the block loads
+constexpr int kParSmem = 200 * 1024;  // parents of a box at most
 
 }  // namespace orsp

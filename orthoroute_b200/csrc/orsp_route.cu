@@ -194,6 +194,7 @@ struct RouteBt {
   bool shared;     // snapshot groups: nets may share edges, so only the usage is counted here
   int32_t *owner;  // snapshot groups with another round to come: marks of the edges used
   LiveParams lp;
+  orsp::LatParents par;  // recorded parents (dynamic shared memory holds a box's)
 };
 
 // Steps 3 and 4, one block per net of the group (block j: net order[j]).  Warp
@@ -207,7 +208,8 @@ struct RouteBt {
 // edge u -> v of path_to_edges), commits it and reverses the path.
 // Bound by the walk's chain of loads and by the launch: the commit as a launch
 // of its own cost 2.1 us of a 100 x 100 x 4 net's 40.
-__global__ void __launch_bounds__(kWalkBlock) route_backtrace_kernel(RouteBt p) {
+__global__ void __launch_bounds__(orsp::kParBlock) route_backtrace_kernel(const __grid_constant__ RouteBt p) {
+  extern __shared__ __align__(16) uint8_t s_par[];
   __shared__ int s_len;
   const int j = blockIdx.x;
   if (p.active && !p.active[j]) return;
@@ -218,6 +220,10 @@ __global__ void __launch_bounds__(kWalkBlock) route_backtrace_kernel(RouteBt p) 
   int32_t *edges = p.net_edges + (int64_t)k * p.cap;
   int32_t *len_out = p.net_lens + k;
   const int serr = *p.search_err;
+  if (p.par.par) {
+    orsp::lat_load_parents(p.par, B, s_par);
+    __syncthreads();
+  }
   if (threadIdx.x < 32) {
     int len = 0;
     if (!serr) {
@@ -234,7 +240,8 @@ __global__ void __launch_bounds__(kWalkBlock) route_backtrace_kernel(RouteBt p) 
       };
       if (src >= 0 && dst_in && dst != src) {
         auto at_src = [src](int64_t v, unsigned d) { return v == src && d == 0u; };
-        len = lat_walk_warp(p.geom, B, p.w4, dget, at_src, x, y, z, nodes, p.cap);
+        if (p.par.par) len = orsp::lat_walk_parents(p.geom, B, p.par, s_par, src, x, y, z, nodes, p.cap);
+        else len = lat_walk_warp(p.geom, B, p.w4, dget, at_src, x, y, z, nodes, p.cap);
       }
     }
     if (threadIdx.x == 0) {
@@ -531,6 +538,7 @@ static int route_nets_impl(orsp_graph *g, int32_t M, const int32_t *src_h, const
     opt.fill_box_only = true;
     opt.copy_ctl = false;
     opt.gathered = kept;
+    opt.parents = true;
     rc = run_lattice_boxes(g, cost_d, n, d_src + a, nullptr, n, boxes_o.data() + (size_t)a * 6, d_box + a, g->dist,
                            st, &opt);
     if (rc) return rc;
@@ -552,7 +560,13 @@ static int route_nets_impl(orsp_graph *g, int32_t M, const int32_t *src_h, const
     bt.search_err = opt.err_d;
     bt.route_err = route_err;
     bt.lp = lp;
-    route_backtrace_kernel<<<n, kWalkBlock, 0, st>>>(bt);
+    if (opt.par_d) {
+      bt.par = {opt.par_d, opt.par_tile_bytes};
+      ORSP_CUDA(cudaFuncSetAttribute(route_backtrace_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kParSmem));
+      route_backtrace_kernel<<<n, kParBlock, opt.par_smem, st>>>(bt);
+    } else {
+      route_backtrace_kernel<<<n, kWalkBlock, 0, st>>>(bt);
+    }
     ORSP_CUDA(cudaGetLastError());
     return rc;
   };

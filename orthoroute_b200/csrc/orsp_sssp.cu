@@ -373,6 +373,7 @@ struct LatBacktraceParams {
   const unsigned *lat_ctl;
   unsigned *lat_ctl_h;
   int lat_words;
+  orsp::LatParents par;  // recorded parents (dynamic shared memory holds the box's)
 };
 
 __device__ __forceinline__ void lat_outcome(const LatBacktraceParams &p, int err, int len, int status) {
@@ -384,7 +385,8 @@ __device__ __forceinline__ void lat_outcome(const LatBacktraceParams &p, int err
   }
 }
 
-__global__ void __launch_bounds__(orsp::kWalkBlock) lat_backtrace_kernel(LatBacktraceParams p) {
+__global__ void __launch_bounds__(orsp::kParBlock) lat_backtrace_kernel(const __grid_constant__ LatBacktraceParams p) {
+  extern __shared__ __align__(16) uint8_t s_par[];
   __shared__ int s_len;
   const LatBox &B = p.box;
   const int32_t dst = p.dst_d ? *p.dst_d : p.dst;
@@ -410,9 +412,14 @@ __global__ void __launch_bounds__(orsp::kWalkBlock) lat_backtrace_kernel(LatBack
     for (int i = 0; i < nseeds; ++i) hit |= seeds[i] == v && f_bits(seed_cost ? seed_cost[i] : 0.0f) == d;
     return hit;
   };
+  if (p.par.par) {
+    orsp::lat_load_parents(p.par, B, s_par);
+    __syncthreads();
+  }
   if (threadIdx.x < 32) {
     int len;
-    if (p.rank_map) len = lat_walk_warp(p.geom, B, p.w4, dget, at_start, x, y, z, p.path_out, p.path_cap,
+    if (p.par.par) len = orsp::lat_walk_parents(p.geom, B, p.par, s_par, seeds[0], x, y, z, p.path_out, p.path_cap);
+    else if (p.rank_map) len = lat_walk_warp(p.geom, B, p.w4, dget, at_start, x, y, z, p.path_out, p.path_cap,
                                         orsp::LatRankRoi{p.rank_map});
     else len = lat_walk_warp(p.geom, B, p.w4, dget, at_start, x, y, z, p.path_out, p.path_cap);
     if (threadIdx.x == 0) s_len = len;
@@ -666,6 +673,7 @@ static int sssp_impl(orsp_graph *g, const float *cost_d, int32_t nseeds, const i
     roi_map_d = g->box_g2r;
   }
   LatOptions lopt;
+  lopt.parents = dst >= 0 && !dist_out_d && nseeds == 1 && !seed_cost_d;
   lopt.copy_ctl = dst < 0;  // with a target the backtrace reports for both
   if (lattice && dst < 0) ORSP_CUDA(cudaMemsetAsync(g->ctl, 0, sizeof(SsspCtl), st));
   if (lattice_roi) {
@@ -701,6 +709,8 @@ static int sssp_impl(orsp_graph *g, const float *cost_d, int32_t nseeds, const i
     b.box.z0 = bx[4];
     b.box.z1 = bx[5];
     b.box.dbase = -1;
+    b.box.ntx = (bx[1] - bx[0] + 16) / 16;
+    b.box.nty = (bx[3] - bx[2] + 16) / 16;
     b.seeds = seeds_d;
     b.seed_cost = seed_cost_d;
     b.nseeds = nseeds;
@@ -708,7 +718,13 @@ static int sssp_impl(orsp_graph *g, const float *cost_d, int32_t nseeds, const i
     b.path_out = path_out_d;
     b.path_cap = path_cap;
     lat_report(g, lopt, &b);
-    lat_backtrace_kernel<<<1, orsp::kWalkBlock, 0, st>>>(b);
+    if (lopt.par_d) {
+      b.par = {lopt.par_d, lopt.par_tile_bytes};
+      ORSP_CUDA(cudaFuncSetAttribute(lat_backtrace_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kParSmem));
+      lat_backtrace_kernel<<<1, kParBlock, lopt.par_smem, st>>>(b);
+    } else {
+      lat_backtrace_kernel<<<1, kWalkBlock, 0, st>>>(b);
+    }
     ORSP_CUDA(cudaGetLastError());
   } else if (dst >= 0) {
     BacktraceParams b{};

@@ -7,6 +7,7 @@
 // float32 numpy expression of the reference function it replaces (numpy >= 2
 // keeps Python-float scalars "weak", so every operand is rounded to float32).
 #include <algorithm>
+#include <cstring>
 #include <initializer_list>
 
 #include "accounting.cuh"
@@ -35,6 +36,18 @@ struct alignas(sizeof(T) * V) Vec {
 template <int V, typename T>
 __device__ __forceinline__ Vec<V, T> ldv(const T *p, int64_t i) {
   return *reinterpret_cast<const Vec<V, T> *>(p + i * V);
+}
+// The same from an array that the launch does not write.
+template <int V, typename T>
+__device__ __forceinline__ Vec<V, T> ldr(const T *p, int64_t i) {
+  Vec<V, T> x;
+  if constexpr (sizeof(x) == 16) {
+    const uint4 u = __ldg(reinterpret_cast<const uint4 *>(p + i * V));
+    memcpy(&x, &u, 16);
+  } else {
+    x = ldv<V>(p, i);
+  }
+  return x;
 }
 template <int V, typename T>
 __device__ __forceinline__ void stv(T *p, int64_t i, const Vec<V, T> &x) {
@@ -83,11 +96,31 @@ __device__ __forceinline__ float cost_of(const CostParams &p, int64_t e, float b
   return total;
 }
 
-template <int V, bool BIAS>
-__global__ void update_costs_kernel(int64_t first, int64_t n, CostParams p) {
+// One whole-array update: op.at<V>(i) is its step on the V edges from V i.  The
+// last E mod V edges go along in the same launch, one a thread (a launch of
+// their own for each update made small arrays slower than single edges were).
+template <int V, class Op>
+__global__ void edges_kernel(int64_t E, Op op) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = first / V + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < first / V + n; i += stride) {
-    const Vec<V, float> b = ldv<V>(p.base, i), m = ldv<V>(p.ema, i), c = ldv<V>(p.cap, i), h = ldv<V>(p.hist, i);
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t n = E / V;
+  for (int64_t i = t; i < n; i += stride) op.template at<V>(i);
+  if (V > 1 && t < E % V) op.template at<1>(E - 1 - t);
+}
+template <class Op>
+int over_edges(int64_t E, bool vec, const Op &op, cudaStream_t st) {
+  if (vec) edges_kernel<4><<<grid_for((E + 3) / 4), 256, 0, st>>>(E, op);
+  else edges_kernel<1><<<grid_for(E), 256, 0, st>>>(E, op);
+  ORSP_CUDA(cudaGetLastError());
+  return ORSP_OK;
+}
+
+template <bool BIAS>
+struct CostOp {
+  CostParams p;
+  template <int V>
+  __device__ __forceinline__ void at(int64_t i) const {
+    const Vec<V, float> b = ldr<V>(p.base, i), m = ldr<V>(p.ema, i), c = ldr<V>(p.cap, i), h = ldr<V>(p.hist, i);
     Vec<V, uint8_t> l{}, k{};
     if (BIAS) {
       l = ldv<V>(p.layer, i);
@@ -98,25 +131,27 @@ __global__ void update_costs_kernel(int64_t first, int64_t n, CostParams p) {
     for (int j = 0; j < V; ++j) o.v[j] = cost_of<BIAS>(p, i * V + j, b.v[j], m.v[j], c.v[j], h.v[j], l.v[j], k.v[j]);
     stv<V>(p.out, i, o);
   }
-}
+};
 
 // The live costs of all edges (edges == nullptr, V edges per step).
-template <int V>
-__global__ void live_costs_all_kernel(int64_t first, int64_t n, const float *__restrict__ base,
-                                      const int32_t *__restrict__ usage, const float *__restrict__ cap,
-                                      const float *__restrict__ hist, float pres_fac, float hist_w, float via_mult,
-                                      float base_w, int jitter, float *__restrict__ out) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = first / V + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < first / V + n; i += stride) {
-    const Vec<V, float> b = ldv<V>(base, i), c = ldv<V>(cap, i), h = ldv<V>(hist, i);
-    const Vec<V, int32_t> u = ldv<V>(usage, i);
+struct LiveCostOp {
+  const float *base;
+  const int32_t *usage;
+  const float *cap, *hist;
+  float pres_fac, hist_w, via_mult, base_w;
+  int jitter;
+  float *out;
+  template <int V>
+  __device__ __forceinline__ void at(int64_t i) const {
+    const Vec<V, float> b = ldr<V>(base, i), c = ldr<V>(cap, i), h = ldr<V>(hist, i);
+    const Vec<V, int32_t> u = ldr<V>(usage, i);
     Vec<V, float> o;
 #pragma unroll
     for (int j = 0; j < V; ++j)
       o.v[j] = orsp::live_cost_of(i * V + j, b.v[j], u.v[j], c.v[j], h.v[j], pres_fac, hist_w, via_mult, base_w, jitter);
     stv<V>(out, i, o);
   }
-}
+};
 
 __global__ void live_costs_kernel(int64_t n, const int32_t *__restrict__ edges, const float *__restrict__ base,
                                   const int32_t *__restrict__ usage, const float *__restrict__ cap,
@@ -149,29 +184,29 @@ __global__ void live_costs_paths_kernel(int32_t K, const int32_t *__restrict__ p
 }
 
 // EdgeAccountant.update_present_ema (UPF:963-971).
-template <int V>
-__global__ void ema_kernel(int64_t first, int64_t n, const float *__restrict__ present, float *__restrict__ ema,
-                           float beta, float omb) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = first / V + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < first / V + n; i += stride) {
-    const Vec<V, float> p = ldv<V>(present, i);
+struct EmaOp {
+  const float *present;
+  float *ema, beta, omb;
+  template <int V>
+  __device__ __forceinline__ void at(int64_t i) const {
+    const Vec<V, float> p = ldr<V>(present, i);
     Vec<V, float> m = ldv<V>(ema, i);
 #pragma unroll
     for (int j = 0; j < V; ++j) m.v[j] = __fadd_rn(__fmul_rn(beta, p.v[j]), __fmul_rn(omb, m.v[j]));
     stv<V>(ema, i, m);
   }
-}
+};
 
 // EdgeAccountant.update_history (UPF:898-961).
-template <int V>
-__global__ void history_kernel(int64_t first, int64_t n, float *__restrict__ hist,
-                               const float *__restrict__ present, const float *__restrict__ cap,
-                               const float *__restrict__ base, float gain, float cap_mult, float decay) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = first / V + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < first / V + n; i += stride) {
-    const Vec<V, float> p = ldv<V>(present, i), c = ldv<V>(cap, i);
+struct HistoryOp {
+  float *hist;
+  const float *present, *cap, *base;
+  float gain, cap_mult, decay;
+  template <int V>
+  __device__ __forceinline__ void at(int64_t i) const {
+    const Vec<V, float> p = ldr<V>(present, i), c = ldr<V>(cap, i);
     Vec<V, float> h = ldv<V>(hist, i), b{};
-    if (base) b = ldv<V>(base, i);
+    if (base) b = ldr<V>(base, i);
 #pragma unroll
     for (int j = 0; j < V; ++j) {
       const float kept = __fmul_rn(h.v[j], decay);
@@ -186,7 +221,7 @@ __global__ void history_kernel(int64_t first, int64_t n, float *__restrict__ his
     }
     stv<V>(hist, i, h);
   }
-}
+};
 
 // EdgeAccountant.compute_overuse (UPF:838-876), edge part.  acc: the float64
 // sum, the count, and the number of blocks done; the last block writes the
@@ -249,35 +284,18 @@ __global__ void overuse_kernel(int64_t E, const float *__restrict__ present, con
   }
 }
 
-template <int V>
-__global__ void present_from_usage_kernel(int64_t first, int64_t n, const int32_t *__restrict__ usage,
-                                          float *__restrict__ present) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = first / V + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < first / V + n; i += stride) {
-    const Vec<V, int32_t> u = ldv<V>(usage, i);
+struct PresentOp {
+  const int32_t *usage;
+  float *present;
+  template <int V>
+  __device__ __forceinline__ void at(int64_t i) const {
+    const Vec<V, int32_t> u = ldr<V>(usage, i);
     Vec<V, float> p;
 #pragma unroll
     for (int j = 0; j < V; ++j) p.v[j] = (float)u.v[j];
     stv<V>(present, i, p);
   }
-}
-
-// Launches `four(first, n)` over the n groups of four edges from edge `first`
-// when the arrays are aligned for it, and `one(first, n)` over the n single
-// edges left.
-template <class Four, class One>
-int over_edges(int64_t E, bool vec, Four four, One one) {
-  const int64_t n4 = vec ? E / 4 : 0;
-  if (n4) {
-    four((int64_t)0, n4);
-    ORSP_CUDA(cudaGetLastError());
-  }
-  if (E > 4 * n4) {
-    one(4 * n4, E - 4 * n4);
-    ORSP_CUDA(cudaGetLastError());
-  }
-  return ORSP_OK;
-}
+};
 
 __global__ void commit_kernel(int64_t n, const int32_t *__restrict__ edges,
                               int32_t *__restrict__ usage, float *__restrict__ present,
@@ -362,27 +380,15 @@ extern "C" int orsp_update_costs(int64_t E, const float *base, const float *ema,
   if (E == 0) return ORSP_OK;
   const CostParams p{base, ema, cap, hist, layer, kind, lbias, pres_fac, hist_w, via_mult, base_w, add_jitter, out};
   cudaStream_t st = (cudaStream_t)stream;
-  return over_edges(
-      E, aligned_to(16, {base, ema, cap, hist, out}) && aligned_to(4, {layer, kind}),
-      [&](int64_t a, int64_t n) {
-        if (lbias) update_costs_kernel<4, true><<<grid_for(n), 256, 0, st>>>(a, n, p);
-        else update_costs_kernel<4, false><<<grid_for(n), 256, 0, st>>>(a, n, p);
-      },
-      [&](int64_t a, int64_t n) {
-        if (lbias) update_costs_kernel<1, true><<<grid_for(n), 256, 0, st>>>(a, n, p);
-        else update_costs_kernel<1, false><<<grid_for(n), 256, 0, st>>>(a, n, p);
-      });
+  const bool vec = aligned_to(16, {base, ema, cap, hist, out}) && aligned_to(4, {layer, kind});
+  return lbias ? over_edges(E, vec, CostOp<true>{p}, st) : over_edges(E, vec, CostOp<false>{p}, st);
 }
 
 extern "C" int orsp_update_present_ema(int64_t E, const float *present, float *ema,
                                        float beta, float omb, uintptr_t stream) {
   if (E < 0 || (E > 0 && (!present || !ema))) { set_error("ema: NULL array"); return ORSP_ERR_ARG; }
   if (E == 0) return ORSP_OK;
-  cudaStream_t st = (cudaStream_t)stream;
-  return over_edges(
-      E, aligned_to(16, {present, ema}),
-      [&](int64_t a, int64_t n) { ema_kernel<4><<<grid_for(n), 256, 0, st>>>(a, n, present, ema, beta, omb); },
-      [&](int64_t a, int64_t n) { ema_kernel<1><<<grid_for(n), 256, 0, st>>>(a, n, present, ema, beta, omb); });
+  return over_edges(E, aligned_to(16, {present, ema}), EmaOp{present, ema, beta, omb}, (cudaStream_t)stream);
 }
 
 extern "C" int orsp_update_history(int64_t E, float *hist, const float *present,
@@ -390,15 +396,8 @@ extern "C" int orsp_update_history(int64_t E, float *hist, const float *present,
                                    float cap_mult, float decay, uintptr_t stream) {
   if (E < 0 || (E > 0 && (!hist || !present || !cap))) { set_error("history: NULL array"); return ORSP_ERR_ARG; }
   if (E == 0) return ORSP_OK;
-  cudaStream_t st = (cudaStream_t)stream;
-  return over_edges(
-      E, aligned_to(16, {hist, present, cap, base}),
-      [&](int64_t a, int64_t n) {
-        history_kernel<4><<<grid_for(n), 256, 0, st>>>(a, n, hist, present, cap, base, gain, cap_mult, decay);
-      },
-      [&](int64_t a, int64_t n) {
-        history_kernel<1><<<grid_for(n), 256, 0, st>>>(a, n, hist, present, cap, base, gain, cap_mult, decay);
-      });
+  return over_edges(E, aligned_to(16, {hist, present, cap, base}),
+                    HistoryOp{hist, present, cap, base, gain, cap_mult, decay}, (cudaStream_t)stream);
 }
 
 namespace orsp {
@@ -441,11 +440,7 @@ extern "C" int orsp_present_from_usage(int64_t E, const int32_t *usage, float *p
                                        uintptr_t stream) {
   if (E < 0 || (E > 0 && (!usage || !present))) { set_error("present_from_usage: NULL array"); return ORSP_ERR_ARG; }
   if (E == 0) return ORSP_OK;
-  cudaStream_t st = (cudaStream_t)stream;
-  return over_edges(
-      E, aligned_to(16, {usage, present}),
-      [&](int64_t a, int64_t n) { present_from_usage_kernel<4><<<grid_for(n), 256, 0, st>>>(a, n, usage, present); },
-      [&](int64_t a, int64_t n) { present_from_usage_kernel<1><<<grid_for(n), 256, 0, st>>>(a, n, usage, present); });
+  return over_edges(E, aligned_to(16, {usage, present}), PresentOp{usage, present}, (cudaStream_t)stream);
 }
 
 extern "C" int orsp_commit_edges(int64_t n, const int32_t *edges, int32_t *usage,
@@ -507,16 +502,8 @@ extern "C" int orsp_update_costs_live(int64_t E, const int32_t *edges, int64_t n
   if (n == 0) return ORSP_OK;
   cudaStream_t st = (cudaStream_t)stream;
   if (!edges)
-    return over_edges(
-        E, aligned_to(16, {base, usage, cap, hist, out}),
-        [&](int64_t a, int64_t m) {
-          live_costs_all_kernel<4><<<grid_for(m), 256, 0, st>>>(a, m, base, usage, cap, hist, pres_fac, hist_w,
-                                                                via_mult, base_w, add_jitter, out);
-        },
-        [&](int64_t a, int64_t m) {
-          live_costs_all_kernel<1><<<grid_for(m), 256, 0, st>>>(a, m, base, usage, cap, hist, pres_fac, hist_w,
-                                                                via_mult, base_w, add_jitter, out);
-        });
+    return over_edges(E, aligned_to(16, {base, usage, cap, hist, out}),
+                      LiveCostOp{base, usage, cap, hist, pres_fac, hist_w, via_mult, base_w, add_jitter, out}, st);
   live_costs_kernel<<<grid_for(n), 256, 0, st>>>(n, edges, base, usage, cap, hist, pres_fac, hist_w, via_mult, base_w,
                                                  add_jitter, out);
   ORSP_CUDA(cudaGetLastError());

@@ -1257,6 +1257,52 @@ __host__ __device__ constexpr int pw_x_bytes() { return PL_X * PL_Y * CIN * 2; }
 template <int COUT>
 __host__ __device__ constexpr int pw_g_bytes() { return PL_X * PL_ROWS * COUT * 2; }
 
+// The CTA's share of dW pair by pair, where its accumulators are not finite:
+// the tiles are padded with zeros on both sides, and a zero meets an infinity
+// or a NaN of the border there that no pair of the sum holds.  The pairs are X[v
+// + tap] and G[v] for v in the grid (X zero outside it), as the zero-padded
+// convolution has them; rows and planes of X just outside the grid go with the
+// border tiles.  Every warp takes 32 rows (dx, ci) x 16 columns of a (dz, dy).
+template <int CIN, int COUT>
+__device__ __noinline__ void wgrad_pairs(const __nv_bfloat16 *__restrict__ X, const __nv_bfloat16 *__restrict__ dY,
+                                         const __nv_bfloat16 *__restrict__ Yo, float *__restrict__ dW, int D, int H,
+                                         int W, const PlanePlan &plan) {
+  constexpr int MT = (3 * CIN + 31) / 32, CT = COUT / 16;
+  const int lane = threadIdx.x & 31;
+  for (int task = threadIdx.x >> 5; task < MT * CT * 9; task += PW_THREADS / 32) {
+    const int m = task % MT * 32 + lane, c0 = task / MT % CT * 16, dz = task / (MT * CT) / 3, dy = task / (MT * CT) % 3;
+    const int dx = m / CIN, ci = m % CIN;
+    float acc[16] = {};
+    for (int u = blockIdx.x; u < plan.units; u += gridDim.x) {
+      const PlaneUnit un(plan, u, D);
+      const int y0 = un.y * PL_Y, ylo = y0 == 0 ? -1 : y0, yhi = y0 + PL_Y >= H ? H : y0 + PL_Y - 1;
+      const int zlo = un.z0 == 0 ? -1 : un.z0, zhi = un.z1 == D ? D : un.z1 - 1;
+      const int x0 = un.x * PL_X, x1 = min(x0 + PL_X, W);
+      for (int zx = max(zlo, dz - 1); zx <= min(zhi, D - 2 + dz); ++zx)
+        for (int yx = max(ylo, dy - 1); yx <= min(yhi, H - 2 + dy); ++yx) {
+          const bool row = dx < 3 && zx >= 0 && zx < D && yx >= 0 && yx < H;
+          const int64_t g0 = (static_cast<int64_t>(zx - dz + 1) * H + (yx - dy + 1)) * W;
+          const int64_t r0 = row ? (static_cast<int64_t>(zx) * H + yx) * W : 0;
+          for (int x = x0; x < x1; ++x) {
+            const int xx = x + dx - 1;
+            const float xv =
+                row && xx >= 0 && xx < W ? __bfloat162float(X[(r0 + xx) * CIN + ci]) : 0.0f;
+            const __nv_bfloat16 *g = dY + (g0 + x) * COUT + c0;
+            const __nv_bfloat16 *k = Yo ? Yo + (g0 + x) * COUT + c0 : nullptr;
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+              const float gv = !k || __bfloat162float(k[q]) > 0.0f ? __bfloat162float(g[q]) : 0.0f;
+              acc[q] = fmaf(xv, gv, acc[q]);
+            }
+          }
+        }
+    }
+    if (dx < 3)
+      for (int q = 0; q < 16; ++q)
+        atomicAdd(dW + (static_cast<int64_t>(dz * 9 + dy * 3 + dx) * CIN + ci) * COUT + c0 + q, acc[q]);
+  }
+}
+
 // Weight gradient: for each plane z' of X, row y' and voxel x of a tile,
 //   D[dz][(dx, ci)][(dy, co)] += X[z'][y'][x + dx][ci] G[z' - dz][y' - dy][x][co]
 // as M = 128 (three dx blocks of CIN channels, the rest of M unused) by N = 3
@@ -1268,16 +1314,18 @@ __host__ __device__ constexpr int pw_g_bytes() { return PL_X * PL_ROWS * COUT * 
 template <int CIN, int COUT, bool MASK>
 __global__ void __launch_bounds__(PW_THREADS, 1) wgrad_planes_kernel(
     const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmg,
-    const __grid_constant__ CUtensorMap tmm, float *__restrict__ dW, int D, PlanePlan plan) {
+    const __grid_constant__ CUtensorMap tmm, const __nv_bfloat16 *__restrict__ X, const __nv_bfloat16 *__restrict__ dY,
+    const __nv_bfloat16 *__restrict__ Yo, float *__restrict__ dW, int D, int H, int W, PlanePlan plan) {
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ PlaneBars pb;
+  __shared__ int s_bad;  // an accumulator is not finite
   constexpr int XB = pw_x_bytes<CIN>(), GB = pw_g_bytes<COUT>(), NG = 4, N = 3 * COUT;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   unsigned char *const xs = sm;               // [2][3] shifted X planes
   unsigned char *const gs = xs + 6 * XB;      // [NG] G planes
   unsigned char *const ms = gs + NG * GB;     // [2] mask planes (MASK)
   if (tid == 0) {
-    pb.abort = 0;
+    pb.abort = s_bad = 0;
     for (int b = 0; b < NG; ++b) {
       mbar_init(&pb.full[b], 1);
       mbar_init(&pb.ready[b], PL_MASK);
@@ -1412,43 +1460,66 @@ __global__ void __launch_bounds__(PW_THREADS, 1) wgrad_planes_kernel(
         }
       }
     }
-  } else if (any) {
-    // ------------------------------------------------------------ epilogue
-    const int qd = warp & 3, mrow = qd * 32 + lane, dx = mrow / CIN, ci = mrow % CIN;
-    // accumulators that some plane of this CTA wrote: a plane has no G plane
-    // above it at the top of the grid, none below at the bottom
-    bool used[3] = {false, true, false};
+  }
+  // ---------------------------------------------------------------- epilogue
+  // Warps 6 to 9, a TMEM quarter each (32 rows of (dx, ci)): they look at the
+  // accumulators first and add them to dW when the whole CTA has seen that all
+  // are finite.
+  const int qd = warp & 3, mrow = qd * 32 + lane, dx = mrow / CIN, ci = mrow % CIN;
+  const bool sums = any && warp >= 2 + PL_MASK / 32 && qd * 32 < 3 * CIN;
+  // accumulators that some plane of this CTA wrote: a plane has no G plane
+  // above it at the top of the grid, none below at the bottom
+  bool used[3] = {false, true, false};
+  if (sums) {
     for (int u = blockIdx.x; u < plan.units; u += gridDim.x) {
       const PlaneUnit un(plan, u, D);
       used[0] = used[0] || un.z0 < D - 1;
       used[2] = used[2] || un.z1 > 1;
     }
-    if (qd * 32 < 3 * CIN && plane_wait(pb, &pb.accf[0], 0) && !pb.abort) {
-      __syncwarp();
-      tc_fence_after();
+  }
+  auto accumulators = [&](auto each) {  // each(dz, first column, 16 values)
 #pragma unroll
-      for (int dz = 0; dz < 3; ++dz) {
-        if (!used[dz]) continue;
-        for (int c0 = 0; c0 < N; c0 += 16) {
-          uint32_t r[16];
-          tmem_ld16(tmem + (static_cast<uint32_t>(qd * 32) << 16) + static_cast<uint32_t>(dz * N + c0), r);
-          const int dy = 2 - c0 / COUT;  // block 0 pairs row y' with G row y' - 1
-          if (dx < 3) {
-            float *dst = dW + (static_cast<int64_t>(dz * 9 + dy * 3 + dx) * CIN + ci) * COUT + c0 % COUT;
-            if ((reinterpret_cast<uintptr_t>(dW) & 15) == 0) {
-#pragma unroll
-              for (int k = 0; k < 16; k += 4)
-                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + k),
-                             "f"(__uint_as_float(r[k])), "f"(__uint_as_float(r[k + 1])),
-                             "f"(__uint_as_float(r[k + 2])), "f"(__uint_as_float(r[k + 3]))
-                             : "memory");
-            } else {
-#pragma unroll
-              for (int k = 0; k < 16; ++k) atomicAdd(dst + k, __uint_as_float(r[k]));
-            }
-          }
-        }
+    for (int dz = 0; dz < 3; ++dz) {
+      if (!used[dz]) continue;
+      for (int c0 = 0; c0 < N; c0 += 16) {
+        uint32_t r[16];
+        tmem_ld16(tmem + (static_cast<uint32_t>(qd * 32) << 16) + static_cast<uint32_t>(dz * N + c0), r);
+        each(dz, c0, r);
       }
+    }
+  };
+  if (sums && plane_wait(pb, &pb.accf[0], 0) && !pb.abort) {
+    __syncwarp();
+    tc_fence_after();
+    bool bad = false;
+    accumulators([&](int, int, const uint32_t (&r)[16]) {
+#pragma unroll
+      for (int k = 0; k < 16; ++k) bad = bad || (r[k] & 0x7f800000u) == 0x7f800000u;
+    });
+    if (bad && dx < 3) s_bad = 1;
+    tc_fence_before();
+  }
+  __syncthreads();
+  if (any && !pb.abort) {
+    if (s_bad) {
+      wgrad_pairs<CIN, COUT>(X, dY, MASK ? Yo : nullptr, dW, D, H, W, plan);
+    } else if (sums) {
+      tc_fence_after();
+      accumulators([&](int dz, int c0, const uint32_t (&r)[16]) {
+        const int dy = 2 - c0 / COUT;  // block 0 pairs row y' with G row y' - 1
+        if (dx >= 3) return;
+        float *dst = dW + (static_cast<int64_t>(dz * 9 + dy * 3 + dx) * CIN + ci) * COUT + c0 % COUT;
+        if ((reinterpret_cast<uintptr_t>(dW) & 15) == 0) {
+#pragma unroll
+          for (int k = 0; k < 16; k += 4)
+            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + k), "f"(__uint_as_float(r[k])),
+                         "f"(__uint_as_float(r[k + 1])), "f"(__uint_as_float(r[k + 2])), "f"(__uint_as_float(r[k + 3]))
+                         : "memory");
+        } else {
+#pragma unroll
+          for (int k = 0; k < 16; ++k) atomicAdd(dst + k, __uint_as_float(r[k]));
+        }
+      });
     }
   }
   tc_fence_before();
@@ -1604,7 +1675,8 @@ static int wgrad_planes(const void *X, const void *dY, const void *Yo, float *dW
   };
   auto kfn = Yo ? pick(std::true_type()) : pick(std::false_type());
   ORSP_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kfn<<<std::min(plan.units, sms), PW_THREADS, smem, st>>>(tx, tg, tm, dW, D, plan);
+  kfn<<<std::min(plan.units, sms), PW_THREADS, smem, st>>>(
+      tx, tg, tm, (const __nv_bfloat16 *)X, (const __nv_bfloat16 *)dY, (const __nv_bfloat16 *)Yo, dW, D, H, W, plan);
   ORSP_CUDA(cudaGetLastError());
   return ORSP_OK;
 }

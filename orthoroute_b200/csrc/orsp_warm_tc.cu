@@ -912,12 +912,37 @@ struct PlanePlan {
 
 struct PlaneUnit {
   int x, y, z0, z1;  // column, planes [z0, z1)
+  __device__ __forceinline__ PlaneUnit() {}
   __device__ __forceinline__ PlaneUnit(const PlanePlan &pl, int u, int D) {
     const int cols = pl.nxs * pl.nys, c = u % cols;
     x = c % pl.nxs;
     y = c / pl.nxs;
     z0 = (u / cols) * pl.zc;
     z1 = min(D, z0 + pl.zc);
+  }
+};
+
+// The weight gradient's tiles: a CTA's share is a range of all columns' planes,
+// one column after the other, and shares differ by one plane at most.  Its
+// rounding error is that of the longest sums: chunks of one length gave some
+// CTAs 24 planes of 200 x 200 x 18 and others 18 (9 and 4 of 72 x 112 x 17).
+struct PlaneShare {
+  int at, end;
+  __device__ __forceinline__ PlaneShare(const PlanePlan &pl, int D) {
+    const int64_t n = static_cast<int64_t>(pl.nxs) * pl.nys * D;
+    at = static_cast<int>(n * blockIdx.x / gridDim.x);
+    end = static_cast<int>(n * (blockIdx.x + 1) / gridDim.x);
+  }
+  __device__ __forceinline__ bool more() const { return at < end; }
+  __device__ __forceinline__ PlaneUnit next(const PlanePlan &pl, int D) {
+    PlaneUnit u;
+    const int c = at / D;
+    u.x = c % pl.nxs;
+    u.y = c / pl.nxs;
+    u.z0 = at - c * D;
+    u.z1 = min(D, u.z0 + end - at);
+    at += u.z1 - u.z0;
+    return u;
   }
 };
 
@@ -1252,6 +1277,14 @@ __global__ void __launch_bounds__(pc_threads<MASK>(), 1) conv3d_planes_kernel(
 
 constexpr int PW_THREADS = 64 + PL_MASK + 128;  // TMA, MMA, mask warps, four epilogue warps
 
+// TMEM column of the accumulator of dz for even (0) and odd (1) planes of a
+// share: 6 x 48 columns for 16 output channels; 5 x 96 of 512 for 32, the last dz
+// has one.
+template <int COUT>
+__host__ __device__ constexpr int pw_acc(int dz, int odd) {
+  return 3 * COUT * (COUT == 16 || dz < 2 ? 2 * dz + odd : 4);
+}
+
 template <int CIN>
 __host__ __device__ constexpr int pw_x_bytes() { return PL_X * PL_Y * CIN * 2; }  // one shifted X plane
 template <int COUT>
@@ -1273,8 +1306,8 @@ __device__ __noinline__ void wgrad_pairs(const __nv_bfloat16 *__restrict__ X, co
     const int m = task % MT * 32 + lane, c0 = task / MT % CT * 16, dz = task / (MT * CT) / 3, dy = task / (MT * CT) % 3;
     const int dx = m / CIN, ci = m % CIN;
     float acc[16] = {};
-    for (int u = blockIdx.x; u < plan.units; u += gridDim.x) {
-      const PlaneUnit un(plan, u, D);
+    for (PlaneShare sh(plan, D); sh.more();) {
+      const PlaneUnit un = sh.next(plan, D);
       const int y0 = un.y * PL_Y, ylo = y0 == 0 ? -1 : y0, yhi = y0 + PL_Y >= H ? H : y0 + PL_Y - 1;
       const int zlo = un.z0 == 0 ? -1 : un.z0, zhi = un.z1 == D ? D : un.z1 - 1;
       const int x0 = un.x * PL_X, x1 = min(x0 + PL_X, W);
@@ -1309,8 +1342,15 @@ __device__ __noinline__ void wgrad_pairs(const __nv_bfloat16 *__restrict__ X, co
 // COUT (three dy blocks) MMAs over K = 16 voxels; both operands are M- or
 // N-major (channels contiguous).  The dx blocks are three TMA loads of the X
 // plane, one voxel apart, the dy blocks the G plane one row apart, so one MMA
-// serves nine taps.  The three accumulators (dz) stay in TMEM over all of a
-// CTA's tiles and are added to dW once, four values per atomic.
+// serves nine taps.  The accumulators (dz) stay in TMEM over a CTA's share and
+// are added to dW once, four values per atomic (adding them twice, in halves of
+// the share, took 10 us more).  The rounding error of a sum in TMEM grows with
+// its length to the power 1.5, so the planes alternate between two
+// accumulators of a dz where TMEM holds them (pw_acc), which are added before
+// they leave.
+// Error of dW against 64 bits, 200 x 200 x 18, 32 -> 32 channels: 2.34e-6 with
+// chunks of one length and one accumulator, 2.34e-6 with even shares, 1.55e-6 with
+// both; 144 x 184 x 12, 32 -> 16: 1.18e-6, 8.8e-7, 4.4e-7.
 template <int CIN, int COUT, bool MASK>
 __global__ void __launch_bounds__(PW_THREADS, 1) wgrad_planes_kernel(
     const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmg,
@@ -1339,7 +1379,7 @@ __global__ void __launch_bounds__(PW_THREADS, 1) wgrad_planes_kernel(
     mbar_init(&pb.accf[0], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  constexpr uint32_t ncols = 3 * N <= 256 ? 256u : 512u;
+  constexpr uint32_t ncols = 512;
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&pb.tmem)),
                  "r"(ncols)
@@ -1350,7 +1390,6 @@ __global__ void __launch_bounds__(PW_THREADS, 1) wgrad_planes_kernel(
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = pb.tmem;
-  const bool any = static_cast<int>(blockIdx.x) < plan.units;
 
   if (warp == 0) {
     if (lane == 0) {
@@ -1367,8 +1406,8 @@ __global__ void __launch_bounds__(PW_THREADS, 1) wgrad_planes_kernel(
         ++n;
         return true;
       };
-      for (int u = blockIdx.x; u < plan.units && ok; u += gridDim.x) {
-        const PlaneUnit un(plan, u, D);
+      for (PlaneShare sh(plan, D); sh.more() && ok;) {
+        const PlaneUnit un = sh.next(plan, D);
         const int zhi = min(un.z1, D - 1);
         int zg = max(un.z0 - 1, 0);
         for (int z = un.z0; z < un.z1 && ok; ++z, ++m) {
@@ -1389,10 +1428,10 @@ __global__ void __launch_bounds__(PW_THREADS, 1) wgrad_planes_kernel(
     const uint32_t idesc = umma_idesc_bf16_mn(TC_M, N);
     const uint64_t x0d = plane_desc<CIN>(smem_addr(xs), XB), g0d = plane_desc<COUT>(smem_addr(gs), PL_X * COUT * 2);
     int b = 0, par = 0, m = 0;
-    uint32_t used[3] = {0, 0, 0};
+    uint32_t used[3][2] = {};
     bool ok = true;
-    for (int u = blockIdx.x; u < plan.units && ok; u += gridDim.x) {
-      const PlaneUnit un(plan, u, D);
+    for (PlaneShare sh(plan, D); sh.more() && ok;) {
+      const PlaneUnit un = sh.next(plan, D);
       int bz[3] = {-1, -1, -1};  // G planes below, at and above z
       auto next = [&]() {
         ok = ok && plane_wait(pb, MASK ? &pb.ready[b] : &pb.full[b], par);
@@ -1410,6 +1449,7 @@ __global__ void __launch_bounds__(PW_THREADS, 1) wgrad_planes_kernel(
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
+        const bool odd = m & 1;
         if (elect_lane()) {
 #pragma unroll
           for (int dz = 0; dz < 3; ++dz) {  // tap dz - 1: the G plane at z - (dz - 1)
@@ -1417,8 +1457,8 @@ __global__ void __launch_bounds__(PW_THREADS, 1) wgrad_planes_kernel(
             if (g < 0) continue;
             uint64_t ad = x0d + static_cast<uint64_t>((m & 1) * (3 * XB / 16));
             uint64_t bd = g0d + static_cast<uint64_t>(g * (GB / 16));
-            const uint32_t acc = tmem + static_cast<uint32_t>(dz * N);
-            uint32_t add = used[dz];
+            const uint32_t acc = tmem + static_cast<uint32_t>(odd ? pw_acc<COUT>(dz, 1) : pw_acc<COUT>(dz, 0));
+            uint32_t add = odd ? used[dz][1] : used[dz][0];
 #pragma unroll
             for (int k = 0; k < PL_Y * 2; ++k) {
               mma_bf16(acc, ad, bd, idesc, add);
@@ -1437,7 +1477,10 @@ __global__ void __launch_bounds__(PW_THREADS, 1) wgrad_planes_kernel(
         __syncwarp();
 #pragma unroll
         for (int dz = 0; dz < 3; ++dz)
-          if (bz[2 - dz] >= 0) used[dz] = 1;
+          if (bz[2 - dz] >= 0) {
+            if (!odd || pw_acc<COUT>(dz, 0) == pw_acc<COUT>(dz, 1)) used[dz][0] = 1;
+            if (odd || pw_acc<COUT>(dz, 0) == pw_acc<COUT>(dz, 1)) used[dz][1] = 1;
+          }
       }
     }
     if (elect_lane()) mma_commit(&pb.accf[0]);  // after every MMA of the CTA, also after a failed wait
@@ -1447,8 +1490,8 @@ __global__ void __launch_bounds__(PW_THREADS, 1) wgrad_planes_kernel(
     if (MASK) {
       int n = 0;
       bool ok = true;
-      for (int u = blockIdx.x; u < plan.units && ok; u += gridDim.x) {
-        const PlaneUnit un(plan, u, D);
+      for (PlaneShare sh(plan, D); sh.more() && ok;) {
+        const PlaneUnit un = sh.next(plan, D);
         for (int z = max(un.z0 - 1, 0); z <= min(un.z1, D - 1) && ok; ++z, ++n) {
           const int b = n % NG;
           ok = plane_wait(pb, &pb.full[b], (n / NG) & 1);
@@ -1466,25 +1509,49 @@ __global__ void __launch_bounds__(PW_THREADS, 1) wgrad_planes_kernel(
   // accumulators first and add them to dW when the whole CTA has seen that all
   // are finite.
   const int qd = warp & 3, mrow = qd * 32 + lane, dx = mrow / CIN, ci = mrow % CIN;
-  const bool sums = any && warp >= 2 + PL_MASK / 32 && qd * 32 < 3 * CIN;
+  const bool sums = warp >= 2 + PL_MASK / 32 && qd * 32 < 3 * CIN;
   // accumulators that some plane of this CTA wrote: a plane has no G plane
   // above it at the top of the grid, none below at the bottom
-  bool used[3] = {false, true, false};
+  bool used[3][2] = {};
   if (sums) {
-    for (int u = blockIdx.x; u < plan.units; u += gridDim.x) {
-      const PlaneUnit un(plan, u, D);
-      used[0] = used[0] || un.z0 < D - 1;
-      used[2] = used[2] || un.z1 > 1;
+    int m = 0;
+    for (PlaneShare sh(plan, D); sh.more();) {
+      const PlaneUnit un = sh.next(plan, D);
+      for (int z = un.z0; z < un.z1; ++z, ++m)
+#pragma unroll
+        for (int dz = 0; dz < 3; ++dz) {
+          const bool w = dz == 1 || (dz == 0 ? z < D - 1 : z > 0);
+          if (pw_acc<COUT>(dz, 0) == pw_acc<COUT>(dz, 1) || !(m & 1)) used[dz][0] = used[dz][0] || w;
+          else used[dz][1] = used[dz][1] || w;
+        }
     }
   }
-  auto accumulators = [&](auto each) {  // each(dz, first column, 16 values)
+  auto accumulators = [&](auto each) {  // each(dz, dy, first channel, 16 values)
+    const uint32_t t0 = tmem + (static_cast<uint32_t>(qd * 32) << 16);
 #pragma unroll
     for (int dz = 0; dz < 3; ++dz) {
-      if (!used[dz]) continue;
-      for (int c0 = 0; c0 < N; c0 += 16) {
-        uint32_t r[16];
-        tmem_ld16(tmem + (static_cast<uint32_t>(qd * 32) << 16) + static_cast<uint32_t>(dz * N + c0), r);
-        each(dz, c0, r);
+      if (!used[dz][0] && !used[dz][1]) continue;
+      const bool both = used[dz][0] && used[dz][1];
+      for (int blk = 0; blk < 3; ++blk) {  // block 0 pairs row y' with G row y' - 1
+        // all columns of a block in flight at a time
+        const uint32_t t1 = t0 + static_cast<uint32_t>(blk * COUT + pw_acc<COUT>(dz, used[dz][0] ? 0 : 1));
+        const uint32_t t2 = both ? t0 + static_cast<uint32_t>(blk * COUT + pw_acc<COUT>(dz, 1)) : t1;
+        uint32_t r[COUT / 16][16], o[COUT / 16][16];
+#pragma unroll
+        for (int c = 0; c < COUT / 16; ++c) {
+          tmem_ld16_async(t1 + c * 16, r[c]);
+          tmem_ld16_async(t2 + c * 16, o[c]);
+        }
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int c = 0; c < COUT / 16; ++c) {
+#pragma unroll
+          for (int k = 0; k < 16; ++k) {
+            asm volatile("" : "+r"(r[c][k]), "+r"(o[c][k]));  // (no use of them before the wait)
+            if (both) r[c][k] = __float_as_uint(__uint_as_float(r[c][k]) + __uint_as_float(o[c][k]));
+          }
+          each(dz, 2 - blk, c * 16, r[c]);
+        }
       }
     }
   };
@@ -1492,7 +1559,7 @@ __global__ void __launch_bounds__(PW_THREADS, 1) wgrad_planes_kernel(
     __syncwarp();
     tc_fence_after();
     bool bad = false;
-    accumulators([&](int, int, const uint32_t (&r)[16]) {
+    accumulators([&](int, int, int, const uint32_t (&r)[16]) {
 #pragma unroll
       for (int k = 0; k < 16; ++k) bad = bad || (r[k] & 0x7f800000u) == 0x7f800000u;
     });
@@ -1500,15 +1567,14 @@ __global__ void __launch_bounds__(PW_THREADS, 1) wgrad_planes_kernel(
     tc_fence_before();
   }
   __syncthreads();
-  if (any && !pb.abort) {
+  if (!pb.abort) {
     if (s_bad) {
       wgrad_pairs<CIN, COUT>(X, dY, MASK ? Yo : nullptr, dW, D, H, W, plan);
     } else if (sums) {
       tc_fence_after();
-      accumulators([&](int dz, int c0, const uint32_t (&r)[16]) {
-        const int dy = 2 - c0 / COUT;  // block 0 pairs row y' with G row y' - 1
+      accumulators([&](int dz, int dy, int c0, const uint32_t (&r)[16]) {
         if (dx >= 3) return;
-        float *dst = dW + (static_cast<int64_t>(dz * 9 + dy * 3 + dx) * CIN + ci) * COUT + c0 % COUT;
+        float *dst = dW + (static_cast<int64_t>(dz * 9 + dy * 3 + dx) * CIN + ci) * COUT + c0;
         if ((reinterpret_cast<uintptr_t>(dW) & 15) == 0) {
 #pragma unroll
           for (int k = 0; k < 16; k += 4)
@@ -1663,8 +1729,9 @@ static int wgrad_planes(const void *X, const void *dY, const void *Yo, float *dW
   int dev = 0, sms = 0;
   ORSP_CUDA(cudaGetDevice(&dev));
   ORSP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const PlanePlan plan = plane_plan((W + PL_X - 1) / PL_X, (H + PL_Y - 1) / PL_Y, D, sms);
-  if (plan.units <= 0) return ORSP_NO_PATH;
+  const PlanePlan plan{(W + PL_X - 1) / PL_X, (H + PL_Y - 1) / PL_Y, 0, 0};
+  const int64_t nplanes = (int64_t)plan.nxs * plan.nys * D;
+  if (nplanes > INT32_MAX) return ORSP_NO_PATH;
   const size_t xb = Cin == 32 ? pw_x_bytes<32>() : pw_x_bytes<16>(), gb = Cout == 32 ? pw_g_bytes<32>() : pw_g_bytes<16>();
   // (the unused rows of M read past the third X plane, within the allocation)
   const size_t smem = std::max(6 * xb + 4 * gb + (Yo ? 2 * gb : 0), 3 * xb + 128 / Cin * xb);
@@ -1675,7 +1742,7 @@ static int wgrad_planes(const void *X, const void *dY, const void *Yo, float *dW
   };
   auto kfn = Yo ? pick(std::true_type()) : pick(std::false_type());
   ORSP_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kfn<<<std::min(plan.units, sms), PW_THREADS, smem, st>>>(
+  kfn<<<(int)std::min<int64_t>(nplanes, sms), PW_THREADS, smem, st>>>(
       tx, tg, tm, (const __nv_bfloat16 *)X, (const __nv_bfloat16 *)dY, (const __nv_bfloat16 *)Yo, dW, D, H, W, plan);
   ORSP_CUDA(cudaGetLastError());
   return ORSP_OK;

@@ -32,7 +32,7 @@ ORSP_API int orsp_warm_conv3d(const void *X, const void *mask, const void *Wt, c
  * K-major layout and the fp32 accumulator in tensor memory (128 voxels x
  * Cout per tile), persistent CTAs.  Cin and Cout multiples of 16, Cout <= 64,
  * and all 27 x Cin x Cout weights within shared memory (Cin x Cout <= 2048
- * for Cout <= 32; Cin <= 32 for Cout = 64).  A wait that expires (2 s) is
+ * for Cout <= 32; Cin <= 32 for Cout = 64).  A wait that expires (2 s, ORSP_WAIT_NS) is
  * recorded for orsp_warm_tc_status. */
 ORSP_API int orsp_warm_conv3d_tc(const void *X, const void *mask, const void *Wt, const float *bias, void *Y,
                                  float *Yf, int32_t D, int32_t H, int32_t W, int32_t Cin, int32_t Cout,

@@ -42,6 +42,13 @@ constexpr int TC_M = 128;        // voxels per tile: the MMA's M and the accumul
 constexpr int TC_THREADS = 128;  // four warps, one per 32-lane quarter of TMEM
 constexpr unsigned long long TC_WAIT_NS = 2000000000ull;
 
+// Bound of one wait of a launch (ORSP_WAIT_NS).  What a launch still waits for
+// when it has given up, its copies and MMAs in flight, keeps TC_WAIT_NS.
+inline unsigned long long tc_wait_ns() {
+  const char *s = getenv("ORSP_WAIT_NS");
+  return s && *s ? strtoull(s, nullptr, 10) : TC_WAIT_NS;
+}
+
 __device__ int g_tc_err = 0;     // set by a kernel whose wait expired (orsp_warm_tc_status)
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p) {
@@ -451,7 +458,7 @@ template <int CG>
 __global__ void __launch_bounds__(WS_THREADS, 1) conv3d_tc_ws_kernel(
     const __nv_bfloat16 *__restrict__ X, const __nv_bfloat16 *__restrict__ Mk, const __nv_bfloat16 *__restrict__ Wt,
     const float *__restrict__ bias, __nv_bfloat16 *__restrict__ Y, float *__restrict__ Yf, int D, int H, int W,
-    int Cin, int Cout, int relu, int NS) {
+    int Cin, int Cout, int relu, int NS, unsigned long long wait_ns) {
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ volatile int s_abort;
   const int KC = Cin >> 4;
@@ -540,13 +547,17 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv3d_tc_ws_kernel(
     for (;;) {
       if (mbar_try(a, static_cast<uint32_t>(parity))) return true;
       if (s_abort) return false;
-      if (dev_globaltimer() - t0 > TC_WAIT_NS) {
+      if (dev_globaltimer() - t0 > wait_ns) {
         s_abort = 1;
         atomicExch(&g_tc_err, 1);
         return false;
       }
     }
   };
+  // the same by a whole warp, whose lanes go on or give up together: one lane
+  // may find the phase complete and another the abort flag, and what follows
+  // (tcgen05.ld) takes all of them
+  auto wait_warp = [&](unsigned long long *bar, int parity) { return __all_sync(0xffffffffu, wait(bar, parity)) != 0; };
   const int LAG = NS - 2 < 4 ? NS - 2 : 4;
 
   if (warp < 8) {
@@ -604,7 +615,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv3d_tc_ws_kernel(
     bool ok = true;
     // drains tile ep_T (accumulator ep_T & 1) and frees the accumulator
     auto drain = [&]() -> bool {
-      if (!wait(accf + (ep_T & 1), (ep_T >> 1) & 1)) return false;
+      if (!wait_warp(accf + (ep_T & 1), (ep_T >> 1) & 1)) return false;
       tc_fence_after();
       epilogue(et.tx, et.y, et.z, ep_T & 1);
       tc_fence_before();
@@ -617,7 +628,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv3d_tc_ws_kernel(
     for (int s = 0; s < nst32 + LAG && ok; ++s) {
       if (s < nst32) {
         // the buffer's previous stage must have been consumed
-        if (s >= NS && !wait(empty + ci.buf, ci.par ^ 1)) {
+        if (s >= NS && !wait_warp(empty + ci.buf, ci.par ^ 1)) {
           ok = false;
           break;
         }
@@ -1027,6 +1038,7 @@ struct PlaneBars {
   unsigned long long accf[2], acce[2];
   uint32_t tmem;
   volatile int abort;
+  unsigned long long wait_ns;
 };
 
 // Waits for `parity` of a barrier, bounded; ends early when another role has
@@ -1038,12 +1050,19 @@ __device__ __forceinline__ bool plane_wait(PlaneBars &pb, void *bar, int parity)
   for (;;) {
     if (mbar_try(a, static_cast<uint32_t>(parity))) return true;
     if (pb.abort) return false;
-    if (dev_globaltimer() - t0 > TC_WAIT_NS) {
+    if (dev_globaltimer() - t0 > pb.wait_ns) {
       pb.abort = 1;
       atomicExch(&g_tc_err, 1);
       return false;
     }
   }
+}
+
+// The same by a whole warp, whose lanes go on or give up together: one lane may
+// find the phase complete and another the abort flag, and what follows (MMA
+// issue, tcgen05.ld, shuffles) takes all of them.
+__device__ __forceinline__ bool plane_wait_warp(PlaneBars &pb, void *bar, int parity) {
+  return __all_sync(0xffffffffu, plane_wait(pb, bar, parity)) != 0;
 }
 
 // TMA, MMA, mask warps, sixteen epilogue warps
@@ -1062,7 +1081,8 @@ template <int CIN, bool MASK>
 __global__ void __launch_bounds__(pc_threads<MASK>(), 1) conv3d_planes_kernel(
     const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmm,
     const __nv_bfloat16 *__restrict__ Wt, const float *__restrict__ bias, __nv_bfloat16 *__restrict__ Y,
-    float *__restrict__ Yf, int D, int H, int W, int Cout, int relu, PlanePlan plan, int NB) {
+    float *__restrict__ Yf, int D, int H, int W, int Cout, int relu, PlanePlan plan, int NB,
+    unsigned long long wait_ns) {
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ PlaneBars pb;
   constexpr int KC = CIN / 16, PB = plane_bytes<CIN>(), EPI = 2 + (MASK ? PL_MASK / 32 : 0);  // first epilogue warp
@@ -1087,6 +1107,7 @@ __global__ void __launch_bounds__(pc_threads<MASK>(), 1) conv3d_planes_kernel(
   }
   if (tid == 0) {
     pb.abort = 0;
+    pb.wait_ns = wait_ns;
     for (int b = 0; b < NB; ++b) {
       mbar_init(&pb.full[b], 1);
       mbar_init(&pb.ready[b], PL_MASK);
@@ -1193,6 +1214,7 @@ __global__ void __launch_bounds__(pc_threads<MASK>(), 1) conv3d_planes_kernel(
     }
     // after a failed wait the MMAs in flight get one more bounded wait
     if (!ok && step > 0) mbar_wait(smem_addr(&pb.accf[(step - 1) & 1]), ((step - 1) >> 1) & 1);
+    __syncwarp();
   } else if (warp < EPI) {
     // ---------------------------------------------------------------- mask
     if (MASK) {
@@ -1228,9 +1250,8 @@ __global__ void __launch_bounds__(pc_threads<MASK>(), 1) conv3d_planes_kernel(
       const bool in = lane >= 1 && lane <= 30 && x < W && y < H;
       for (int z = un.z0; z < un.z1; ++z, ++step) {
         const int a = step & 1;
-        ok = plane_wait(pb, &pb.accf[a], (step >> 1) & 1);
+        ok = plane_wait_warp(pb, &pb.accf[a], (step >> 1) & 1);
         if (!ok) break;
-        __syncwarp();
         tc_fence_after();
         const uint32_t t0 =
             tmem + (static_cast<uint32_t>(qd * 32) << 16) + static_cast<uint32_t>((a * 2 + j) * N + c * 16);
@@ -1355,7 +1376,8 @@ template <int CIN, int COUT, bool MASK>
 __global__ void __launch_bounds__(PW_THREADS, 1) wgrad_planes_kernel(
     const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmg,
     const __grid_constant__ CUtensorMap tmm, const __nv_bfloat16 *__restrict__ X, const __nv_bfloat16 *__restrict__ dY,
-    const __nv_bfloat16 *__restrict__ Yo, float *__restrict__ dW, int D, int H, int W, PlanePlan plan) {
+    const __nv_bfloat16 *__restrict__ Yo, float *__restrict__ dW, int D, int H, int W, PlanePlan plan,
+    unsigned long long wait_ns) {
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ PlaneBars pb;
   __shared__ int s_bad;  // an accumulator is not finite
@@ -1366,6 +1388,7 @@ __global__ void __launch_bounds__(PW_THREADS, 1) wgrad_planes_kernel(
   unsigned char *const ms = gs + NG * GB;     // [2] mask planes (MASK)
   if (tid == 0) {
     pb.abort = s_bad = 0;
+    pb.wait_ns = wait_ns;
     for (int b = 0; b < NG; ++b) {
       mbar_init(&pb.full[b], 1);
       mbar_init(&pb.ready[b], PL_MASK);
@@ -1486,6 +1509,7 @@ __global__ void __launch_bounds__(PW_THREADS, 1) wgrad_planes_kernel(
     if (elect_lane()) mma_commit(&pb.accf[0]);  // after every MMA of the CTA, also after a failed wait
     __syncwarp();
     if (!ok) mbar_wait(smem_addr(&pb.accf[0]), 0);
+    __syncwarp();
   } else if (warp < 2 + PL_MASK / 32) {
     if (MASK) {
       int n = 0;
@@ -1555,8 +1579,7 @@ __global__ void __launch_bounds__(PW_THREADS, 1) wgrad_planes_kernel(
       }
     }
   };
-  if (sums && plane_wait(pb, &pb.accf[0], 0) && !pb.abort) {
-    __syncwarp();
+  if (sums && plane_wait_warp(pb, &pb.accf[0], 0)) {
     tc_fence_after();
     bool bad = false;
     accumulators([&](int, int, int, const uint32_t (&r)[16]) {
@@ -1715,7 +1738,7 @@ static int conv3d_planes(const void *X, const void *mask, const void *Wt, const 
                        : (mask ? conv3d_planes_kernel<16, true> : conv3d_planes_kernel<16, false>);
   ORSP_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   kfn<<<std::min(plan.units, sms), mask ? pc_threads<true>() : pc_threads<false>(), smem, st>>>(tx, tm, (const __nv_bfloat16 *)Wt, bias, (__nv_bfloat16 *)Y,
-                                                           Yf, D, H, W, Cout, relu, plan, nb);
+                                                           Yf, D, H, W, Cout, relu, plan, nb, tc_wait_ns());
   ORSP_CUDA(cudaGetLastError());
   return ORSP_OK;
 }
@@ -1743,7 +1766,8 @@ static int wgrad_planes(const void *X, const void *dY, const void *Yo, float *dW
   auto kfn = Yo ? pick(std::true_type()) : pick(std::false_type());
   ORSP_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   kfn<<<(int)std::min<int64_t>(nplanes, sms), PW_THREADS, smem, st>>>(
-      tx, tg, tm, (const __nv_bfloat16 *)X, (const __nv_bfloat16 *)dY, (const __nv_bfloat16 *)Yo, dW, D, H, W, plan);
+      tx, tg, tm, (const __nv_bfloat16 *)X, (const __nv_bfloat16 *)dY, (const __nv_bfloat16 *)Yo, dW, D, H, W, plan,
+      tc_wait_ns());
   ORSP_CUDA(cudaGetLastError());
   return ORSP_OK;
 }
@@ -1789,13 +1813,13 @@ extern "C" int orsp_warm_conv3d_tc(const void *X, const void *mask, const void *
   // stages over through mbarriers); ORSP_WARM_TC_WS=0: the kernel with one
   // block barrier per stage
   if (!stage_barrier) {
-    decltype(kfn) kws = Cin == 16 ? conv3d_tc_ws_kernel<2> : Cin == 32 ? conv3d_tc_ws_kernel<4>
+    auto kws = Cin == 16 ? conv3d_tc_ws_kernel<2> : Cin == 32 ? conv3d_tc_ws_kernel<4>
                                                                        : conv3d_tc_ws_kernel<8>;
     const size_t smem_ws = ws_smem_bytes(Cin, Cout, ns);
     ORSP_CUDA(cudaFuncSetAttribute(kws, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_ws));
     kws<<<grid, WS_THREADS, smem_ws, (cudaStream_t)stream>>>((const __nv_bfloat16 *)X, (const __nv_bfloat16 *)mask,
                                                              (const __nv_bfloat16 *)Wt, bias, (__nv_bfloat16 *)Y, Yf,
-                                                             D, H, W, Cin, Cout, relu, ns);
+                                                             D, H, W, Cin, Cout, relu, ns, tc_wait_ns());
     ORSP_CUDA(cudaGetLastError());
     return ORSP_OK;
   }

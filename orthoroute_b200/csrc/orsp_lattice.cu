@@ -1708,13 +1708,19 @@ struct OwnShared {
   int pub[4];                  // sides with publications not yet sent as messages
   volatile int stop, rel;      // the search is over; the tile is given back once it is idle
   volatile int idle, out;      // no work at the last look; the tile's distances are written
+  volatile int quit;           // the launch has failed: the workers leave, idle or not
   int tile;
   LatBox box;
 };
 
 // The cycles of an owned tile, from the halo values na / nb until it is idle
-// and asked to stop.  pa / pb: the boundary values last published; snap: the
-// inbox count read before na and nb.  Returns the number of cycles.
+// and asked to stop, or the launch has failed.  (A tile can stay busy for good:
+// costs whose sum around a loop is negative lower its distances until the
+// floats saturate.  Every kQuitCycles cycles, under a millisecond, the workers
+// look whether to leave all the same.)  pa / pb: the boundary values last
+// published; snap: the inbox count read before na and nb.  Returns the number
+// of cycles.
+constexpr unsigned kQuitCycles = 1024;
 template <int NZM, bool CV, bool ZS>
 __device__ __forceinline__ unsigned own_cycles(const OwnParams &o, const LatBox &B, const RunGeom &G,
                                                const RunTile<NZM, ZS> &R, RunShared &S, OwnShared &Q, float *sd,
@@ -1809,7 +1815,7 @@ __device__ __forceinline__ unsigned own_cycles(const OwnParams &o, const LatBox 
     }
     const bool zany = tile_sync_or<NW, true>(mz != 0);
     dirty = run && (((G.isv ? S.colz[k][G.rl] : S.rowz[k][G.rl]) >> G.rz) & 1u);
-    ++cycles;
+    if (++cycles % kQuitCycles == 0 && tile_sync_or<NW, true>(Q.quit != 0)) break;
     idle = !any && !zany;
     if (tid == 0) {
       // a cycle without a change answers the request read before its halo loads
@@ -1886,7 +1892,7 @@ __global__ void __launch_bounds__(RunTile<NZM, ZS>::NW + 32, MINB)
   if (tid < 32) S.clear();
   if (tid == 0) {
     Q.req = Q.ack = 0;
-    Q.stop = Q.rel = 0;
+    Q.stop = Q.rel = Q.quit = 0;
     S.start();
     S.lap(-1);
   }
@@ -1937,7 +1943,8 @@ __global__ void __launch_bounds__(RunTile<NZM, ZS>::NW + 32, MINB)
       int stop = 0;
       if (lane == 0) {
         in = ld_acquire_u32(&o.inbox[t]);
-        stop = ld_acquire_u32((const unsigned *)o.done) != 0 || ld_acquire_u32((const unsigned *)&p.ctl->err) != 0;
+        if (ld_acquire_u32((const unsigned *)&p.ctl->err)) stop = Q.quit = 1;
+        if (ld_acquire_u32((const unsigned *)o.done)) stop = 1;
       }
       in = __shfl_sync(ORSP_FULL_MASK, in, 0);
       if (asked == got && in != got) {
@@ -1958,7 +1965,7 @@ __global__ void __launch_bounds__(RunTile<NZM, ZS>::NW + 32, MINB)
       }
       if (lane == 0 && (spins & 31u) == 31u && dev_globaltimer() - t_start > min(p.wait_ns * 4, p.budget_ns)) {
         atomicCAS(&p.ctl->err, DEV_OK, DEV_ERR_TIMEOUT);
-        stop = 1;
+        stop = Q.quit = 1;
       }
       if (__shfl_sync(ORSP_FULL_MASK, stop, 0)) break;
     }
@@ -2104,7 +2111,7 @@ __global__ void __launch_bounds__(RunTile<NZM, true>::NW + 32, 2)
           atomicExch(&p.tstate[t], 2);
           if (bi != box) Q.box = load_box(p, bi);
           Q.req = Q.ack = got;
-          Q.stop = Q.rel = Q.idle = Q.out = 0;
+          Q.stop = Q.rel = Q.idle = Q.out = Q.quit = 0;
         }
         box = bi;
         if (lane < 4) Q.pub[lane] = 0;
@@ -2158,8 +2165,10 @@ __global__ void __launch_bounds__(RunTile<NZM, true>::NW + 32, 2)
         if (lane == 2) v = ld_acquire_u32((const unsigned *)&ctl->err);
         if (lane == 3) v = ld_acquire_u32((const unsigned *)&ctl->avail);
         const unsigned in = __shfl_sync(ORSP_FULL_MASK, v, 0);
-        over = __shfl_sync(ORSP_FULL_MASK, v, 1) == 0u || __shfl_sync(ORSP_FULL_MASK, v, 2) != 0u;
+        const bool failed = __shfl_sync(ORSP_FULL_MASK, v, 2) != 0u;
+        over = failed || __shfl_sync(ORSP_FULL_MASK, v, 1) == 0u;
         const int waiting = (int)__shfl_sync(ORSP_FULL_MASK, v, 3);  // < 0: free CTAs
+        if (failed && lane == 0) Q.quit = 1;
         if (over && lane == 0) Q.stop = 1;
         if (asked == got && in != got) {
           asked = in;

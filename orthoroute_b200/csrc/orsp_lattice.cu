@@ -1610,6 +1610,9 @@ __device__ __forceinline__ void visit_runs(const LatParams &p, int t, const LatB
 // not come yet is covered by the sender, which still owes that message.  The
 // seeds' tiles start with one message each, sent by the launch.
 //
+// An owner waits for messages as long as the search runs, so what bounds its
+// wait is the launch's time (ORSP_BUDGET_NS), not that of a single wait.
+//
 // Measured, search kernel, queue schedule with run visits -> owners: 49 tiles
 // of 18 layers 193 -> 57 us, 100 x 100 x 4 board 77 (before run visits) -> 19
 // us, 91 tiles of a 200 x 200 x 6 column-via lattice 248 -> 133 us.
@@ -1963,7 +1966,7 @@ __global__ void __launch_bounds__(RunTile<NZM, ZS>::NW + 32, MINB)
           if (lane == 0) atomicExch(o.done, 1);
         }
       }
-      if (lane == 0 && (spins & 31u) == 31u && dev_globaltimer() - t_start > min(p.wait_ns * 4, p.budget_ns)) {
+      if (lane == 0 && (spins & 31u) == 31u && dev_globaltimer() - t_start > p.budget_ns) {
         atomicCAS(&p.ctl->err, DEV_OK, DEV_ERR_TIMEOUT);
         stop = Q.quit = 1;
       }
@@ -2065,7 +2068,7 @@ __global__ void __launch_bounds__(RunTile<NZM, true>::NW + 32, 2)
   if (tid >= NW) {
     // ------------------------------------------------------------ helper
     const unsigned long long t_start = dev_globaltimer();
-    const unsigned long long limit = min(p.wait_ns * 4, p.budget_ns);
+    const unsigned long long limit = p.budget_ns;
     const int lane = tid - NW;
     int box = -1;
     bool have = false;  // a place in the queue is taken: pos

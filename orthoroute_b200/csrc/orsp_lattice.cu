@@ -1905,42 +1905,39 @@ __global__ void __launch_bounds__(RunTile<NZM, ZS>::NW + 32, MINB)
     // ------------------------------------------------------------ helper
     const int lane = tid - NW;
     unsigned sent = 0, got = 0, asked = 0;
+    // messages to the neighbours on the sides in m, the sent count first.  The
+    // lanes that took the sides' flags fence, each behind the boundary values
+    // published before its flag, and lane 0 counts the messages after them: a
+    // neighbour that sees its count reads those values
+    auto send = [&](unsigned m) {
+      sent += __popc(m);
+      if (lane == 0) __stcg(&o.sent[t], sent);
+      __threadfence();
+      __syncwarp();
+      if (lane == 0) {
+        if (m & 1u) atomicAdd(&o.inbox[t - 1], 1u);
+        if (m & 2u) atomicAdd(&o.inbox[t + 1], 1u);
+        if (m & 4u) atomicAdd(&o.inbox[t - B.ntx], 1u);
+        if (m & 8u) atomicAdd(&o.inbox[t + B.ntx], 1u);
+      }
+    };
     for (unsigned spins = 0;; ++spins) {
-      // publications become messages: one lane per side, the sent count first
+      // publications become messages: one lane per side
       const bool pub = lane < 4 && atomicExch(&Q.pub[lane], 0) != 0;
       const unsigned pm = __ballot_sync(ORSP_FULL_MASK, pub);
       const bool acked = asked != got && __shfl_sync(ORSP_FULL_MASK, Q.ack, 0) == asked;
       if (acked) {
         // everything published up to the answer: flags raised since the
-        // exchange above are part of it
+        // exchange above are part of it (what lane 0 saw, all lanes follow)
+        __syncwarp();
         __threadfence_block();
         const bool more = lane < 4 && atomicExch(&Q.pub[lane], 0) != 0;
-        const unsigned mm = __ballot_sync(ORSP_FULL_MASK, more);
-        const unsigned both = pm | mm;
-        if (both) {
-          sent += __popc(both);
-          if (lane == 0) __stcg(&o.sent[t], sent);
-          __threadfence();
-          __syncwarp();
-          if (lane == 0) {
-            if (both & 1u) atomicAdd(&o.inbox[t - 1], 1u);
-            if (both & 2u) atomicAdd(&o.inbox[t + 1], 1u);
-            if (both & 4u) atomicAdd(&o.inbox[t - B.ntx], 1u);
-            if (both & 8u) atomicAdd(&o.inbox[t + B.ntx], 1u);
-          }
-        }
+        const unsigned both = pm | __ballot_sync(ORSP_FULL_MASK, more);
+        if (both) send(both);
         got = asked;
         if (lane == 0) asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&o.got[t]), "r"(got) : "memory");
       } else if (pm) {
-        sent += __popc(pm);
-        if (lane == 0) {
-          __stcg(&o.sent[t], sent);
-          __threadfence();
-          if (pm & 1u) atomicAdd(&o.inbox[t - 1], 1u);
-          if (pm & 2u) atomicAdd(&o.inbox[t + 1], 1u);
-          if (pm & 4u) atomicAdd(&o.inbox[t - B.ntx], 1u);
-          if (pm & 8u) atomicAdd(&o.inbox[t + B.ntx], 1u);
-        }
+        send(pm);
       }
       unsigned in = 0;
       int stop = 0;
@@ -2149,6 +2146,7 @@ __global__ void __launch_bounds__(RunTile<NZM, true>::NW + 32, 2)
         const bool acked = asked != got && __shfl_sync(ORSP_FULL_MASK, Q.ack, 0) == asked;
         const bool out = __shfl_sync(ORSP_FULL_MASK, Q.out, 0) != 0;
         const bool rest = __shfl_sync(ORSP_FULL_MASK, Q.idle, 0) != 0;
+        __syncwarp();  // what lane 0 saw, all lanes follow
         __threadfence_block();
         // everything published up to the answer is sent before the count is
         // dealt with
@@ -2662,6 +2660,7 @@ __global__ void __launch_bounds__(RunTile<NZM, ZS>::NW + 32, MINB) lattice_spec_
     for (unsigned spins = 0;; ++spins) {
       // (one lane reads it: the warp takes the branch as one)
       if (!finished && __shfl_sync(0xffffffffu, s_done, 0) == k) {
+        __syncwarp();  // what lane 0 saw, all lanes follow
         finish_visit<GOAL>(p, cur, s_box[k & 1], s_act[k & 1], lane);
         ++visits;
         finished = true;

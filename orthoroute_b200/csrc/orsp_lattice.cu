@@ -34,6 +34,7 @@
 
 #include "common.cuh"
 #include "fastdiv.cuh"
+#include "launch_cache.cuh"
 #include "lattice_walk.cuh"
 
 namespace {
@@ -2857,45 +2858,23 @@ int launch_persistent(orsp::Graph *g, void *kfn, int threads, size_t smem, int w
   // largest tile once per (kernel, device), never lowered, so a launch with a
   // smaller tile does not invalidate a cached larger one.  The occupancy is
   // cached per (kernel, block, shared memory, device).
-  struct OccEntry {
-    void *fn;
-    int threads, device;
-    size_t smem;
-    int occ;
-  };
-  struct CapEntry {
-    void *fn;
-    int device;
-  };
-  static OccEntry occ_cache[64];
-  static int occ_n = 0;
-  static CapEntry cap_set[32];
-  static int cap_n = 0;
-  static std::mutex occ_mu;
-  int occ = -1;
-  {
-    std::lock_guard<std::mutex> lock(occ_mu);
-    bool capped = false;
-    for (int i = 0; i < cap_n; ++i) capped = capped || (cap_set[i].fn == kfn && cap_set[i].device == g->device);
-    if (!capped) {
-      // the opt-in maximum less the kernel's static shared memory
-      cudaFuncAttributes fa{};
-      ORSP_CUDA(cudaFuncGetAttributes(&fa, kfn));
-      int optin = 0;
-      ORSP_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, g->device));
-      ORSP_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     optin - (int)fa.sharedSizeBytes));
-      if (cap_n < 32) cap_set[cap_n++] = CapEntry{kfn, g->device};
-    }
-    for (int i = 0; i < occ_n; ++i)
-      if (occ_cache[i].fn == kfn && occ_cache[i].threads == threads && occ_cache[i].smem == smem &&
-          occ_cache[i].device == g->device)
-        occ = occ_cache[i].occ;
-    if (occ < 0) {
-      ORSP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kfn, threads, smem));
-      if (occ_n < 64) occ_cache[occ_n++] = OccEntry{kfn, threads, g->device, smem, occ};
-    }
-  }
+  static orsp::LaunchCache caps, occupancies;
+  int cap = 0, occ = 0;
+  int rc = caps.get(kfn, 0, 0, g->device, &cap, [&](int *bytes) {
+    // the opt-in maximum less the kernel's static shared memory
+    cudaFuncAttributes fa{};
+    ORSP_CUDA(cudaFuncGetAttributes(&fa, kfn));
+    ORSP_CUDA(cudaDeviceGetAttribute(bytes, cudaDevAttrMaxSharedMemoryPerBlockOptin, g->device));
+    *bytes -= (int)fa.sharedSizeBytes;
+    ORSP_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, *bytes));
+    return ORSP_OK;
+  });
+  if (rc) return rc;
+  rc = occupancies.get(kfn, threads, smem, g->device, &occ, [&](int *blocks) {
+    ORSP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, kfn, threads, smem));
+    return ORSP_OK;
+  });
+  if (rc) return rc;
   if (occ < 1) {
     orsp::set_error("lattice search: kernel does not fit on an SM");
     return ORSP_ERR_ARG;

@@ -1731,12 +1731,15 @@ static int conv3d_planes(const void *X, const void *mask, const void *Wt, const 
   if (plan.units <= 0) return ORSP_NO_PATH;
   const size_t pb = Cin == 32 ? plane_bytes<32>() : plane_bytes<16>();
   const size_t wb = Cin == 32 ? pc_weight_bytes<32>(Cout) : pc_weight_bytes<16>(Cout);
-  const size_t room = 224 * 1024 - wb - (mask ? 2 * pb : 0);
+  // (the attribute is the kernel's, for all threads: a size that fits every
+  // launch, so that one does not lower it between another's setting and launch)
+  constexpr size_t kSmem = 224 * 1024;
+  const size_t room = kSmem - wb - (mask ? 2 * pb : 0);
   const int nb = (int)std::min<size_t>(PL_MAXB, room / pb);
   const size_t smem = nb * pb + (mask ? 2 * pb : 0) + wb;
   auto kfn = Cin == 32 ? (mask ? conv3d_planes_kernel<32, true> : conv3d_planes_kernel<32, false>)
                        : (mask ? conv3d_planes_kernel<16, true> : conv3d_planes_kernel<16, false>);
-  ORSP_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  ORSP_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
   kfn<<<std::min(plan.units, sms), mask ? pc_threads<true>() : pc_threads<false>(), smem, st>>>(tx, tm, (const __nv_bfloat16 *)Wt, bias, (__nv_bfloat16 *)Y,
                                                            Yf, D, H, W, Cout, relu, plan, nb, tc_wait_ns());
   ORSP_CUDA(cudaGetLastError());

@@ -1836,8 +1836,9 @@ __device__ __forceinline__ unsigned own_cycles(const OwnParams &o, const LatBox 
 // values on chip.  The walk then reads half a byte per cell from shared memory
 // instead of distances and weights through L2, and no distances are written:
 // routing 270 nets twice on 100 x 100 x 4 13.3 -> 12.3 ms, one net 87 -> 81 us.
-// Only where a box's parents fit the walk's shared memory (kParSmem: 97 tiles of
-// 18 layers, every owner launch of up to 5) and nothing else reads distances.
+// Only where a box's parents fit the walk's shared memory (kParSmem: 88 tiles of
+// 18 layers, 266 of 5, every owner launch of up to 4) and nothing else reads
+// distances.
 template <int NZM, bool ZS>
 __device__ __forceinline__ void record_parents(const RunGeom &G, const RunTile<NZM, ZS> &R, const float *sd,
                                                const float2 *wp, const float2 *wz, uint8_t *par) {

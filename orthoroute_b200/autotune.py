@@ -4,7 +4,8 @@ The batch kernel has two implementations and a few knobs:
 
 * one CTA per search (block-local near-far): bucket width delta, CTAs per SM;
 * tile sweeps over many boxes per launch, each box with its own distance
-  slice: tile width 16 or 32.
+  slice, in tiles 16 wide.  (A plan's tile width of 32 stands for the depth up
+  to which such a tile would fit: deeper boxes then take one CTA each.)
 
 Which is fastest depends on the ROI size and on the mix: small boxes fit a
 CTA's shared memory and finish in a few rounds, large boxes need many SMs,
@@ -17,12 +18,15 @@ plan may only change the time), and installs the fastest plan on the graph
 """
 from __future__ import annotations
 
+import ctypes
 from dataclasses import dataclass, field
 from typing import Dict, List, Sequence
 
 import numpy as np
 import torch
 
+from . import _lib
+from ._lib import check
 from .solver import DeviceGraph
 
 DEFAULT_EDGES = (4096, 32768, 262144)  # bucket upper bounds (nodes); the last bucket is open
@@ -44,6 +48,15 @@ def _candidates(mean_cost: float, is_lattice: bool) -> List[dict]:
         for tw in (16, 32):
             out.append({"impl": 1, "delta": 0.0, "ctas_per_sm": 0, "tile_w": tw})
     return out
+
+
+def _sweep_widths(depths: np.ndarray) -> tuple:
+    """The plans' tile widths that tell boxes of these depths apart: the two
+    sweep the same boxes, in the same launch, unless one is too deep for the
+    wider tile."""
+    deepest = ctypes.c_int32()
+    check(_lib.load().orsp_lattice_max_layers(32, ctypes.byref(deepest)), "orsp_lattice_max_layers")
+    return (16, 32) if int(np.max(depths, initial=0)) > deepest.value else (16,)
 
 
 def _name(c: dict) -> str:
@@ -82,9 +95,9 @@ def tune_batch(dg: DeviceGraph, cost: torch.Tensor, src: torch.Tensor, dst: torc
     Stage 2, whole plans on a sample of `sample` searches drawn from the whole
     workload (so that buckets share the GPU as they do in the real run): every
     bucket on one CTA per search, or the buckets from a size threshold up on
-    tile sweeps (tile width 16 or 32).  Every candidate must return the same
-    paths as the first.  boxes: host int32[K, 6]; src/dst/cost: device
-    tensors.  Installs the fastest plan on `dg` unless install=False."""
+    tile sweeps (with tile width 32 too, where it leaves boxes out that are too
+    deep for it).  Every candidate must return the same paths as the first.
+    boxes: host int32[K, 6]; src/dst/cost: device tensors.  Installs the fastest plan on `dg` unless install=False."""
     boxes = np.ascontiguousarray(boxes, dtype=np.int32)
     K = len(boxes)
     vol = (boxes[:, 1] - boxes[:, 0] + 1).astype(np.int64) * (boxes[:, 3] - boxes[:, 2] + 1) * \
@@ -132,8 +145,9 @@ def tune_batch(dg: DeviceGraph, cost: torch.Tensor, src: torch.Tensor, dst: torc
     b = torch.from_numpy(boxes[pick]).to(src.device)
     plans = {"default": None, "cta": [{"max_nodes": int(ub), **c} for ub, c in zip(bounds, cta_best)]}
     if getattr(dg, "lattice_kind", int(dg.is_lattice)) == 1:  # batched tile sweeps need adjacent-layer vias
+        widths = _sweep_widths(boxes[pick, 5] - boxes[pick, 4] + 1)
         for cut in range(len(bounds)):
-            for tw in (16, 32):
+            for tw in widths:
                 plans[f"sweeps>={cut}/tile{tw}"] = [
                     {"max_nodes": int(ub), **(c if i < cut else {"impl": 1, "delta": 0.0, "ctas_per_sm": 0,
                                                                   "tile_w": tw})}

@@ -819,7 +819,7 @@ struct LayerLists {
   int box;
 };
 
-template <int TX, int TY, bool PRIV, bool SPEC, bool DEEP = false, bool TMA = false, bool CV = false>
+template <int TX, int TY, bool PRIV, bool DEEP = false, bool TMA = false, bool CV = false>
 __device__ __forceinline__ void process_tile(const LatParams &p, int t, float *sd, LayerLists &L, int *s_flags,
                                              int *s_act, int *s_nb = nullptr, bool warm = false,
                                              TmaCtx *tma = nullptr) {
@@ -835,7 +835,7 @@ __device__ __forceinline__ void process_tile(const LatParams &p, int t, float *s
     L.nv = nv;
     L.box = bi;
   }
-  tile_sync<TX * TY, SPEC>();
+  __syncthreads();
   const int *s_hl = L.hl, *s_vl = L.vl;
   const int nh = L.nh, nv = L.nv;
   constexpr int SX = TX + 3;
@@ -1003,7 +1003,7 @@ __device__ __forceinline__ void process_tile(const LatParams &p, int t, float *s
       sd[z * PS + yy * SX + xx] = v;
     }
   }
-  tile_sync<TX * TY, SPEC>();
+  __syncthreads();
   unsigned long long ts1 = 0;
   if (threadIdx.x == 0) ts1 = dev_globaltimer();
 
@@ -1061,7 +1061,7 @@ __device__ __forceinline__ void process_tile(const LatParams &p, int t, float *s
       }
     }
     if (chg) s_flags[cyc % 3] = 1;
-    tile_sync<TX * TY, SPEC>();
+    __syncthreads();
     if (cyc > 0 && !s_flags[cyc % 3] && !s_flags[3 + (cyc - 1) % 3]) { converged = true; break; }
     chg = false;
     for (int c = threadIdx.x; c < tw * th; c += (TX * TY)) {
@@ -1075,7 +1075,7 @@ __device__ __forceinline__ void process_tile(const LatParams &p, int t, float *s
       }
     }
     if (chg) s_flags[3 + cyc % 3] = 1;
-    tile_sync<TX * TY, SPEC>();
+    __syncthreads();
     if (!s_flags[cyc % 3] && !s_flags[3 + cyc % 3]) { converged = true; break; }
   }
   unsigned long long ts2 = 0;
@@ -1112,7 +1112,7 @@ __device__ __forceinline__ void process_tile(const LatParams &p, int t, float *s
     }
   }
   if (threadIdx.x == 0 && !converged) s_act[4] = 1;
-  tile_sync<TX * TY, SPEC>();
+  __syncthreads();
   if (threadIdx.x == 0) {
     const unsigned long long ts3 = dev_globaltimer();
     atomicAdd(&p.ctl->ns[0], ts1 - ts0);
@@ -2318,7 +2318,7 @@ __global__ void __launch_bounds__(TX * TY, 1) lattice_tile_kernel(LatParams p) {
       __syncthreads();
       if (ti >= (int)n_in) break;
       const int t = __ldcg(&inl[ti]);
-      process_tile<TX, TY, PRIV, false>(p, t, sd, s_layers, s_flags, s_act);
+      process_tile<TX, TY, PRIV>(p, t, sd, s_layers, s_flags, s_act);
       if (threadIdx.x == 0) {
         int nb[5];
         const int k = revisit_list(p, t, s_act, nb);
@@ -2470,7 +2470,7 @@ __global__ void __launch_bounds__(NZM > 0 ? RunTile<NZM ? NZM : 1, ZS>::NW : TX 
     __syncthreads();
     if (t < 0) break;
     if constexpr (NZM > 0) visit_runs<NZM, PRIV, false, CV, ZS>(p, t, s_box, sd, R, s_run, s_act, s_nb, warm);
-    else process_tile<TX, TY, PRIV, false, DEEP, TMA, CV>(p, t, sd, s_layers, s_flags, s_act, s_nb, warm, &tma);
+    else process_tile<TX, TY, PRIV, DEEP, TMA, CV>(p, t, sd, s_layers, s_flags, s_act, s_nb, warm, &tma);
     // neighbours are activated by threads 0..3 in parallel, after this
     // tile's distances are visible
     unsigned long long ta = 0;

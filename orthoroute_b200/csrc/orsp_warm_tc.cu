@@ -887,10 +887,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) wgrad_tc_kernel(
 //    9 x Cin / 16 of 96, whose tensor time covers their operand reads;
 //  - warps are specialised: TMA, MMA, ReLU-mask (in place in shared memory,
 //    only when a mask is given), epilogue on a second accumulator pair.
-// Measured, 32 -> 32 channels: 400 x 400 x 18 forward 1 259 -> 172 us (925
+// Measured, 32 -> 32 channels: 400 x 400 x 18 forward 1 259 -> 177 us (900
 // TFLOP/s; 100 us of it are the MMAs, 59 clocks each, the rest the hand-overs
 // between the steps and the last, partial round of tiles); 200 x 200 x 18 with
-// the ReLU mask: weight gradient 1 982 -> 68 us, input gradient 660 -> 60 us.
+// the ReLU mask: weight gradient 1 982 -> 70 us, input gradient 660 -> 60 us.
 // Every wait is bounded; one that expires sets the abort flag that ends the
 // others, the TMA thread waits (bounded) for its loads in flight, and TMEM is
 // freed.  No load is multicast.
@@ -1038,19 +1038,18 @@ struct PlaneBars {
   unsigned long long accf[2], acce[2];
   uint32_t tmem;
   volatile int abort;
-  unsigned long long wait_ns;
 };
 
 // Waits for `parity` of a barrier, bounded; ends early when another role has
 // given up, and makes the others give up when it expires.
-__device__ __forceinline__ bool plane_wait(PlaneBars &pb, void *bar, int parity) {
+__device__ __forceinline__ bool plane_wait(PlaneBars &pb, unsigned long long wait_ns, void *bar, int parity) {
   const uint32_t a = smem_addr(bar);
   if (mbar_try(a, static_cast<uint32_t>(parity))) return true;
   const unsigned long long t0 = dev_globaltimer();
   for (;;) {
     if (mbar_try(a, static_cast<uint32_t>(parity))) return true;
     if (pb.abort) return false;
-    if (dev_globaltimer() - t0 > pb.wait_ns) {
+    if (dev_globaltimer() - t0 > wait_ns) {
       pb.abort = 1;
       atomicExch(&g_tc_err, 1);
       return false;
@@ -1058,11 +1057,16 @@ __device__ __forceinline__ bool plane_wait(PlaneBars &pb, void *bar, int parity)
   }
 }
 
-// The same by a whole warp, whose lanes go on or give up together: one lane may
-// find the phase complete and another the abort flag, and what follows (MMA
-// issue, tcgen05.ld, shuffles) takes all of them.
-__device__ __forceinline__ bool plane_wait_warp(PlaneBars &pb, void *bar, int parity) {
-  return __all_sync(0xffffffffu, plane_wait(pb, bar, parity)) != 0;
+// The same for a whole warp, whose lanes go on or give up together: waiting by
+// themselves, one may find the phase complete and another the abort flag, and
+// what follows (tcgen05.ld, shuffles) takes all of them.  Lane 0 waits for all
+// (a vote on every lane's wait: 181.7 us for 400 x 400 x 18, 32 -> 32, this 177.1).
+__device__ __forceinline__ bool plane_wait_warp(PlaneBars &pb, unsigned long long wait_ns, void *bar, int parity) {
+  int ok = 1;
+  if ((threadIdx.x & 31) == 0) ok = plane_wait(pb, wait_ns, bar, parity);
+  ok = __shfl_sync(0xffffffffu, ok, 0);
+  __syncwarp();  // what lane 0 has waited for is visible to all
+  return ok != 0;
 }
 
 // TMA, MMA, mask warps, sixteen epilogue warps
@@ -1107,7 +1111,6 @@ __global__ void __launch_bounds__(pc_threads<MASK>(), 1) conv3d_planes_kernel(
   }
   if (tid == 0) {
     pb.abort = 0;
-    pb.wait_ns = wait_ns;
     for (int b = 0; b < NB; ++b) {
       mbar_init(&pb.full[b], 1);
       mbar_init(&pb.ready[b], PL_MASK);
@@ -1142,8 +1145,8 @@ __global__ void __launch_bounds__(pc_threads<MASK>(), 1) conv3d_planes_kernel(
         const PlaneUnit un(plan, u, D);
         for (int z = max(un.z0 - 1, 0); z <= min(un.z1, D - 1); ++z, ++n) {
           const int b = n % NB;
-          if (n >= NB && !plane_wait(pb, &pb.empty[b], (n / NB - 1) & 1)) { ok = false; break; }
-          if (MASK && n >= 2 && !plane_wait(pb, &pb.mfree[n & 1], ((n >> 1) - 1) & 1)) { ok = false; break; }
+          if (n >= NB && !plane_wait(pb, wait_ns, &pb.empty[b], (n / NB - 1) & 1)) { ok = false; break; }
+          if (MASK && n >= 2 && !plane_wait(pb, wait_ns, &pb.mfree[n & 1], ((n >> 1) - 1) & 1)) { ok = false; break; }
           mbar_expect(&pb.full[b], MASK ? 2 * PB : PB);
           const int x = un.x * (PL_X - 2) - 1, y = un.y * PL_Y - 1;
           tma_load_4d(smem_addr(planes + static_cast<size_t>(b) * PB), &tmx, smem_addr(&pb.full[b]), x, y, z);
@@ -1165,7 +1168,7 @@ __global__ void __launch_bounds__(pc_threads<MASK>(), 1) conv3d_planes_kernel(
       // buffers of the planes below, at and above z (-1: outside the grid)
       int bz[3] = {-1, -1, -1};
       auto next = [&]() {  // the next plane of the unit, when it has landed
-        ok = ok && plane_wait(pb, MASK ? &pb.ready[b] : &pb.full[b], par);
+        ok = ok && plane_wait(pb, wait_ns, MASK ? &pb.ready[b] : &pb.full[b], par);
         const int got = b;
         if (++b == NB) b = 0, par ^= 1;
         return got;
@@ -1177,7 +1180,7 @@ __global__ void __launch_bounds__(pc_threads<MASK>(), 1) conv3d_planes_kernel(
         bz[0] = bz[1];
         bz[1] = bz[2];
         bz[2] = z + 1 < D ? next() : -1;
-        if (ok && step >= 2) ok = plane_wait(pb, &pb.acce[a], ((step >> 1) - 1) & 1);
+        if (ok && step >= 2) ok = plane_wait(pb, wait_ns, &pb.acce[a], ((step >> 1) - 1) & 1);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
@@ -1224,7 +1227,7 @@ __global__ void __launch_bounds__(pc_threads<MASK>(), 1) conv3d_planes_kernel(
         const PlaneUnit un(plan, u, D);
         for (int z = max(un.z0 - 1, 0); z <= min(un.z1, D - 1) && ok; ++z, ++n) {
           const int b = n % NB;
-          ok = plane_wait(pb, &pb.full[b], (n / NB) & 1);
+          ok = plane_wait(pb, wait_ns, &pb.full[b], (n / NB) & 1);
           if (!ok) break;
           mask_plane<PB>(planes + static_cast<size_t>(b) * PB, masks + (n & 1) * PB, tid - 64);
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -1250,7 +1253,7 @@ __global__ void __launch_bounds__(pc_threads<MASK>(), 1) conv3d_planes_kernel(
       const bool in = lane >= 1 && lane <= 30 && x < W && y < H;
       for (int z = un.z0; z < un.z1; ++z, ++step) {
         const int a = step & 1;
-        ok = plane_wait_warp(pb, &pb.accf[a], (step >> 1) & 1);
+        ok = plane_wait_warp(pb, wait_ns, &pb.accf[a], (step >> 1) & 1);
         if (!ok) break;
         tc_fence_after();
         const uint32_t t0 =
@@ -1388,7 +1391,6 @@ __global__ void __launch_bounds__(PW_THREADS, 1) wgrad_planes_kernel(
   unsigned char *const ms = gs + NG * GB;     // [2] mask planes (MASK)
   if (tid == 0) {
     pb.abort = s_bad = 0;
-    pb.wait_ns = wait_ns;
     for (int b = 0; b < NG; ++b) {
       mbar_init(&pb.full[b], 1);
       mbar_init(&pb.ready[b], PL_MASK);
@@ -1421,8 +1423,8 @@ __global__ void __launch_bounds__(PW_THREADS, 1) wgrad_planes_kernel(
       bool ok = true;
       auto load_g = [&](const PlaneUnit &un, int z) {
         const int b = n % NG;
-        if (n >= NG && !plane_wait(pb, &pb.empty[b], (n / NG - 1) & 1)) return false;
-        if (MASK && n >= 2 && !plane_wait(pb, &pb.mfree[n & 1], ((n >> 1) - 1) & 1)) return false;
+        if (n >= NG && !plane_wait(pb, wait_ns, &pb.empty[b], (n / NG - 1) & 1)) return false;
+        if (MASK && n >= 2 && !plane_wait(pb, wait_ns, &pb.mfree[n & 1], ((n >> 1) - 1) & 1)) return false;
         mbar_expect(&pb.full[b], MASK ? 2 * GB : GB);
         tma_load_4d(smem_addr(gs + b * GB), &tmg, smem_addr(&pb.full[b]), un.x * PL_X, un.y * PL_Y - 1, z);
         if (MASK) tma_load_4d(smem_addr(ms + (n & 1) * GB), &tmm, smem_addr(&pb.full[b]), un.x * PL_X, un.y * PL_Y - 1, z);
@@ -1436,7 +1438,7 @@ __global__ void __launch_bounds__(PW_THREADS, 1) wgrad_planes_kernel(
         for (int z = un.z0; z < un.z1 && ok; ++z, ++m) {
           while (ok && zg <= min(z + 1, zhi)) ok = load_g(un, zg++);
           const int b = m & 1;
-          if (!ok || (m >= 2 && !plane_wait(pb, &pb.xempty[b], ((m >> 1) - 1) & 1))) { ok = false; break; }
+          if (!ok || (m >= 2 && !plane_wait(pb, wait_ns, &pb.xempty[b], ((m >> 1) - 1) & 1))) { ok = false; break; }
           mbar_expect(&pb.xfull[b], 3 * XB);
           for (int dx = 0; dx < 3; ++dx)
             tma_load_4d(smem_addr(xs + (b * 3 + dx) * XB), &tmx, smem_addr(&pb.xfull[b]), un.x * PL_X + dx - 1,
@@ -1457,7 +1459,7 @@ __global__ void __launch_bounds__(PW_THREADS, 1) wgrad_planes_kernel(
       const PlaneUnit un = sh.next(plan, D);
       int bz[3] = {-1, -1, -1};  // G planes below, at and above z
       auto next = [&]() {
-        ok = ok && plane_wait(pb, MASK ? &pb.ready[b] : &pb.full[b], par);
+        ok = ok && plane_wait(pb, wait_ns, MASK ? &pb.ready[b] : &pb.full[b], par);
         const int got = b;
         if (++b == NG) b = 0, par ^= 1;
         return got;
@@ -1468,7 +1470,7 @@ __global__ void __launch_bounds__(PW_THREADS, 1) wgrad_planes_kernel(
         bz[0] = bz[1];
         bz[1] = bz[2];
         bz[2] = z + 1 < D ? next() : -1;
-        if (ok) ok = plane_wait(pb, &pb.xfull[m & 1], (m >> 1) & 1);
+        if (ok) ok = plane_wait(pb, wait_ns, &pb.xfull[m & 1], (m >> 1) & 1);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
@@ -1518,7 +1520,7 @@ __global__ void __launch_bounds__(PW_THREADS, 1) wgrad_planes_kernel(
         const PlaneUnit un = sh.next(plan, D);
         for (int z = max(un.z0 - 1, 0); z <= min(un.z1, D - 1) && ok; ++z, ++n) {
           const int b = n % NG;
-          ok = plane_wait(pb, &pb.full[b], (n / NG) & 1);
+          ok = plane_wait(pb, wait_ns, &pb.full[b], (n / NG) & 1);
           if (!ok) break;
           mask_plane<GB>(gs + b * GB, ms + (n & 1) * GB, tid - 64);
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -1579,7 +1581,7 @@ __global__ void __launch_bounds__(PW_THREADS, 1) wgrad_planes_kernel(
       }
     }
   };
-  if (sums && plane_wait_warp(pb, &pb.accf[0], 0)) {
+  if (sums && plane_wait_warp(pb, wait_ns, &pb.accf[0], 0)) {
     tc_fence_after();
     bool bad = false;
     accumulators([&](int, int, int, const uint32_t (&r)[16]) {

@@ -55,14 +55,13 @@ C3_GROUP, C3_REPAIR = 32, 3
 BLOCKED = 0.05
 SEED = 20261203
 # DRAM bytes (read + write) per lattice node and source of the tile search in
-# a many-source launch (lattice_spec_kernel, two CTAs per SM), from ncu
-# (dram__bytes_read.sum + dram__bytes_write.sum) on a 4-source launch of the
-# 1000x1000x12 lattice (bench.py --profile-case --per-launch 4), with the
-# scheduler warp's L2 prefetch: 971.27 + 178.85 MB for 4 x 12.0 M
-# node-sources.  Every search settles every node;
+# a many-source launch (lattice_spec_kernel<12>, run visits, two CTAs per SM),
+# from ncu (dram__bytes_read.sum + dram__bytes_write.sum) on a 4-source launch of
+# the 1000x1000x12 lattice (bench.py --profile-case --per-launch 4): 934.72 +
+# 177.19 MB for 4 x 12.0 M node-sources.  Every search settles every node;
 # the traffic is the distance slices read and written about once plus the
 # shared weights, so it grows with the sources per launch.
-LAT_DRAM_BYTES_PER_NODE = (971.270912e6 + 178.853888e6) / (4 * 1000 * 1000 * 12)
+LAT_DRAM_BYTES_PER_NODE = (934.723328e6 + 177.192448e6) / (4 * 1000 * 1000 * 12)
 
 
 def _peaks():
@@ -749,8 +748,8 @@ def sweep_c4(dev, nsearch: int = 4096):
     3 % blocked), box sides log-uniform per axis (x, y in [20, 400], z in
     [4, 16]), source and target uniform in each box.  Three runs of the same
     searches: one search per launch (orsp_sssp_box), the default batch plan
-    (one CTA per search), and the plan the autotuner picks per ROI-size
-    bucket; the paths must be identical."""
+    (tile sweeps), and the plan the autotuner picks per ROI-size bucket; the
+    paths must be identical."""
     import torch
 
     from orthoroute_b200.autotune import tune_batch
@@ -965,10 +964,11 @@ def run_ours(args, world, rank, local):
         visits_per_tile = single["visits_per_tile"]
     value = total_edges / (ms_max / 1e3) / 1e9
     # the tile-search kernel of the timed step: many-source launches of up
-    # to 12 layers take the warp-specialised schedule (ORSP_LAT_SPEC overrides)
+    # to 18 layers take the warp-specialised schedule (ORSP_LAT_SPEC overrides),
+    # single searches visiting owners
     spec_env = os.environ.get("ORSP_LAT_SPEC")
-    spec = (spec_env not in (None, "") and spec_env != "0") if spec_env not in (None, "") else bool(per and lat.nz <= 12)
-    timed_kernel = "lattice_spec_kernel" if spec else "lattice_async_kernel"
+    spec = (spec_env not in (None, "") and spec_env != "0") if spec_env not in (None, "") else bool(per and lat.nz <= 18)
+    timed_kernel = "lattice_spec_kernel" if spec else "lattice_async_kernel" if per else "lattice_live_kernel"
     avg_kernel_ms = kernel_ms / launches
     bytes_per_launch = bytes_alg / len(sources) * srcs_per_launch
     achieved = bytes_per_launch / (avg_kernel_ms / 1e3) / 1e9
@@ -1046,9 +1046,9 @@ def run_ours(args, world, rank, local):
         "sources_per_launch": per if per else 1,
         "e2e": {"value": round(e2e_value, 4), "unit": "GTEPS",
                 "h2d_bytes_per_step": int(w.nbytes), "d2h_bytes_per_step": int(lat.N * 4 * len(sources))},
-        # per launch: fill, seed and the tile search (the weight gather ran
-        # before the timed region, once for the unchanged weights)
-        "gpu_launches": int(launches * 3),
+        # per launch: fill, queue, seed and the tile search (the weight gather
+        # ran before the timed region, once for the unchanged weights)
+        "gpu_launches": int(launches * 4),
         "single_search": single,
         "visits_per_tile": round(visits_per_tile, 2),
         "roofline": {"bound": "hbm", "achieved": round(achieved, 2), "peak": peak, "unit": "GB/s",
@@ -1119,7 +1119,7 @@ def run_reference(args, world, rank, local):
 def profile_case(args):
     """A small case of the timed kernel for ncu captures: the bench lattice
     and weights, three orsp_sssp_sources launches of --per-launch new sources
-    each (capture the third: -k regex:lattice_async -s 2 -c 1).  Prints one
+    each (capture the third: -k regex:lattice_spec -s 2 -c 1).  Prints one
     line; no timing."""
     import torch
 

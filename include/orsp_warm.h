@@ -39,8 +39,10 @@ ORSP_API int orsp_warm_conv3d_tc(const void *X, const void *mask, const void *Wt
                                  int32_t relu, uintptr_t stream);
 
 /* The weight and bias gradients of orsp_warm_wgrad on the tensor cores
- * (tcgen05.mma, both operands MN-major, one TMEM accumulator per group of
- * 128 / Cin taps, partial sums added to dW with fp32 atomics).  Cin, Cout
+ * (tcgen05.mma, both operands MN-major, accumulators in TMEM, partial sums
+ * added to dW with fp32 atomics; 16 and 32 channels by planes with TMA loads).
+ * Infinities and NaN reach the elements whose sum over the grid's voxels,
+ * zero-padded X times the gradient, holds them.  Cin, Cout
  * multiples of 16, at most 64, with ceil(27 Cin / 128) x Cout <= 512
  * accumulator columns. */
 ORSP_API int orsp_warm_wgrad_tc(const void *X, const void *dY, const void *Yo, float *dW, float *db, int32_t D,

@@ -17,10 +17,11 @@
 //   - the epilogue reads the accumulator with tcgen05.ld (warps w and w + 4
 //     share TMEM lanes 32 (w % 4) .., i.e. those voxels, and split the output
 //     channels), adds the bias, applies the ReLU and stores bf16 or fp32.
-// The weight gradient (wgrad_tc_kernel) is a second tcgen05 GEMM.
+// The weight gradient (wgrad_tc_kernel) is a second tcgen05 GEMM.  Layers of 16
+// and 32 channels take the plane kernels (TMA loads) at the end of the file.
 // Every mbarrier wait is bounded by the global timer; on expiry the kernel
-// records an error, waits once more (bounded) for its MMAs, frees its TMEM
-// and returns.  Single-GPU code: no multicast.
+// records an error, waits once more (bounded) for what is in flight, frees its
+// TMEM and returns.  Single-GPU code: no multicast.
 #include <cstdlib>
 #include <algorithm>
 #include <climits>

@@ -262,7 +262,8 @@ ORSP_API int orsp_sssp_batch_ranges(orsp_graph *g, const float *cost_d, int32_t 
  *            otherwise.  tile_w[i] (16 or 32) only bounds the depth of the
  *            boxes swept (orsp_lattice_max_layers); tiles are 16 wide.
  * nb = 0 restores the default: tile sweeps for boxes of up to 18 layers on
- * H/V lattices with adjacent vias, impl 0 otherwise.  Every plan gives the
+ * H/V lattices with adjacent vias (small ones beside deeper boxes may go along
+ * with those), impl 0 otherwise.  Every plan gives the
  * same paths, bit for bit; the plan only changes the time.  No counterpart in
  * the reference. */
 ORSP_API int orsp_batch_set_plan(orsp_graph *g, int32_t nb, const int64_t *max_nodes, const int32_t *impl,

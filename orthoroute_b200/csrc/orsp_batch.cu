@@ -17,6 +17,7 @@
 // path_len = -2 and are re-run by the host wrapper with larger queues.
 #include <algorithm>
 #include <climits>
+#include <cmath>
 #include <cstdlib>
 #include <vector>
 
@@ -806,9 +807,35 @@ static int run_batch(orsp_graph *g, const float *cost_d, int32_t K, const int32_
   // against 1.38, 512 of up to 400 x 400 x 16: 1.9 against 19.3).  Column-via
   // and deeper boxes keep one CTA per search: not measured.
   const bool sweep_all = !range_mode && g->plan_nb == 0 && g->lattice_ok && !g->cvia;
+  // Beside deeper boxes, which take a launch of one CTA per search in any case,
+  // boxes whose distances that launch keeps in shared memory, no larger than the
+  // largest deep one, go along in it when it then takes no longer; a sweep of
+  // their own adds its time.  One CTA searches such a box of n nodes in about
+  // sqrt(n) (144 nodes 70 us, 1 600 165, 10 000 465, 22 500 675), so the launch
+  // takes no longer while their sum per CTA stays below that of the largest deep
+  // box.  Apart -> together: 8 deep boxes of 20 x 20 x 25 (alone 465 us) with 64
+  // of 20 x 20 x 8 566 -> 465 us, with 2 048 of 6 x 6 x 4 686 -> 530 us; one of 8
+  // x 8 x 25 with 64 of 6 x 6 x 4 258 -> 180 us.  Where the rule says apart: that
+  // one with 2 048 of 6 x 6 x 4 399 against 529 us, with 64 of 20 x 20 x 8 263
+  // against 343 us; one of 60 x 60 x 25 with 250 of 60 x 60 x 12 1.08 against 1.73 ms.
+  int64_t along = 0;  // nodes of the largest box that goes along; 0: none does
+  if (sweep_all) {
+    int64_t deep = 0;
+    double sum = 0.0;
+    for (int32_t k = 0; k < K; ++k) {
+      const int32_t *b = &bb[(size_t)per * k];
+      if (b[5] - b[4] >= 18) deep = std::max(deep, box_volume(b, 0));
+    }
+    along = std::min<int64_t>(deep, env_int("ORSP_BATCH_SMEM_NODES", 24 * 1024));
+    for (int32_t k = 0; along > 0 && k < K; ++k) {
+      const int64_t v = box_volume(&bb[(size_t)per * k], 0);
+      if (v <= along) sum += std::sqrt((double)v);
+    }
+    if (sum > 2.0 * g->num_sms * std::sqrt((double)deep)) along = 0;
+  }
   auto swept = [&](int i, int32_t k) {
     const int32_t *b = &bb[(size_t)per * k];
-    if (sweep_all) return b[5] - b[4] < 18;
+    if (sweep_all) return b[5] - b[4] < 18 && box_volume(b, 0) > along;
     return tuned && g->plan_impl[i] == 1 && g->lattice_ok && !(g->cvia && g->plan_tile[i] != 16) &&
            tile_ok(k, g->plan_tile[i]);
   };
